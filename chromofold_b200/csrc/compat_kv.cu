@@ -12,6 +12,7 @@
 
 #include "cf_device_common.cuh"
 #include "chromofold_b200/compat_kv.h"
+#include "compat_paged_mma.cuh"
 
 namespace cfb {
 // Implemented in flat_rans_decode.cu
@@ -88,6 +89,7 @@ constexpr uint32_t kCompatSlots = 4;
 constexpr uint32_t kCompatSlotFloats = 512u * 1024u;   // 2 MiB per slot
 constexpr uint32_t kCompatMaxSplits = 64;
 __device__ float g_compat_partials[kCompatSlots * kCompatSlotFloats];
+__device__ uint32_t g_compat_arrived[kCompatSlots * kPagedMmaCounters];   // zero between calls
 
 __global__ void __launch_bounds__(kThreads) compat_paged_attention_kernel(cf_kv_paged_attention_desc desc,
                                                                           uint32_t batch_tokens, uint32_t splits,
@@ -495,6 +497,7 @@ struct CompatSlots {
     bool made = false;
     cudaEvent_t done[cfb::kCompatSlots] = {};
     float *base = nullptr;
+    uint32_t *arrived = nullptr;
     uint32_t next = 0;
     int sm_count = 0;
 };
@@ -508,11 +511,7 @@ extern "C" cf_status cf_kv_paged_attention_async(const cf_kv_paged_attention_des
     if (valid != CF_OK) return valid;
     if (d->gqa_group_size > cfb::kMaxGroup) return CF_ERR_UNSUPPORTED;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const uint32_t batch_tokens = cfb::kBatchSymbols / d->head_dim;
-    const cfb::Smem lay = cfb::smem_layout(d->gqa_group_size, d->head_dim, batch_tokens);
-    if (cudaFuncSetAttribute(cfb::compat_paged_attention_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(lay.total)) != cudaSuccess)
-        return CF_ERR_CUDA;
+    const bool mma = cfb::paged_mma_supports(*d);
     int device = 0;
     if (cudaGetDevice(&device) != cudaSuccess) return CF_ERR_CUDA;
     uint32_t splits = 1, slot = 0;
@@ -522,17 +521,18 @@ extern "C" cf_status cf_kv_paged_attention_async(const cf_kv_paged_attention_des
     if (capture != cudaStreamCaptureStatusNone) slots = nullptr;   // a captured call keeps to one launch and no events
     if (slots) {
         std::lock_guard<std::mutex> guard(slots->lock);
-        if (!slots->made) {   // first call on this device: events, the array's address, the SM count
+        if (!slots->made) {   // first call on this device: events, the arrays' addresses, the SM count
             for (cudaEvent_t &e : slots->done)
                 if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) return CF_ERR_CUDA;
             if (cudaGetSymbolAddress(reinterpret_cast<void **>(&slots->base), cfb::g_compat_partials) != cudaSuccess ||
+                cudaGetSymbolAddress(reinterpret_cast<void **>(&slots->arrived), cfb::g_compat_arrived) != cudaSuccess ||
                 cudaDeviceGetAttribute(&slots->sm_count, cudaDevAttrMultiProcessorCount, device) != cudaSuccess)
                 return CF_ERR_CUDA;
             slots->made = true;
         }
         const uint64_t pairs = static_cast<uint64_t>(d->query_count) * d->kv_head_count;
         const uint64_t room = cfb::kCompatSlotFloats / (static_cast<uint64_t>(d->query_count) * d->query_head_count * (d->head_dim + 2u));
-        const uint64_t wanted = (2ull * slots->sm_count + pairs - 1) / pairs;
+        const uint64_t wanted = mma ? cfb::paged_mma_splits(*d, slots->sm_count) : (2ull * slots->sm_count + pairs - 1) / pairs;
         splits = static_cast<uint32_t>(std::max<uint64_t>(1, std::min({wanted, room, static_cast<uint64_t>(cfb::kCompatMaxSplits)})));
         if (splits > 1) {
             slot = slots->next++ % cfb::kCompatSlots;
@@ -540,13 +540,22 @@ extern "C" cf_status cf_kv_paged_attention_async(const cf_kv_paged_attention_des
         }
     }
     float *partials = splits > 1 ? slots->base + static_cast<size_t>(slot) * cfb::kCompatSlotFloats : nullptr;
-    cfb::compat_paged_attention_kernel<<<dim3(d->query_count, d->kv_head_count, splits), cfb::kThreads, lay.total, s>>>(
-        *d, batch_tokens, splits, partials);
-    if (splits > 1) {
-        cfb::compat_combine_kernel<<<dim3(d->query_count, d->query_head_count), 128, 0, s>>>(d->output, partials, d->query_head_count,
-                                                                                          d->head_dim, splits);
-        if (cudaEventRecord(slots->done[slot], s) != cudaSuccess) return CF_ERR_CUDA;
+    if (mma) {   // head_dim 128 and 64; the splits are merged by the kernel itself
+        uint32_t *arrived = splits > 1 ? slots->arrived + slot * cfb::kPagedMmaCounters : nullptr;
+        if (cfb::launch_paged_mma(*d, splits, partials, arrived, s) != cudaSuccess) return CF_ERR_CUDA;
+    } else {
+        const uint32_t batch_tokens = cfb::kBatchSymbols / d->head_dim;
+        const cfb::Smem lay = cfb::smem_layout(d->gqa_group_size, d->head_dim, batch_tokens);
+        if (cudaFuncSetAttribute(cfb::compat_paged_attention_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 static_cast<int>(lay.total)) != cudaSuccess)
+            return CF_ERR_CUDA;
+        cfb::compat_paged_attention_kernel<<<dim3(d->query_count, d->kv_head_count, splits), cfb::kThreads, lay.total, s>>>(
+            *d, batch_tokens, splits, partials);
+        if (splits > 1)
+            cfb::compat_combine_kernel<<<dim3(d->query_count, d->query_head_count), 128, 0, s>>>(d->output, partials, d->query_head_count,
+                                                                                              d->head_dim, splits);
     }
+    if (splits > 1 && cudaEventRecord(slots->done[slot], s) != cudaSuccess) return CF_ERR_CUDA;
     return cudaPeekAtLastError() == cudaSuccess ? CF_OK : CF_ERR_CUDA;
 }
 

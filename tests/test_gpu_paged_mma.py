@@ -1,0 +1,106 @@
+"""cf_kv_paged_attention_async at head_dim 128 and 64 (csrc/compat_paged_mma.cu) against fp64 softmax over the dequantised
+rows, where the tiles and branches of the tensor-core form begin and end: row counts around the 16-row tile, page sizes
+around the 16-token group, windows, tails, every code width it loads directly, and the ones it decodes first."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from compat_types import DevicePage, PagedAttentionDesc
+
+pytestmark = pytest.mark.gpu
+
+
+def _pack(sym, bits):
+    """Symbols MSB-first in u32 words, two words of slack."""
+    per = 32 // bits
+    s = np.concatenate([sym.astype(np.uint64).ravel(), np.zeros(-sym.size % per, np.uint64)]).reshape(-1, per)
+    shifts = (32 - bits - bits * np.arange(per)).astype(np.uint64)
+    return np.concatenate([(s << shifts).sum(1).astype(np.uint32), np.zeros(2, np.uint32)])
+
+
+# (bits, head_dim, q heads, kv heads, page sizes, tail, query tokens, window, zero point, what is special)
+CASES = [
+    (4, 128, 4, 1, [16], 0, 1, 0, 8, ""),
+    (4, 128, 32, 8, [128] * 9, 5, 1, 0, 8, ""),
+    (4, 64, 14, 2, [1, 15, 17, 31], 1, 3, 0, 8, ""),
+    (8, 128, 8, 8, [33, 16, 128], 17, 16, 0, 128, ""),
+    (8, 64, 16, 1, [64, 2], 0, 5, 20, 128, ""),
+    (4, 128, 5, 1, [128, 128, 128], 127, 7, 100, 8, ""),
+    (4, 128, 4, 1, [], 40, 9, 0, 8, ""),
+    (8, 128, 2, 2, [48], 16, 60, 33, 128, ""),
+    (4, 128, 32, 8, [40, 24], 3, 2, 0, 8, "unaligned"),
+    (2, 64, 4, 2, [20, 12], 2, 1, 0, 1, ""),
+    (0, 128, 8, 2, [40, 9], 4, 3, 0, 128, ""),
+    (0, 64, 7, 1, [100], 0, 1, 30, 128, ""),
+    (8, 128, 4, 1, [32, 32], 6, 2, 0, 2000, ""),
+    (4, 128, 4, 1, [64, 64], 6, 2, 0, 8, "magnitudes"),
+]
+
+
+@pytest.mark.parametrize("case", CASES, ids=str)
+def test_paged_attention_on_the_tensor_cores(native, oracle, case):
+    import torch
+    from helpers import hist_of, laplace_codes
+    from test_gpu_compat import _softmax_attention
+    bits, d, hq, hkv, sizes, tail, nq, window, zp, special = case
+    rng = np.random.default_rng(CASES.index(case))
+    dev = lambda a: torch.from_numpy(np.array(a, copy=True)).cuda()
+    pages, keep, begin, sealed = [], [], 0, sum(sizes)
+    dense_k, dense_v = np.zeros((hkv, sealed, d)), np.zeros((hkv, sealed, d))
+    for tokens in sizes:
+        for h in range(hkv):
+            ks, vs = rng.uniform(0.005, 0.02, d).astype(np.float32), rng.uniform(0.005, 0.02, tokens).astype(np.float32)
+            if zp == 2000:
+                ks, vs = ks / 2000, vs / 2000
+            if special == "magnitudes":
+                ks, vs = ks * 10.0 ** rng.uniform(-5, 1, d).astype(np.float32), vs * 10.0 ** rng.uniform(-6, 4, tokens).astype(np.float32)
+            n = tokens * d
+            if bits:
+                syms = [rng.integers(0, 1 << bits, n).astype(np.uint8) for _ in range(2)]
+                words, offs, luts = [_pack(s, bits) for s in syms], [np.zeros((n + 63) // 64, np.int32)] * 2, [np.zeros(1 << bits, np.int32)] * 2
+            else:
+                syms = [(laplace_codes(rng, n, b).astype(np.int16) + 128).astype(np.uint8) for b in (9.0, 14.0)]
+                cbs = [oracle.codebook_from_hist(hist_of(s)) for s in syms]
+                coded = [oracle.huff_encode(s, 64, cb) for s, cb in zip(syms, cbs)]
+                words, offs, luts = [np.concatenate([w, np.zeros(2, np.uint32)]) for w, _ in coded], [o for _, o in coded], [cb.np("lut") for cb in cbs]
+            dense_k[h, begin:begin + tokens] = (syms[0].reshape(tokens, d).astype(np.float64) - zp) * ks[None, :]
+            dense_v[h, begin:begin + tokens] = (syms[1].reshape(tokens, d).astype(np.float64) - zp) * vs[:, None]
+            shift = 1 if special == "unaligned" else 0
+            held = [dev(np.concatenate([np.zeros(shift, np.uint32), w]).view(np.int32)) for w in words] + [dev(x) for x in (*offs, *luts, ks, vs)]
+            keep.append(held)
+            pg = DevicePage()
+            pg.k_words, pg.v_words = held[0].data_ptr() + 4 * shift, held[1].data_ptr() + 4 * shift
+            pg.k_block_offsets, pg.v_block_offsets, pg.k_lut, pg.v_lut, pg.k_scales, pg.v_scales = [x.data_ptr() for x in held[2:]]
+            pg.token_begin, pg.token_count, pg.head_dim, pg.block_size = begin, tokens, d, 64
+            pg.k_max_code_length = pg.v_max_code_length = bits or 12
+            pg.zero_point, pg.kv_head, pg.fixed_code_length = zp, h, bits
+            pages.append(pg)
+        begin += tokens
+    q = rng.standard_normal((nq, hq, d)).astype(np.float32)
+    tk, tv = (rng.standard_normal((max(tail, 1), hkv, d)).astype(np.float32) for _ in range(2))
+    if special == "magnitudes":
+        tv *= 1e3
+    out = torch.full((nq, hq, d), 3.0, device="cuda")
+    d_q, d_tk, d_tv = dev(q), dev(tk), dev(tv)
+    desc = PagedAttentionDesc()
+    desc.struct_size, desc.abi_version = C.sizeof(desc), 0
+    if pages:
+        d_pages = dev(np.frombuffer(bytes((DevicePage * len(pages))(*pages)), np.uint8))
+        desc.pages, desc.page_count = d_pages.data_ptr(), len(pages)
+    desc.kv_head_count, desc.query_head_count, desc.gqa_group_size = hkv, hq, hq // hkv
+    desc.active_k, desc.active_v, desc.active_token_begin, desc.active_token_count = d_tk.data_ptr(), d_tv.data_ptr(), sealed, tail
+    first = sealed + tail - nq
+    desc.queries, desc.output, desc.query_token_begin, desc.query_count = d_q.data_ptr(), out.data_ptr(), first, nq
+    desc.head_dim, desc.causal_window, desc.softmax_scale = d, window, 1.0 / np.sqrt(d)
+    for _ in range(2):   # twice: the splits' arrival counters are left at zero
+        out.fill_(3.0)
+        assert native.lib().cf_kv_paged_attention_async(C.byref(desc), None) == 0
+    torch.cuda.synchronize()
+    pos = [first + i for i in range(nq)]
+    want = _softmax_attention(np.concatenate([dense_k, tk[:tail].transpose(1, 0, 2)], axis=1),
+                              np.concatenate([dense_v, tv[:tail].transpose(1, 0, 2)], axis=1), q, pos,
+                              [max(0, p + 1 - window) if window else 0 for p in pos], 1.0 / np.sqrt(d), hq // hkv)
+    got = out.cpu().numpy()
+    assert np.isfinite(got).all()
+    assert np.abs(got - want).max() <= 1e-5 * np.abs(want).max(), np.abs(got - want).max() / np.abs(want).max()
