@@ -27,6 +27,7 @@ namespace {
 constexpr int kMmaWarps = 8;
 constexpr int kMmaThreads = kMmaWarps * 32;
 constexpr float kLog2e = 1.4426950408889634f;
+constexpr uint32_t kTailWeight = 3;
 constexpr float kWeightScale = 32768.0f;   // weights are at most 1 (times a relative V scale of at most 1)
 
 template <int D>
@@ -149,50 +150,52 @@ __device__ __noinline__ void decode_group(const uint32_t *words, const int32_t *
     }
 }
 
-// The running state of one warp: rows g and g + 8 of the CTA's sixteen (g = lane / 4), tokens and channels by lane % 4.
-template <int D>
+// The running state of one warp: rows g and g + 8 of the CTA's sixteen (g = lane / 4), tokens and channels by lane % 4. With
+// NR = 1 the tile has at most eight rows (a decode step) and nothing is kept or computed for the upper half.
+template <int D, int NR>
 struct Rows {
     float acc[D / 8][4];   // n-tile j: channel g' * D / 8 + j of column g' = 2 (lane & 3) + {0, 1}, rows g | g + 8
-    float m[2], l[2];      // l: this lane's tokens only
+    float m[NR], l[NR];    // l: this lane's tokens only
     float v_unit;          // O is kept in units of v_unit / kWeightScale; 0 = nothing accumulated yet
 
-    __device__ __forceinline__ void rescale(float f0, float f1) {
-#pragma unroll
-        for (int j = 0; j < D / 8; ++j) {
-            acc[j][0] *= f0, acc[j][1] *= f0;
-            acc[j][2] *= f1, acc[j][3] *= f1;
-        }
-    }
     // Online softmax over the 16 tokens whose scores (log2 units, -inf = not visible) are in s[tile][row pair]; the weights
     // replace the scores, times factor(tile, column) of their token.
     template <class Factor>
     __device__ __forceinline__ void softmax(float (&s)[2][4], float unit, Factor factor) {
-        float r0 = fmaxf(fmaxf(s[0][0], s[0][1]), fmaxf(s[1][0], s[1][1])), r1 = fmaxf(fmaxf(s[0][2], s[0][3]), fmaxf(s[1][2], s[1][3]));
-#pragma unroll
-        for (int o = 1; o <= 2; o <<= 1) {
-            r0 = fmaxf(r0, __shfl_xor_sync(0xffffffffu, r0, o));
-            r1 = fmaxf(r1, __shfl_xor_sync(0xffffffffu, r1, o));
-        }
-        const float n0 = fmaxf(m[0], r0), n1 = fmaxf(m[1], r1);
-        const float z0 = n0 == -CUDART_INF_F ? 0.0f : n0, z1 = n1 == -CUDART_INF_F ? 0.0f : n1;
-        const float a0 = exp2f(m[0] - z0), a1 = exp2f(m[1] - z1);
         const float f = v_unit == unit ? 1.0f : __fdividef(v_unit, unit);   // powers of two
-        if (!__all_sync(0xffffffffu, a0 * f == 1.0f && a1 * f == 1.0f)) rescale(a0 * f, a1 * f);
         v_unit = unit;
-        m[0] = n0, m[1] = n1;
-        float l0 = 0.0f, l1 = 0.0f;
+        float a[NR], z[NR];
+        bool moved = false;
 #pragma unroll
-        for (int tile = 0; tile < 2; ++tile)
+        for (int r = 0; r < NR; ++r) {
+            float top = fmaxf(fmaxf(s[0][2 * r], s[0][2 * r + 1]), fmaxf(s[1][2 * r], s[1][2 * r + 1]));
+            top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1));
+            top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 2));
+            const float next = fmaxf(m[r], top);
+            z[r] = next == -CUDART_INF_F ? 0.0f : next;
+            a[r] = exp2f(m[r] - z[r]);
+            m[r] = next;
+            moved = moved || a[r] * f != 1.0f;
+        }
+        if (__any_sync(0xffffffffu, moved)) {
 #pragma unroll
-            for (int c = 0; c < 2; ++c) {
-                const float p0 = exp2f(s[tile][c] - z0), p1 = exp2f(s[tile][2 + c] - z1);
-                l0 += p0, l1 += p1;
-                const float k = factor(tile, c);
-                s[tile][c] = p0 * k;
-                s[tile][2 + c] = p1 * k;
-            }
-        l[0] = l[0] * a0 + l0;
-        l[1] = l[1] * a1 + l1;
+            for (int j = 0; j < D / 8; ++j)
+#pragma unroll
+                for (int r = 0; r < NR; ++r) acc[j][2 * r] *= a[r] * f, acc[j][2 * r + 1] *= a[r] * f;
+        }
+#pragma unroll
+        for (int r = 0; r < NR; ++r) {
+            float sum = 0.0f;
+#pragma unroll
+            for (int tile = 0; tile < 2; ++tile)
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    const float p = exp2f(s[tile][2 * r + c] - z[r]);
+                    sum += p;
+                    s[tile][2 * r + c] = p * factor(tile, c);
+                }
+            l[r] = l[r] * a[r] + sum;
+        }
     }
 };
 
@@ -202,10 +205,10 @@ __device__ __forceinline__ float power_above(float v) {
 }
 
 // One 16-token group of a page. kBits: width of the words at `k` / `v` (the page's own, or the decoded bytes of the group).
-template <int D, int kBits, bool kDecoded>
-__device__ __forceinline__ void page_group(Rows<D> &st, const cf_kv_device_page &page, uint32_t t0, const uint8_t *planes, uint8_t *symbols,
-                                           const float (&inv_scale)[2], const float (&query_sum)[2], const CodeBias &bias,
-                                           const uint32_t (&qtok)[2], const uint32_t (&first)[2], uint32_t lane) {
+template <int D, int NR, int kBits, bool kDecoded>
+__device__ __forceinline__ void page_group(Rows<D, NR> &st, const cf_kv_device_page &page, uint32_t t0, const uint8_t *planes, uint8_t *symbols,
+                                           const float (&inv_scale)[NR], const float (&query_sum)[NR], const CodeBias &bias,
+                                           const uint32_t (&qtok)[NR], const uint32_t (&first)[NR], uint32_t lane) {
     using L = MmaLayout<D>;
     constexpr int kKWords = D / 4 * kBits / 32, kVWords = D / 8 * kBits / 32;   // words of a lane's share of one token
     constexpr uint32_t kRowBytes = D * kBits / 8;
@@ -253,9 +256,12 @@ __device__ __forceinline__ void page_group(Rows<D> &st, const cf_kv_device_page 
 #pragma unroll
     for (int step = 0; step < static_cast<int>(L::kSteps); ++step) {
         const uint2 h0 = *reinterpret_cast<const uint2 *>(planes + ((step * 16u + g) * 4u + t) * 8u);
-        const uint2 h1 = *reinterpret_cast<const uint2 *>(planes + ((step * 16u + g + 8u) * 4u + t) * 8u);
         const uint2 l0 = *reinterpret_cast<const uint2 *>(planes + L::kPlane + ((step * 16u + g) * 4u + t) * 8u);
-        const uint2 l1 = *reinterpret_cast<const uint2 *>(planes + L::kPlane + ((step * 16u + g + 8u) * 4u + t) * 8u);
+        uint2 h1 = make_uint2(0u, 0u), l1 = make_uint2(0u, 0u);
+        if constexpr (NR == 2) {
+            h1 = *reinterpret_cast<const uint2 *>(planes + ((step * 16u + g + 8u) * 4u + t) * 8u);
+            l1 = *reinterpret_cast<const uint2 *>(planes + L::kPlane + ((step * 16u + g + 8u) * 4u + t) * 8u);
+        }
 #pragma unroll
         for (int tile = 0; tile < 2; ++tile) {
             uint32_t b0, b1;
@@ -289,7 +295,7 @@ __device__ __forceinline__ void page_group(Rows<D> &st, const cf_kv_device_page 
             top = fmaxf(top, fabsf(scale[tile][c]));
             const uint32_t in_page = t0 + 8u * tile + 2u * t + c, token = page.token_begin + in_page;
 #pragma unroll
-            for (int r = 0; r < 2; ++r) {
+            for (int r = 0; r < NR; ++r) {
                 const float x = s[tile][2 * r + c] - bias.rest * query_sum[r];
                 s[tile][2 * r + c] = in_page < count && token >= first[r] && token <= qtok[r] ? x * inv_scale[r] : -CUDART_INF_F;
             }
@@ -299,22 +305,21 @@ __device__ __forceinline__ void page_group(Rows<D> &st, const cf_kv_device_page 
     const float unit = top > st.v_unit ? power_above(top) : st.v_unit, to_unit = kWeightScale / unit;
     st.softmax(s, unit, [&](int tile, int c) { return scale[tile][c] * to_unit; });
     if (bias.rest != 0.0f) {   // sum_t w_t (c_t - zp) = sum_t w_t (c_t - 1024) - rest * sum_t w_t
-        float w0 = s[0][0] + s[0][1] + s[1][0] + s[1][1], w1 = s[0][2] + s[0][3] + s[1][2] + s[1][3];
 #pragma unroll
-        for (int o = 1; o <= 2; o <<= 1) {
-            w0 += __shfl_xor_sync(0xffffffffu, w0, o);
-            w1 += __shfl_xor_sync(0xffffffffu, w1, o);
-        }
+        for (int r = 0; r < NR; ++r) {
+            float w = s[0][2 * r] + s[0][2 * r + 1] + s[1][2 * r] + s[1][2 * r + 1];
+            w += __shfl_xor_sync(0xffffffffu, w, 1);
+            w += __shfl_xor_sync(0xffffffffu, w, 2);
 #pragma unroll
-        for (int j = 0; j < D / 8; ++j) {
-            st.acc[j][0] -= bias.rest * w0, st.acc[j][1] -= bias.rest * w0;
-            st.acc[j][2] -= bias.rest * w1, st.acc[j][3] -= bias.rest * w1;
+            for (int j = 0; j < D / 8; ++j) st.acc[j][2 * r] -= bias.rest * w, st.acc[j][2 * r + 1] -= bias.rest * w;
         }
     }
     // O += P V
     uint32_t ph[4], pl[4];   // A fragments: (row g, tile 0) (row g + 8, tile 0) (row g, tile 1) (row g + 8, tile 1)
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
+        ph[i] = pl[i] = 0u;
+        if (NR == 1 && (i & 1)) continue;
         const float w0 = s[i >> 1][2 * (i & 1)], w1 = s[i >> 1][2 * (i & 1) + 1];
         ph[i] = pack_half2(w0, w1);
         const float2 back = unpack_half2(ph[i]);
@@ -345,17 +350,17 @@ __device__ __forceinline__ void page_group(Rows<D> &st, const cf_kv_device_page 
 }
 
 // One 16-token group of the fp32 tail ([token][kv head][D]; paged_kv_attention.cu:154-166).
-template <int D>
-__device__ __forceinline__ void tail_group(Rows<D> &st, const cf_kv_paged_attention_desc &desc, uint32_t kv_head, uint32_t t0, const float *q_rows,
-                                           const uint32_t (&qtok)[2], const uint32_t (&first)[2], uint32_t lane) {
+template <int D, int NR>
+__device__ __forceinline__ void tail_group(Rows<D, NR> &st, const cf_kv_paged_attention_desc &desc, uint32_t kv_head, uint32_t t0, const float *q_rows,
+                                           const uint32_t (&qtok)[NR], const uint32_t (&first)[NR], uint32_t lane) {
     const uint32_t g = lane >> 2, t = lane & 3u, count = desc.active_token_count;
     const size_t stride = static_cast<size_t>(desc.kv_head_count) * D;
     const float *k0 = desc.active_k + static_cast<size_t>(kv_head) * D, *v0 = desc.active_v + static_cast<size_t>(kv_head) * D;
     float s[2][4] = {};
-#pragma unroll 1
+#pragma unroll 2
     for (uint32_t step = 0; step < D / 16u; ++step) {   // 16 channels: two k8 steps
         const float4 qa = *reinterpret_cast<const float4 *>(q_rows + ((step * 16u + g) * 4u + t) * 4u);
-        const float4 qb = *reinterpret_cast<const float4 *>(q_rows + ((step * 16u + g + 8u) * 4u + t) * 4u);
+        const float4 qb = NR == 2 ? *reinterpret_cast<const float4 *>(q_rows + ((step * 16u + g + 8u) * 4u + t) * 4u) : make_float4(0.f, 0.f, 0.f, 0.f);
         uint32_t ah[2][4], al[2][4];
         tf32_split(qa.x, ah[0][0], al[0][0]), tf32_split(qb.x, ah[0][1], al[0][1]);
         tf32_split(qa.y, ah[0][2], al[0][2]), tf32_split(qb.y, ah[0][3], al[0][3]);
@@ -375,14 +380,14 @@ __device__ __forceinline__ void tail_group(Rows<D> &st, const cf_kv_paged_attent
         for (int c = 0; c < 2; ++c) {
             const uint32_t in_tail = t0 + 8u * tile + 2u * t + c, token = desc.active_token_begin + in_tail;
 #pragma unroll
-            for (int r = 0; r < 2; ++r)
+            for (int r = 0; r < NR; ++r)
                 if (!(in_tail < count && token >= first[r] && token <= qtok[r])) s[tile][2 * r + c] = -CUDART_INF_F;
         }
     const float unit = st.v_unit == 0.0f ? 1.0f : st.v_unit, to_unit = kWeightScale / unit;
     st.softmax(s, unit, [&](int, int) { return to_unit; });
 #pragma unroll 1
     for (int tile = 0; tile < 2; ++tile) {   // k index t = token 2t, t + 4 = token 2t + 1 of the tile
-        const float w0 = tile ? s[1][0] : s[0][0], w1 = tile ? s[1][1] : s[0][1], w2 = tile ? s[1][2] : s[0][2], w3 = tile ? s[1][3] : s[0][3];
+        const float w0 = tile ? s[1][0] : s[0][0], w1 = tile ? s[1][1] : s[0][1], w2 = NR == 1 ? 0.0f : tile ? s[1][2] : s[0][2], w3 = NR == 1 ? 0.0f : tile ? s[1][3] : s[0][3];
         uint32_t ah[4], al[4];
         tf32_split(w0, ah[0], al[0]), tf32_split(w2, ah[1], al[1]);
         tf32_split(w1, ah[2], al[2]), tf32_split(w3, ah[3], al[3]);
@@ -401,7 +406,7 @@ __device__ __forceinline__ void tail_group(Rows<D> &st, const cf_kv_paged_attent
 }
 
 // Grid: (16-row tile, kv head, split). 128 registers: two CTAs per SM.
-template <int D>
+template <int D, int NR>
 __global__ void __launch_bounds__(kMmaThreads, 2) paged_mma_kernel(cf_kv_paged_attention_desc desc, uint32_t splits, float *partials,
                                                                   uint32_t *arrived) {
     using L = MmaLayout<D>;
@@ -439,6 +444,7 @@ __global__ void __launch_bounds__(kMmaThreads, 2) paged_mma_kernel(cf_kv_paged_a
     __syncthreads();
     for (uint32_t i = tid; i < 16u * (D / 4u); i += kMmaThreads) {   // (step, row, lane & 3) -> four channels
         const uint32_t tt = i & 3u, row = (i >> 2) & 15u, step = i >> 6;
+        if (NR == 1 && row >= 8u) continue;
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
         if (row0 + row < rows_total) {
             const uint32_t r = row0 + row;
@@ -472,24 +478,31 @@ __global__ void __launch_bounds__(kMmaThreads, 2) paged_mma_kernel(cf_kv_paged_a
         }
     __syncthreads();
 
-    Rows<D> st;
+    Rows<D, NR> st;
 #pragma unroll
     for (int j = 0; j < D / 8; ++j) st.acc[j][0] = st.acc[j][1] = st.acc[j][2] = st.acc[j][3] = 0.0f;
-    st.m[0] = st.m[1] = -CUDART_INF_F;
-    st.l[0] = st.l[1] = 0.0f;
     st.v_unit = 0.0f;
-    uint32_t qtok[2], first[2];
+    uint32_t qtok[NR], first[NR];
 #pragma unroll
-    for (int r = 0; r < 2; ++r) {
+    for (int r = 0; r < NR; ++r) {
+        st.m[r] = -CUDART_INF_F;
+        st.l[r] = 0.0f;
         qtok[r] = desc.query_token_begin + min(row0 + g + 8u * r, last_row) / G;
         first[r] = window_begin(qtok[r], desc.causal_window);
     }
 
-    // This warp's share of the groups: pages first, then the tail.
-    const uint64_t total = static_cast<uint64_t>(page_groups) + (desc.active_token_count + 15u) / 16u;
+    // This warp's share of the groups: pages first, then the tail, one of whose groups (fp32 loads, three products) weighs
+    // as much as kTailWeight of the pages' and belongs to the warp its first unit falls to.
+    const uint64_t total = static_cast<uint64_t>(page_groups) + kTailWeight * ((desc.active_token_count + 15u) / 16u);
     const uint32_t workers = splits * kMmaWarps, worker = split * kMmaWarps + warp;
-    uint64_t at_group = total * worker / workers;
-    const uint64_t end_group = total * (worker + 1u) / workers;
+    uint64_t at_group, end_group;
+    if (total < (1u << 22)) {   // at most 512 workers: 32-bit divisions do
+        at_group = static_cast<uint32_t>(total) * worker / workers;
+        end_group = static_cast<uint32_t>(total) * (worker + 1u) / workers;
+    } else {
+        at_group = total * worker / workers;
+        end_group = total * (worker + 1u) / workers;
+    }
     uint32_t m_at = 0;
     if (at_group < end_group && at_group < page_groups) {   // the last page that starts at or before the first group
         uint32_t lo = 0, hi = matches;
@@ -504,14 +517,25 @@ __global__ void __launch_bounds__(kMmaThreads, 2) paged_mma_kernel(cf_kv_paged_a
         const uint32_t g0 = static_cast<uint32_t>(at_group) - prefix[m_at];
         const uint32_t page_end = m_at + 1u < matches ? prefix[m_at + 1u] : page_groups;
         const uint32_t stop = static_cast<uint32_t>(min(end_group, static_cast<uint64_t>(page_end))) - prefix[m_at];
+        if (page.fixed_code_length != 0u && lane < 24u) {   // the first two groups' bytes on their way while the rows are scaled
+            const uint32_t row_bytes = D * page.fixed_code_length / 8u, bytes = min(32u, page.token_count - 16u * g0) * row_bytes;
+            const uint32_t *words = lane & 1u ? page.v_words : page.k_words;
+            if ((lane >> 1) * 512u < bytes) {
+                const uint8_t *at = reinterpret_cast<const uint8_t *>(words) + 16u * g0 * row_bytes + (lane >> 1) * 512u;
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(at));
+                if ((lane >> 1) * 512u + 128u < bytes) asm volatile("prefetch.global.L2 [%0];" ::"l"(at + 128));
+                if ((lane >> 1) * 512u + 256u < bytes) asm volatile("prefetch.global.L2 [%0];" ::"l"(at + 256));
+                if ((lane >> 1) * 512u + 384u < bytes) asm volatile("prefetch.global.L2 [%0];" ::"l"(at + 384));
+            }
+        }
         // The page's K scales onto the rows. A power of two is taken out of every row: one above (largest |q|) * (largest scale),
         // which is at most a few binary orders above the largest term (the residue's range absorbs those).
-        float inv_scale[2], query_sum[2], row_scale[2], top = 0.0f;
+        float inv_scale[NR], query_sum[NR], row_scale[NR], top = 0.0f;
 #pragma unroll
         for (uint32_t c = 0; c < D / 32u; ++c) top = fmaxf(top, fabsf(page.k_scales[lane + 32u * c]));
         top = warp_max(top);
 #pragma unroll
-        for (int r = 0; r < 2; ++r) {
+        for (int r = 0; r < NR; ++r) {
             const float bound = __uint_as_float(q_top[g + 8 * r]) * top;
             const uint32_t e = min(max(__float_as_uint(bound) >> 23, 30u), 225u);   // 2^(e - 127) <= bound < 2^(e - 126)
             row_scale[r] = __uint_as_float((267u - e) << 23);                       // 2^(140 - e): terms below 2^14
@@ -523,7 +547,7 @@ __global__ void __launch_bounds__(kMmaThreads, 2) paged_mma_kernel(cf_kv_paged_a
         for (int step = 0; step < static_cast<int>(L::kSteps); ++step) {
             const float4 ks = load4(page.k_scales + t * (D / 4) + 4 * step);
 #pragma unroll
-            for (int r = 0; r < 2; ++r) {
+            for (int r = 0; r < NR; ++r) {
                 const uint32_t at_row = (step * 16u + g + 8u * r) * 4u + t;
                 const float4 q = *reinterpret_cast<const float4 *>(q_rows + at_row * 4u);
                 const float x0 = q.x * ks.x * row_scale[r], x1 = q.y * ks.y * row_scale[r], x2 = q.z * ks.z * row_scale[r], x3 = q.w * ks.w * row_scale[r];
@@ -535,7 +559,7 @@ __global__ void __launch_bounds__(kMmaThreads, 2) paged_mma_kernel(cf_kv_paged_a
             }
         }
 #pragma unroll
-        for (int r = 0; r < 2; ++r)
+        for (int r = 0; r < NR; ++r)
 #pragma unroll
             for (int o = 1; o <= 2; o <<= 1) query_sum[r] += __shfl_xor_sync(0xffffffffu, query_sum[r], o);
         __syncwarp();
@@ -546,35 +570,37 @@ __global__ void __launch_bounds__(kMmaThreads, 2) paged_mma_kernel(cf_kv_paged_a
             const uint32_t t0 = 16u * n, begin = page.token_begin + t0;
             if (begin > newest || begin + 16u <= oldest_visible) continue;
             if (aligned && page.fixed_code_length == 4u)
-                page_group<D, 4, false>(st, page, t0, planes, symbols, inv_scale, query_sum, bias, qtok, first, lane);
+                page_group<D, NR, 4, false>(st, page, t0, planes, symbols, inv_scale, query_sum, bias, qtok, first, lane);
             else if (aligned && page.fixed_code_length == 8u)
-                page_group<D, 8, false>(st, page, t0, planes, symbols, inv_scale, query_sum, bias, qtok, first, lane);
+                page_group<D, NR, 8, false>(st, page, t0, planes, symbols, inv_scale, query_sum, bias, qtok, first, lane);
             else
-                page_group<D, 8, true>(st, page, t0, planes, symbols, inv_scale, query_sum, bias, qtok, first, lane);
+                page_group<D, NR, 8, true>(st, page, t0, planes, symbols, inv_scale, query_sum, bias, qtok, first, lane);
         }
         at_group = static_cast<uint64_t>(prefix[m_at]) + stop;
         ++m_at;
     }
     for (; at_group < end_group; ++at_group) {
-        const uint32_t t0 = 16u * static_cast<uint32_t>(at_group - page_groups), begin = desc.active_token_begin + t0;
+        const uint32_t unit = static_cast<uint32_t>(at_group - page_groups);
+        if (unit % kTailWeight != 0u) continue;
+        const uint32_t t0 = 16u * (unit / kTailWeight), begin = desc.active_token_begin + t0;
         if (begin > newest || begin + 16u <= oldest_visible) continue;
-        tail_group<D>(st, desc, kv_head, t0, q_rows, qtok, first, lane);
+        tail_group<D, NR>(st, desc, kv_head, t0, q_rows, qtok, first, lane);
     }
 
     // ---- merge: the warps' (max, sum, O) in shared memory, then the CTA's rows to the output or to its split's partials ----
     const float o_unit = st.v_unit * (1.0f / kWeightScale);
 #pragma unroll
-    for (int r = 0; r < 2; ++r)
+    for (int r = 0; r < NR; ++r)
 #pragma unroll
         for (int o = 1; o <= 2; o <<= 1) st.l[r] += __shfl_xor_sync(0xffffffffu, st.l[r], o);
     if (t == 0) {
-        state[warp * 16u + g] = make_float2(st.m[0], st.l[0]);
-        state[warp * 16u + g + 8u] = make_float2(st.m[1], st.l[1]);
+#pragma unroll
+        for (int r = 0; r < NR; ++r) state[warp * 16u + g + 8u * r] = make_float2(st.m[r], st.l[r]);
     }
     __syncwarp();
     float *mine_o = reinterpret_cast<float *>(planes);   // [16][D]; channel c * (D / 8) + j of column c = 2t + {0, 1}
 #pragma unroll
-    for (int r = 0; r < 2; ++r) {
+    for (int r = 0; r < NR; ++r) {
         if (row0 + g + 8u * r >= rows_total) continue;
 #pragma unroll
         for (int j = 0; j < D / 8; j += 4) {
@@ -585,6 +611,8 @@ __global__ void __launch_bounds__(kMmaThreads, 2) paged_mma_kernel(cf_kv_paged_a
         }
     }
     __syncthreads();
+    // partials: weighted sums [query row][split][D], then (max, sum) [query row][split]
+    float2 *partial_ml = reinterpret_cast<float2 *>(partials + static_cast<size_t>(desc.query_count) * desc.query_head_count * splits * D);
     for (uint32_t i = tid; i < 16u * D; i += kMmaThreads) {
         const uint32_t row = i / D, d = i % D, r = row0 + row;
         if (r >= rows_total) break;
@@ -603,9 +631,8 @@ __global__ void __launch_bounds__(kMmaThreads, 2) paged_mma_kernel(cf_kv_paged_a
         }
         const size_t out_row = static_cast<size_t>(r / G) * desc.query_head_count + kv_head * G + r % G;
         if (splits > 1) {
-            float *dst = partials + (out_row * splits + split) * (D + 2u);
-            if (d == 0) dst[0] = m, dst[1] = l;
-            dst[2 + d] = a;
+            if (d == 0) partial_ml[out_row * splits + split] = make_float2(m, l);
+            partials[(out_row * splits + split) * D + d] = a;
         } else {
             desc.output[out_row * D + d] = l > 0.0f ? a / l : 0.0f;   // no visible token: zeros (paged_kv_attention.cu:170-173)
         }
@@ -619,32 +646,62 @@ __global__ void __launch_bounds__(kMmaThreads, 2) paged_mma_kernel(cf_kv_paged_a
     __syncthreads();
     if (!s_last) return;
     __threadfence();
-    float *weight = reinterpret_cast<float *>(smem + L::kOffWarps);   // [16 rows][splits], then 1 / sum per row
-    float *inverse = weight + 16u * splits;
-    for (uint32_t row = warp; row < 16u && row0 + row < rows_total; row += kMmaWarps) {
+    float *weight = reinterpret_cast<float *>(smem + L::kOffWarps);   // [row of the tile][split]
+    const uint32_t tile_rows = min(16u, rows_total - row0);
+    for (uint32_t row = warp; row < tile_rows; row += kMmaWarps) {   // at most 64 splits: two per lane
         const uint32_t r = row0 + row;
-        const float *src = partials + (static_cast<size_t>(r / G) * desc.query_head_count + kv_head * G + r % G) * splits * (D + 2u);
-        float m = -CUDART_INF_F, l = 0.0f;
-        for (uint32_t i = lane; i < splits; i += 32u) m = fmaxf(m, __ldcg(src + i * (D + 2u)));
-        m = warp_max(m);
-        for (uint32_t i = lane; i < splits; i += 32u) {
-            const float ms = __ldcg(src + i * (D + 2u)), w = ms == -CUDART_INF_F ? 0.0f : exp2f(ms - m);
-            weight[row * splits + i] = w;
-            l += __ldcg(src + i * (D + 2u) + 1u) * w;
-        }
-        l = warp_sum(l);
-        if (lane == 0) inverse[row] = l > 0.0f ? 1.0f / l : 0.0f;
+        const float2 *ml = partial_ml + (static_cast<size_t>(r / G) * desc.query_head_count + kv_head * G + r % G) * splits;
+        const float2 ml0 = lane < splits ? __ldcg(ml + lane) : make_float2(-CUDART_INF_F, 0.0f);
+        const float2 ml1 = lane + 32u < splits ? __ldcg(ml + lane + 32u) : make_float2(-CUDART_INF_F, 0.0f);
+        const float m = warp_max(fmaxf(ml0.x, ml1.x));
+        const float w0 = ml0.x == -CUDART_INF_F ? 0.0f : exp2f(ml0.x - m), w1 = ml1.x == -CUDART_INF_F ? 0.0f : exp2f(ml1.x - m);
+        const float l = warp_sum(ml0.y * w0 + ml1.y * w1), inverse = l > 0.0f ? 1.0f / l : 0.0f;   // no visible token: zeros
+        if (lane < splits) weight[row * splits + lane] = w0 * inverse;
+        if (lane + 32u < splits) weight[row * splits + lane + 32u] = w1 * inverse;
     }
     __syncthreads();
-    for (uint32_t i = tid; i < 16u * D; i += kMmaThreads) {
-        const uint32_t row = i / D, d = i % D, r = row0 + row;
-        if (r >= rows_total) break;
+    // D / 4 threads hold a row, four channels each; where the tile has few rows several such groups share a row's splits, so
+    // that a decode step has (nearly) all of them in flight at once.
+    constexpr uint32_t kRowThreads = D / 4u, kGroups = kMmaThreads / kRowThreads;
+    const uint32_t group = tid / kRowThreads, quad = tid % kRowThreads, shares = max(1u, kGroups / tile_rows), share = group % shares;
+    float4 *meet = reinterpret_cast<float4 *>(smem + L::kOffWarps + 16u * 64u * 4u);
+    for (uint32_t row = group / shares; row < tile_rows; row += kGroups / shares) {
+        const uint32_t r = row0 + row;
         const size_t out_row = static_cast<size_t>(r / G) * desc.query_head_count + kv_head * G + r % G;
-        const float *src = partials + out_row * splits * (D + 2u) + 2u + d;
-        float a = 0.0f;
-#pragma unroll 8
-        for (uint32_t k = 0; k < splits; ++k) a += __ldcg(src + k * (D + 2u)) * weight[row * splits + k];
-        desc.output[out_row * D + d] = a * inverse[row];
+        const float4 *src = reinterpret_cast<const float4 *>(partials + out_row * splits * D) + quad;
+        float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (uint32_t k0 = share; k0 < splits; k0 += 8u * shares) {   // eight loads in flight whatever is left
+            float4 x[8];
+#pragma unroll
+            for (uint32_t i = 0; i < 8u; ++i) {
+                const uint32_t k = k0 + i * shares;
+                x[i] = k < splits ? __ldcg(src + k * kRowThreads) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+#pragma unroll
+            for (uint32_t i = 0; i < 8u; ++i) {
+                const float w = weight[row * splits + min(k0 + i * shares, splits - 1u)];
+                a.x += x[i].x * w, a.y += x[i].y * w, a.z += x[i].z * w, a.w += x[i].w * w;
+            }
+        }
+        if (shares == 1u) {
+            float *out = desc.output + out_row * D + 4u * quad;
+            out[0] = a.x, out[1] = a.y, out[2] = a.z, out[3] = a.w;
+        } else {
+            meet[tid] = a;
+        }
+    }
+    if (shares > 1u) {   // one pass above: group / shares is the row
+        __syncthreads();
+        const uint32_t row = group / shares, r = row0 + row;
+        if (share == 0 && row < tile_rows) {
+            float4 a = meet[tid];
+            for (uint32_t k = 1; k < shares; ++k) {
+                const float4 x = meet[tid + k * kRowThreads];
+                a.x += x.x, a.y += x.y, a.z += x.z, a.w += x.w;
+            }
+            float *out = desc.output + (static_cast<size_t>(r / G) * desc.query_head_count + kv_head * G + r % G) * D + 4u * quad;
+            out[0] = a.x, out[1] = a.y, out[2] = a.z, out[3] = a.w;
+        }
     }
     if (tid == 0) *counter = 0u;
 }
@@ -666,18 +723,23 @@ cudaError_t launch_paged_mma(const cf_kv_paged_attention_desc &d, uint32_t split
     cudaError_t e;
     LauncherState *state = launcher_state(table, &e);
     if (!state) return e;
+    using Kernel = void (*)(cf_kv_paged_attention_desc, uint32_t, float *, uint32_t *);
+    static constexpr Kernel kernels[2][2] = {{paged_mma_kernel<64, 1>, paged_mma_kernel<64, 2>}, {paged_mma_kernel<128, 1>, paged_mma_kernel<128, 2>}};
     if (!state->configured) {   // room for the largest descriptor list
-        e = cudaFuncSetAttribute(paged_mma_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(MmaLayout<128>::bytes(CF_KV_CUDA_MAX_PAGES_PER_LAUNCH)));
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(paged_mma_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     static_cast<int>(MmaLayout<64>::bytes(CF_KV_CUDA_MAX_PAGES_PER_LAUNCH)));
-        if (e != cudaSuccess) return e;
+        for (int wide = 0; wide < 2; ++wide)
+            for (int rows = 0; rows < 2; ++rows) {
+                e = cudaFuncSetAttribute(kernels[wide][rows], cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         static_cast<int>(wide ? MmaLayout<128>::bytes(CF_KV_CUDA_MAX_PAGES_PER_LAUNCH)
+                                                               : MmaLayout<64>::bytes(CF_KV_CUDA_MAX_PAGES_PER_LAUNCH)));
+                if (e != cudaSuccess) return e;
+            }
         state->configured = true;
     }
-    const dim3 grid(static_cast<uint32_t>((static_cast<uint64_t>(d.query_count) * d.gqa_group_size + 15u) / 16u), d.kv_head_count, splits);
-    if (d.head_dim == 128) paged_mma_kernel<128><<<grid, kMmaThreads, MmaLayout<128>::bytes(d.page_count), stream>>>(d, splits, partials, arrived);
-    else paged_mma_kernel<64><<<grid, kMmaThreads, MmaLayout<64>::bytes(d.page_count), stream>>>(d, splits, partials, arrived);
+    const uint64_t rows = static_cast<uint64_t>(d.query_count) * d.gqa_group_size;
+    const dim3 grid(static_cast<uint32_t>((rows + 15u) / 16u), d.kv_head_count, splits);
+    const bool wide = d.head_dim == 128;
+    kernels[wide][rows > 8u]<<<grid, kMmaThreads, wide ? MmaLayout<128>::bytes(d.page_count) : MmaLayout<64>::bytes(d.page_count), stream>>>(
+        d, splits, partials, arrived);
     return cudaPeekAtLastError();
 }
 
