@@ -72,62 +72,136 @@ inline KiviLayout kivi_layout(uint32_t tokens, uint32_t dim, uint32_t bits) {
     return l;
 }
 
-// One CTA per page. rows: K / V as [token][row_stride floats], this head's `dim` values first in each row.
-__global__ void __launch_bounds__(256) kivi_quantise_kernel(const float *k_rows, const float *v_rows, uint32_t row_stride,
-                                                            uint32_t tokens, uint32_t dim, uint32_t bits, uint8_t *block,
-                                                            KiviLayout lay, uint32_t *status) {
-    extern __shared__ float scales[];   // [dim] K scales | [tokens] V scales
-    float *k_scale = scales, *v_scale = scales + dim;
+// The pages of one append: rows are numbered from the first unsealed one; the first tail_rows of them are already in the
+// tail ([token][row_stride floats], this head's `dim` values first in each row), the others just arrived in the stage
+// ([token][dim]). CTA p makes page p of rows p * tokens ..; the rows after the last page become the new tail.
+constexpr uint32_t kKiviPagesPerLaunch = 64;
+struct KiviJob {
+    const float *stage_k, *stage_v;
+    float *tail_k, *tail_v;
+    uint32_t row_stride, tail_rows, tokens, dim, bits, pages, rest_rows;
+    uint32_t *first_bad;                       // host-mapped: lowest page that holds a non-finite value (its page is not to be used)
+    uint8_t *block[kKiviPagesPerLaunch];
+};
+
+// Bound: latency of two passes over a page (64 KB + 64 KB at 128 x 128, the second out of L1) and, on one SM per page, an
+// IEEE division per value. 32 warps, a token per warp and four channels per lane, so that a pass is a handful of
+// independent 16-byte loads per thread: 50 us with 256 threads that walked the tokens of a channel one by one, 14 us now.
+__global__ void __launch_bounds__(1024) kivi_quantise_kernel(const __grid_constant__ KiviJob job, KiviLayout lay) {
+    extern __shared__ uint32_t magnitudes[];   // [dim] K | [tokens] V absmax as float bits, then the scales in their place
+    const uint32_t tokens = job.tokens, dim = job.dim, bits = job.bits, page = blockIdx.x, first_row = page * tokens;
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    uint32_t *k_mag = magnitudes, *v_mag = magnitudes + dim;
     const int qmax = (1 << (bits - 1)) - 1, zero = 1 << (bits - 1);
-    int bad = 0;
-    for (uint32_t d = threadIdx.x; d < dim; d += blockDim.x) {   // per channel over the tokens
-        float m = 0.0f;
-        for (uint32_t t = 0; t < tokens; ++t) {
-            const float x = k_rows[static_cast<size_t>(t) * row_stride + d];
-            bad |= !isfinite(x);
-            m = fmaxf(m, fabsf(x));
+    auto k_row = [&](uint32_t t) {
+        const uint32_t r = first_row + t;
+        return r < job.tail_rows ? job.tail_k + static_cast<size_t>(r) * job.row_stride : job.stage_k + static_cast<size_t>(r - job.tail_rows) * dim;
+    };
+    auto v_row = [&](uint32_t t) {
+        const uint32_t r = first_row + t;
+        return r < job.tail_rows ? job.tail_v + static_cast<size_t>(r) * job.row_stride : job.stage_v + static_cast<size_t>(r - job.tail_rows) * dim;
+    };
+    for (uint32_t i = threadIdx.x; i < dim; i += blockDim.x) k_mag[i] = 0u;
+    __syncthreads();
+    const bool quads = dim % 4u == 0 && dim <= 128u;   // rows are 16-byte aligned then
+    if (quads) {
+        uint32_t km[4] = {0u, 0u, 0u, 0u};
+#pragma unroll 4
+        for (uint32_t t = warp; t < tokens; t += warps) {
+            uint32_t vm = 0u;
+            if (4u * lane < dim) {
+                const uint4 k = *reinterpret_cast<const uint4 *>(k_row(t) + 4u * lane), v = *reinterpret_cast<const uint4 *>(v_row(t) + 4u * lane);
+                km[0] = max(km[0], k.x & 0x7fffffffu), km[1] = max(km[1], k.y & 0x7fffffffu);
+                km[2] = max(km[2], k.z & 0x7fffffffu), km[3] = max(km[3], k.w & 0x7fffffffu);
+                vm = max(max(v.x & 0x7fffffffu, v.y & 0x7fffffffu), max(v.z & 0x7fffffffu, v.w & 0x7fffffffu));
+            }
+            vm = __reduce_max_sync(0xffffffffu, vm);
+            if (lane == 0) v_mag[t] = vm;
         }
-        k_scale[d] = m == 0.0f ? 1.0f : __fdiv_rn(m, static_cast<float>(qmax));
+        if (4u * lane < dim)
+            for (int j = 0; j < 4; ++j) atomicMax(&k_mag[4u * lane + j], km[j]);
+    } else {
+        for (uint32_t t = warp; t < tokens; t += warps) {
+            uint32_t vm = 0u;
+            for (uint32_t d = lane; d < dim; d += 32u) {
+                atomicMax(&k_mag[d], __float_as_uint(k_row(t)[d]) & 0x7fffffffu);
+                vm = max(vm, __float_as_uint(v_row(t)[d]) & 0x7fffffffu);
+            }
+            vm = __reduce_max_sync(0xffffffffu, vm);
+            if (lane == 0) v_mag[t] = vm;
+        }
     }
-    for (uint32_t t = threadIdx.x / 32u; t < tokens; t += blockDim.x / 32u) {   // per token over the channels: a warp each
-        float m = 0.0f;
-        for (uint32_t d = threadIdx.x % 32u; d < dim; d += 32u) {
-            const float x = v_rows[static_cast<size_t>(t) * row_stride + d];
-            bad |= !isfinite(x);
-            m = fmaxf(m, fabsf(x));
-        }
-        for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-        if (threadIdx.x % 32u == 0) v_scale[t] = m == 0.0f ? 1.0f : __fdiv_rn(m, static_cast<float>(qmax));
+    __syncthreads();
+    int bad = 0;
+    for (uint32_t i = threadIdx.x; i < dim + tokens; i += blockDim.x) {   // dim K channels, then tokens V rows
+        const uint32_t m = magnitudes[i];
+        bad |= m >= 0x7f800000u;   // inf and NaN lie above every finite magnitude
+        const float scale = m == 0u ? 1.0f : __fdiv_rn(__uint_as_float(m), static_cast<float>(qmax));
+        magnitudes[i] = __float_as_uint(scale);
     }
     if (__syncthreads_or(bad)) {   // kv_gpu_fixture.cpp:13: a non-finite value is an error; nothing of the page is used
-        if (threadIdx.x == 0) atomicOr(status, 1u);
+        if (threadIdx.x == 0) atomicMin_system(job.first_bad, page);
         return;
     }
+    const float *k_scale = reinterpret_cast<const float *>(k_mag), *v_scale = reinterpret_cast<const float *>(v_mag);
     const uint32_t per_word = 32u / bits;
+    uint8_t *block = job.block[page];
     uint32_t *kw = reinterpret_cast<uint32_t *>(block + lay.k_words), *vw = reinterpret_cast<uint32_t *>(block + lay.v_words);
-    const uint64_t symbols = static_cast<uint64_t>(tokens) * dim;
-    auto symbol = [&](float x, float scale) {
-        const int q = max(-(qmax + 1), min(qmax, __float2int_rn(__fdiv_rn(x, scale))));   // lrint(x / scale), clamped
-        return static_cast<uint32_t>(q + zero);
+    // lrint(x / scale), clamped. x * (1 / scale) is within 1.5 * 2^-23 * |q| of the quotient, so where it is further than 2^-14
+    // from every half-integer both round alike, and only the few values closer than that take the division.
+    auto symbol = [&](float x, float scale, float rcp) {
+        float y = x * rcp, n = rintf(y);
+        if (!(fabsf(fabsf(y - n) - 0.5f) >= 6.103515625e-05f) || rcp > 1e37f) n = rintf(__fdiv_rn(x, scale));
+        return static_cast<uint32_t>(max(-(qmax + 1), min(qmax, __float2int_rn(n))) + zero);
     };
-    for (uint32_t w = threadIdx.x; w < lay.word_count; w += blockDim.x) {
-        uint32_t kword = 0, vword = 0;
-        for (uint32_t j = 0; j < per_word; ++j) {
-            const uint64_t i = static_cast<uint64_t>(w) * per_word + j;
-            if (i >= symbols) break;
-            const uint32_t t = static_cast<uint32_t>(i / dim), d = static_cast<uint32_t>(i % dim);
-            const uint32_t shift = (32u - bits) - j * bits;
-            kword |= symbol(k_rows[static_cast<size_t>(t) * row_stride + d], k_scale[d]) << shift;
-            vword |= symbol(v_rows[static_cast<size_t>(t) * row_stride + d], v_scale[t]) << shift;
+    if (quads && dim % per_word == 0) {   // a word is four or eight channels of one token
+        const uint32_t row_words = dim / per_word;
+        for (uint32_t w = threadIdx.x; w < lay.word_count; w += blockDim.x) {
+            const uint32_t t = w / row_words, d0 = (w % row_words) * per_word;
+            const float *k = k_row(t) + d0, *v = v_row(t) + d0;
+            const float vs = v_scale[t], vr = __frcp_rn(vs);
+            uint32_t kword = 0, vword = 0;
+            for (uint32_t j = 0; j < per_word; j += 4u) {
+                const float4 a = *reinterpret_cast<const float4 *>(k + j), b = *reinterpret_cast<const float4 *>(v + j);
+                const float *ks = k_scale + d0 + j;
+                const uint32_t ks4[4] = {symbol(a.x, ks[0], __frcp_rn(ks[0])), symbol(a.y, ks[1], __frcp_rn(ks[1])),
+                                         symbol(a.z, ks[2], __frcp_rn(ks[2])), symbol(a.w, ks[3], __frcp_rn(ks[3]))};
+                const uint32_t vs4[4] = {symbol(b.x, vs, vr), symbol(b.y, vs, vr), symbol(b.z, vs, vr), symbol(b.w, vs, vr)};
+#pragma unroll
+                for (int c = 0; c < 4; ++c) kword = kword << bits | ks4[c], vword = vword << bits | vs4[c];
+            }
+            kw[w] = kword;
+            vw[w] = vword;
         }
-        kw[w] = kword;
-        vw[w] = vword;
+    } else {
+        const uint64_t symbols = static_cast<uint64_t>(tokens) * dim;
+        for (uint32_t w = threadIdx.x; w < lay.word_count; w += blockDim.x) {
+            uint32_t kword = 0, vword = 0;
+            for (uint32_t j = 0; j < per_word; ++j) {
+                const uint64_t i = static_cast<uint64_t>(w) * per_word + j;
+                if (i >= symbols) break;
+                const uint32_t t = static_cast<uint32_t>(i / dim), d = static_cast<uint32_t>(i % dim);
+                const uint32_t shift = (32u - bits) - j * bits;
+                kword |= symbol(k_row(t)[d], k_scale[d], __frcp_rn(k_scale[d])) << shift;
+                vword |= symbol(v_row(t)[d], v_scale[t], __frcp_rn(v_scale[t])) << shift;
+            }
+            kw[w] = kword;
+            vw[w] = vword;
+        }
     }
     for (uint32_t d = threadIdx.x; d < dim; d += blockDim.x) reinterpret_cast<float *>(block + lay.k_scales)[d] = k_scale[d];
     for (uint32_t t = threadIdx.x; t < tokens; t += blockDim.x) reinterpret_cast<float *>(block + lay.v_scales)[t] = v_scale[t];
     for (uint32_t b = threadIdx.x; b < lay.block_count; b += blockDim.x) {
         reinterpret_cast<int32_t *>(block + lay.k_offsets)[b] = static_cast<int32_t>(b * 64u * bits);
         reinterpret_cast<int32_t *>(block + lay.v_offsets)[b] = static_cast<int32_t>(b * 64u * bits);
+    }
+    if (page != 0) return;
+    __syncthreads();   // the tail's old rows have been read: the rows after the last page take their place
+    const uint32_t from = job.pages * tokens - job.tail_rows;
+    for (uint32_t i = threadIdx.x; i < job.rest_rows * dim; i += blockDim.x) {
+        const size_t at = static_cast<size_t>(i / dim) * job.row_stride + i % dim;
+        job.tail_k[at] = job.stage_k[static_cast<size_t>(from) * dim + i];
+        job.tail_v[at] = job.stage_v[static_cast<size_t>(from) * dim + i];
     }
 }
 
@@ -185,9 +259,16 @@ struct cf_llama_kv_adapter {
     std::vector<std::unique_ptr<DeviceBuffer<cf_kv_device_page>>> kivi_descs;   // per layer, device
     std::vector<std::vector<cf_kv_device_page>> kivi_host_descs;                // per layer, the same on the host
     uint64_t kivi_resident_bytes = 0;
+    DeviceBuffer<float> kivi_stage;          // rows of an append that fills pages: [K rows | V rows]
+    float *kivi_pinned = nullptr;            // the same on their way from the caller's pageable memory
+    size_t kivi_stage_floats = 0;            // of one of the two streams
+    uint32_t *kivi_first_bad = nullptr;      // host-mapped word the quantiser reports to
+    static constexpr size_t kKiviStageBytes = 4u << 20;   // rows staged at a time (at least one page)
 
     ~cf_llama_kv_adapter() {
         for (uint8_t *c : kivi_chunks) cudaFree(c);
+        if (kivi_pinned) cudaFreeHost(kivi_pinned);
+        if (kivi_first_bad) cudaFreeHost(kivi_first_bad);
     }
     size_t kivi_row_floats() const { return static_cast<size_t>(opt.kv_head_count) * opt.head_dim; }
     float *kivi_tail(DeviceBuffer<float> &buffer, uint32_t layer) const {
@@ -219,7 +300,7 @@ struct cf_llama_kv_adapter {
         for (uint32_t v = 0; v < levels; ++v) lut[v] = static_cast<int32_t>(v | (kivi_bits << 8));
         kivi_lut.ensure(levels, s);
         cuda_check(cudaMemcpy(kivi_lut.ptr, lut.data(), levels * 4, cudaMemcpyHostToDevice), "upload lut");
-        status.ensure(1, s);
+        cuda_check(cudaHostAlloc(reinterpret_cast<void **>(&kivi_first_bad), sizeof(uint32_t), cudaHostAllocMapped), "cudaHostAlloc");
         kivi_descs.clear();
         for (uint32_t l = 0; l < opt.layer_count; ++l) {
             kivi_descs.push_back(std::make_unique<DeviceBuffer<cf_kv_device_page>>());
@@ -247,49 +328,130 @@ struct cf_llama_kv_adapter {
         kivi_resident_bytes = 0;
         for (auto &d : kivi_host_descs) d.clear();
     }
-    // Quantise the tail rows of (layer, kv_head) into one page (the reference's seal_full_pages / flush for one head).
-    void kivi_seal(uint32_t layer, uint32_t kv_head, cudaStream_t s) {
+    // Quantise `pages` pages of `tokens` rows of (layer, kv_head): the rows of the tail, then the staged ones; `rest` staged rows
+    // after them become the tail. One launch and one synchronisation: the reference quantises on the host and throws at
+    // once, and so does this front. Returns the pages that were sealed: fewer than asked if the next one holds NaN or Inf.
+    uint32_t kivi_seal(uint32_t layer, uint32_t kv_head, uint32_t pages, uint32_t tokens, uint32_t rest, cudaStream_t s) {
+        HeadState &h = head(layer, kv_head);
+        const uint32_t D = opt.head_dim;
+        const KiviLayout lay = kivi_layout(tokens, D, kivi_bits);
+        KiviJob job{};
+        job.stage_k = kivi_stage.ptr;
+        job.stage_v = kivi_stage.ptr + kivi_stage_floats;
+        job.tail_k = kivi_tail(kivi_tail_k, layer) + static_cast<size_t>(kv_head) * D;
+        job.tail_v = kivi_tail(kivi_tail_v, layer) + static_cast<size_t>(kv_head) * D;
+        job.row_stride = static_cast<uint32_t>(kivi_row_floats());
+        job.tail_rows = h.tail;
+        job.tokens = tokens;
+        job.dim = D;
+        job.bits = kivi_bits;
+        job.pages = pages;
+        job.rest_rows = rest;
+        job.first_bad = kivi_first_bad;
+        const size_t chunk_index = kivi_chunk_index, chunk_used = kivi_chunk_used;
+        for (uint32_t p = 0; p < pages; ++p) job.block[p] = kivi_take(lay.total);
+        *kivi_first_bad = pages;
+        kivi_quantise_kernel<<<pages, 1024, (static_cast<size_t>(D) + tokens) * sizeof(float), s>>>(job, lay);
+        cuda_check(cudaGetLastError(), "page quantise launch");
+        std::vector<cf_kv_device_page> &host = kivi_host_descs[layer];
+        const size_t first = host.size();
+        for (uint32_t p = 0; p < pages; ++p) {
+            const uint8_t *block = job.block[p];
+            cf_kv_device_page page{};
+            page.k_words = reinterpret_cast<const uint32_t *>(block + lay.k_words);
+            page.v_words = reinterpret_cast<const uint32_t *>(block + lay.v_words);
+            page.k_scales = reinterpret_cast<const float *>(block + lay.k_scales);
+            page.v_scales = reinterpret_cast<const float *>(block + lay.v_scales);
+            page.k_block_offsets = reinterpret_cast<const int32_t *>(block + lay.k_offsets);
+            page.v_block_offsets = reinterpret_cast<const int32_t *>(block + lay.v_offsets);
+            page.k_lut = page.v_lut = kivi_lut.ptr;
+            page.token_begin = h.next_token - h.tail + p * tokens;
+            page.token_count = tokens;
+            page.head_dim = D;
+            page.block_size = 64;
+            page.k_max_code_length = page.v_max_code_length = page.fixed_code_length = kivi_bits;
+            page.zero_point = 1u << (kivi_bits - 1);
+            page.kv_head = kv_head;
+            host.push_back(page);
+        }
+        DeviceBuffer<cf_kv_device_page> &dev = *kivi_descs[layer];
+        dev.ensure(host.size(), s);   // (entries past the list's length are never read: a refused page's is overwritten later)
+        cuda_check(cudaMemcpyAsync(dev.ptr + first, host.data() + first, pages * sizeof(cf_kv_device_page), cudaMemcpyHostToDevice, s), "publish pages");
+        cuda_check(cudaStreamSynchronize(s), "cudaStreamSynchronize");
+        const uint32_t first_bad = *static_cast<volatile uint32_t *>(kivi_first_bad), sealed = std::min(pages, first_bad);
+        if (sealed < pages) {   // the page blocks after the last good page are handed out again
+            host.resize(first + sealed);
+            kivi_chunk_index = chunk_index;
+            kivi_chunk_used = chunk_used;
+            for (uint32_t p = 0; p < sealed; ++p) kivi_take(lay.total);
+        }
+        // EncodedKvPage::resident_bytes: words, offsets, both LUTs, scales
+        kivi_resident_bytes += sealed * (8ull * lay.word_count + 8ull * lay.block_count + 8ull * (1u << kivi_bits) + 4ull * (D + tokens));
+        if (sealed && tokens < opt.page_size) h.flushed_partial = true;
+        h.sealed += sealed * tokens;
+        sealed_tiles += sealed;
+        return sealed;
+    }
+    void kivi_flush(uint32_t layer, uint32_t kv_head, cudaStream_t s) {
         HeadState &h = head(layer, kv_head);
         if (h.tail == 0) return;
-        const uint32_t D = opt.head_dim, tokens = h.tail;
-        const KiviLayout lay = kivi_layout(tokens, D, kivi_bits);
-        uint8_t *block = kivi_take(lay.total);
-        cuda_check(cudaMemsetAsync(status.ptr, 0, 4, s), "clear status");
-        const size_t smem = (static_cast<size_t>(D) + tokens) * sizeof(float);
-        kivi_quantise_kernel<<<1, 256, smem, s>>>(kivi_tail(kivi_tail_k, layer) + static_cast<size_t>(kv_head) * D,
-                                                  kivi_tail(kivi_tail_v, layer) + static_cast<size_t>(kv_head) * D,
-                                                  static_cast<uint32_t>(kivi_row_floats()), tokens, D, kivi_bits, block, lay, status.ptr);
-        cuda_check(cudaGetLastError(), "page quantise launch");
-        uint32_t bad = 0;   // the reference quantises on the host and throws at once; so does this front
-        cuda_check(cudaMemcpyAsync(&bad, status.ptr, 4, cudaMemcpyDeviceToHost, s), "read status");
-        cuda_check(cudaStreamSynchronize(s), "cudaStreamSynchronize");
-        if (bad) throw std::invalid_argument("invalid quantization input");
-        cf_kv_device_page page{};
-        page.k_words = reinterpret_cast<const uint32_t *>(block + lay.k_words);
-        page.v_words = reinterpret_cast<const uint32_t *>(block + lay.v_words);
-        page.k_scales = reinterpret_cast<const float *>(block + lay.k_scales);
-        page.v_scales = reinterpret_cast<const float *>(block + lay.v_scales);
-        page.k_block_offsets = reinterpret_cast<const int32_t *>(block + lay.k_offsets);
-        page.v_block_offsets = reinterpret_cast<const int32_t *>(block + lay.v_offsets);
-        page.k_lut = page.v_lut = kivi_lut.ptr;
-        page.token_begin = h.next_token - h.tail;
-        page.token_count = tokens;
-        page.head_dim = D;
-        page.block_size = 64;
-        page.k_max_code_length = page.v_max_code_length = page.fixed_code_length = kivi_bits;
-        page.zero_point = 1u << (kivi_bits - 1);
-        page.kv_head = kv_head;
-        std::vector<cf_kv_device_page> &host = kivi_host_descs[layer];
-        host.push_back(page);
-        DeviceBuffer<cf_kv_device_page> &dev = *kivi_descs[layer];
-        dev.ensure(host.size(), s);
-        cuda_check(cudaMemcpyAsync(dev.ptr + host.size() - 1, &host.back(), sizeof page, cudaMemcpyHostToDevice, s), "publish page");
-        // EncodedKvPage::resident_bytes: words, offsets, both LUTs, scales
-        kivi_resident_bytes += 8ull * lay.word_count + 8ull * lay.block_count + 8ull * (1u << kivi_bits) + 4ull * (D + tokens);
-        if (h.tail < opt.page_size) h.flushed_partial = true;
-        h.sealed += h.tail;
+        if (kivi_seal(layer, kv_head, 1, h.tail, 0, s) == 0) throw std::invalid_argument("invalid quantization input");
         h.tail = 0;
-        ++sealed_tiles;
+    }
+    // `take` host rows into the tail ([token][kv head][dim]: the layout the attention reads).
+    void kivi_rows_to_tail(uint32_t layer, uint32_t kv_head, const float *keys, const float *values, uint32_t take, cudaStream_t s) {
+        if (take == 0) return;
+        HeadState &h = head(layer, kv_head);
+        const size_t row = kivi_row_floats(), D = opt.head_dim, at = static_cast<size_t>(h.tail) * row + static_cast<size_t>(kv_head) * D;
+        cuda_check(cudaMemcpy2DAsync(kivi_tail(kivi_tail_k, layer) + at, row * 4, keys, D * 4, D * 4, take, cudaMemcpyHostToDevice, s), "append keys");
+        cuda_check(cudaMemcpy2DAsync(kivi_tail(kivi_tail_v, layer) + at, row * 4, values, D * 4, D * 4, take, cudaMemcpyHostToDevice, s), "append values");
+        h.tail += take;
+        h.next_token += take;
+    }
+    // Host rows of (layer, kv_head): those that only lengthen the tail are copied there; those that complete pages are staged,
+    // as many pages at a time as the stage holds, and quantised by one launch.
+    void kivi_append(uint32_t layer, uint32_t kv_head, const float *keys, const float *values, uint32_t token_count, cudaStream_t s) {
+        HeadState &h = head(layer, kv_head);
+        const uint32_t T = tile_tokens, D = opt.head_dim;
+        uint32_t done = 0;
+        while (done < token_count) {
+            const uint32_t left = token_count - done;
+            if (h.tail + left < T) {
+                kivi_rows_to_tail(layer, kv_head, keys + static_cast<size_t>(done) * D, values + static_cast<size_t>(done) * D, left, s);
+                return;
+            }
+            const uint32_t room = std::max<uint32_t>(1u, std::min<uint32_t>(kKiviPagesPerLaunch, static_cast<uint32_t>(kKiviStageBytes / (4ull * T * D))));
+            const uint32_t pages = std::min<uint32_t>(room, (h.tail + left) / T);
+            const bool last = pages == (h.tail + left) / T;
+            const uint32_t rows = last ? left : pages * T - h.tail, rest = last ? h.tail + left - pages * T : 0u;
+            const size_t floats = static_cast<size_t>(rows) * D;
+            if (floats > kivi_stage_floats) {
+                const size_t wanted = std::max(floats, kivi_stage_floats * 2);
+                if (kivi_pinned) cudaFreeHost(kivi_pinned);   // every launch that read it has been waited for
+                kivi_pinned = nullptr;
+                kivi_stage_floats = 0;
+                cuda_check(cudaHostAlloc(reinterpret_cast<void **>(&kivi_pinned), 2 * wanted * sizeof(float), cudaHostAllocDefault), "cudaHostAlloc");
+                kivi_stage.ensure(2 * wanted, s);
+                kivi_stage_floats = wanted;
+            }
+            const float *source[2] = {keys + static_cast<size_t>(done) * D, values + static_cast<size_t>(done) * D};
+            for (int stream = 0; stream < 2; ++stream) {   // the copy of K crosses the bus while V is gathered
+                std::memcpy(kivi_pinned + stream * kivi_stage_floats, source[stream], floats * sizeof(float));
+                cuda_check(cudaMemcpyAsync(kivi_stage.ptr + stream * kivi_stage_floats, kivi_pinned + stream * kivi_stage_floats, floats * sizeof(float),
+                                           cudaMemcpyHostToDevice, s), "stage rows");
+            }
+            const uint32_t sealed = kivi_seal(layer, kv_head, pages, T, rest, s);
+            if (sealed < pages) {   // pages before the refused one stay; its rows become the (full) tail, as if appended page by page
+                const uint32_t skip = sealed ? sealed * T - h.tail : 0u, keep = sealed ? 0u : h.tail;
+                if (sealed) h.next_token += skip;
+                h.tail = keep;
+                kivi_rows_to_tail(layer, kv_head, source[0] + static_cast<size_t>(skip) * D, source[1] + static_cast<size_t>(skip) * D, T - keep, s);
+                throw std::invalid_argument("invalid quantization input");
+            }
+            h.tail = rest;
+            h.next_token += rows;
+            done += rows;
+        }
     }
 
     HeadState &head(uint32_t layer, uint32_t h) { return heads[static_cast<size_t>(layer) * opt.kv_head_count + h]; }
@@ -539,21 +701,8 @@ extern "C" int cf_llama_kv_append(cf_llama_kv_adapter *adapter, uint32_t layer, 
             h.next_token = token_begin;
         }
         const uint32_t D = adapter->opt.head_dim, T = adapter->tile_tokens;
-        if (adapter->kivi) {   // rows into the [token][kv head][dim] tail the attention reads; a full tail becomes a page
-            const size_t row = adapter->kivi_row_floats();
-            uint32_t done = 0;
-            while (done < token_count) {
-                const uint32_t take = std::min(token_count - done, T - h.tail);
-                const size_t at = static_cast<size_t>(h.tail) * row + static_cast<size_t>(kv_head) * D;
-                cuda_check(cudaMemcpy2DAsync(adapter->kivi_tail(adapter->kivi_tail_k, layer) + at, row * 4, keys + static_cast<size_t>(done) * D,
-                                             D * 4ull, D * 4ull, take, cudaMemcpyHostToDevice, s), "append keys");
-                cuda_check(cudaMemcpy2DAsync(adapter->kivi_tail(adapter->kivi_tail_v, layer) + at, row * 4, values + static_cast<size_t>(done) * D,
-                                             D * 4ull, D * 4ull, take, cudaMemcpyHostToDevice, s), "append values");
-                h.tail += take;
-                h.next_token += take;
-                done += take;
-                if (h.tail == T) adapter->kivi_seal(layer, kv_head, s);
-            }
+        if (adapter->kivi) {
+            adapter->kivi_append(layer, kv_head, keys, values, token_count, s);
             h.appended += token_count;
             return;
         }
@@ -711,7 +860,7 @@ extern "C" int cf_llama_kv_flush(cf_llama_kv_adapter *adapter, void *stream) {
     return guarded(adapter, [&] {
         for (uint32_t layer = 0; layer < adapter->opt.layer_count; ++layer)
             for (uint32_t h = 0; h < adapter->opt.kv_head_count; ++h) {
-                if (adapter->kivi) adapter->kivi_seal(layer, h, static_cast<cudaStream_t>(stream));
+                if (adapter->kivi) adapter->kivi_flush(layer, h, static_cast<cudaStream_t>(stream));
                 else adapter->seal_tail(layer, h, static_cast<cudaStream_t>(stream));
             }
     });

@@ -7,6 +7,7 @@ import numpy as np
 import pytest
 
 from compat_types import DevicePage, PagedAttentionDesc
+from test_gpu_compat import _read_device
 
 pytestmark = pytest.mark.gpu
 
@@ -104,3 +105,83 @@ def test_paged_attention_on_the_tensor_cores(native, oracle, case):
     got = out.cpu().numpy()
     assert np.isfinite(got).all()
     assert np.abs(got - want).max() <= 1e-5 * np.abs(want).max(), np.abs(got - want).max() / np.abs(want).max()
+
+
+# ---- the adapter's page quantiser (csrc/adapter.cu): several pages per launch --------------------------------------------
+def _quantised(x, axis, bits):
+    """The reference fixture's rule (src/runtime/kv_gpu_fixture.cpp:12-16, 46-95) in fp32: one scale along `axis`."""
+    qmax = (1 << (bits - 1)) - 1
+    m = np.abs(x).max(axis=axis, keepdims=True)
+    scale = np.where(m == 0, np.float32(1), m / np.float32(qmax)).astype(np.float32)
+    return (np.clip(np.rint(x / scale), -(qmax + 1), qmax) + (1 << (bits - 1))).astype(np.uint8), scale.ravel()
+
+
+def _adapter(native, heads, d, page, bits):
+    from compat_types import LlamaKvOptions
+    lib = native.lib()
+    lib.cf_llama_kv_create.restype = C.c_void_p
+    opt = LlamaKvOptions(C.sizeof(LlamaKvOptions), 1, 1, heads, heads, d, page, 1, bits)
+    handle = C.c_void_p(lib.cf_llama_kv_create(C.byref(opt)))
+    assert handle.value
+    return lib, handle
+
+
+def _append(lib, handle, head, begin, k, v):
+    return lib.cf_llama_kv_append(handle, 0, head, begin, C.c_void_p(k.ctypes.data), C.c_void_p(v.ctypes.data), k.shape[0], None)
+
+
+@pytest.mark.parametrize("d,page,bits,pieces", [(128, 128, 4, [1, 500, 300]), (64, 16, 8, [1100]), (48, 32, 4, [31, 1, 33]), (30, 16, 4, [50]),
+                                                (128, 256, 8, [255, 2, 600])], ids=str)
+def test_adapter_pages_of_multi_page_appends_are_exact(native, d, page, bits, pieces):
+    import torch
+    rng = np.random.default_rng(d + page)
+    lib, handle = _adapter(native, 2, d, page, bits)
+    total = sum(pieces)
+    k = (rng.standard_normal((2, total, d)) * 10.0 ** rng.uniform(-3, 2, (1, total, 1))).astype(np.float32)
+    v = (rng.standard_normal((2, total, d)) * 10.0 ** rng.uniform(-3, 2, (1, 1, d))).astype(np.float32)
+    k[0, :, 3] = 0.0
+    at = 0
+    for n in pieces:
+        for h in range(2):
+            kk, vv = np.ascontiguousarray(k[h, at:at + n]), np.ascontiguousarray(v[h, at:at + n])
+            assert _append(lib, handle, h, at, kk, vv) == 0
+        at += n
+    seen = {0: 0, 1: 0}
+    for i in range(2 * (total // page)):
+        pg = DevicePage()
+        assert lib.cf_b200_llama_kv_reference_page(handle, 0, i, C.byref(pg)) == 0
+        h = pg.kv_head
+        assert pg.token_begin == seen[h] and pg.token_count == page
+        rows = slice(seen[h], seen[h] + page)
+        seen[h] += page
+        ks, kscale = _quantised(k[h, rows], 0, bits)
+        vs, vscale = _quantised(v[h, rows], 1, bits)
+        words = (page * d * bits + 31) // 32
+        for ptr, want in ((pg.k_words, _pack(ks, bits)[:words]), (pg.v_words, _pack(vs, bits)[:words])):
+            assert np.array_equal(_read_device(ptr, words, np.uint32), want)
+        assert np.array_equal(_read_device(pg.k_scales, d, np.float32), kscale) and np.array_equal(_read_device(pg.v_scales, page, np.float32), vscale)
+    assert lib.cf_b200_llama_kv_reference_page(handle, 0, 2 * (total // page), C.byref(DevicePage())) == -1
+    lib.cf_llama_kv_destroy(handle)
+
+
+def test_adapter_append_keeps_the_pages_before_a_refused_one(native):
+    """Five pages in one append, NaN in the fourth: the first three are sealed, the fourth's rows are the full tail and every
+    further append fails, as when the rows came page by page."""
+    from compat_types import LlamaKvStats
+    rng = np.random.default_rng(3)
+    lib, handle = _adapter(native, 1, 64, 16, 4)
+    lib.cf_llama_kv_last_error.restype = C.c_char_p
+    k, v = (rng.standard_normal((85, 64)).astype(np.float32) for _ in range(2))
+    v[3 * 16 + 2, 7] = np.nan
+    assert _append(lib, handle, 0, 0, k[:5], v[:5]) == 0
+    assert _append(lib, handle, 0, 5, k[5:], v[5:]) == -1 and lib.cf_llama_kv_last_error(handle) == b"invalid quantization input"
+    stats = LlamaKvStats()
+    assert lib.cf_llama_kv_get_stats(handle, C.byref(stats)) == 0
+    assert (stats.sealed_pages, stats.sealed_tokens, stats.active_tokens) == (3, 48, 16)
+    assert _append(lib, handle, 0, 64, k[64:66], v[64:66]) == -1
+    assert lib.cf_llama_kv_clear(handle) == 0 and _append(lib, handle, 0, 0, k[:48], v[:48]) == 0
+    pg = DevicePage()
+    assert lib.cf_b200_llama_kv_reference_page(handle, 0, 2, C.byref(pg)) == 0 and pg.token_begin == 32
+    ks, _ = _quantised(k[32:48], 0, 4)
+    assert np.array_equal(_read_device(pg.k_words, 128, np.uint32), _pack(ks, 4)[:128])
+    lib.cf_llama_kv_destroy(handle)
