@@ -10,13 +10,13 @@
 #include <map>
 #include <memory>
 #include <mutex>
-#include <set>
 #include <stdexcept>
 #include <string>
 #include <unordered_set>
 #include <vector>
 
 #include "chromofold_b200/compat_mscache.h"
+#include "ms_internal.h"
 
 static_assert(sizeof(cf_sequence_attention_item) == sizeof(cf_ms_batch_item), "the two batch item layouts are one");
 
@@ -306,11 +306,33 @@ extern "C" int cf_sequence_append_async(cf_multisequence_cache *c, int64_t id, u
     });
 }
 
+// cf_sequence_append_async for any number of dense fp32 rows, cut at page boundaries: `applicable` is false (and nothing done)
+// where the pages of the store and of the caller's positions do not coincide or a speculation holds the tail open; the rows
+// then have to go page by page.
+static int append_rows(cf_multisequence_cache *c, int64_t id, uint32_t layer, uint32_t token_begin, const float *keys, const float *values,
+                       uint32_t token_count, void *stream, bool *applicable) {
+    *applicable = true;
+    return guarded(c, [&] {
+        SequenceState &q = find(c, id);
+        const bool empty = total_tokens(c, id) == 0;
+        const uint32_t base = empty ? token_begin : q.base;
+        if (q.speculation.active || base % c->config.page_size != 0) {
+            *applicable = false;
+            return;
+        }
+        q.base = base;
+        if (token_begin < base) throw std::runtime_error("non-contiguous sequence append");
+        device_check(c, cfb_engine::ms_append_rows(c->device, id, layer, token_begin - base, keys, values, token_count, stream));
+        maybe_audit(c);
+    });
+}
+
 extern "C" int cf_multisequence_attention_async(cf_multisequence_cache *c, const cf_sequence_attention_item *items,
                                                 uint32_t item_count, void *stream) {
     if (!c || !items || item_count == 0) return -1;
     return guarded(c, [&] {
-        std::set<int64_t> observed;
+        std::vector<int64_t> observed;
+        observed.reserve(item_count);
         bool rebased = false;
         for (uint32_t i = 0; i < item_count; ++i) {
             const cf_sequence_attention_item &item = items[i];
@@ -320,8 +342,10 @@ extern "C" int cf_multisequence_attention_async(cf_multisequence_cache *c, const
                 throw std::runtime_error("invalid sequence attention item");
             if (item.query_token_begin < it->second.base) throw std::runtime_error("query position lies before the sequence's first token");
             rebased = rebased || it->second.base != 0;
-            observed.insert(item.sequence_id);
+            observed.push_back(item.sequence_id);
         }
+        std::sort(observed.begin(), observed.end());
+        observed.erase(std::unique(observed.begin(), observed.end()), observed.end());
         ++c->counters.batches_dispatched;
         c->counters.sequences_per_batch_peak = std::max<uint64_t>(c->counters.sequences_per_batch_peak, observed.size());
         if (!rebased) {
@@ -548,6 +572,10 @@ extern "C" int cf_llama_server_append_layer_async(cf_llama_server_runtime *r, in
     if (layer >= r->config.layer_count) return server_fail(r, "layer index is out of range");
     const uint64_t row = static_cast<uint64_t>(r->config.kv_head_count) * r->config.head_dim;
     uint32_t done = 0;
+    bool at_once = false;
+    if (append_rows(r->cache, id, layer, token_begin, key, value, token_count, stream, &at_once) != 0)
+        return server_fail(r, cf_multisequence_last_error(r->cache));
+    if (at_once) done = token_count;
     while (done < token_count) {   // page by page: an append never crosses a page boundary
         const uint32_t position = token_begin + done;
         const uint32_t chunk = std::min(token_count - done, r->config.page_size - position % r->config.page_size);
@@ -576,12 +604,12 @@ extern "C" int cf_llama_server_execute_batch_async(cf_llama_server_runtime *r, c
     std::lock_guard<std::mutex> guard(r->mutex);
     if (r->shutting_down) return server_fail(r, "server runtime is shutting down");
     if (r->stats.dense_nodes_scheduled != 0) return server_fail(r, "dense attention node scheduled while the sealed-KV backend is active");
-    std::unordered_set<int64_t> ids;
+    bool several = false;
     for (uint32_t i = 0; i < batch->attention_item_count; ++i) {
         if (!r->live.count(batch->attention_items[i].sequence_id)) return server_fail(r, "batch references unknown sequence");
-        ids.insert(batch->attention_items[i].sequence_id);
+        several = several || batch->attention_items[i].sequence_id != batch->attention_items[0].sequence_id;
     }
-    if (ids.size() > 1) ++r->stats.interleaved_batches;
+    if (several) ++r->stats.interleaved_batches;
     if (cf_multisequence_attention_async(r->cache, batch->attention_items, batch->attention_item_count, stream) != 0)
         return server_fail(r, cf_multisequence_last_error(r->cache));
     r->error.clear();

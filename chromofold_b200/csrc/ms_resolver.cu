@@ -12,12 +12,15 @@
 #include "chromofold_b200/compat_ms.h"
 #include "cf_device_common.cuh"
 #include "engine_common.cuh"
+#include "ms_internal.h"
+#include "seal_params.cuh"
 
 using namespace cfb_engine;
 
 namespace {
 
 constexpr uint32_t kMaxBatchTokens = 2048;
+constexpr size_t kPendingBatches = 64;   // batches whose snapshots may be out before finished ones are let go without being asked
 
 struct SharedPage;
 // `page` is the entry of cf_ms_cuda_resolver::pages for page_id (entries of that map do not move; set when the reference
@@ -26,6 +29,7 @@ struct PageRef { uint64_t page_id; int64_t logical_begin; uint32_t tokens; uint3
 struct SharedPage {
     uint64_t logical_refs = 0, in_flight_refs = 0, resident_bytes = 0, seal_generation = 0;
     bool retired = false;
+    mutable uint64_t observed = 0;    // scratch of the audit
     uint64_t record_bytes = 0;        // what the sealer wrote into the page's arena slot
     std::vector<uint32_t> store_ids;  // page ids of its tiles in the arena's directory
 };
@@ -67,6 +71,24 @@ __global__ void unpack_reference_page_kernel(cf_device_page_descriptor page, flo
     const uint64_t dst = (static_cast<uint64_t>(h) * capacity + t) * page.head_dim + d;
     tail_k[dst] = k;
     tail_v[dst] = v;
+}
+
+// Rows into the fp32 tail of one (layer, slot) ([kv head][capacity][dim], from tail row `row0`; z = 0: keys, z = 1: values) and,
+// with them, the counts a reader of the sequence goes by: one launch per append.
+__global__ void append_tail_kernel(cf_device_tensor_view keys, cf_device_tensor_view values, float *tail_k, float *tail_v, uint32_t capacity,
+                                   uint32_t row0, uint32_t *sealed_at, uint32_t sealed, uint32_t *tail_at, uint32_t tail) {
+    if (blockIdx.x == 0 && blockIdx.z == 0 && threadIdx.x == 0) {
+        *sealed_at = sealed;
+        *tail_at = tail;
+    }
+    const cf_device_tensor_view &view = blockIdx.z ? values : keys;
+    const uint64_t count = static_cast<uint64_t>(view.token_count) * view.head_count * view.head_dim;
+    const uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (i >= count) return;
+    const uint32_t d = i % view.head_dim, h = (i / view.head_dim) % view.head_count;
+    const uint32_t t = i / (static_cast<uint64_t>(view.head_dim) * view.head_count);
+    const float v = load_scalar(view.data, t * view.token_stride_bytes + h * view.head_stride_bytes + d * view.element_stride_bytes, view.scalar_type);
+    (blockIdx.z ? tail_v : tail_k)[(static_cast<uint64_t>(h) * capacity + row0 + t) * view.head_dim + d] = v;
 }
 
 struct ItemIo {   // one batch item's query view and output placement, as the gather / scatter kernels see them
@@ -128,12 +150,17 @@ struct cf_ms_cuda_resolver {
     bool ready = false;
     Buffer<uint8_t> arena, workspace;
     Buffer<uint64_t> page_dir;
-    Buffer<uint32_t> page_table, sealed, tails, jobs, status, slot_list, positions;   // tables are [layer][slot]
+    Buffer<uint32_t> page_table, sealed, tails, jobs, status, slot_list;   // tables are [layer][slot]
     Buffer<float> tail_k, tail_v, scratch_k, scratch_v, q_dense, o_dense;          // tails are [layer][slot][Hkv][page][D]
     Buffer<cf_b200_codebook_tables> tables;
     Buffer<unsigned long long> cursor;
     Buffer<ItemIo> item_io;
+    Buffer<uint32_t> seal_report;        // what a bulk seal wrote per (tile, kv head), and the device status word
+    std::vector<cudaEvent_t> free_events;
 
+    ~cf_ms_cuda_resolver() {
+        for (cudaEvent_t e : free_events) cudaEventDestroy(e);
+    }
     size_t page_values() const { return static_cast<size_t>(config.kv_head_count) * config.page_size * config.head_dim; }
     size_t max_record_bytes() const { return 16 + 2 * ((static_cast<size_t>(tile) * config.head_dim + 15) / 16 * 16); }
     size_t row(uint32_t layer, uint32_t slot) const { return static_cast<size_t>(layer) * slot_capacity + slot; }
@@ -151,11 +178,7 @@ struct cf_ms_cuda_resolver {
         page_dir.ensure(static_cast<size_t>(4096) * config.kv_head_count, s);
         scratch_k.ensure(page_values(), s);
         scratch_v.ensure(page_values(), s);
-        slot_list.ensure(kMaxBatchTokens, s);
-        positions.ensure(kMaxBatchTokens, s);
-        item_io.ensure(1024, s);
-        q_dense.ensure(static_cast<size_t>(kMaxBatchTokens) * config.query_head_count * config.head_dim, s);
-        o_dense.ensure(q_dense.count, s);
+        slot_list.ensure(2 * kMaxBatchTokens, s);   // slots, then positions
         cf_b200_sealed_attention_desc d{};
         d.kv_head_count = config.kv_head_count;
         d.query_head_count = config.query_head_count;
@@ -216,11 +239,17 @@ struct cf_ms_cuda_resolver {
         return slot;
     }
 
-    void push_scalars(const Sequence &q, uint32_t layer, cudaStream_t s) {
+    // The sequence's counts to the device, with rows for its tail (views of no tokens: the counts alone).
+    void push_rows(const Sequence &q, uint32_t layer, const cf_device_tensor_view &keys, const cf_device_tensor_view &values, uint32_t row0, cudaStream_t s) {
         const LayerSeq &L = q.layers[layer];
-        cuda_check(cudaMemcpyAsync(sealed.ptr + row(layer, q.slot), &L.sealed_tokens, 4, cudaMemcpyHostToDevice, s), "sealed count");
-        cuda_check(cudaMemcpyAsync(tails.ptr + row(layer, q.slot), &L.active_count, 4, cudaMemcpyHostToDevice, s), "tail count");
+        const uint64_t count = static_cast<uint64_t>(keys.token_count) * keys.head_count * keys.head_dim;
+        const size_t base = row(layer, q.slot) * page_values();
+        append_tail_kernel<<<dim3(static_cast<unsigned>(std::max<uint64_t>(1, (count + 255) / 256)), 1, count ? 2 : 1), 256, 0, s>>>(
+            keys, values, tail_k.ptr + base, tail_v.ptr + base, config.page_size, row0, sealed.ptr + row(layer, q.slot), L.sealed_tokens,
+            tails.ptr + row(layer, q.slot), L.active_count);
+        cuda_check(cudaGetLastError(), "append sequence rows");
     }
+    void push_scalars(const Sequence &q, uint32_t layer, cudaStream_t s) { push_rows(q, layer, {}, {}, 0, s); }
 
     void release_snapshot(const Snapshot &snap) {
         if (snap.lazy) {   // never written down: the list it pinned is still there (a drop would have materialised it)
@@ -299,6 +328,67 @@ void retire_if_unreferenced(cf_ms_cuda_resolver *r, SharedPage &page) {
     r->counters.pending_reclamation_bytes_peak = std::max(r->counters.pending_reclamation_bytes_peak, r->counters.pending_reclamation_bytes);
 }
 
+// Snapshots of finished batches let go, their events kept for the next ones (cf_ms_cuda_reclaim_async, and by itself once
+// many are out: a server that only decodes would otherwise keep one event per batch for ever).
+void release_finished(cf_ms_cuda_resolver *r) {
+    size_t kept = 0;
+    for (size_t i = 0; i < r->pending.size(); ++i) {
+        Pending &p = r->pending[i];
+        const cudaError_t status = cudaEventQuery(p.event);
+        if (status == cudaErrorNotReady) {
+            if (kept != i) r->pending[kept] = std::move(p);
+            ++kept;
+            continue;
+        }
+        cuda_check(status, "query snapshot release event");
+        for (const Snapshot &snap : p.snapshots) r->release_snapshot(snap);
+        r->free_events.push_back(p.event);
+        p.event = nullptr;
+    }
+    r->pending.resize(kept);
+}
+
+// Retired pages nobody reads any more give their arena slots back; the directory rows of their tiles go back to "not there"
+// (runs of neighbouring slots in one memset).
+void reclaim_pages(cf_ms_cuda_resolver *r, cudaStream_t s) {
+    std::vector<uint32_t> slots;
+    for (auto it = r->pages.begin(); it != r->pages.end();) {
+        SharedPage &page = it->second;
+        if (page.retired && page.logical_refs == 0 && page.in_flight_refs == 0) {
+            if (!page.store_ids.empty()) slots.push_back((page.store_ids.front() - 1u) / r->tiles_per_page);
+            r->live_record_bytes -= std::min<uint64_t>(r->live_record_bytes, page.record_bytes);
+            r->counters.pending_reclamation_bytes -= page.resident_bytes;
+            ++r->counters.pages_reclaimed;
+            it = r->pages.erase(it);
+        } else {
+            ++it;
+        }
+    }
+    std::sort(slots.begin(), slots.end());
+    const size_t slot_entries = static_cast<size_t>(r->tiles_per_page) * r->config.kv_head_count;
+    for (size_t i = 0; i < slots.size();) {
+        size_t n = 1;
+        while (i + n < slots.size() && slots[i + n] == slots[i] + n) ++n;
+        if (r->ready)
+            cuda_check(cudaMemsetAsync(r->page_dir.ptr + slots[i] * slot_entries + r->config.kv_head_count, 0, n * slot_entries * sizeof(uint64_t), s),
+                       "clear directory rows");
+        i += n;
+    }
+    r->free_page_slots.insert(r->free_page_slots.end(), slots.rbegin(), slots.rend());
+}
+
+// `wanted` more page slots are about to be taken: where the free ones do not cover them and the arena would have to grow,
+// what can be reclaimed is reclaimed first, so that a server that resets its slots but never asks for reclamation stays
+// within the memory its live pages need.
+void recycle_before_growth(cf_ms_cuda_resolver *r, size_t wanted, cudaStream_t s) {
+    if (r->free_page_slots.size() >= wanted) return;
+    const uint64_t slot_units = static_cast<uint64_t>(r->tiles_per_page) * r->config.kv_head_count * (r->max_record_bytes() / 16u);
+    const uint64_t end = 1ull + (r->next_page_slot + wanted - r->free_page_slots.size()) * slot_units;
+    if (end * 16u + 4096 <= r->arena.count || r->counters.pages_retired == r->counters.pages_reclaimed) return;
+    release_finished(r);
+    reclaim_pages(r, s);
+}
+
 // Seal `token_count` fp32 rows laid out [kv head][page_size][dim] at src_k / src_v into format-v1 records (one launch),
 // append their ids to the sequence's page-table row of `layer` and return the number of tiles. The first page of a
 // layer also calibrates the layer's shared codebooks from its own codes.
@@ -308,6 +398,7 @@ uint32_t seal_rows(cf_ms_cuda_resolver *r, Sequence &q, uint32_t layer, const fl
     const uint32_t n = (token_count + r->tile - 1) / r->tile;
     r->grow_stride(L.tiles + n, s);
     if (n > r->tiles_per_page) throw std::invalid_argument("more rows than a page holds");
+    recycle_before_growth(r, 1, s);
     const bool recycled = !r->free_page_slots.empty();
     const uint32_t page_slot = recycled ? r->free_page_slots.back() : r->next_page_slot;
     const uint64_t slot_units = static_cast<uint64_t>(r->tiles_per_page) * r->config.kv_head_count * (r->max_record_bytes() / 16u);
@@ -393,6 +484,128 @@ uint32_t seal_rows(cf_ms_cuda_resolver *r, Sequence &q, uint32_t layer, const fl
     cuda_check(cudaMemcpyAsync(r->page_table.ptr + r->row(layer, q.slot) * r->stride + L.tiles, host.data() + n, n * 4,
                                cudaMemcpyHostToDevice, s), "publish page ids");
     return n;
+}
+
+void append_to_active(cf_ms_cuda_resolver *r, Sequence &q, uint32_t layer, uint32_t token_begin, const cf_device_tensor_view &keys,
+                      const cf_device_tensor_view &values, cudaStream_t s) {
+    LayerSeq &L = q.layers[layer];
+    if (L.partial_last) throw std::invalid_argument("a layer whose last page is short cannot grow");
+    if (token_begin != L.sealed_tokens + L.active_count) throw std::invalid_argument("non-contiguous sequence append");
+    if (L.active_count + keys.token_count > r->config.page_size)
+        throw std::invalid_argument("append crosses sequence active-page boundary");
+    r->ensure_ready(s);
+    const uint32_t row0 = L.active_count;
+    if (!row0) L.active_begin = L.sealed_tokens;
+    L.active_count += keys.token_count;
+    ++L.active_generation;
+    r->push_rows(q, layer, keys, values, row0, s);
+}
+
+// The bookkeeping of a page that has been sealed into `n` tiles and holds the layer's next `tokens` tokens.
+void book_sealed_page(cf_ms_cuda_resolver *r, Sequence &q, uint32_t layer, SharedPage &&page, uint32_t tokens, uint32_t n) {
+    LayerSeq &L = q.layers[layer];
+    page.logical_refs = 1;
+    ++r->ref_increments;
+    page.resident_bytes = static_cast<uint64_t>(n) * r->config.kv_head_count * r->max_record_bytes();
+    const uint64_t page_id = r->next_page_id++;
+    L.pages.push_back({page_id, static_cast<int64_t>(L.sealed_tokens), tokens, L.tiles, n});
+    L.pages.back().page = &r->pages.emplace(page_id, std::move(page)).first->second;
+    L.tiles += n;
+    L.sealed_tokens += tokens;
+    L.partial_last = tokens % r->tile != 0;
+    L.active_count = 0;
+    L.active_begin = L.sealed_tokens;
+    ++L.descriptor_generation;
+    ++q.topology_generation;
+    ++r->counters.pages_registered;
+    ++r->counters.descriptor_tables_built;
+}
+
+void seal_active_page(cf_ms_cuda_resolver *r, Sequence &q, uint32_t layer, cudaStream_t s) {
+    LayerSeq &L = q.layers[layer];
+    if (!L.active_count) throw std::invalid_argument("no active rows to seal");
+    if (L.partial_last) throw std::invalid_argument("a short page can only be the last page of a layer");
+    r->ensure_ready(s);
+    const size_t base = r->row(layer, q.slot) * r->page_values();
+    SharedPage page;
+    const uint32_t n = seal_rows(r, q, layer, r->tail_k.ptr + base, r->tail_v.ptr + base, L.active_count, page, s);
+    book_sealed_page(r, q, layer, std::move(page), L.active_count, n);
+    r->push_scalars(q, layer, s);
+}
+
+// Up to kBulkPages full pages straight from dense rows [token][kv head][dim]: one launch, one synchronisation for the outcome
+// (a page with NaN or Inf must be refused by the call that brings it). Returns the pages sealed; fewer than asked if the next
+// one was refused. The caller pushes the counts.
+uint32_t seal_pages_in_place(cf_ms_cuda_resolver *r, Sequence &q, uint32_t layer, const float *keys, const float *values, uint32_t pages, cudaStream_t s) {
+    LayerSeq &L = q.layers[layer];
+    const uint32_t H = r->config.kv_head_count, tiles = pages * r->tiles_per_page;
+    cfb::SealParams p{};
+    p.kv_head_count = H;
+    p.head_dim = r->config.head_dim;
+    p.page_tokens = r->tile;
+    p.block_size = 64;
+    p.coder = engine_coder(r->tile * r->config.head_dim);
+    p.codebook_id = layer;
+    p.k_tables = r->tables.ptr + 2 * layer;
+    p.v_tables = r->tables.ptr + 2 * layer + 1;
+    p.tail_k = keys;
+    p.tail_v = values;
+    p.tail_type = CF_B200_F32;
+    p.row_stride = static_cast<uint64_t>(H) * r->config.head_dim;
+    p.head_stride = r->config.head_dim;
+    p.job_count = tiles;
+    if (!r->calibrated[layer] || !cfb::seal_blocks_supports(p)) return 0;   // the page-by-page way calibrates, and takes every geometry
+    r->grow_stride(L.tiles + tiles, s);
+    recycle_before_growth(r, pages, s);
+    cfb::SealPlacement place{};
+    place.tiles_per_page = r->tiles_per_page;
+    place.record_units = static_cast<uint32_t>(r->max_record_bytes() / 16u);
+    const size_t recycled = std::min<size_t>(pages, r->free_page_slots.size());
+    for (uint32_t i = 0; i < pages; ++i)
+        place.page_slot[i] = i < recycled ? r->free_page_slots[r->free_page_slots.size() - 1u - i] : r->next_page_slot + (i - static_cast<uint32_t>(recycled));
+    const uint64_t slots_after = r->next_page_slot + (pages - recycled);
+    r->arena.ensure((1ull + slots_after * r->tiles_per_page * H * place.record_units) * 16u + 4096, s);
+    r->page_dir.ensure((static_cast<size_t>(slots_after) * r->tiles_per_page + 2) * H, s);
+    const size_t words = static_cast<size_t>(tiles) * H + 1u;
+    r->seal_report.ensure(words, s);
+    p.arena = r->arena.ptr;
+    p.arena_units = r->arena.count / 16;
+    p.page_dir = r->page_dir.ptr;
+    p.status = r->status.ptr;
+    place.used = r->seal_report.ptr;
+    place.table_row = r->page_table.ptr + r->row(layer, q.slot) * r->stride + L.tiles;
+    if (cfb::launch_seal_placed(p, place, s) != cudaSuccess) throw std::runtime_error("seal launch rejected");
+    std::vector<uint32_t> used(words);
+    cuda_check(cudaMemcpyAsync(used.data(), r->seal_report.ptr, words * sizeof(uint32_t), cudaMemcpyDeviceToHost, s), "read seal report");
+    cuda_check(cudaStreamSynchronize(s), "seal validation sync");
+    r->device_status_seen |= used[words - 1u];   // the status word as the launch found it
+    uint32_t good = 0;
+    for (; good < pages; ++good) {
+        uint64_t units = 0;
+        bool refused = false;
+        for (uint32_t i = 0; i < r->tiles_per_page * H; ++i) {
+            const uint32_t u = used[static_cast<size_t>(good) * r->tiles_per_page * H + i];
+            refused = refused || u == cfb::kSealRefused;
+            units += u;
+        }
+        if (refused) break;
+        SharedPage page;
+        for (uint32_t j = 0; j < r->tiles_per_page; ++j) page.store_ids.push_back(place.page_slot[good] * r->tiles_per_page + 1u + j);
+        page.record_bytes = units * 16ull;
+        r->live_record_bytes += page.record_bytes;
+        book_sealed_page(r, q, layer, std::move(page), r->config.page_size, r->tiles_per_page);
+    }
+    if (good < pages) {   // whatever the refused page and those after it did publish goes back to "not there"; their slots stay free
+        r->device_status_seen |= CF_B200_DEVSTAT_NONFINITE;
+        for (uint32_t i = good; i < pages; ++i)
+            cuda_check(cudaMemsetAsync(r->page_dir.ptr + (static_cast<size_t>(place.page_slot[i]) * r->tiles_per_page + 1u) * H, 0,
+                                       static_cast<size_t>(r->tiles_per_page) * H * sizeof(uint64_t), s), "unpublish refused page");
+        cuda_check(cudaMemsetAsync(r->status.ptr, 0, 4, s), "clear status");
+    }
+    const size_t taken = std::min<size_t>(good, recycled);
+    r->free_page_slots.resize(r->free_page_slots.size() - taken);
+    r->next_page_slot += good - static_cast<uint32_t>(taken);
+    return good;
 }
 
 }  // namespace
@@ -530,23 +743,7 @@ extern "C" int cf_b200_ms_append_active_async(cf_ms_cuda_resolver *r, int64_t id
             values->head_count != r->config.kv_head_count || keys->head_dim != r->config.head_dim ||
             values->head_dim != r->config.head_dim || keys->token_count == 0)
             throw std::invalid_argument("append tensor topology mismatch");
-        Sequence &q = it->second;
-        LayerSeq &L = q.layers[layer];
-        if (L.partial_last) throw std::invalid_argument("a layer whose last page is short cannot grow");
-        if (token_begin != L.sealed_tokens + L.active_count) throw std::invalid_argument("non-contiguous sequence append");
-        if (L.active_count + keys->token_count > r->config.page_size)
-            throw std::invalid_argument("append crosses sequence active-page boundary");
-        r->ensure_ready(s);
-        const uint64_t count = static_cast<uint64_t>(keys->token_count) * keys->head_count * keys->head_dim;
-        const int blocks = static_cast<int>((count + 255) / 256);
-        const size_t base = r->row(layer, q.slot) * r->page_values();
-        rows_to_tail_kernel<<<blocks, 256, 0, s>>>(*keys, r->tail_k.ptr + base, r->config.page_size, L.active_count);
-        rows_to_tail_kernel<<<blocks, 256, 0, s>>>(*values, r->tail_v.ptr + base, r->config.page_size, L.active_count);
-        cuda_check(cudaGetLastError(), "append sequence rows");
-        if (!L.active_count) L.active_begin = L.sealed_tokens;
-        L.active_count += keys->token_count;
-        ++L.active_generation;
-        r->push_scalars(q, layer, s);
+        append_to_active(r, it->second, layer, token_begin, *keys, *values, s);
     });
 }
 
@@ -556,30 +753,52 @@ extern "C" int cf_b200_ms_seal_active_async(cf_ms_cuda_resolver *r, int64_t id, 
         cudaStream_t s = static_cast<cudaStream_t>(stream);
         auto it = r->sequences.find(id);
         if (it == r->sequences.end() || layer >= it->second.layers.size()) throw std::invalid_argument("seal target is invalid");
+        seal_active_page(r, it->second, layer, s);
+    });
+}
+
+int cfb_engine::ms_append_rows(cf_ms_cuda_resolver *r, int64_t id, uint32_t layer, uint32_t token_begin, const float *keys, const float *values,
+                               uint32_t token_count, void *stream) {
+    return locked(r, true, [&] {
+        cudaStream_t s = static_cast<cudaStream_t>(stream);
+        auto it = r->sequences.find(id);
+        if (it == r->sequences.end() || layer >= it->second.layers.size()) throw std::invalid_argument("append target is invalid");
         Sequence &q = it->second;
         LayerSeq &L = q.layers[layer];
-        if (!L.active_count) throw std::invalid_argument("no active rows to seal");
-        if (L.partial_last) throw std::invalid_argument("a short page can only be the last page of a layer");
+        if (L.partial_last) throw std::invalid_argument("a layer whose last page is short cannot grow");
+        if (token_begin != L.sealed_tokens + L.active_count) throw std::invalid_argument("non-contiguous sequence append");
         r->ensure_ready(s);
-        const size_t base = r->row(layer, q.slot) * r->page_values();
-        SharedPage page;
-        const uint32_t n = seal_rows(r, q, layer, r->tail_k.ptr + base, r->tail_v.ptr + base, L.active_count, page, s);
-        page.logical_refs = 1;
-        ++r->ref_increments;
-        page.resident_bytes = static_cast<uint64_t>(n) * r->config.kv_head_count * r->max_record_bytes();
-        const uint64_t page_id = r->next_page_id++;
-        L.pages.push_back({page_id, static_cast<int64_t>(L.sealed_tokens), L.active_count, L.tiles, n});
-        L.pages.back().page = &r->pages.emplace(page_id, std::move(page)).first->second;
-        L.tiles += n;
-        L.sealed_tokens += L.active_count;
-        L.partial_last = L.active_count % r->tile != 0;
-        L.active_count = 0;
-        L.active_begin = L.sealed_tokens;
-        ++L.descriptor_generation;
-        r->push_scalars(q, layer, s);
-        ++q.topology_generation;
-        ++r->counters.pages_registered;
-        ++r->counters.descriptor_tables_built;
+        const uint32_t T = r->config.page_size;
+        const size_t row = static_cast<size_t>(r->config.kv_head_count) * r->config.head_dim;
+        cf_device_tensor_view view{};
+        view.scalar_type = CF_DEVICE_F32;
+        view.head_count = r->config.kv_head_count;
+        view.head_dim = r->config.head_dim;
+        view.element_stride_bytes = 4;
+        view.head_stride_bytes = 4ull * view.head_dim;
+        view.token_stride_bytes = 4ull * row;
+        uint32_t done = 0;
+        while (done < token_count) {
+            const uint32_t left = token_count - done;
+            if (L.active_count == 0 && left >= T) {
+                const uint32_t room = std::max<uint32_t>(1u, std::min<uint32_t>(cfb::kBulkPages, (1u << 20) / (r->tiles_per_page * r->config.kv_head_count)));
+                const uint32_t asked = std::min(left / T, room);
+                const uint32_t sealed = seal_pages_in_place(r, q, layer, keys + done * row, values + done * row, asked, s);
+                done += sealed * T;
+                if (sealed == asked) {
+                    if (token_count - done < 1u || token_count - done >= T) r->push_scalars(q, layer, s);   // else with the rows below
+                    continue;
+                }
+            }
+            cf_device_tensor_view k = view, v = view;   // rows that start, continue or complete a page by way of the tail
+            k.token_count = v.token_count = std::min(token_count - done, T - L.active_count);
+            k.data = keys + done * row;
+            v.data = values + done * row;
+            const uint32_t position = L.sealed_tokens + L.active_count;
+            append_to_active(r, q, layer, position, k, v, s);
+            done += k.token_count;
+            if (L.active_count == T) seal_active_page(r, q, layer, s);   // (throws for a page with NaN or Inf, its rows active)
+        }
     });
 }
 
@@ -838,31 +1057,54 @@ extern "C" int cf_ms_cuda_execute_batch_async(cf_ms_cuda_resolver *r, const cf_m
         r->ensure_ready(s);
 
         // rows of the batch, grouped by layer: [layer 0 items..., layer 1 items..., ...]
+        const uint32_t Hq = r->config.query_head_count, D = r->config.head_dim;
+        const size_t row_values = static_cast<size_t>(Hq) * D;
         std::vector<ItemIo> io(item_count);
-        std::vector<uint32_t> slots, positions, order;
+        std::vector<uint32_t> rows(2 * total_rows);   // slots, then positions
         std::vector<std::pair<uint32_t, uint32_t>> layer_rows(r->config.layer_count, {0u, 0u});  // first row, count
+        // Usually the items' queries are the rows of one dense fp32 tensor and their outputs those of another: the kernels
+        // then read and write those directly; otherwise the rows are gathered into and scattered from dense copies.
+        const void *q_base = nullptr, *o_base = nullptr;
+        bool dense = true;
+        uint32_t at = 0;
         for (uint32_t layer = 0; layer < r->config.layer_count; ++layer) {
-            layer_rows[layer].first = static_cast<uint32_t>(slots.size());
+            layer_rows[layer].first = at;
             for (uint32_t i = 0; i < item_count; ++i) {
                 const cf_ms_batch_item &it = items[i];
                 if (it.layer != layer) continue;
-                io[i] = ItemIo{it.query, it.output, it.output_type, static_cast<uint32_t>(slots.size()),
+                io[i] = ItemIo{it.query, it.output, it.output_type, at,
                                it.output_token_stride_bytes, it.output_head_stride_bytes, it.output_element_stride_bytes};
+                if (!q_base) q_base = it.query.data, o_base = it.output;
+                const uint64_t head_bytes = 4ull * D, token_bytes = head_bytes * Hq;
+                const bool one = it.query.token_count == 1;
+                dense = dense && it.query.scalar_type == CF_DEVICE_F32 && it.output_type == CF_DEVICE_F32 &&
+                        it.query.element_stride_bytes == 4 && it.output_element_stride_bytes == 4 && it.query.head_stride_bytes == head_bytes &&
+                        it.output_head_stride_bytes == head_bytes && (one || (it.query.token_stride_bytes == token_bytes && it.output_token_stride_bytes == token_bytes)) &&
+                        static_cast<const char *>(it.query.data) == static_cast<const char *>(q_base) + at * token_bytes &&
+                        static_cast<const char *>(it.output) == static_cast<const char *>(o_base) + at * token_bytes;
                 const uint32_t slot = r->sequences.at(it.sequence_id).slot;
-                for (uint32_t t = 0; t < it.query.token_count; ++t) {
-                    slots.push_back(slot);
-                    positions.push_back(it.query_token_begin + t);
+                for (uint32_t t = 0; t < it.query.token_count; ++t, ++at) {
+                    rows[at] = slot;
+                    rows[total_rows + at] = it.query_token_begin + t;
                 }
                 if (it.query.token_count == 1) ++r->counters.decode_items; else ++r->counters.prefill_items;
             }
-            layer_rows[layer].second = static_cast<uint32_t>(slots.size()) - layer_rows[layer].first;
+            layer_rows[layer].second = at - layer_rows[layer].first;
         }
-        cuda_check(cudaMemcpyAsync(r->item_io.ptr, io.data(), io.size() * sizeof(ItemIo), cudaMemcpyHostToDevice, s), "upload batch items");
-        cuda_check(cudaMemcpyAsync(r->slot_list.ptr, slots.data(), slots.size() * 4, cudaMemcpyHostToDevice, s), "upload batch slots");
-        cuda_check(cudaMemcpyAsync(r->positions.ptr, positions.data(), positions.size() * 4, cudaMemcpyHostToDevice, s), "upload batch positions");
-        const uint32_t Hq = r->config.query_head_count, D = r->config.head_dim;
-        gather_queries_kernel<<<dim3(8, item_count), 256, 0, s>>>(r->item_io.ptr, r->q_dense.ptr, Hq, D);
-        cuda_check(cudaGetLastError(), "query gather launch");
+        dense = dense && ((reinterpret_cast<uintptr_t>(q_base) | reinterpret_cast<uintptr_t>(o_base)) & 15u) == 0;
+        if (!dense) {   // (taken when a batch first needs them)
+            r->item_io.ensure(1024, s);
+            r->q_dense.ensure(static_cast<size_t>(kMaxBatchTokens) * row_values, s);
+            r->o_dense.ensure(r->q_dense.count, s);
+        }
+        const float *q_rows = dense ? static_cast<const float *>(q_base) : r->q_dense.ptr;
+        float *o_rows = dense ? static_cast<float *>(const_cast<void *>(o_base)) : r->o_dense.ptr;
+        cuda_check(cudaMemcpyAsync(r->slot_list.ptr, rows.data(), rows.size() * 4, cudaMemcpyHostToDevice, s), "upload batch rows");
+        if (!dense) {
+            cuda_check(cudaMemcpyAsync(r->item_io.ptr, io.data(), io.size() * sizeof(ItemIo), cudaMemcpyHostToDevice, s), "upload batch items");
+            gather_queries_kernel<<<dim3(8, item_count), 256, 0, s>>>(r->item_io.ptr, r->q_dense.ptr, Hq, D);
+            cuda_check(cudaGetLastError(), "query gather launch");
+        }
         float softmax_scale = items[0].softmax_scale;
         uint32_t window = items[0].causal_window;
         for (uint32_t i = 1; i < item_count; ++i)
@@ -894,9 +1136,9 @@ extern "C" int cf_ms_cuda_execute_batch_async(cf_ms_cuda_resolver *r, const cf_m
             d.tail_tokens = r->tails.ptr + r->row(layer, 0);
             d.tail_type = CF_B200_F32;
             d.tail_capacity = r->config.page_size;
-            d.query_positions = r->positions.ptr + first;
-            d.queries = r->q_dense.ptr + static_cast<size_t>(first) * Hq * D;
-            d.output = r->o_dense.ptr + static_cast<size_t>(first) * Hq * D;
+            d.query_positions = r->slot_list.ptr + total_rows + first;
+            d.queries = q_rows + first * row_values;
+            d.output = o_rows + first * row_values;
             d.query_type = CF_B200_F32;
             d.output_type = CF_B200_F32;
             d.softmax_scale = softmax_scale;
@@ -912,14 +1154,22 @@ extern "C" int cf_ms_cuda_execute_batch_async(cf_ms_cuda_resolver *r, const cf_m
             if (cf_b200_sealed_attention_async(&d, s) != CF_OK) throw std::runtime_error("multi-sequence attention launch rejected");
             ++r->counters.sequence_attention_launches;
         }
-        scatter_outputs_kernel<<<dim3(8, item_count), 256, 0, s>>>(r->item_io.ptr, r->o_dense.ptr, Hq, D);
-        cuda_check(cudaGetLastError(), "output scatter launch");
+        if (!dense) {
+            scatter_outputs_kernel<<<dim3(8, item_count), 256, 0, s>>>(r->item_io.ptr, r->o_dense.ptr, Hq, D);
+            cuda_check(cudaGetLastError(), "output scatter launch");
+        }
         {   // one event for the batch: every snapshot of it is released when the batch's last kernel is done
+            if (r->pending.size() >= kPendingBatches) release_finished(r);
             Pending p;
-            cuda_check(cudaEventCreateWithFlags(&p.event, cudaEventDisableTiming), "create snapshot release event");
+            if (r->free_events.empty()) {
+                cuda_check(cudaEventCreateWithFlags(&p.event, cudaEventDisableTiming), "create snapshot release event");
+            } else {
+                p.event = r->free_events.back();
+                r->free_events.pop_back();
+            }
             const cudaError_t recorded = cudaEventRecord(p.event, s);
             if (recorded != cudaSuccess) {
-                cudaEventDestroy(p.event);
+                r->free_events.push_back(p.event);
                 cuda_check(recorded, "record snapshot release event");
             }
             r->counters.snapshot_release_events += snapshots.size();
@@ -971,32 +1221,8 @@ extern "C" int cf_ms_cuda_sequence_remove_async(cf_ms_cuda_resolver *r, int64_t 
 extern "C" int cf_ms_cuda_reclaim_async(cf_ms_cuda_resolver *r, void *stream) {
     if (!r) return -1;
     return locked(r, true, [&] {
-        for (auto it = r->pending.begin(); it != r->pending.end();) {
-            const cudaError_t status = cudaEventQuery(it->event);
-            if (status == cudaErrorNotReady) { ++it; continue; }
-            cuda_check(status, "query snapshot release event");
-            for (const Snapshot &snap : it->snapshots) r->release_snapshot(snap);
-            cudaEventDestroy(it->event);
-            it = r->pending.erase(it);
-        }
-        for (auto it = r->pages.begin(); it != r->pages.end();) {
-            SharedPage &page = it->second;
-            if (page.retired && page.logical_refs == 0 && page.in_flight_refs == 0) {
-                // the directory rows of its tiles go back to "not there"; its arena slot is handed to the next page sealed
-                for (uint32_t id : page.store_ids)
-                    if (r->ready)
-                        cuda_check(cudaMemsetAsync(r->page_dir.ptr + static_cast<size_t>(id) * r->config.kv_head_count, 0,
-                                                   r->config.kv_head_count * sizeof(uint64_t), static_cast<cudaStream_t>(stream)),
-                                   "clear directory rows");
-                if (!page.store_ids.empty()) r->free_page_slots.push_back((page.store_ids.front() - 1u) / r->tiles_per_page);
-                r->live_record_bytes -= std::min<uint64_t>(r->live_record_bytes, page.record_bytes);
-                r->counters.pending_reclamation_bytes -= page.resident_bytes;
-                ++r->counters.pages_reclaimed;
-                it = r->pages.erase(it);
-            } else {
-                ++it;
-            }
-        }
+        release_finished(r);
+        reclaim_pages(r, static_cast<cudaStream_t>(stream));
     });
 }
 
@@ -1032,23 +1258,30 @@ extern "C" int cf_ms_cuda_shift_sequence(cf_ms_cuda_resolver *r, int64_t id, uin
 extern "C" int cf_ms_cuda_audit(const cf_ms_cuda_resolver *r) {
     if (!r) return -1;
     std::lock_guard<std::mutex> guard(r->mutex);
-    std::unordered_map<uint64_t, uint64_t> observed;
-    std::unordered_map<uint32_t, int> slots;
+    for (const auto &entry : r->pages) entry.second.observed = 0;
+    std::vector<bool> slots;
     for (const auto &[id, q] : r->sequences) {
-        if (id != q.id || ++slots[q.slot] > 1) return -1;
+        if (q.slot >= slots.size()) slots.resize(q.slot + 1u);
+        if (id != q.id || slots[q.slot]) return -1;
+        slots[q.slot] = true;
         for (const auto &layer : q.layers) {
             uint32_t tokens = 0;
             for (const auto &ref : layer.pages) {
-                auto page = r->pages.find(ref.page_id);
-                if (page == r->pages.end() || page->second.retired) return -1;
-                ++observed[ref.page_id];
+                const SharedPage *page = ref.page;
+                if (!page) {
+                    auto found = r->pages.find(ref.page_id);
+                    if (found == r->pages.end()) return -1;
+                    page = &found->second;
+                }
+                if (page->retired) return -1;
+                ++page->observed;
                 tokens += ref.tokens;
             }
             if (tokens != layer.sealed_tokens) return -1;
         }
     }
     for (const auto &[id, page] : r->pages)
-        if (!page.retired && page.logical_refs != observed[id]) return -1;
+        if (!page.retired && page.logical_refs != page.observed) return -1;
     return r->counters.cross_sequence_contamination == 0 && r->counters.dense_fallback_launches == 0 ? 0 : -1;
 }
 

@@ -289,6 +289,8 @@ __global__ void __launch_bounds__(kThreads, 2) seal_blocks_kernel(const __grid_c
     for (uint32_t i = tid; i < 512u; i += kThreads) {
         s_enc[i] = coder_entry(i < 256u ? p.k_tables : p.v_tables, i & 255u, rans);
     }
+    if constexpr (kPlaced)
+        if (blockIdx.x == 0 && tid == 0) place.used[p.job_count * p.kv_head_count] = *p.status;
     __syncthreads();
     const uint32_t head_bytes = rans ? align_up_u32(6u * G::kBlocks, 4u) : align_up_u32(2u * G::kBlocks, 4u);
     const uint32_t before = head_bytes + (split ? G::kSyms / 2u : 0u);   // block table, then the raw low-nibble plane, then the payload
@@ -356,7 +358,7 @@ __global__ void __launch_bounds__(kThreads, 2) seal_blocks_kernel(const __grid_c
         }
         if (rows == 0 || k_mag >= 0x7f800000u || v_mag >= 0x7f800000u) {   // finite validation failed: nothing is published
             if (lane == 0) {
-                if (p.status) atomicOr(p.status, CF_B200_DEVSTAT_NONFINITE);
+                if (!kPlaced && p.status) atomicOr(p.status, CF_B200_DEVSTAT_NONFINITE);
                 if constexpr (kPlaced) place.used[job * heads + head_at] = kSealRefused;
             }
             continue;

@@ -34,7 +34,8 @@ constexpr uint32_t kBulkPages = 512;   // pages per launch: the list travels wit
 struct SealPlacement {
     uint32_t tiles_per_page, record_units;   // 16-byte units of the largest record
     uint32_t *table_row;                     // the sequence's page-table row at its first new tile
-    uint32_t *used;                          // host-mapped [tile][kv head]: record units, or kSealRefused for a non-finite tile
+    uint32_t *used;                          // [tile][kv head]: record units, or kSealRefused for a non-finite tile; behind
+                                             // them the status word as the launch found it
     uint32_t page_slot[kBulkPages];
 };
 constexpr uint32_t kSealRefused = 0xffffffffu;
