@@ -36,7 +36,9 @@ struct AttentionParams {
     // split-KV
     uint8_t *workspace;
     WorkspaceLayout layout;
-    uint32_t min_pages_per_unit;    // 0 = the plan kernel chooses (default_pages_per_unit)
+    uint32_t min_pages_per_unit;    // 0 = the line of pages is cut evenly over plan_warps (PageLine)
+    uint32_t plan_warps;            // warps (any-geometry kernel: CTAs) that are resident at once in the attention kernel
+    uint32_t unit_lanes;            // units that share a stretch: kv heads x passes over a kv head's query group
     uint32_t shared_prefix_pages;   // the caller's hint, already zeroed when the launch cannot use it
     uint32_t sm_count;
     uint32_t decode_probe;          // 1 = measurement: decode every page, fold the symbols into a checksum, no attention;
@@ -53,15 +55,15 @@ struct AttentionParams {
 __device__ __forceinline__ PlanHeader *plan_header(const AttentionParams &p) {
     return reinterpret_cast<PlanHeader *>(p.workspace);
 }
-__device__ __forceinline__ uint32_t *chunk_prefix(const AttentionParams &p) {
+__device__ __forceinline__ uint32_t *line_prefix(const AttentionParams &p) {
     return reinterpret_cast<uint32_t *>(p.workspace + p.layout.prefix_offset);
 }
-__device__ __forceinline__ ChunkInfo *chunk_info(const AttentionParams &p) {
-    return reinterpret_cast<ChunkInfo *>(p.workspace + p.layout.info_offset);
+__device__ __forceinline__ SeqInfo *seq_info(const AttentionParams &p) {
+    return reinterpret_cast<SeqInfo *>(p.workspace + p.layout.info_offset);
 }
-__device__ __forceinline__ float *partial_ptr(const AttentionParams &p, uint32_t chunk, uint32_t local_q_head) {
+__device__ __forceinline__ float *partial_ptr(const AttentionParams &p, uint32_t slot, uint32_t local_q_head) {
     return reinterpret_cast<float *>(p.workspace + p.layout.partials_offset) +
-           (static_cast<uint64_t>(chunk) * (p.kv_head_span * p.group) + local_q_head) * p.layout.partial_stride_floats;
+           (static_cast<uint64_t>(slot) * (p.kv_head_span * p.group) + local_q_head) * p.layout.partial_stride_floats;
 }
 // Shared-prefix partial of (cell, batch entry, local query head); cells as SharedSplit numbers them.
 __device__ __forceinline__ float *shared_partial_ptr(const AttentionParams &p, uint32_t chunk, uint32_t seq, uint32_t local_q_head) {
@@ -86,27 +88,61 @@ __device__ __forceinline__ float load_tail(const void *base, uint32_t type, uint
 __device__ __forceinline__ void raise_status(const AttentionParams &p, uint32_t bits) {
     if (p.status) atomicOr(p.status, bits);
 }
-// Sequence that owns chunk `c`: the last s with chunk_prefix[s] <= c.
-__device__ __forceinline__ uint32_t sequence_of_chunk(const uint32_t *prefix, uint32_t seq_count, uint32_t c) {
+// The sequence that holds line position x: the last s with line_prefix[s] <= x. Whole warps, 32 probes at a time.
+__device__ __forceinline__ uint32_t sequence_at(const uint32_t *prefix, uint32_t seq_count, uint32_t x, uint32_t lane) {
     uint32_t lo = 0, hi = seq_count;
-    while (hi - lo > 1) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (prefix[mid] <= c) lo = mid; else hi = mid;
+    while (hi - lo > 1u) {
+        const uint32_t step = (hi - lo + 31u) / 32u, at = lo + (lane + 1u) * step;
+        const uint32_t below = __popc(__ballot_sync(0xffffffffu, at < hi && __ldcg(prefix + at) <= x));
+        lo += below * step;
+        hi = min(lo + step, hi);
     }
     return lo;
+}
+// The part of a stretch inside one sequence: positions [x, x_end) of the line, pages [page, page_end) of the entry.
+struct LineRun {
+    uint32_t x, x_end, seq, page, page_end;
+    SeqInfo info;
+};
+// The run that starts at position x and ends at x_stop (the stretch's end) at the latest. Whole warps.
+__device__ __forceinline__ LineRun run_at(const AttentionParams &p, uint32_t x, uint32_t x_stop, uint32_t grain, uint32_t lane) {
+    LineRun run;
+    run.x = x;
+    run.seq = sequence_at(line_prefix(p), p.seq_count, x, lane);
+    const uint4 *src = reinterpret_cast<const uint4 *>(seq_info(p) + run.seq);
+    const uint4 a = __ldcg(src), b = __ldcg(src + 1);
+    run.info.slot = a.x, run.info.sealed = a.y, run.info.qpos = a.z, run.info.tail = a.w;
+    run.info.first_page = b.x, run.info.page_end = b.y, run.info.row = b.z, run.info.line_begin = b.w;
+    const uint32_t length = b.y - b.x, positions = grain == 1u ? length : (length + grain - 1u) / grain;
+    run.x_end = min(x_stop, b.w + positions);
+    run.page = b.x + (x - b.w) * grain;
+    run.page_end = min(b.x + (run.x_end - b.w) * grain, b.y);
+    return run;
+}
+// The plan's line, past every level-1 cache: the kernels that read it may have started before the plan kernel ended.
+__device__ __forceinline__ PageLine plan_line(const AttentionParams &p) {
+    const uint4 *src = reinterpret_cast<const uint4 *>(p.workspace);
+    const uint4 a = __ldcg(src), b = __ldcg(src + 1);
+    PageLine line;
+    line.positions = a.x, line.grain = a.y, line.stretches = a.z, line.base = a.w;
+    line.longer = b.x, line.pieces = b.y, line.by_position = b.z;
+    return line;
 }
 #endif
 
 // Implemented in sealed_attention.cu
 cf_status sealed_attention_stages(const cf_b200_sealed_attention_desc *d, uint32_t stages, void *stream, bool output_on_peer);
+// dependent: the kernel before it on the stream belongs to the same call and lets this one start early.
 cudaError_t launch_plan(const AttentionParams &p, cudaStream_t stream);
-cudaError_t launch_combine(const AttentionParams &p, cudaStream_t stream);
+cudaError_t launch_combine(const AttentionParams &p, cudaStream_t stream, bool dependent);
 cudaError_t launch_generic_attention(const AttentionParams &p, cudaStream_t stream);
+constexpr uint32_t kGenericCtasPerSm = 4;
 // Implemented in sealed_attention_lanes.cu
 bool lanes_kernel_supports(const AttentionParams &p);
-cudaError_t launch_lanes_attention(const AttentionParams &p, cudaStream_t stream);
+void lanes_plan_shape(const AttentionParams &p, uint32_t sm_count, uint32_t *warps, uint32_t *unit_lanes);
+cudaError_t launch_lanes_attention(const AttentionParams &p, cudaStream_t stream, bool dependent, bool after_prefix);
 // Implemented in sealed_attention_prefix.cu
-cudaError_t launch_prefix_attention(const AttentionParams &p, cudaStream_t stream);
+cudaError_t launch_prefix_attention(const AttentionParams &p, cudaStream_t stream, bool dependent);
 // Implemented in dense_attention.cu
 cudaError_t launch_dense_attention(const AttentionParams &p, cudaStream_t stream);
 

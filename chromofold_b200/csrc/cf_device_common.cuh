@@ -15,23 +15,55 @@ constexpr int kZero = CF_B200_ZERO_POINT;
 
 __host__ __device__ inline uint32_t align_up_u32(uint32_t v, uint32_t a) { return (v + a - 1) / a * a; }
 
-// Split-KV workspace. One chunk = `pages_per_unit` consecutive pages of one sequence; one unit = (chunk, kv head).
+// Split-KV workspace.
 //   [0, 64)                       PlanHeader
-//   [64, 64 + 4*(seq_count+1))    chunk_prefix: number of chunks before each sequence
+//   [64, 64 + 4*(seq_count+1))    line_prefix: line positions before each sequence (see PageLine)
+//   [info_offset, ...)            SeqInfo[seq_count]
 //   [shared_offset, ...)          shared-prefix partials, per (cell, sequence, local query head), when asked for (SharedSplit)
-//   [partials_offset, ...)        per chunk and local query head: float m, float l, float acc[head_dim]
+//   [partials_offset, ...)        per partial slot and local query head: float m, float l, float acc[head_dim]
+//
+// The pages a launch reads (per kv head) form one line: the visible pages of sequence 0, then those of sequence 1, ... The line is
+// cut into `stretches` of equal length, to within one page, one for every warp that can be resident: each warp then reads the
+// same number of pages whatever the sequences' lengths. (Units of one size handed out in rounds left the last round partly empty.)
+// A stretch inside one sequence leaves one partial per piece, a piece being at most kPiecePages, which bounds how far the tensor
+// cores' fp32 sums can drift. A caller who fixes the pages per unit gets that many pages per position, one position per stretch
+// and no position shared by two sequences, so that the cut depends on nothing but the sequence itself.
+struct PageLine {
+    uint32_t positions;              // of the whole line
+    uint32_t grain;                  // pages per position
+    uint32_t stretches, base, longer;   // stretch length; the first `longer` stretches have one position more
+    uint32_t pieces;                 // per stretch, at most `base`
+    uint32_t by_position;            // 1: partial slots are numbered by position (the caller's pages per unit)
+    __host__ __device__ uint32_t begin(uint32_t j) const { return j * base + (j < longer ? j : longer); }
+    __host__ __device__ uint32_t length(uint32_t j) const { return base + (j < longer ? 1u : 0u); }
+    __host__ __device__ uint32_t stretch_of(uint32_t x) const {
+        const uint32_t split = longer * (base + 1u);
+        return x < split ? x / (base + 1u) : longer + (x - split) / base;
+    }
+    // piece of stretch j that holds position x, and where the piece ends
+    __host__ __device__ uint32_t piece_of(uint32_t j, uint32_t x) const {
+        return pieces == 1u ? 0u : static_cast<uint32_t>((static_cast<uint64_t>(x - begin(j) + 1u) * pieces - 1ull) / length(j));
+    }
+    __host__ __device__ uint32_t piece_end(uint32_t j, uint32_t piece) const {
+        return begin(j) + static_cast<uint32_t>(static_cast<uint64_t>(length(j)) * (piece + 1u) / pieces);
+    }
+    // The slot of the partial over the positions of sequence s around x. Along the line the numbers rise by one with every piece
+    // inside a sequence, and by one or two where a sequence starts.
+    __host__ __device__ uint32_t slot(uint32_t j, uint32_t piece, uint32_t x, uint32_t s) const {
+        return by_position ? x : j * pieces + piece + s;
+    }
+};
+constexpr uint32_t kPiecePages = 32;
+
 struct PlanHeader {
-    uint32_t chunk_count;
-    uint32_t pages_per_unit;
-    uint32_t next_unit;      // work counter for the attention kernel; the plan kernel clears it
-    uint32_t chunk_capacity;
-    uint32_t overflow;
+    PageLine line;
+    uint32_t next_unit;               // work counter of the attention kernel; the plan kernel clears it
     uint32_t shared_pages;            // pages at the head of every sequence that the shared-prefix kernel handles (0 = none)
     uint32_t shared_ctas;             // CTAs of the shared-prefix kernel that take a share of it (0 = none), and
     uint32_t shared_rounds;           // rounds of eight pages that the shared pages make for one (kv head, row tile)
-    uint32_t reserved_shared;         // unused
-    uint32_t pad[7];
+    uint32_t pad[5];
 };
+static_assert(sizeof(PlanHeader) == 64, "the header has 64 bytes of the workspace");
 
 // How the shared-prefix kernel's work is cut. The rounds of all (kv head, row tile) pairs form one line, head-tile major:
 // round x belongs to head-tile x / rounds. CTA b of `ctas` takes the rounds [first_round(b), first_round(b + 1)): every CTA
@@ -58,21 +90,22 @@ __host__ __device__ inline uint32_t shared_split_ctas(uint32_t rounds, uint32_t 
     return head_tiles * (cells - 1u);
 }
 
-// What a (chunk, kv head) unit needs to start, written per chunk by the plan kernel so that the attention kernel's
-// warps read one 32-byte record instead of searching the chunk prefix and chasing four dependent loads.
-struct ChunkInfo {
-    uint32_t seq, slot, sealed, qpos;      // batch entry, its sequence slot, its sealed tokens, its query position
-    uint32_t page_begin, reserved[3];      // first page (index into the slot's page-table row) of the chunk
+// What is known of a batch entry, written by the plan kernel so that later kernels read two 16-byte words instead of chasing
+// slot -> counts -> position.
+struct SeqInfo {
+    uint32_t slot, sealed, qpos, tail;          // sequence slot, sealed tokens, query position, unsealed tokens
+    uint32_t first_page, page_end, row, line_begin;   // visible pages [first_page, page_end) outside the shared prefix; query /
+                                                      // output row; first position on the line
 };
-static_assert(sizeof(ChunkInfo) == 32, "one chunk record is two 16-byte loads");
+static_assert(sizeof(SeqInfo) == 32, "an entry's record is two 16-byte loads");
 
 struct WorkspaceLayout {
     uint64_t prefix_offset;
+    uint64_t info_offset;            // SeqInfo[seq_count]
     uint64_t shared_offset;          // 0 = no room was set aside for shared-prefix partials
     uint64_t partials_offset;
-    uint64_t partial_stride_floats;  // per (chunk, local query head)
-    uint64_t chunk_capacity;
-    uint64_t info_offset;            // ChunkInfo[chunk_capacity], behind the partials
+    uint64_t partial_stride_floats;  // per (partial slot, local query head)
+    uint64_t chunk_capacity;         // partial slots
 };
 
 __host__ __device__ inline WorkspaceLayout workspace_layout(uint32_t seq_count, uint32_t local_q_heads,
@@ -80,7 +113,8 @@ __host__ __device__ inline WorkspaceLayout workspace_layout(uint32_t seq_count, 
                                                             bool shared_prefix = false) {
     WorkspaceLayout w;
     w.prefix_offset = sizeof(PlanHeader);
-    w.partials_offset = (w.prefix_offset + 4ull * (seq_count + 1) + 255ull) / 256ull * 256ull;
+    w.info_offset = (w.prefix_offset + 4ull * (seq_count + 1) + 31ull) / 32ull * 32ull;
+    w.partials_offset = (w.info_offset + sizeof(SeqInfo) * seq_count + 255ull) / 256ull * 256ull;
     w.partial_stride_floats = head_dim + 2ull;
     w.shared_offset = 0;
     if (shared_prefix) {
@@ -88,10 +122,8 @@ __host__ __device__ inline WorkspaceLayout workspace_layout(uint32_t seq_count, 
         w.partials_offset += (static_cast<uint64_t>(CF_B200_SHARED_CHUNKS_MAX) * seq_count * local_q_heads *
                               w.partial_stride_floats * 4ull + 255ull) / 256ull * 256ull;
     }
-    const uint64_t per_chunk = w.partial_stride_floats * 4ull * local_q_heads;
-    w.chunk_capacity = workspace_bytes > w.partials_offset + 32ull
-                           ? (workspace_bytes - w.partials_offset - 32ull) / (per_chunk + sizeof(ChunkInfo)) : 0;
-    w.info_offset = (w.partials_offset + w.chunk_capacity * per_chunk + 31ull) / 32ull * 32ull;
+    const uint64_t per_slot = w.partial_stride_floats * 4ull * local_q_heads;
+    w.chunk_capacity = workspace_bytes > w.partials_offset ? (workspace_bytes - w.partials_offset) / per_slot : 0;
     return w;
 }
 
@@ -118,13 +150,13 @@ inline LauncherState *launcher_state(LauncherState (&table)[64], cudaError_t *er
     return state;
 }
 
-// The unit size the WORKSPACE is sized for when the caller leaves the choice to the library: 16 pages, or fewer (down
-// to 4) when the batch is so small that units of 16 pages would not give every resident warp of the attention kernel
-// (148 SMs x 16 warps) about four units. (The plan kernel makes the actual choice, among the sizes that fit.)
-__host__ __device__ inline uint32_t default_pages_per_unit(uint64_t total_pages, uint32_t kv_head_span) {
-    const uint64_t slots = 4ull * 148ull * 16ull;
-    const uint64_t wanted = (total_pages * kv_head_span + slots - 1ull) / slots;
-    return static_cast<uint32_t>(wanted < 4ull ? 4ull : wanted > 16ull ? 16ull : wanted);
+// Partial slots a launch over at most total_pages pages can need: with the library's own cut one per stretch (a warp of the 148 x
+// 16 resident ones, for one kv head of the span), per kPiecePages pages and per sequence; with the caller's one per unit.
+__host__ __device__ inline uint64_t partial_slots_for(uint64_t total_pages, uint32_t seq_count, uint32_t kv_head_span, uint32_t min_pages_per_unit) {
+    if (min_pages_per_unit) return total_pages / min_pages_per_unit + seq_count + 1ull;   // each sequence may round up once
+    const uint64_t warps = 148ull * 16ull / (kv_head_span ? kv_head_span : 1u) + 1ull;
+    const uint64_t stretches = total_pages < warps ? total_pages : warps;
+    return stretches + (total_pages + stretches) / kPiecePages + seq_count + 1ull;
 }
 
 // A device pointer against the current device: false when it is memory of ANOTHER GPU. Kernels are launched on the
@@ -147,6 +179,28 @@ __host__ __device__ inline uint32_t window_begin(uint32_t query_token, uint32_t 
 }
 
 #ifdef __CUDACC__
+
+// Kernels of one call that follow each other on a stream are launched so that the later one may start before the earlier one has
+// ended (programmatic dependent launch): it sets itself up, reads what the call's caller provided, and waits with
+// wait_for_previous_kernel() before it touches anything the earlier kernel writes. The earlier kernel says with
+// allow_dependent_launch() that its own blocks are placed. Both are no-ops in a kernel launched the ordinary way.
+__device__ __forceinline__ void wait_for_previous_kernel() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void allow_dependent_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <class... KernelArgs, class... Args>
+inline cudaError_t launch_kernel(void (*kernel)(KernelArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, bool dependent, Args... args) {
+    cudaLaunchConfig_t config = {};
+    config.gridDim = grid;
+    config.blockDim = block;
+    config.dynamicSmemBytes = smem;
+    config.stream = stream;
+    cudaLaunchAttribute attribute;
+    attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attribute.val.programmaticStreamSerializationAllowed = 1;
+    config.attrs = &attribute;
+    config.numAttrs = dependent ? 1 : 0;
+    return cudaLaunchKernelEx(&config, kernel, static_cast<KernelArgs>(args)...);
+}
 
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll

@@ -80,9 +80,8 @@ __global__ void __launch_bounds__(kThreads, 1) dense_attention_kernel(AttentionP
     __syncthreads();
 
     PlanHeader *hdr = plan_header(p);
-    const uint32_t *prefix = chunk_prefix(p);
-    const uint32_t unit_count = hdr->chunk_count * p.kv_head_span;
-    const uint32_t pages_per_unit = hdr->pages_per_unit;
+    const PageLine line = plan_line(p);
+    const uint32_t unit_count = line.stretches * p.kv_head_span;
     const uint32_t G = p.group, g = lane >> 2, t = lane & 3u;
     const float scale = p.softmax_scale * kLog2e;
     uint32_t phase_bits = 0u;
@@ -92,19 +91,14 @@ __global__ void __launch_bounds__(kThreads, 1) dense_attention_kernel(AttentionP
         if (lane == 0) unit = atomicAdd(&hdr->next_unit, 1u);
         unit = __shfl_sync(0xffffffffu, unit, 0);
         if (unit >= unit_count) break;
-        const uint32_t chunk = unit / p.kv_head_span;
+        const uint32_t stretch = unit / p.kv_head_span;
         const uint32_t head_local = unit % p.kv_head_span;
         const uint32_t kv_head = p.kv_head_begin + head_local;
-        const uint32_t seq = sequence_of_chunk(prefix, p.seq_count, chunk);
-        const uint32_t slot = slot_of(p, seq);
-        const uint32_t sealed = p.seq_sealed_tokens[slot];
-        const uint32_t qpos = query_position(p, seq, sealed, 0u);
+        // the caller's (or the default) pages per unit: a stretch is one position, inside one sequence
+        const LineRun run = run_at(p, line.begin(stretch), line.begin(stretch + 1u), line.grain, lane);
+        const uint32_t seq = run.seq, slot = run.info.slot, sealed = run.info.sealed, qpos = run.info.qpos;
         const uint32_t first_token = window_begin(qpos, p.causal_window);
-        const uint32_t pages = min((sealed + 15u) / 16u, qpos / 16u + 1u);
-        const uint32_t first_page = min(first_token / 16u, pages);
-        const uint32_t page_begin = first_page + (chunk - prefix[seq]) * pages_per_unit;
-        const uint32_t page_end = min(page_begin + pages_per_unit, pages);
-        const uint32_t n_pages = page_end > page_begin ? page_end - page_begin : 0u;
+        const uint32_t page_begin = run.page, n_pages = run.page_end - run.page;
         const uint32_t *table_row = p.page_table + static_cast<uint64_t>(slot) * p.page_table_stride;
 
         // Q fragments: row g = query head g of the group; this lane's channels are chunks t, t+4, t+8, t+12
@@ -219,7 +213,7 @@ __global__ void __launch_bounds__(kThreads, 1) dense_attention_kernel(AttentionP
         l += __shfl_xor_sync(0xffffffffu, l, 1);
         l += __shfl_xor_sync(0xffffffffu, l, 2);
         if (g < G) {
-            float *dst = partial_ptr(p, chunk, head_local * G + g);
+            float *dst = partial_ptr(p, line.slot(stretch, 0u, run.x, seq), head_local * G + g);
             if (t == 0) {
                 dst[0] = m_run;
                 dst[1] = l;
@@ -293,6 +287,6 @@ extern "C" cf_status cf_b200_dense_attention_async(const cf_b200_dense_attention
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (cfb::launch_plan(p, s) != cudaSuccess) return CF_ERR_CUDA;
     if (cfb::launch_dense_attention(p, s) != cudaSuccess) return CF_ERR_CUDA;
-    if (cfb::launch_combine(p, s) != cudaSuccess) return CF_ERR_CUDA;
+    if (cfb::launch_combine(p, s, false) != cudaSuccess) return CF_ERR_CUDA;
     return CF_OK;
 }

@@ -8,6 +8,7 @@
 // (max, sum, weighted) triples are merged with the rule of cf_online_softmax_merge (src/runtime/kv_runtime.cpp:219-243).
 
 #include <atomic>
+#include <cstddef>
 #include <math_constants.h>
 
 #include "attention_params.cuh"
@@ -20,61 +21,76 @@ namespace {
 
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr int kPlanThreads = 1024;
-constexpr uint32_t kPlanCache = 2048;   // batch entries whose page ranges the plan kernel keeps in shared memory
 constexpr int kGenericThreads = 128;
 constexpr uint32_t kGenericMaxGroup = 16;
 
 // ---------------------------------------------------------------------------------------------------------------
-// Plan: how many chunks each sequence gets. One block.
+// Plan: every entry's record, the line of pages and its cut (PageLine). One block.
+//
+// Bound by the chain of dependent loads slot -> counts -> record, once per entry, and a block scan; the kernels behind it set
+// themselves up meanwhile (see launch_kernel). It used to write a record per unit of pages as well and to try 32 unit sizes:
+// 5.2 us for one sequence and 9.4 us for 64, against 3.5 and 4.3 us now.
 // ---------------------------------------------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t visible_pages(const AttentionParams &p, uint32_t seq, uint32_t *first_page,
-                                                  uint32_t shared_pages = 0) {
-    const uint32_t slot = slot_of(p, seq);
-    const uint32_t sealed = p.seq_sealed_tokens[slot];
-    const uint32_t tail = p.tail_tokens ? p.tail_tokens[slot] : 0u;
-    const uint32_t qpos = query_position(p, seq, sealed, tail);
-    const uint32_t pages = min((sealed + p.page_tokens - 1u) / p.page_tokens, qpos / p.page_tokens + 1u);
-    const uint32_t first = min(max(window_begin(qpos, p.causal_window) / p.page_tokens, shared_pages), pages);
-    if (first_page) *first_page = first;
-    return pages - first;
-}
 
 // Shared-prefix hint, part one: block s compares the first `shared_prefix_pages` ids of entry s's page-table row with the
-// first entry's and leaves the result (1 = differs) in the entry's cell of the chunk-prefix array, which the plan kernel
+// first entry's and leaves the result (1 = differs) in the entry's cell of the line-prefix array, which the plan kernel
 // reads before it overwrites the array with the real prefix sums.
 __global__ void __launch_bounds__(256) verify_prefix_kernel(AttentionParams p) {
+    allow_dependent_launch();
     const uint32_t s = blockIdx.x;
     const uint32_t *row0 = p.page_table + static_cast<uint64_t>(slot_of(p, 0)) * p.page_table_stride;
     const uint32_t *row = p.page_table + static_cast<uint64_t>(slot_of(p, s)) * p.page_table_stride;
     int bad = 0;
     for (uint32_t pg = threadIdx.x; pg < p.shared_prefix_pages; pg += blockDim.x) bad |= row[pg] != row0[pg];
     bad = __syncthreads_or(bad);
-    if (threadIdx.x == 0) chunk_prefix(p)[s] = bad ? 1u : 0u;
+    if (threadIdx.x == 0) line_prefix(p)[s] = bad ? 1u : 0u;
+}
+
+// Inclusive sum over the block (whole warps, at most 32 of them); *total gets the block's sum.
+__device__ __forceinline__ uint32_t block_scan(uint32_t value, uint32_t *warp_totals, uint32_t *total) {
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, warps = blockDim.x >> 5;
+    uint32_t incl = value;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t up = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= static_cast<uint32_t>(o)) incl += up;
+    }
+    __syncthreads();   // the previous use of warp_totals is over
+    if (lane == 31u) warp_totals[warp] = incl;
+    __syncthreads();
+    uint32_t v = lane < warps ? warp_totals[lane] : 0u;   // every warp sums the totals for itself
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t up = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= static_cast<uint32_t>(o)) v += up;
+    }
+    *total = __shfl_sync(0xffffffffu, v, 31);
+    const uint32_t before = __shfl_sync(0xffffffffu, v, warp ? warp - 1u : 0u);
+    return incl + (warp ? before : 0u);
 }
 
 __global__ void __launch_bounds__(kPlanThreads) plan_kernel(AttentionParams p) {
-    __shared__ uint32_t scan[kPlanThreads];
     __shared__ uint32_t warp_totals[kPlanThreads / 32];
-    __shared__ uint32_t s_visible[kPlanCache], s_first[kPlanCache];
-    __shared__ uint32_t s_total;
-    static_assert(kPlanThreads == 1024, "the block scan below is 32 warps of 32 lanes");
+    allow_dependent_launch();
     const uint32_t tid = threadIdx.x;
-    const uint32_t per_thread = (p.seq_count + kPlanThreads - 1) / kPlanThreads;
+    const uint32_t per_thread = (p.seq_count + blockDim.x - 1) / blockDim.x;
     const uint32_t begin = min(tid * per_thread, p.seq_count);
     const uint32_t end = min(begin + per_thread, p.seq_count);
     PlanHeader *hdr = plan_header(p);
-    uint32_t *prefix = chunk_prefix(p);
+    uint32_t *prefix = line_prefix(p);
+    SeqInfo *info = seq_info(p);
 
     // Shared prefix: taken only if every listed sequence has the pages sealed and its page-table row starts with the
     // same ids as the first sequence's (compared by verify_prefix_kernel, result per entry in prefix[]). The pages are
-    // then cut into chunks for the shared-prefix kernel and left out of the per-sequence chunks below.
+    // then left to the shared-prefix kernel and taken off the line.
     uint32_t shared = p.shared_prefix_pages;
     if (shared) {
         int bad = 0;
+        wait_for_previous_kernel();
         for (uint32_t s = begin; s < end; ++s) {   // the pages must be sealed and wholly visible to the entry's query token
             const uint32_t slot = slot_of(p, s), sealed = p.seq_sealed_tokens[slot];
             const uint32_t qpos = query_position(p, s, sealed, p.tail_tokens ? p.tail_tokens[slot] : 0u);
-            if (sealed / p.page_tokens < shared || qpos + 1u < shared * p.page_tokens || prefix[s] != 0u) bad = 1;
+            if (sealed / p.page_tokens < shared || qpos + 1u < shared * p.page_tokens || __ldcg(prefix + s) != 0u) bad = 1;
         }
         if (__syncthreads_or(bad)) {
             shared = 0;
@@ -86,141 +102,67 @@ __global__ void __launch_bounds__(kPlanThreads) plan_kernel(AttentionParams p) {
         const uint32_t row_tiles = (p.seq_count * p.group + 127u) / 128u;
         shared_rounds = (shared + 7u) / 8u;
         shared_ctas = shared_split_ctas(shared_rounds, p.kv_head_span * row_tiles, p.sm_count, CF_B200_SHARED_CHUNKS_MAX);
-        if (shared_ctas == 0u) shared = 0;   // no CTA to take it: the pages stay with the per-sequence chunks
+        if (shared_ctas == 0u) shared = 0;   // no CTA to take it: the pages stay on the line
     }
 
-    // The visible page range of every batch entry is needed by each pass below; it costs a chain of dependent loads
-    // (slot, sealed tokens, tail tokens, query position), so batches of up to kPlanCache entries keep it in shared memory.
-    const bool cached = p.seq_count <= kPlanCache;
-    if (cached) {
-        for (uint32_t s = tid; s < p.seq_count; s += kPlanThreads) {
-            uint32_t first_page;
-            s_visible[s] = visible_pages(p, s, &first_page, shared);
-            s_first[s] = first_page;
-        }
-        __syncthreads();
-    }
-    auto visible_of = [&](uint32_t s, uint32_t *first_page) {
-        if (!cached) return visible_pages(p, s, first_page, shared);
-        if (first_page) *first_page = s_first[s];
-        return s_visible[s];
-    };
-
-    uint32_t pages_per_unit = p.min_pages_per_unit;
-    uint32_t overflow = 0;
-    uint32_t local = 0;  // chunks of this thread's sequences at the current pages_per_unit
-    if (pages_per_unit == 0u) {
-        // The library's choice. Units are equal-sized and handed out dynamically to W resident warps, so a launch lasts
-        // about ceil(units / W) rounds of one unit each; a unit costs its pages plus a start-up worth about three
-        // quarters of a page. Warp w scores the candidate 4 + w pages per unit over all sequences; the cheapest that
-        // fits the workspace wins (ties: the larger unit, fewer partials to merge). A launch too small to give every
-        // warp a unit comes out at 4.
-        const uint32_t warp = tid >> 5, lane = tid & 31u, candidate = 4u + warp;
-        uint64_t units = 0;
-        for (uint32_t s = lane; s < p.seq_count; s += 32u) units += (visible_of(s, nullptr) + candidate - 1u) / candidate;
-        for (int o = 16; o > 0; o >>= 1) units += __shfl_xor_sync(0xffffffffu, units, o);
-        const uint32_t pass_heads = p.group <= 4u ? 4u : p.query_type == CF_B200_F32 ? 4u : 8u;
-        const uint64_t warps = 16ull * (p.sm_count ? p.sm_count : 148u);
-        const uint64_t rounds = (units * p.kv_head_span * ((p.group + pass_heads - 1u) / pass_heads) + warps - 1ull) / warps;
-        uint64_t cost = rounds * (4ull * candidate + 3ull);
-        if (units > p.layout.chunk_capacity || units == 0) cost = ~0ull;
-        if (lane == 0) reinterpret_cast<unsigned long long *>(scan)[warp] = cost;   // 32 x 8 bytes of the scan array
-        __syncthreads();
-        if (tid == 0) {
-            uint32_t best = 16u;
-            unsigned long long best_cost = ~0ull;
-            for (uint32_t w = 0; w < kPlanThreads / 32; ++w) {
-                const unsigned long long c = reinterpret_cast<unsigned long long *>(scan)[w];
-                if (c <= best_cost && c != ~0ull) {
-                    best_cost = c;
-                    best = 4u + w;
-                }
-            }
-            s_total = best;
-        }
-        __syncthreads();
-        pages_per_unit = s_total;
-        __syncthreads();
-    }
-    for (int attempt = 0; attempt < 32; ++attempt) {
-        local = 0;
-        for (uint32_t s = begin; s < end; ++s) local += (visible_of(s, nullptr) + pages_per_unit - 1u) / pages_per_unit;
-        // inclusive scan over the block: inside each warp with shuffles, then over the 32 warp totals
-        uint32_t incl = local;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t up = __shfl_up_sync(0xffffffffu, incl, o);
-            if ((tid & 31u) >= static_cast<uint32_t>(o)) incl += up;
-        }
-        __syncthreads();                          // the previous use of warp_totals is over
-        if ((tid & 31u) == 31u) warp_totals[tid >> 5] = incl;
-        __syncthreads();
-        if (tid < 32u) {
-            uint32_t v = warp_totals[tid];
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t up = __shfl_up_sync(0xffffffffu, v, o);
-                if (tid >= static_cast<uint32_t>(o)) v += up;
-            }
-            warp_totals[tid] = v;
-            if (tid == 31u) s_total = v;
-        }
-        __syncthreads();
-        scan[tid] = incl + ((tid >> 5) ? warp_totals[(tid >> 5) - 1u] : 0u);
-        __syncthreads();
-        if (s_total <= p.layout.chunk_capacity) break;
-        if (attempt == 31 || pages_per_unit >= (1u << 30)) { overflow = 1; break; }
-        pages_per_unit <<= 1;
-    }
-    // Chunk prefix per sequence, and every chunk's start-up record (the attention kernel's warps read that record, not
-    // the prefix). Few sequences with many chunks each: a warp per sequence writes the records side by side; many
-    // sequences with few chunks: every thread writes those of its own sequences.
-    uint32_t running = scan[tid] - local;
-    ChunkInfo *info = chunk_info(p);
-    const bool by_warp = !overflow && s_total >= 8ull * p.seq_count;
+    uint32_t local = 0;   // pages of this thread's sequences
     for (uint32_t s = begin; s < end; ++s) {
-        prefix[s] = overflow ? 0u : running;
-        uint32_t first_page;
-        const uint32_t chunks = (visible_of(s, &first_page) + pages_per_unit - 1u) / pages_per_unit;
-        if (!overflow && !by_warp && chunks) {
-            const uint32_t slot = slot_of(p, s), sealed = p.seq_sealed_tokens[slot];
-            const uint32_t qpos = query_position(p, s, sealed, p.tail_tokens ? p.tail_tokens[slot] : 0u);
-            for (uint32_t k = 0; k < chunks; ++k) {
-                uint4 *dst = reinterpret_cast<uint4 *>(info + running + k);
-                dst[0] = make_uint4(s, slot, sealed, qpos);
-                dst[1] = make_uint4(first_page + k * pages_per_unit, row_of(p, s), 0u, 0u);
-            }
-        }
-        running += chunks;
+        const uint32_t slot = slot_of(p, s), row = row_of(p, s);
+        const uint32_t sealed = p.seq_sealed_tokens[slot], tail = p.tail_tokens ? p.tail_tokens[slot] : 0u;
+        const uint32_t qpos = query_position(p, s, sealed, tail);
+        const uint32_t pages = min((sealed + p.page_tokens - 1u) / p.page_tokens, qpos / p.page_tokens + 1u);
+        const uint32_t first = min(max(window_begin(qpos, p.causal_window) / p.page_tokens, shared), pages);
+        reinterpret_cast<uint4 *>(info + s)[0] = make_uint4(slot, sealed, qpos, tail);
+        reinterpret_cast<uint4 *>(info + s)[1] = make_uint4(first, pages, row, 0u);
+        local += pages - first;
     }
-    if (by_warp) {
-        __syncthreads();   // prefix[] is complete
-        for (uint32_t s = tid >> 5; s < p.seq_count; s += kPlanThreads / 32) {
-            const uint32_t c0 = prefix[s], c1 = s + 1u < p.seq_count ? prefix[s + 1u] : s_total;
-            if (c1 == c0) continue;
-            uint32_t first_page;
-            visible_of(s, &first_page);
-            const uint32_t slot = slot_of(p, s), sealed = p.seq_sealed_tokens[slot];
-            const uint32_t qpos = query_position(p, s, sealed, p.tail_tokens ? p.tail_tokens[slot] : 0u);
-            const uint32_t row = row_of(p, s);
-            for (uint32_t c = c0 + (tid & 31u); c < c1; c += 32u) {
-                uint4 *dst = reinterpret_cast<uint4 *>(info + c);
-                dst[0] = make_uint4(s, slot, sealed, qpos);
-                dst[1] = make_uint4(first_page + (c - c0) * pages_per_unit, row, 0u, 0u);
-            }
+    PageLine line = {};
+    line.grain = 1;
+    line.by_position = p.min_pages_per_unit != 0u;
+    uint32_t incl, total;
+    const uint32_t capacity = static_cast<uint32_t>(min(p.layout.chunk_capacity, static_cast<uint64_t>(0x7fffffffu)));
+    if (!line.by_position) {
+        // One stretch per resident warp for the units of a stretch (kv heads x passes), where there is a page for each and a
+        // partial slot: the last slot is stretches * pieces + seq_count - 2. The capacity is at least seq_count.
+        incl = block_scan(local, warp_totals, &total);
+        const uint32_t room = capacity - (p.seq_count - 1u);
+        line.stretches = min(min(max(p.plan_warps / p.unit_lanes, 1u), total), room);
+        if (line.stretches) {
+            line.base = total / line.stretches;
+            line.longer = total % line.stretches;
+            const uint32_t longest = line.base + (line.longer ? 1u : 0u);
+            line.pieces = min(max(min((longest + kPiecePages - 1u) / kPiecePages, room / line.stretches), 1u), line.base);
         }
+    } else {
+        line.grain = p.min_pages_per_unit;
+        for (;;) {   // units grow until every one has a slot; from one unit per sequence on they do
+            local = 0;
+            for (uint32_t s = begin; s < end; ++s) {
+                const uint4 pages = reinterpret_cast<const uint4 *>(info + s)[1];   // this thread's own record
+                local += (pages.y - pages.x + line.grain - 1u) / line.grain;
+            }
+            incl = block_scan(local, warp_totals, &total);
+            if (total <= capacity || line.grain >= (1u << 30)) break;
+            line.grain <<= 1;
+        }
+        line.stretches = total;
+        line.base = line.pieces = 1;
+    }
+    line.positions = total;
+    uint32_t running = incl - local;
+    for (uint32_t s = begin; s < end; ++s) {
+        const uint4 pages = reinterpret_cast<const uint4 *>(info + s)[1];
+        prefix[s] = running;
+        info[s].line_begin = running;
+        running += line.grain == 1u ? pages.y - pages.x : (pages.y - pages.x + line.grain - 1u) / line.grain;
     }
     if (tid == 0) {
-        prefix[p.seq_count] = overflow ? 0u : s_total;
-        hdr->chunk_count = overflow ? 0u : s_total;
-        hdr->pages_per_unit = pages_per_unit;
+        prefix[p.seq_count] = total;
+        hdr->line = line;
         hdr->next_unit = 0;
-        hdr->chunk_capacity = static_cast<uint32_t>(min(p.layout.chunk_capacity, static_cast<uint64_t>(0xffffffffu)));
-        hdr->overflow = overflow;
-        hdr->shared_pages = overflow ? 0u : shared;
-        hdr->shared_ctas = overflow ? 0u : shared_ctas;
+        hdr->shared_pages = shared;
+        hdr->shared_ctas = shared_ctas;
         hdr->shared_rounds = shared_rounds;
-        if (overflow) raise_status(p, CF_B200_DEVSTAT_WORKSPACE);
     }
 }
 
@@ -234,7 +176,7 @@ __device__ __forceinline__ float load_query(const AttentionParams &p, uint32_t s
 }
 
 // ---------------------------------------------------------------------------------------------------------------
-// Any-geometry attention kernel: one CTA per (chunk, kv head) unit. Each page record is copied to shared memory,
+// Any-geometry attention kernel: one CTA per (stretch, kv head) unit. Each page record is copied to shared memory,
 // both streams are decoded to symbols there (one thread per block), then scores and the online-softmax update
 // are computed from shared memory. Built for coverage of every legal geometry, not for speed.
 // ---------------------------------------------------------------------------------------------------------------
@@ -274,9 +216,8 @@ __global__ void __launch_bounds__(kGenericThreads) generic_attention_kernel(Atte
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     const uint32_t D = p.head_dim, T = p.page_tokens, G = p.group;
     PlanHeader *hdr = plan_header(p);
-    const uint32_t *prefix = chunk_prefix(p);
-    const uint32_t unit_count = hdr->chunk_count * p.kv_head_span;
-    const uint32_t pages_per_unit = hdr->pages_per_unit;
+    const PageLine line = plan_line(p);
+    const uint32_t unit_count = line.stretches * p.kv_head_span;
     const uint32_t max_part_units = align_up_u32(p.symbols, 16u) / 16u;
 
     for (;;) {
@@ -285,22 +226,20 @@ __global__ void __launch_bounds__(kGenericThreads) generic_attention_kernel(Atte
         __syncthreads();
         const uint32_t unit = s_unit;
         if (unit >= unit_count) break;
-        const uint32_t chunk = unit / p.kv_head_span;
+        const uint32_t stretch = unit / p.kv_head_span;
         const uint32_t head_local = unit % p.kv_head_span;
         const uint32_t kv_head = p.kv_head_begin + head_local;
-        const uint32_t seq = sequence_of_chunk(prefix, p.seq_count, chunk);
-        const uint32_t slot = slot_of(p, seq);
-        const uint32_t sealed = p.seq_sealed_tokens[slot];
-        const uint32_t tail = p.tail_tokens ? p.tail_tokens[slot] : 0u;
-        const uint32_t qpos = query_position(p, seq, sealed, tail);
+        for (uint32_t x = line.begin(stretch), x_end = line.begin(stretch + 1u); x < x_end;) {
+        const uint32_t piece = line.piece_of(stretch, x);
+        const LineRun run = run_at(p, x, min(line.piece_end(stretch, piece), x_end), line.grain, lane);
+        const uint32_t seq = run.seq, slot = run.info.slot, sealed = run.info.sealed, qpos = run.info.qpos;
         const uint32_t first_token = window_begin(qpos, p.causal_window);
-        uint32_t first_page;
-        const uint32_t vis = visible_pages(p, seq, &first_page);
-        const uint32_t page_begin = first_page + (chunk - prefix[seq]) * pages_per_unit;
-        const uint32_t page_end = min(page_begin + pages_per_unit, first_page + vis);
+        const uint32_t page_begin = run.page, page_end = run.page_end;
+        x = run.x_end;
+        __syncthreads();   // the previous run's results are written
 
         for (uint32_t i = tid; i < G * D; i += kGenericThreads) {
-            q[i] = load_query(p, row_of(p, seq), kv_head * G + i / D, i % D) * (p.softmax_scale * kLog2e);
+            q[i] = load_query(p, run.info.row, kv_head * G + i / D, i % D) * (p.softmax_scale * kLog2e);
             acc[i] = 0.0f;
         }
         if (tid < G) {
@@ -400,131 +339,341 @@ __global__ void __launch_bounds__(kGenericThreads) generic_attention_kernel(Atte
         __syncthreads();
         for (uint32_t i = tid; i < G * D; i += kGenericThreads) {
             const uint32_t g = i / D, d = i % D;
-            float *dst = partial_ptr(p, chunk, head_local * G + g);
+            float *dst = partial_ptr(p, line.slot(stretch, piece, run.x, seq), head_local * G + g);
             dst[2 + d] = acc[i];
             if (d == 0) {
                 dst[0] = ml[2 * g];
                 dst[1] = ml[2 * g + 1];
             }
         }
+        }
     }
 }
 
 // ---------------------------------------------------------------------------------------------------------------
-// Combine: merge the chunk partials of one (sequence, query head) with the unsealed tail and write the output.
+// Combine: merge the partials of every (entry, query head) row with the unsealed tail and write the output.
+//
+// A CTA serves R rows: the query heads of one kv head, for one entry or, in multi-query calls, for several entries of one
+// slot. The tail's K and V rows are then read once per CTA instead of once per row (at 500 rows over a tail of up to 127
+// tokens those reads were all of the 274 us this stage took). A launch with too few rows for that, one or a few
+// sequences, gives each row a CTA of its own (R = 1), whose warps share out the row's partials.
+//
+// Every sum has an order of its own that the shape of the CTA does not change, so that a row's result depends on nothing
+// but the row: partials are added up in 32 consecutive strands and the strands in order, tail tokens in eight interleaved
+// strands.
 // ---------------------------------------------------------------------------------------------------------------
-#ifndef CFB_COMBINE_THREADS
-#define CFB_COMBINE_THREADS 128   // = the largest head_dim: thread d owns output channel d; more threads only wait
-#endif
-constexpr int kCombineThreads = CFB_COMBINE_THREADS;
-constexpr int kCombineWarps = kCombineThreads / 32;
+constexpr uint32_t kStrands = 32;
 
-__global__ void __launch_bounds__(kCombineThreads) combine_kernel(AttentionParams p) {
-    extern __shared__ float tail_scores[];  // [tail_capacity]
-    __shared__ float s_m[kCombineWarps], s_l[kCombineWarps];
-    __shared__ float s_acc[kCombineWarps][128];
-    const uint32_t seq = blockIdx.x;
-    const uint32_t local_q = blockIdx.y;
-    const uint32_t G = p.group, D = p.head_dim;
-    const uint32_t kv_head = p.kv_head_begin + local_q / G;
-    const uint32_t q_head = kv_head * G + local_q % G;
+// Sums of V values over the warp, V a power of two up to 32: lane l gets the sum of value l / (32 / V).
+template <int V>
+__device__ __forceinline__ float sum_many(float (&v)[V], uint32_t lane) {
+    int o = 16;
+#pragma unroll
+    for (int h = V / 2; h >= 1; h /= 2) {
+        const bool upper = (lane & static_cast<uint32_t>(o)) != 0u;
+#pragma unroll
+        for (int i = 0; i < h; ++i) {
+            const float sent = upper ? v[i] : v[i + h], kept = upper ? v[i + h] : v[i];
+            v[i] = kept + __shfl_xor_sync(0xffffffffu, sent, o);
+        }
+        o >>= 1;
+    }
+#pragma unroll
+    for (int rest = V; rest < 32; rest *= 2) {
+        v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+        o >>= 1;
+    }
+    return v[0];
+}
+
+template <int R, int kThreads>
+struct CombineSmem {   // offsets in floats
+    static constexpr int kGroups = kThreads / 128;          // thread groups of one thread per channel
+    static constexpr int kRowStride = R == 1 ? 1 : R + 4;   // of a tail token's weights: 16-byte aligned, banks spread
+    static constexpr int kQ = 0;                            // [R][128]
+    static constexpr int kTail = kQ + R * 128;              // [groups (2 for one group)][R][128] sums of weighted V rows
+    static constexpr int kTailGroups = kGroups < 2 ? 2 : kGroups;
+    static constexpr int kStrand = kTail + kTailGroups * R * 128;   // R = 1: [strand][128]
+    static constexpr int kWeights = kStrand + (R == 1 ? static_cast<int>(kStrands) * 128 : 0);   // [tail_capacity][kRowStride]
+    static size_t bytes(uint32_t tail_capacity) { return (kWeights + static_cast<size_t>(tail_capacity) * kRowStride) * 4u; }
+};
+
+template <int R, int kThreads>
+__global__ void __launch_bounds__(kThreads) combine_kernel(AttentionParams p, uint32_t cta_entries, uint32_t cta_heads) {
+    using S = CombineSmem<R, kThreads>;
+    constexpr int kWarps = kThreads / 32, kGroups = S::kGroups, kGroupStrands = 8 / kGroups;
+    extern __shared__ __align__(16) float smem_f[];
+    float *q = smem_f + S::kQ, *tail_acc = smem_f + S::kTail, *weights = smem_f + S::kWeights;
+    __shared__ uint32_t e_slot[R], e_sealed[R], e_qpos[R], e_tail[R], e_row[R];
+    __shared__ float tail_m[R], tail_l[R];
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    const uint32_t slot = slot_of(p, seq);
-    const uint32_t sealed = p.seq_sealed_tokens[slot];
-    const uint32_t C = p.tail_capacity;  // rows per (slot, kv head) in the tails
-    const uint32_t tail = p.tail_tokens ? min(p.tail_tokens[slot], C) : 0u;
-    const uint32_t qpos = query_position(p, seq, sealed, p.tail_tokens ? p.tail_tokens[slot] : 0u);
-    const uint32_t first_token = window_begin(qpos, p.causal_window);
-    const uint32_t *prefix = chunk_prefix(p);
-    const uint32_t c0 = prefix[seq], c1 = prefix[seq + 1];
-    const uint32_t row = row_of(p, seq);   // of the query and output tensors
+    const uint32_t G = p.group, D = p.head_dim, C = p.tail_capacity;   // C: rows per (slot, kv head) in the tails
+    const uint32_t entry0 = blockIdx.x * cta_entries, entries = min(cta_entries, p.seq_count - entry0);
+    const uint32_t head0 = blockIdx.y * cta_heads, rows = entries * cta_heads;   // local query heads; row = entry * heads + head
+    const uint32_t kv_head = p.kv_head_begin + head0 / G;
+    auto q_head_of = [&](uint32_t r) { return p.kv_head_begin * G + head0 + r % cta_heads; };
 
-    // tail scores (binary16 rows, one warp per token)
-    for (uint32_t t = warp; t < tail; t += kCombineThreads / 32) {
-        const uint64_t tail_row = ((static_cast<uint64_t>(slot) * p.kv_head_count + kv_head) * C + t) * D;
-        float dot = 0.0f;
-        for (uint32_t d = lane; d < D; d += 32) dot += load_query(p, row, q_head, d) * load_tail(p.tail_k, p.tail_type, tail_row + d);
-        dot = warp_sum(dot);
-        if (lane == 0)
-            tail_scores[t] = (sealed + t >= first_token && sealed + t <= qpos) ? dot * p.softmax_scale * kLog2e : -CUDART_INF_F;
+    if (tid < entries) {
+        const uint32_t seq = entry0 + tid, slot = slot_of(p, seq), row = row_of(p, seq);
+        const uint32_t sealed = p.seq_sealed_tokens[slot], tail = p.tail_tokens ? p.tail_tokens[slot] : 0u;
+        e_slot[tid] = slot;
+        e_sealed[tid] = sealed;
+        e_qpos[tid] = query_position(p, seq, sealed, tail);
+        e_tail[tid] = min(tail, C);
+        e_row[tid] = row;
     }
     __syncthreads();
+    uint32_t any_tail = 0;
+    for (uint32_t e = 0; e < entries; ++e) any_tail |= e_tail[e];
 
-    // Chunk partials: every warp merges its share of the chunks in one pass (running max, rescale on the way), four
-    // channels per lane, so that many independent loads are in flight; the warps' results meet in shared memory.
-    {
-        float wm = -CUDART_INF_F, wl = 0.0f, wa[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-        for (uint32_t c = c0 + warp; c < c1; c += kCombineWarps) {
-            const float *part = partial_ptr(p, c, local_q);
-            const float pm = part[0], pl = part[1];
-            float pa[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) pa[j] = lane + 32u * j < D ? part[2 + lane + 32u * j] : 0.0f;
-            if (pm == -CUDART_INF_F) continue;
-            const float nm = fmaxf(wm, pm);
-            const float so = exp2f(wm - nm), sn = exp2f(pm - nm);  // wm = -inf gives so = 0
-            wl = wl * so + pl * sn;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) wa[j] = wa[j] * so + pa[j] * sn;
-            wm = nm;
+    if (any_tail) {
+        for (uint32_t i = tid; i < R * 128u; i += kThreads) {
+            const uint32_t r = i >> 7, d = i & 127u;
+            q[i] = r < rows && d < D ? load_query(p, e_row[r / cta_heads], q_head_of(r), d) : 0.0f;
         }
-        // the shared prefix's partials, same rule: one per CTA of the shared-prefix kernel that met the row's head-tile
-        const PlanHeader *hdr = plan_header(p);
-        uint32_t cells = 0;
-        if (hdr->shared_pages != 0u && hdr->shared_ctas != 0u) {
+        __syncthreads();
+        // Scores. Consecutive entries of one slot share the pass over its rows: two tokens per warp at a time, four channels
+        // per lane, the sums of all rows reduced together.
+        for (uint32_t e0 = 0, e1; e0 < entries; e0 = e1) {
+            for (e1 = e0 + 1u; e1 < entries && e_slot[e1] == e_slot[e0]; ++e1) {}
+            const uint32_t tail = e_tail[e0], sealed = e_sealed[e0];
+            const uint64_t base = (static_cast<uint64_t>(e_slot[e0]) * p.kv_head_count + kv_head) * C;
+            for (uint32_t t0 = 2u * warp; t0 < tail; t0 += 2u * kWarps) {
+                float k0[4], k1[4], sums[2 * R];
+#pragma unroll
+                for (uint32_t j = 0; j < 4; ++j) {
+                    const uint32_t d = lane + 32u * j;
+                    k0[j] = d < D ? load_tail(p.tail_k, p.tail_type, (base + t0) * D + d) : 0.0f;
+                    k1[j] = d < D && t0 + 1u < tail ? load_tail(p.tail_k, p.tail_type, (base + t0 + 1u) * D + d) : 0.0f;
+                }
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    float a = 0.0f, b = 0.0f;
+#pragma unroll
+                    for (uint32_t j = 0; j < 4; ++j) {
+                        const float qv = q[r * 128 + lane + 32u * j];
+                        a = fmaf(qv, k0[j], a);
+                        b = fmaf(qv, k1[j], b);
+                    }
+                    sums[r] = a;
+                    sums[R + r] = b;
+                }
+                const float sum = sum_many<2 * R>(sums, lane);
+                const uint32_t value = lane / (16u / R), r = value % R, t = t0 + value / R;
+                if (lane % (16u / R) == 0u && t < tail && r < rows && r / cta_heads >= e0 && r / cta_heads < e1) {
+                    const uint32_t qpos = e_qpos[r / cta_heads], token = sealed + t;
+                    const bool visible = token >= window_begin(qpos, p.causal_window) && token <= qpos;
+                    weights[t * S::kRowStride + r] = visible ? sum * p.softmax_scale * kLog2e : -CUDART_INF_F;
+                }
+            }
+        }
+        __syncthreads();
+        // softmax of every row over its tail: scores become weights relative to the row's largest
+        for (uint32_t r = warp; r < R; r += kWarps) {
+            const uint32_t tail = r < rows ? e_tail[r / cta_heads] : 0u;
+            float m = -CUDART_INF_F, l = 0.0f;
+            for (uint32_t t = lane; t < tail; t += 32u) m = fmaxf(m, weights[t * S::kRowStride + r]);
+            m = warp_max(m);
+            for (uint32_t t = lane; t < tail; t += 32u) {
+                const float s = weights[t * S::kRowStride + r], w = s == -CUDART_INF_F ? 0.0f : exp2f(s - m);
+                weights[t * S::kRowStride + r] = w;
+                l += w;
+            }
+            l = warp_sum(l);
+            if (lane == 0) {
+                tail_m[r] = m;
+                tail_l[r] = l;
+            }
+        }
+        __syncthreads();
+        // weighted V rows: a thread per channel, thread group g takes the token strands g, g + groups, ... of eight
+        const uint32_t d = tid & 127u, grp = tid >> 7;
+        float acc[kGroupStrands][R];
+#pragma unroll
+        for (int k = 0; k < kGroupStrands; ++k)
+#pragma unroll
+            for (int r = 0; r < R; ++r) acc[k][r] = 0.0f;
+        for (uint32_t e0 = 0, e1; e0 < entries; e0 = e1) {
+            for (e1 = e0 + 1u; e1 < entries && e_slot[e1] == e_slot[e0]; ++e1) {}
+            const uint32_t tail = e_tail[e0];
+            const bool whole = e0 == 0u && e1 == entries;   // one slot: every row takes every token
+            const uint64_t base = (static_cast<uint64_t>(e_slot[e0]) * p.kv_head_count + kv_head) * C;
+            for (uint32_t t0 = 0; t0 < tail; t0 += 8u) {
+                float v[kGroupStrands];
+#pragma unroll
+                for (int k = 0; k < kGroupStrands; ++k) {
+                    const uint32_t t = t0 + grp + static_cast<uint32_t>(k * kGroups);
+                    v[k] = t < tail && d < D ? load_tail(p.tail_v, p.tail_type, (base + t) * D + d) : 0.0f;
+                }
+#pragma unroll
+                for (int k = 0; k < kGroupStrands; ++k) {
+                    const uint32_t t = t0 + grp + static_cast<uint32_t>(k * kGroups);
+                    if (t >= tail) continue;
+#pragma unroll
+                    for (int r = 0; r < R; ++r) {
+                        const float w = whole || (r / cta_heads >= e0 && r / cta_heads < e1) ? weights[t * S::kRowStride + r] : 0.0f;
+                        if (w != 0.0f) acc[k][r] = fmaf(w, v[k], acc[k][r]);   // a token the row does not see may hold anything
+                    }
+                }
+            }
+        }
+        // ((s0 + s2) + (s4 + s6)) and ((s1 + s3) + (s5 + s7)), added below
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            if constexpr (kGroups == 1) {
+                tail_acc[r * 128 + d] = (acc[0][r] + acc[2][r]) + (acc[4][r] + acc[6][r]);
+                tail_acc[(R + r) * 128 + d] = (acc[1][r] + acc[3][r]) + (acc[5][r] + acc[7][r]);
+            } else if constexpr (kGroups == 2) {
+                tail_acc[(grp * R + r) * 128 + d] = (acc[0][r] + acc[1][r]) + (acc[2][r] + acc[3][r]);
+            } else {
+                tail_acc[(grp * R + r) * 128 + d] = acc[0][r];
+            }
+        }
+    } else if (tid < R) {
+        tail_m[tid] = -CUDART_INF_F;
+        tail_l[tid] = 0.0f;
+    }
+    __syncthreads();
+    auto tail_sum = [&](uint32_t r, uint32_t d) {
+        if (!any_tail) return 0.0f;
+        float h[2];
+        for (int i = 0; i < 2; ++i) {
+            if constexpr (S::kTailGroups == 2) h[i] = tail_acc[(i * R + r) * 128 + d];
+            else h[i] = (tail_acc[i * 128 + d] + tail_acc[(i + 2) * 128 + d]) + (tail_acc[(i + 4) * 128 + d] + tail_acc[(i + 6) * 128 + d]);
+        }
+        return h[0] + h[1];
+    };
+    auto store = [&](uint32_t r, uint32_t d, float value) {
+        const uint64_t i = (static_cast<uint64_t>(e_row[r / cta_heads]) * p.query_head_count + q_head_of(r)) * D + d;
+        if (p.output_type == CF_B200_F16) reinterpret_cast<__half *>(p.output)[i] = __float2half_rn(value);
+        else reinterpret_cast<float *>(p.output)[i] = value;
+    };
+
+    // ---- the partials: what the attention kernels wrote ----
+    wait_for_previous_kernel();
+    const PageLine line = plan_line(p);
+    const uint4 more = __ldcg(reinterpret_cast<const uint4 *>(p.workspace) + 2);   // shared_pages.. of the header, see below
+    static_assert(sizeof(PageLine) == 28 && offsetof(PlanHeader, shared_pages) == 32 && offsetof(PlanHeader, shared_rounds) == 40, "");
+    struct RowPartials { uint32_t first, regular, count, seq, local_q; };
+    auto row_partials = [&](uint32_t r) {
+        RowPartials rp = {};
+        rp.seq = entry0 + r / cta_heads;
+        rp.local_q = head0 + r % cta_heads;
+        const uint32_t a = __ldcg(line_prefix(p) + rp.seq), b = __ldcg(line_prefix(p) + rp.seq + 1u);
+        if (b > a) {
+            const uint32_t j0 = line.stretch_of(a), j1 = line.stretch_of(b - 1u);
+            rp.first = line.slot(j0, line.piece_of(j0, a), a, rp.seq);
+            rp.regular = line.slot(j1, line.piece_of(j1, b - 1u), b - 1u, rp.seq) + 1u - rp.first;
+        }
+        rp.count = rp.regular;
+        if (more.x != 0u && more.y != 0u) {   // the shared prefix's: one per CTA of the shared-prefix kernel that met the row's head-tile
             const uint32_t row_tiles = (p.seq_count * G + 127u) / 128u;
-            const SharedSplit split = {hdr->shared_rounds, p.kv_head_span * row_tiles, hdr->shared_ctas};
-            const uint64_t first = static_cast<uint64_t>((local_q / G) * row_tiles + (seq * G + local_q % G) / 128u) * split.rounds;
-            cells = min(split.cta_of(first + split.rounds - 1u) - split.cta_of(first) + 1u, CF_B200_SHARED_CHUNKS_MAX);
+            const SharedSplit split = {more.z, p.kv_head_span * row_tiles, more.y};
+            const uint64_t first = static_cast<uint64_t>((rp.local_q / G) * row_tiles + (rp.seq * G + rp.local_q % G) / 128u) * split.rounds;
+            rp.count += min(split.cta_of(first + split.rounds - 1u) - split.cta_of(first) + 1u, CF_B200_SHARED_CHUNKS_MAX);
         }
-        for (uint32_t c = warp; c < cells; c += kCombineWarps) {
-            const float *part = shared_partial_ptr(p, c, seq, local_q);
-            const float pm = part[0], pl = part[1];
-            float pa[4];
+        return rp;
+    };
+    auto partial_of = [&](const RowPartials &rp, uint32_t c) {
+        return c < rp.regular ? partial_ptr(p, rp.first + c, rp.local_q) : shared_partial_ptr(p, c - rp.regular, rp.seq, rp.local_q);
+    };
+    // Adds up the partials [begin, end) of a row, a whole number of strands of `strand` each; `emit` gets every strand's sums
+    // (of l, and of this lane's channels lane + 32 j). Eight partials' loads are in flight at a time.
+    auto add_strands = [&](const RowPartials &rp, uint32_t begin, uint32_t end, uint32_t strand, float m, auto emit) {
+        float part[4] = {0.0f, 0.0f, 0.0f, 0.0f}, part_l = 0.0f;
+        uint32_t left = strand;
+        for (uint32_t c0 = begin; c0 < end; c0 += 32u) {
+            float w = 0.0f, wl = 0.0f;   // lane i: weight of partial c0 + i, and its l
+            if (c0 + lane < end) {
+                const float *src = partial_of(rp, c0 + lane);
+                const float pm = __ldcg(src);
+                wl = __ldcg(src + 1);
+                w = pm == -CUDART_INF_F ? 0.0f : exp2f(pm - m);
+            }
+            const uint32_t n = min(32u, end - c0);
+            for (uint32_t i0 = 0; i0 < n; i0 += 8u) {
+                float x[8][4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) pa[j] = lane + 32u * j < D ? part[2 + lane + 32u * j] : 0.0f;
-            if (pm == -CUDART_INF_F) continue;
-            const float nm = fmaxf(wm, pm);
-            const float so = exp2f(wm - nm), sn = exp2f(pm - nm);
-            wl = wl * so + pl * sn;
+                for (int i = 0; i < 8; ++i) {
+                    const float *src = i0 + i < n ? partial_of(rp, c0 + i0 + i) + 2 : nullptr;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) wa[j] = wa[j] * so + pa[j] * sn;
-            wm = nm;
-        }
-        if (lane == 0) {
-            s_m[warp] = wm;
-            s_l[warp] = wl;
-        }
+                    for (uint32_t j = 0; j < 4; ++j) x[i][j] = src && lane + 32u * j < D ? __ldcg(src + lane + 32u * j) : 0.0f;
+                }
 #pragma unroll
-        for (int j = 0; j < 4; ++j) s_acc[warp][lane + 32 * j] = wa[j];
-    }
-    __syncthreads();
-    float m = -CUDART_INF_F;
-    for (int w = 0; w < kCombineWarps; ++w) m = fmaxf(m, s_m[w]);
-    for (uint32_t t = 0; t < tail; ++t) m = fmaxf(m, tail_scores[t]);
-
-    float l = 0.0f, a = 0.0f;
-    if (m != -CUDART_INF_F) {
-        for (int w = 0; w < kCombineWarps; ++w) {
-            if (s_m[w] == -CUDART_INF_F) continue;
-            const float sw = exp2f(s_m[w] - m);
-            l += s_l[w] * sw;
-            if (tid < D) a += s_acc[w][tid] * sw;
+                for (int i = 0; i < 8; ++i) {
+                    if (i0 + i >= n) break;
+                    const float wi = __shfl_sync(0xffffffffu, w, i0 + i), li = __shfl_sync(0xffffffffu, wl, i0 + i);
+                    if (wi != 0.0f) {   // a partial without a visible token says nothing
+                        part_l = fmaf(li, wi, part_l);
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) part[j] = fmaf(x[i][j], wi, part[j]);
+                    }
+                    if (--left == 0u) {
+                        emit(part_l, part);
+                        left = strand;
+                        part_l = part[0] = part[1] = part[2] = part[3] = 0.0f;
+                    }
+                }
+            }
         }
-        for (uint32_t t = 0; t < tail; ++t) {
-            const float s = tail_scores[t];
-            if (s == -CUDART_INF_F) continue;
-            const float w = exp2f(s - m);
-            l += w;
-            if (tid < D)
-                a += w * load_tail(p.tail_v, p.tail_type, ((static_cast<uint64_t>(slot) * p.kv_head_count + kv_head) * C + t) * D + tid);
+        if (left != strand) emit(part_l, part);
+    };
+    if constexpr (R > 1) {   // a warp per row
+        for (uint32_t r = warp; r < rows; r += kWarps) {
+            const RowPartials rp = row_partials(r);
+            float m = -CUDART_INF_F;
+            for (uint32_t c = lane; c < rp.count; c += 32u) m = fmaxf(m, __ldcg(partial_of(rp, c)));
+            m = warp_max(m);
+            float l = 0.0f, a[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            add_strands(rp, 0u, rp.count, (rp.count + kStrands - 1u) / kStrands, m, [&](float pl, const float (&pa)[4]) {
+                l += pl;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) a[j] += pa[j];
+            });
+            const float top = fmaxf(m, tail_m[r]);
+            const float sp = m == -CUDART_INF_F ? 0.0f : exp2f(m - top), st = tail_m[r] == -CUDART_INF_F ? 0.0f : exp2f(tail_m[r] - top);
+            const float total = l * sp + tail_l[r] * st;
+            const float inv = total > 0.0f ? 1.0f / total : 0.0f;   // no visible token: zeros (paged_kv_attention.cu:170-173)
+#pragma unroll
+            for (uint32_t j = 0; j < 4; ++j) {
+                const uint32_t d = lane + 32u * j;
+                if (d < D) store(r, d, (a[j] * sp + tail_sum(r, d) * st) * inv);
+            }
         }
-    }
-    if (tid < D) {
-        const float out = l > 0.0f ? a / l : 0.0f;  // no visible token: zeros (paged_kv_attention.cu:170-173)
-        const uint64_t i = (static_cast<uint64_t>(row) * p.query_head_count + q_head) * D + tid;
-        if (p.output_type == CF_B200_F16) reinterpret_cast<__half *>(p.output)[i] = __float2half_rn(out);
-        else reinterpret_cast<float *>(p.output)[i] = out;
+    } else {   // the CTA's warps share one row's strands
+        constexpr uint32_t kOwn = kStrands / kWarps;
+        __shared__ float warp_m[kWarps], strand_l[kStrands];
+        float *strands = smem_f + S::kStrand;
+        const RowPartials rp = row_partials(0u);
+        const uint32_t strand = (rp.count + kStrands - 1u) / kStrands;
+        const uint32_t begin = min(warp * kOwn * strand, rp.count), end = min(begin + kOwn * strand, rp.count);
+        float m = -CUDART_INF_F;
+        for (uint32_t c = begin + lane; c < end; c += 32u) m = fmaxf(m, __ldcg(partial_of(rp, c)));
+        m = warp_max(m);
+        if (lane == 0) warp_m[warp] = m;
+        __syncthreads();
+        m = warp_max(lane < kWarps ? warp_m[lane] : -CUDART_INF_F);
+        uint32_t k = warp * kOwn;
+        add_strands(rp, begin, end, strand, m, [&](float pl, const float (&pa)[4]) {
+            if (lane == 0) strand_l[k] = pl;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) strands[k * 128u + lane + 32u * j] = pa[j];
+            ++k;
+        });
+        __syncthreads();
+        const uint32_t used = strand ? (rp.count + strand - 1u) / strand : 0u;
+        if (tid < D) {
+            float l = 0.0f, a = 0.0f;
+            for (uint32_t i = 0; i < used; ++i) {
+                l += strand_l[i];
+                a += strands[i * 128u + tid];
+            }
+            const float top = fmaxf(m, tail_m[0]);
+            const float sp = m == -CUDART_INF_F ? 0.0f : exp2f(m - top), st = tail_m[0] == -CUDART_INF_F ? 0.0f : exp2f(tail_m[0] - top);
+            const float total = l * sp + tail_l[0] * st;
+            const float inv = total > 0.0f ? 1.0f / total : 0.0f;
+            store(0u, tid, (a * sp + tail_sum(0u, tid) * st) * inv);
+        }
     }
 }
 
@@ -621,14 +770,42 @@ bool fill_params(const cf_b200_sealed_attention_desc *d, AttentionParams *p) {
 
 cudaError_t launch_plan(const AttentionParams &p, cudaStream_t stream) {
     if (p.shared_prefix_pages) verify_prefix_kernel<<<p.seq_count, 256, 0, stream>>>(p);
-    plan_kernel<<<1, kPlanThreads, 0, stream>>>(p);
-    return cudaPeekAtLastError();
+    const uint32_t threads = p.seq_count <= 128u ? 128u : kPlanThreads;   // small batches: fewer warps to start and to meet
+    return launch_kernel(plan_kernel, 1, threads, 0, stream, p.shared_prefix_pages != 0u, p);
 }
 
-cudaError_t launch_combine(const AttentionParams &p, cudaStream_t stream) {
-    const dim3 grid(p.seq_count, p.kv_head_span * p.group);
-    combine_kernel<<<grid, kCombineThreads, max(p.tail_capacity, 1u) * sizeof(float), stream>>>(p);
-    return cudaPeekAtLastError();
+namespace {
+
+template <int R, int kThreads>
+cudaError_t launch_combine_as(const AttentionParams &p, cudaStream_t stream, bool dependent, uint32_t entries, uint32_t heads) {
+    const dim3 grid((p.seq_count + entries - 1u) / entries, p.kv_head_span * p.group / heads);
+    const size_t smem = CombineSmem<R, kThreads>::bytes(p.tail_capacity);
+    if (smem > 47u * 1024u) {   // tails of thousands of tokens
+        const cudaError_t e = cudaFuncSetAttribute(combine_kernel<R, kThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+        if (e != cudaSuccess) return e;
+    }
+    return launch_kernel(combine_kernel<R, kThreads>, grid, kThreads, smem, stream, dependent, p, entries, heads);
+}
+
+}  // namespace
+
+// Rows per CTA of the combine kernel: a kv head's whole query group where that still makes about a CTA per SM, and in
+// multi-query calls as many entries beside it as make sixteen rows, if their tails are long enough to be worth sharing.
+// Otherwise a CTA per row: of 1024 threads while all of them are resident at once, of 256 beyond that. The tail's weights must
+// fit the 48 KB of shared memory that need no opt-in.
+cudaError_t launch_combine(const AttentionParams &p, cudaStream_t stream, bool dependent) {
+    constexpr uint32_t kEnoughCtas = 120, kSharedBytes = 48 * 1024 - 1024;
+    const uint32_t groups = p.seq_count * p.kv_head_span, G = p.group, C = p.tail_capacity;
+    if (groups >= kEnoughCtas) {
+        const uint32_t entries = p.query_positions && p.seq_slots && C > 16u ? 16u / G : 1u;
+        if (entries > 1u && (groups + entries - 1u) / entries >= kEnoughCtas && CombineSmem<16, 256>::bytes(C) <= kSharedBytes)
+            return launch_combine_as<16, 256>(p, stream, dependent, entries, G);
+        if (G <= 4u && CombineSmem<4, 128>::bytes(C) <= kSharedBytes) return launch_combine_as<4, 128>(p, stream, dependent, 1u, G);
+        if (G <= 8u && CombineSmem<8, 256>::bytes(C) <= kSharedBytes) return launch_combine_as<8, 256>(p, stream, dependent, 1u, G);
+        if (CombineSmem<16, 256>::bytes(C) <= kSharedBytes) return launch_combine_as<16, 256>(p, stream, dependent, 1u, G);
+    }
+    if (groups * G <= 2u * 148u && CombineSmem<1, 1024>::bytes(C) <= kSharedBytes) return launch_combine_as<1, 1024>(p, stream, dependent, 1u, 1u);
+    return launch_combine_as<1, 256>(p, stream, dependent, 1u, 1u);
 }
 
 cudaError_t launch_generic_attention(const AttentionParams &p, cudaStream_t stream) {
@@ -641,7 +818,7 @@ cudaError_t launch_generic_attention(const AttentionParams &p, cudaStream_t stre
     e = cudaFuncSetAttribute(generic_attention_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          static_cast<int>(lay.total));
     if (e != cudaSuccess) return e;
-    generic_attention_kernel<<<sm_count * 4, kGenericThreads, lay.total, stream>>>(p);
+    generic_attention_kernel<<<sm_count * kGenericCtasPerSm, kGenericThreads, lay.total, stream>>>(p);
     return cudaPeekAtLastError();
 }
 
@@ -677,7 +854,7 @@ extern "C" cf_status cf_b200_sealed_attention_validate(const cf_b200_sealed_atte
     const uint32_t span = d->kv_head_span ? d->kv_head_span : d->kv_head_count - d->kv_head_begin;
     const cfb::WorkspaceLayout w = cfb::workspace_layout(d->seq_count, span * (d->query_head_count / d->kv_head_count),
                                                          d->head_dim, d->workspace_bytes, d->shared_prefix_pages != 0);
-    if (w.chunk_capacity < d->seq_count) return CF_ERR_INVALID_ARGUMENT;  // at least one chunk per sequence
+    if (w.chunk_capacity < d->seq_count) return CF_ERR_INVALID_ARGUMENT;  // at least one partial per sequence
     if (d->shared_prefix_pages > d->page_table_stride) return CF_ERR_INVALID_ARGUMENT;
     // reserved0 has one use: the number of page ids the dump buffer of CF_B200_KERNEL_DECODE_DUMP covers
     if ((d->kernel == CF_B200_KERNEL_DECODE_DUMP) != (d->reserved0 != 0)) return CF_ERR_INVALID_ARGUMENT;
@@ -691,10 +868,9 @@ extern "C" cf_status cf_b200_sealed_attention_workspace_bytes(const cf_b200_seal
         return CF_ERR_INVALID_ARGUMENT;
     const uint32_t span = d->kv_head_span ? d->kv_head_span : d->kv_head_count - d->kv_head_begin;
     const uint32_t local_q = span * (d->query_head_count / d->kv_head_count);
-    const uint32_t ppu = d->min_pages_per_unit ? d->min_pages_per_unit : cfb::default_pages_per_unit(total_pages, span);
-    const uint64_t chunks = total_pages / ppu + d->seq_count + 1;  // each sequence may round up once
+    const uint64_t slots = cfb::partial_slots_for(total_pages, d->seq_count, span, d->min_pages_per_unit);
     const cfb::WorkspaceLayout w = cfb::workspace_layout(d->seq_count, local_q, d->head_dim, 0, d->shared_prefix_pages != 0);
-    *out_bytes = w.partials_offset + chunks * (w.partial_stride_floats * 4ull * local_q + sizeof(cfb::ChunkInfo)) + 64ull;
+    *out_bytes = w.partials_offset + slots * (w.partial_stride_floats * 4ull * local_q) + 64ull;
     return CF_OK;
 }
 
@@ -722,25 +898,32 @@ cf_status cfb::sealed_attention_stages(const cf_b200_sealed_attention_desc *d, u
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const bool use_lanes = d->kernel == CF_B200_KERNEL_LANES || probe ||
                            (d->kernel == CF_B200_KERNEL_AUTO && lanes_ok);
-    // the shared-prefix kernel works on rows of 128 = whole query groups and on pages every query token sees in full
-    if (use_lanes && p.block_size == 64 && p.head_dim == 128 && d->row_map == nullptr && p.decode_probe != 1u && d->shared_prefix_pages && d->causal_window == 0 && 128u % p.group == 0) {
-        static cfb::LauncherState table[64];
-        cudaError_t e;
-        const cfb::LauncherState *state = cfb::launcher_state(table, &e);
-        if (!state) return CF_ERR_CUDA;
-        p.shared_prefix_pages = d->shared_prefix_pages;
-        p.sm_count = static_cast<uint32_t>(state->sm_count);
+    static cfb::LauncherState table[64];
+    cudaError_t e;
+    const cfb::LauncherState *state = cfb::launcher_state(table, &e);
+    if (!state) return CF_ERR_CUDA;
+    p.sm_count = static_cast<uint32_t>(state->sm_count);
+    if (use_lanes) {
+        cfb::lanes_plan_shape(p, p.sm_count, &p.plan_warps, &p.unit_lanes);
+    } else {
+        p.plan_warps = p.sm_count * cfb::kGenericCtasPerSm;
+        p.unit_lanes = p.kv_head_span;
     }
-    if ((stages & CF_B200_STAGE_PLAN) && cfb::launch_plan(p, s) != cudaSuccess) return CF_ERR_CUDA;
-    if (stages & CF_B200_STAGE_ATTENTION) {
-        if (p.shared_prefix_pages) {
-            if (cfb::launch_prefix_attention(p, s) != cudaSuccess) return CF_ERR_CUDA;
+    // the shared-prefix kernel works on rows of 128 = whole query groups and on pages every query token sees in full
+    if (use_lanes && p.block_size == 64 && p.head_dim == 128 && d->row_map == nullptr && p.decode_probe != 1u && d->shared_prefix_pages && d->causal_window == 0 && 128u % p.group == 0)
+        p.shared_prefix_pages = d->shared_prefix_pages;
+    const bool plan = (stages & CF_B200_STAGE_PLAN) != 0, attention = (stages & CF_B200_STAGE_ATTENTION) != 0;
+    if (plan && cfb::launch_plan(p, s) != cudaSuccess) return CF_ERR_CUDA;
+    if (attention) {
+        const bool prefix = p.shared_prefix_pages != 0u;
+        if (prefix) {
+            if (cfb::launch_prefix_attention(p, s, plan) != cudaSuccess) return CF_ERR_CUDA;
             g_shared_prefix_launches.fetch_add(1, std::memory_order_relaxed);
         }
-        const cudaError_t e = use_lanes ? cfb::launch_lanes_attention(p, s) : cfb::launch_generic_attention(p, s);
+        e = use_lanes ? cfb::launch_lanes_attention(p, s, plan || prefix, prefix) : cfb::launch_generic_attention(p, s);
         if (e != cudaSuccess) return CF_ERR_CUDA;
     }
-    if ((stages & CF_B200_STAGE_COMBINE) && cfb::launch_combine(p, s) != cudaSuccess) return CF_ERR_CUDA;
+    if ((stages & CF_B200_STAGE_COMBINE) && cfb::launch_combine(p, s, attention && use_lanes) != cudaSuccess) return CF_ERR_CUDA;
     return CF_OK;
 }
 

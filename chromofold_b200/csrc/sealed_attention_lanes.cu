@@ -5,7 +5,7 @@
 //
 // What it computes is what src/cuda/paged_kv_attention.cu:183-276 computes for one query token; how it runs is new:
 //
-//   * One WARP owns one (chunk, kv head) unit. A page record arrives in shared memory as ONE bulk async copy
+//   * One WARP owns one (stretch of the page line, kv head) unit. A page record arrives in shared memory as ONE bulk async copy
 //     (cp.async.bulk + mbarrier), double buffered per warp. Coding tables (rANS slot table, Huffman LUT) are loaded
 //     once per CTA. No thread ever reads page bytes from global memory directly.
 //   * Lane l decodes block l of the K stream and block l of the V stream, interleaved so that the two independent
@@ -17,7 +17,7 @@
 //     contraction lands in its own output column/row. Tensor cores do the whole contraction for the group;
 //     a code is decoded once for all query heads (the reference re-decodes per query head,
 //     paged_kv_attention.cu:205-207).
-//   * Online softmax per page in fp32; partial (max, sum, weighted) per unit goes to the split-KV workspace and is
+//   * Online softmax per page in fp32; partial (max, sum, weighted) per piece of a stretch goes to the split-KV workspace and is
 //     merged by the combine kernel (cf_online_softmax_merge rule, src/runtime/kv_runtime.cpp:219-243).
 //   * Every wait on a copy is bounded; on expiry the warp raises CF_B200_DEVSTAT_WAIT_EXPIRED and leaves.
 
@@ -283,7 +283,7 @@ static_assert(WarpLayout<1>::kSmem <= 232448 && WarpLayout<2>::kSmem <= 232448 &
 // binary16(q - binary16(q)), stored as the rows of group 0 and group 1, the two score fragments are added, and one
 // softmax / P V follows: the scores equal fp32-query scores to 2^-22 relative, at the cost of a second score mma.
 template <int NG, int kMode = kAttend, bool kSplitQ = false, int NB = 32, int kDim = 128>
-__global__ void __launch_bounds__(kThreadsOf<NG, NB>, 1) lanes_attention_kernel(AttentionParams p) {
+__global__ void __launch_bounds__(kThreadsOf<NG, NB>, 1) lanes_attention_kernel(AttentionParams p, uint32_t after_prefix) {
     constexpr bool kProbe = kMode != kAttend;
     static_assert(!kSplitQ || NG == 2, "split queries use the two-group query layout");
     static_assert(NB == 32 || NB == 24 || NB == 16 || NB == 12 || NB == 8 || NB == 4, "blocks per stream");
@@ -318,10 +318,11 @@ __global__ void __launch_bounds__(kThreadsOf<NG, NB>, 1) lanes_attention_kernel(
     }
     __syncthreads();
 
-    PlanHeader *hdr = plan_header(p);
+    // The plan kernel's results. A shared-prefix kernel in front of this one has waited for them before it let this kernel start, and
+    // nothing here needs what it writes: this kernel takes over each SM as that one leaves it, and waits for its end at its own.
+    if (!after_prefix) wait_for_previous_kernel();
+    allow_dependent_launch();
     const uint32_t subgroups = (p.group + kPassHeads - 1u) / kPassHeads;   // 4 NG query heads per pass
-    const uint32_t unit_count = hdr->chunk_count * p.kv_head_span * subgroups;
-    const uint32_t pages_per_unit = hdr->pages_per_unit;
     const uint32_t g = lane >> 2, t = lane & 3u;
     uint32_t phase_bits = 0u;  // bit s: parity the next wait on stage s expects
 
@@ -333,27 +334,42 @@ __global__ void __launch_bounds__(kThreadsOf<NG, NB>, 1) lanes_attention_kernel(
     const uint32_t o_head = g & 3u;                        // O fragments: all of this lane's outputs are one head per group
     const bool row_lo_mine = t == (g >> 2), row_hi_mine = t == (g >> 2) + 2u;   // P rows with lane tag t
 
+    // A unit is a stretch of the page line for one kv head (and one pass over its query group). The library's own cut makes at most
+    // as many units as there are warps: unit u goes to warp u / gridDim of CTA u % gridDim, so that fewer of them spread over the
+    // SMs. More, when the caller fixes the pages per unit, are handed out as warps come free.
+    // One turn of the loop covers a unit's positions inside one sequence and one piece. Between turns only `unit` and `x`, where the
+    // unit goes on (0: at its start), are kept; the line is read again, so that the pages' loop has the registers to itself.
+    uint32_t unit = warp * gridDim.x + blockIdx.x, x = 0u;
     for (;;) {
-        uint32_t unit = 0;
-        if (lane == 0) unit = atomicAdd(&hdr->next_unit, 1u);
-        unit = __shfl_sync(0xffffffffu, unit, 0);
-        if (unit >= unit_count) break;
-        const uint32_t sub = unit % subgroups;
-        const uint32_t chunk = (unit / subgroups) / p.kv_head_span;
-        const uint32_t head_local = (unit / subgroups) % p.kv_head_span;
+        uint32_t partial, page_begin, n_pages, slot, sealed, qpos, q_row, sub, head_local;
+        {
+            const PageLine line = plan_line(p);
+            const uint32_t unit_lanes = p.kv_head_span * subgroups, unit_count = line.stretches * unit_lanes, warps = kWarpsOf<NG, NB> * gridDim.x;
+            uint32_t stretch = unit / unit_lanes;
+            if (x != 0u && x == line.begin(stretch + 1u)) {   // the unit is done
+                if (unit_count <= warps) break;
+                if (lane == 0) unit = warps + atomicAdd(&plan_header(p)->next_unit, 1u);
+                unit = __shfl_sync(0xffffffffu, unit, 0);
+                stretch = unit / unit_lanes;
+                x = 0u;
+            }
+            if (unit >= unit_count) break;
+            if (x == 0u) x = line.begin(stretch);
+            const uint32_t piece = line.piece_of(stretch, x);
+            const LineRun run = run_at(p, x, line.piece_end(stretch, piece), line.grain, lane);
+            partial = line.slot(stretch, piece, x, run.seq);
+            page_begin = run.page;
+            n_pages = run.page_end - run.page;
+            slot = run.info.slot, sealed = run.info.sealed, qpos = run.info.qpos, q_row = run.info.row;
+            x = run.x_end;
+            sub = unit % subgroups;
+            head_local = (unit / subgroups) % p.kv_head_span;
+        }
         const uint32_t kv_head = p.kv_head_begin + head_local;
         const uint32_t G = min(kPassHeads, p.group - kPassHeads * sub);       // query heads served by this pass
         const uint32_t q_head_base = kv_head * p.group + kPassHeads * sub;    // first of them
         const uint32_t out_head_base = head_local * p.group + kPassHeads * sub;
-        // the chunk's start-up record, written by the plan kernel (which also took the shared pages off its front)
-        const uint4 *ci = reinterpret_cast<const uint4 *>(chunk_info(p) + chunk);
-        const uint4 ci0 = ci[0];
-        const uint4 ci1 = ci[1];
-        const uint32_t slot = ci0.y, sealed = ci0.z, qpos = ci0.w, page_begin = ci1.x, q_row = ci1.y;   // ci0.x = batch entry
         const uint32_t first_token = window_begin(qpos, p.causal_window);
-        const uint32_t pages = min((sealed + 15u) / 16u, qpos / 16u + 1u);
-        const uint32_t page_end = min(page_begin + pages_per_unit, pages);
-        const uint32_t n_pages = page_end > page_begin ? page_end - page_begin : 0u;
         const uint32_t *table_row = p.page_table + static_cast<uint64_t>(slot) * p.page_table_stride;
 
         QSrc qs;
@@ -372,7 +388,7 @@ __global__ void __launch_bounds__(kThreadsOf<NG, NB>, 1) lanes_attention_kernel(
         } else if constexpr (kSplitQ) {
             const float2 *qsrc = reinterpret_cast<const float2 *>(
                 reinterpret_cast<const float *>(p.queries) + (static_cast<uint64_t>(q_row) * p.query_head_count + q_head_base) * kDim);
-            __syncwarp();  // the previous unit's readers are done
+            __syncwarp();  // the previous run's readers are done
 #pragma unroll
             for (int j = 0; j < kDim / 16; ++j) {    // 4 heads x kDim / 2 channel pairs; row = head*2 + half, residues 8 rows further
                 const uint32_t i = lane + 32u * j, head = i / (2u * kRowWords);
@@ -389,7 +405,7 @@ __global__ void __launch_bounds__(kThreadsOf<NG, NB>, 1) lanes_attention_kernel(
         } else {
             const uint32_t *qsrc = reinterpret_cast<const uint32_t *>(
                 reinterpret_cast<const __half *>(p.queries) + (static_cast<uint64_t>(q_row) * p.query_head_count + q_head_base) * kDim);
-            __syncwarp();  // the previous unit's readers are done
+            __syncwarp();  // the previous run's readers are done
 #pragma unroll
             for (int j = 0; j < kDim / 8; ++j) {   // 8 heads x kDim / 2 words; row = head*2 + half
                 const uint32_t i = lane + 32u * j, head = i / (2u * kRowWords);
@@ -672,17 +688,16 @@ __global__ void __launch_bounds__(kThreadsOf<NG, NB>, 1) lanes_attention_kernel(
             // give the copies still in flight a bounded chance to land before this warp's buffers go away
             mbar_wait(&bars[0], phase_bits & 1u, p.wait_polls);
             if constexpr (L::kStages == 2) mbar_wait(&bars[1], (phase_bits >> 1) & 1u, p.wait_polls);
-            return;
+            break;
         }
 
         if constexpr (kMode == kDump) {
-        } else if constexpr (kMode == kFold) {   // the checksum of everything the unit decoded, so that the work cannot be dropped
-            uint32_t x = u.vq[0];
+        } else if constexpr (kMode == kFold) {   // the checksum of everything the partial covers, so that the work cannot be dropped
+            uint32_t folded = u.vq[0];
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) x ^= __shfl_xor_sync(0xffffffffu, x, o);
-            if (lane == 0) partial_ptr(p, chunk, out_head_base)[0] = __uint_as_float(x);
+            for (int o = 1; o < 32; o <<= 1) folded ^= __shfl_xor_sync(0xffffffffu, folded, o);
+            if (lane == 0) partial_ptr(p, partial, out_head_base)[0] = __uint_as_float(folded);
         } else {
-        // ---- unit partials ----
 #pragma unroll
         for (int n = 0; n < NS; ++n) {
             float l0 = u.l0[n], l1 = u.l1[n];
@@ -694,18 +709,18 @@ __global__ void __launch_bounds__(kThreadsOf<NG, NB>, 1) lanes_attention_kernel(
             const uint32_t h0 = 4u * n + my_head0;
             if (g == 0 && t < 2) {
                 if (h0 < G) {
-                    float *dst = partial_ptr(p, chunk, out_head_base + h0);
+                    float *dst = partial_ptr(p, partial, out_head_base + h0);
                     dst[0] = u.m0[n];
                     dst[1] = l0;
                 }
                 if (h0 + 1u < G) {
-                    float *dst = partial_ptr(p, chunk, out_head_base + h0 + 1u);
+                    float *dst = partial_ptr(p, partial, out_head_base + h0 + 1u);
                     dst[0] = u.m1[n];
                     dst[1] = l1;
                 }
             }
             if (4u * n + o_head < G) {
-                float *dst = partial_ptr(p, chunk, out_head_base + 4u * n + o_head) + 2;
+                float *dst = partial_ptr(p, partial, out_head_base + 4u * n + o_head) + 2;
 #pragma unroll
                 for (int dd = 0; dd < kVCh; ++dd) {
 #pragma unroll
@@ -719,6 +734,7 @@ __global__ void __launch_bounds__(kThreadsOf<NG, NB>, 1) lanes_attention_kernel(
         }   // !kProbe
         __syncwarp();
     }
+    wait_for_previous_kernel();
 }
 
 }  // namespace
@@ -738,7 +754,7 @@ bool lanes_kernel_supports(const AttentionParams &p) {
 namespace {
 
 template <int NG, int kMode, bool kSplitQ, int NB, int kDim>
-cudaError_t launch_one(const AttentionParams &p, int sm_count, cudaStream_t stream) {
+cudaError_t launch_one(const AttentionParams &p, int sm_count, cudaStream_t stream, bool dependent, bool after_prefix) {
     static std::atomic<uint64_t> configured{0};   // bit = device ordinal
     int device = 0;
     cudaError_t e = cudaGetDevice(&device);
@@ -750,38 +766,47 @@ cudaError_t launch_one(const AttentionParams &p, int sm_count, cudaStream_t stre
         if (e != cudaSuccess) return e;
         configured.fetch_or(bit, std::memory_order_release);
     }
-    lanes_attention_kernel<NG, kMode, kSplitQ, NB, kDim><<<sm_count, kThreadsOf<NG, NB>, WarpLayout<NG, NB>::kSmem, stream>>>(p);
-    return cudaPeekAtLastError();
+    return launch_kernel(lanes_attention_kernel<NG, kMode, kSplitQ, NB, kDim>, sm_count, kThreadsOf<NG, NB>, WarpLayout<NG, NB>::kSmem,
+                         stream, dependent, p, static_cast<uint32_t>(after_prefix));
 }
 
 template <int NB, int kDim = 128>
-cudaError_t launch_for_blocks(const AttentionParams &p, int sm_count, cudaStream_t stream) {
-    if (p.decode_probe == 2u) return launch_one<1, kDump, false, NB, kDim>(p, sm_count, stream);
-    if (p.decode_probe) return launch_one<1, kFold, false, NB, kDim>(p, sm_count, stream);
-    if (p.query_type == CF_B200_F32) return launch_one<2, kAttend, true, NB, kDim>(p, sm_count, stream);
-    if (p.group <= 4) return launch_one<1, kAttend, false, NB, kDim>(p, sm_count, stream);
-    return launch_one<2, kAttend, false, NB, kDim>(p, sm_count, stream);
+cudaError_t launch_for_blocks(const AttentionParams &p, int sm_count, cudaStream_t stream, bool dependent, bool after_prefix) {
+    if (p.decode_probe == 2u) return launch_one<1, kDump, false, NB, kDim>(p, sm_count, stream, dependent, after_prefix);
+    if (p.decode_probe) return launch_one<1, kFold, false, NB, kDim>(p, sm_count, stream, dependent, after_prefix);
+    if (p.query_type == CF_B200_F32) return launch_one<2, kAttend, true, NB, kDim>(p, sm_count, stream, dependent, after_prefix);
+    if (p.group <= 4) return launch_one<1, kAttend, false, NB, kDim>(p, sm_count, stream, dependent, after_prefix);
+    return launch_one<2, kAttend, false, NB, kDim>(p, sm_count, stream, dependent, after_prefix);
 }
 
 }  // namespace
 
-cudaError_t launch_lanes_attention(const AttentionParams &p, cudaStream_t stream) {
+void lanes_plan_shape(const AttentionParams &p, uint32_t sm_count, uint32_t *warps, uint32_t *unit_lanes) {
+    const bool split_q = p.query_type == CF_B200_F32 && !p.decode_probe;
+    const bool eight = !split_q && p.group > 4u && !p.decode_probe;   // query heads per pass: eight, else four
+    const bool staged = p.block_size != 64u || p.head_dim != 128u;
+    const int per_sm = staged ? (split_q || eight ? kWarpsOf<2, 16> : kWarpsOf<1, 16>) : split_q || eight ? kWarpsOf<2> : kWarpsOf<1>;
+    *warps = sm_count * static_cast<uint32_t>(per_sm);
+    *unit_lanes = p.kv_head_span * (eight ? (p.group + 7u) / 8u : (p.group + 3u) / 4u);
+}
+
+cudaError_t launch_lanes_attention(const AttentionParams &p, cudaStream_t stream, bool dependent, bool after_prefix) {
     static LauncherState table[64];
     cudaError_t e;
     LauncherState *state = launcher_state(table, &e);
     if (!state) return e;
     if (p.head_dim == 64) {   // 16 x 64 pages: 16 (or 8) blocks per stream, always staged
-        return p.block_size == 64 ? launch_for_blocks<16, 64>(p, state->sm_count, stream)
-                                  : launch_for_blocks<8, 64>(p, state->sm_count, stream);
+        return p.block_size == 64 ? launch_for_blocks<16, 64>(p, state->sm_count, stream, dependent, after_prefix)
+                                  : launch_for_blocks<8, 64>(p, state->sm_count, stream, dependent, after_prefix);
     }
     if (p.head_dim == 96) {
-        return p.block_size == 64 ? launch_for_blocks<24, 96>(p, state->sm_count, stream)
-                                  : launch_for_blocks<12, 96>(p, state->sm_count, stream);
+        return p.block_size == 64 ? launch_for_blocks<24, 96>(p, state->sm_count, stream, dependent, after_prefix)
+                                  : launch_for_blocks<12, 96>(p, state->sm_count, stream, dependent, after_prefix);
     }
-    if (p.head_dim == 32) return launch_for_blocks<8, 32>(p, state->sm_count, stream);
-    if (p.block_size == 128) return launch_for_blocks<16>(p, state->sm_count, stream);
-    if (p.block_size == 256) return launch_for_blocks<8>(p, state->sm_count, stream);
-    return launch_for_blocks<32>(p, state->sm_count, stream);
+    if (p.head_dim == 32) return launch_for_blocks<8, 32>(p, state->sm_count, stream, dependent, after_prefix);
+    if (p.block_size == 128) return launch_for_blocks<16>(p, state->sm_count, stream, dependent, after_prefix);
+    if (p.block_size == 256) return launch_for_blocks<8>(p, state->sm_count, stream, dependent, after_prefix);
+    return launch_for_blocks<32>(p, state->sm_count, stream, dependent, after_prefix);
 }
 
 }  // namespace cfb

@@ -732,11 +732,14 @@ __global__ void __launch_bounds__(kTcThreads, 1) prefix_attention_kernel(Attenti
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + kOffBars);
     uint32_t *misc = reinterpret_cast<uint32_t *>(smem + kOffMisc);
 
+    load_tables(smem, p, tid, kTcThreads);   // the caller's: needs nothing of the plan kernel
+    wait_for_previous_kernel();
+    // From here on the plan is complete, so the per-sequence kernel may take over every SM this kernel leaves.
+    allow_dependent_launch();
     PlanHeader *hdr = plan_header(p);
     // uniform: nothing shared, the plan refused the hint, or the split leaves this CTA without a share
     if (hdr->shared_pages == 0 || blockIdx.x >= hdr->shared_ctas) return;
 
-    load_tables(smem, p, tid, kTcThreads);
     if (tid == 0) {
         for (uint32_t w = 0; w < kDecodeWarps; ++w) mbar_init(bars + w, 1);   // copies
         mbar_init(bars + kBarFull, kRoundPages);                    // full[0], full[1]: one arrival per page slot of the round
@@ -773,7 +776,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) prefix_attention_kernel(Attenti
 
 }  // namespace
 
-cudaError_t launch_prefix_attention(const AttentionParams &p, cudaStream_t stream) {
+cudaError_t launch_prefix_attention(const AttentionParams &p, cudaStream_t stream, bool dependent) {
     static LauncherState table[64];
     cudaError_t e;
     LauncherState *state = launcher_state(table, &e);
@@ -792,9 +795,8 @@ cudaError_t launch_prefix_attention(const AttentionParams &p, cudaStream_t strea
         }
         state->configured = true;
     }
-    if (p.query_type == CF_B200_F32) prefix_attention_kernel<true><<<sm_count, kTcThreads, kTcSmem, stream>>>(p);
-    else prefix_attention_kernel<false><<<sm_count, kTcThreads, kTcSmem, stream>>>(p);
-    return cudaPeekAtLastError();
+    return launch_kernel(p.query_type == CF_B200_F32 ? prefix_attention_kernel<true> : prefix_attention_kernel<false>, sm_count, kTcThreads,
+                         kTcSmem, stream, dependent, p);
 }
 
 }  // namespace cfb
