@@ -101,13 +101,15 @@ flat_rans_decode_kernel(const uint8_t *data, const int32_t *byte_off, const uint
         b.open(mine + kPartBytes, kPartBytes, lane, table);
 #pragma unroll 4
         for (uint32_t q = 0; q < 16; ++q) {
-            a.reload();
-            b.reload();
             uint32_t ea[4], eb[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                ea[i] = a.symbol();
-                eb[i] = b.symbol();
+                ea[i] = a.symbol(i & 1);
+                eb[i] = b.symbol(i & 1);
+                if (i & 1) {
+                    a.advance();
+                    b.advance();
+                }
             }
             tile[lane * kTileWords + q] = pack_low_bytes(ea[0], ea[1], ea[2], ea[3]);
             tile[(32u + lane) * kTileWords + q] = pack_low_bytes(eb[0], eb[1], eb[2], eb[3]);

@@ -84,58 +84,81 @@ __device__ __forceinline__ uint32_t pack_low_bytes(uint32_t e0, uint32_t e1, uin
     return __byte_perm(__byte_perm(e0, e1, 0x0040), __byte_perm(e2, e3, 0x0040), 0x5410);
 }
 
+__device__ __forceinline__ uint32_t lds_u32(uint32_t address) {
+    uint32_t w;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w) : "r"(address));
+    return w;
+}
+
 // ---- per-lane block decoders: each yields four symbols packed in one register -----------------------------------
-// Both entropy decoders are written without branches so that the K chain and the V chain of a lane interleave in
-// one straight instruction stream. A 64-bit window holds the upcoming stream bits, top aligned; it is reloaded from
-// shared memory once per quad (four symbols), which is as often as it can run dry.
+// The entropy decoders are written without branches so that the K chain and the V chain of a lane interleave in one straight
+// instruction stream. What bounds them is spread over four pipes, so each was shortened on all of them: a step reads its table
+// once (32 unrelated addresses: 3.5 shared-memory wavefronts, which nothing avoids); the stream's next two words sit in
+// registers and are looked at where they are (one byte permute or funnel shift) instead of being shifted along; and every
+// second step a word is fetched by just those lanes that have used one up, on average a third of them, where all lanes used
+// to fetch three words every fourth step.
+// advance() has to be called after every second symbol().
 template <int NB>
 struct RansLaneT {
     static constexpr bool kWholeQuads = false;
     static constexpr uint32_t kHead = (6u * NB + 3u) / 4u * 4u;   // u32 state0[NB] | u16 byte_off[NB]
-    static constexpr int kSymbolsPerReload = 4;   // a symbol takes at most two bytes; the window holds eight
-    uint32_t x, whi, wlo, used;   // state; window (next byte = top byte of whi); bits taken since the reload
-    uint32_t pos;                 // shared-memory byte address of the first byte not yet taken at the last reload
-    uint32_t table;               // shared-memory byte address of the slot table
+    uint32_t x, w0, w1;   // state; the stream word that holds the next byte, and the one after it
+    uint32_t sel;         // byte-permute selector: the next three bytes, first on top (bytes counted from w0's first)
+    uint32_t next;        // shared-memory byte address of the word after w1
+    uint32_t table;       // shared-memory byte address of the slot table
     // The block's start offset is clamped to the part (part_bytes from the record header): whatever the block table
-    // says, the decoder starts inside its own part, and from there a block takes at most 64 * 2 bytes plus one
-    // 12-byte window, which stays inside the warp's own shared memory (part_offsets_ok reports the bad table).
+    // says, the decoder starts inside its own part, and from there a block takes at most 64 * 2 bytes plus two
+    // words, which stays inside the warp's own shared memory (part_offsets_ok reports the bad table).
+    __device__ __forceinline__ void open_at(uint32_t pos, const uint32_t *slot_table) {
+        const uint32_t base = pos & ~3u;
+        w0 = lds_u32(base);
+        w1 = lds_u32(base + 4u);
+        next = base + 8u;
+        sel = (pos & 3u) * 0x1110u + 0x0120u;
+        table = smem_addr(slot_table);
+    }
     __device__ __forceinline__ void open(const uint8_t *part, uint32_t part_bytes, uint32_t lane, const uint32_t *slot_table) {
         x = reinterpret_cast<const uint32_t *>(part)[lane];
         const uint32_t payload = part_bytes > kHead ? part_bytes - kHead : 0u;
-        pos = smem_addr(part) + kHead + min(static_cast<uint32_t>(reinterpret_cast<const uint16_t *>(part + 4 * NB)[lane]), payload);
-        table = smem_addr(slot_table);
-        used = 0;
-    }
-    // Eight bytes starting at `pos`, in stream order, most significant first (the order rans.cu:23 shifts them in).
-    __device__ __forceinline__ void reload() {
-        pos += used >> 3;
-        used = 0;
-        const uint32_t base = pos & ~3u, align = imad(pos & 3u, 0x1111u, 0x0123u);
-        uint32_t w0, w1, w2;
-        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w0) : "r"(base));
-        asm volatile("ld.shared.u32 %0, [%1+4];" : "=r"(w1) : "r"(base));
-        asm volatile("ld.shared.u32 %0, [%1+8];" : "=r"(w2) : "r"(base));
-        whi = __byte_perm(w0, w1, align);
-        wlo = __byte_perm(w1, w2, align);
+        open_at(smem_addr(part) + kHead + min(static_cast<uint32_t>(reinterpret_cast<const uint16_t *>(part + 4 * NB)[lane]), payload), slot_table);
     }
     // src/cuda/rans.cu:20-23: x = freq * (x >> 12) + (x & 4095) - cum, then bytes are shifted in while x < 2^23.
     // The shared-memory table holds e = sym | (slot - cum) << 8 | freq << 20, so e >> 8 = (slot - cum) + freq * 4096
     // and the update is freq * ((x >> 12) - 4096) + (e >> 8): no field of the entry needs masking.
-    // After the update the state is >= 2^11, so the reference's loop runs 0, 1 or 2 times: (clz(state) - 1) / 8.
-    __device__ __forceinline__ uint32_t symbol() {
+    // After the update the state is >= 2^11, so the reference's loop runs 0, 1 or 2 times: (clz(state) - 1) / 8; the lowest
+    // byte of the permuted word is never looked at, so the selector is kept in units that make its step a multiple of 8.
+    __device__ __forceinline__ uint32_t symbol(int) {
         uint32_t e;
         asm volatile("ld.shared.u32 %0, [%1];" : "=r"(e) : "r"(imad(x & (CF_B200_RANS_M - 1u), 4u, table)));
+#ifdef CFB_RANS_MADHI
+        uint32_t t;
+        asm("mad.hi.u32 %0, %1, %2, %3;" : "=r"(t) : "r"(x), "r"(1u << (32 - CF_B200_RANS_PROB_BITS)), "r"(0u - CF_B200_RANS_M));
+        x = imad(e >> 20, t, e >> 8);
+#else
         x = imad(e >> 20, imad(x >> CF_B200_RANS_PROB_BITS, 1u, 0u - CF_B200_RANS_M), e >> 8);
+#endif
         const uint32_t shift = imad(static_cast<uint32_t>(__clz(x)), 1u, 0xffffffffu) & 24u;
-        x = __funnelshift_l(whi, x, shift);
-        whi = __funnelshift_l(wlo, whi, shift);
-        wlo <<= shift;
-        used = imad(shift, 1u, used);
+        x = __funnelshift_l(__byte_perm(w0, w1, sel), x, shift);
+        sel = imad(shift, 0x1110u / 8u, sel);
         return e;
     }
+    // At most three bytes of w0 were used before two symbols, so at most seven of the eight are now: every byte a step looks
+    // at was in w0 or w1.
+    __device__ __forceinline__ void advance() {
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t.reg .u32 t;\n\t"
+            "and.b32 t, %3, 0x4000;\n\tsetp.ne.u32 p, t, 0;\n\t"
+            "@p mov.u32 %0, %1;\n\t"
+            "@p ld.shared.u32 %1, [%2];\n\t"
+            "@p mad.lo.u32 %2, %2, 1, 4;\n\t"
+            "@p mad.lo.u32 %3, %3, 1, 0xffffbbc0;\n\t}"
+            : "+r"(w0), "+r"(w1), "+r"(next), "+r"(sel));
+    }
     __device__ __forceinline__ uint32_t quad(int) {   // quad index: the decoders that need it get it from an unrolled loop
-        reload();
-        const uint32_t e0 = symbol(), e1 = symbol(), e2 = symbol(), e3 = symbol();
+        const uint32_t e0 = symbol(0), e1 = symbol(1);
+        advance();
+        const uint32_t e2 = symbol(0), e3 = symbol(1);
+        advance();
         return pack_low_bytes(e0, e1, e2, e3);
     }
 };
@@ -158,7 +181,7 @@ __device__ __forceinline__ uint32_t merge_split_quad(uint32_t e0, uint32_t e1, u
 template <int NB, int kSyms = 2048>
 struct RansSplitLaneT : RansLaneT<NB> {
     using Base = RansLaneT<NB>;
-    using Base::x; using Base::pos; using Base::table; using Base::used; using Base::kHead;
+    using Base::x; using Base::kHead;
     static constexpr bool kWholeQuads = true;   // callers ask for a quad at a time (the window is refilled inside)
     static constexpr uint32_t kPlaneBytes = kSyms / 2u;   // a nibble per symbol
     uint32_t lo;   // shared-memory byte address of lo[0][lane]
@@ -166,18 +189,12 @@ struct RansSplitLaneT : RansLaneT<NB> {
         x = reinterpret_cast<const uint32_t *>(part)[lane];
         const uint32_t payload = part_bytes > kHead + kPlaneBytes ? part_bytes - kHead - kPlaneBytes : 0u;
         lo = smem_addr(part) + kHead + 4u * lane;
-        pos = smem_addr(part) + kHead + kPlaneBytes + min(static_cast<uint32_t>(reinterpret_cast<const uint16_t *>(part + 4 * NB)[lane]), payload);
-        table = smem_addr(slot_table);
-        used = 0;
+        Base::open_at(smem_addr(part) + kHead + kPlaneBytes + min(static_cast<uint32_t>(reinterpret_cast<const uint16_t *>(part + 4 * NB)[lane]), payload), slot_table);
     }
-    __device__ __forceinline__ uint32_t lo_word(int j) const {
-        uint32_t w;
-        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w) : "r"(lo + 4u * NB * j));
-        return w;
-    }
+    __device__ __forceinline__ uint32_t lo_word(int j) const { return lds_u32(lo + 4u * NB * j); }
     __device__ __forceinline__ uint32_t quad(int q) {   // one stream on its own (mixed-coder records)
-        if ((q & 1) == 0) Base::reload();
-        const uint32_t e0 = Base::symbol(), e1 = Base::symbol();
+        const uint32_t e0 = Base::symbol(0), e1 = Base::symbol(1);
+        Base::advance();
         return merge_split_quad(e0, e1, lo_word(q >> 1) >> (4 * (q & 1)));
     }
 };
@@ -187,42 +204,49 @@ template <int NB>
 struct HuffLaneT {
     static constexpr bool kWholeQuads = false;
     static constexpr uint32_t kHead = (2u * NB + 3u) / 4u * 4u;   // u16 bit_off[NB]
-    static constexpr int kSymbolsPerReload = 5;   // a code takes at most 12 bits; the window holds 64
-    uint32_t whi, wlo, used;   // window of upcoming bits, MSB first; bits taken since the reload
-    uint32_t words, bit;       // shared-memory address of the payload words; bit position at the last reload
+    uint32_t w0, w1, off;   // the stream word that holds the next bit, the one after it, bits of w0 used
+    uint32_t view;          // the next bits, top aligned: 32 of them at an even symbol, what it left of them at the odd one
+    uint32_t next;          // shared-memory byte address of the word after w1
     uint32_t table;
-    // Start offset clamped to the part as in RansLane::open; a block takes at most 64 * 12 bits plus one window.
+    // Start offset clamped to the part as in RansLane::open; a block takes at most a word per two codes, and two words.
+    __device__ __forceinline__ void open_at(uint32_t words, uint32_t bit, const uint16_t *lut) {
+        const uint32_t base = words + ((bit >> 5) << 2);
+        off = bit & 31u;
+        w0 = lds_u32(base);
+        w1 = lds_u32(base + 4u);
+        next = base + 8u;
+        table = smem_addr(lut);
+    }
     __device__ __forceinline__ void open(const uint8_t *part, uint32_t part_bytes, uint32_t lane, const uint16_t *lut) {
         const uint32_t payload_bits = part_bytes > kHead ? (part_bytes - kHead) * 8u : 0u;
-        bit = min(static_cast<uint32_t>(reinterpret_cast<const uint16_t *>(part)[lane]), payload_bits);
-        words = smem_addr(part) + kHead;
-        table = smem_addr(lut);
-        used = 0;
+        open_at(smem_addr(part) + kHead, min(static_cast<uint32_t>(reinterpret_cast<const uint16_t *>(part)[lane]), payload_bits), lut);
     }
-    __device__ __forceinline__ void reload() {
-        bit += used;
-        used = 0;
-        const uint32_t base = words + ((bit >> 5) << 2), off = bit & 31u;
-        uint32_t w0, w1, w2;
-        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w0) : "r"(base));
-        asm volatile("ld.shared.u32 %0, [%1+4];" : "=r"(w1) : "r"(base));
-        asm volatile("ld.shared.u32 %0, [%1+8];" : "=r"(w2) : "r"(base));
-        whi = __funnelshift_l(w1, w0, off);
-        wlo = __funnelshift_l(w2, w1, off);
-    }
-    // include/chromofold/detail/block_huffman_device.cuh:12-19: the next 12 bits, MSB-first, index the LUT.
-    __device__ __forceinline__ uint32_t symbol() {
+    // include/chromofold/detail/block_huffman_device.cuh:12-19: the next 12 bits, MSB-first, index the LUT. A code takes at
+    // most 12 bits, so 32 bits serve two of them.
+    __device__ __forceinline__ uint32_t symbol(int odd) {
+        if (!odd) view = __funnelshift_l(w1, w0, off);
         uint32_t e;
-        asm volatile("ld.shared.u16 %0, [%1];" : "=r"(e) : "r"(imad(whi >> (32u - CF_B200_HUFF_MAXLEN), 2u, table)));
+        asm volatile("ld.shared.u16 %0, [%1];" : "=r"(e) : "r"(imad(view >> (32u - CF_B200_HUFF_MAXLEN), 2u, table)));
         const uint32_t len = e >> 8;
-        whi = __funnelshift_l(wlo, whi, len);
-        wlo <<= len;
-        used = imad(len, 1u, used);
+        if (!odd) view <<= len;
+        off = imad(len, 1u, off);
         return e;
     }
+    __device__ __forceinline__ void advance() {
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "setp.ge.u32 p, %3, 32;\n\t"
+            "@p mov.u32 %0, %1;\n\t"
+            "@p ld.shared.u32 %1, [%2];\n\t"
+            "@p mad.lo.u32 %2, %2, 1, 4;\n\t"
+            "@p mad.lo.u32 %3, %3, 1, 0xffffffe0;\n\t}"
+            : "+r"(w0), "+r"(w1), "+r"(next), "+r"(off));
+    }
     __device__ __forceinline__ uint32_t quad(int) {
-        reload();
-        const uint32_t e0 = symbol(), e1 = symbol(), e2 = symbol(), e3 = symbol();
+        const uint32_t e0 = symbol(0), e1 = symbol(1);
+        advance();
+        const uint32_t e2 = symbol(0), e3 = symbol(1);
+        advance();
         return pack_low_bytes(e0, e1, e2, e3);
     }
 };
@@ -232,26 +256,19 @@ using HuffLane = HuffLaneT<32>;
 template <int NB, int kSyms = 2048>
 struct HuffSplitLaneT : HuffLaneT<NB> {
     using Base = HuffLaneT<NB>;
-    using Base::bit; using Base::words; using Base::table; using Base::used; using Base::kHead;
+    using Base::kHead;
     static constexpr bool kWholeQuads = true;
     static constexpr uint32_t kPlaneBytes = kSyms / 2u;   // a nibble per symbol
     uint32_t lo;
     __device__ __forceinline__ void open(const uint8_t *part, uint32_t part_bytes, uint32_t lane, const uint16_t *lut) {
         const uint32_t payload_bits = part_bytes > kHead + kPlaneBytes ? (part_bytes - kHead - kPlaneBytes) * 8u : 0u;
-        bit = min(static_cast<uint32_t>(reinterpret_cast<const uint16_t *>(part)[lane]), payload_bits);
         lo = smem_addr(part) + kHead + 4u * lane;
-        words = smem_addr(part) + kHead + kPlaneBytes;
-        table = smem_addr(lut);
-        used = 0;
+        Base::open_at(smem_addr(part) + kHead + kPlaneBytes, min(static_cast<uint32_t>(reinterpret_cast<const uint16_t *>(part)[lane]), payload_bits), lut);
     }
-    __device__ __forceinline__ uint32_t lo_word(int j) const {
-        uint32_t w;
-        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w) : "r"(lo + 4u * NB * j));
-        return w;
-    }
+    __device__ __forceinline__ uint32_t lo_word(int j) const { return lds_u32(lo + 4u * NB * j); }
     __device__ __forceinline__ uint32_t quad(int q) {
-        if ((q & 1) == 0) Base::reload();   // four pair symbols take at most 48 bits
-        const uint32_t e0 = Base::symbol(), e1 = Base::symbol();
+        const uint32_t e0 = Base::symbol(0), e1 = Base::symbol(1);
+        Base::advance();
         return merge_split_quad(e0, e1, lo_word(q >> 1) >> (4 * (q & 1)));
     }
 };
@@ -260,7 +277,6 @@ using HuffSplitLane = HuffSplitLaneT<32>;
 template <int NB, int kSyms = 2048>
 struct FixedLaneT {
     static constexpr bool kWholeQuads = true;  // a quad is one word: nothing to interleave
-    static constexpr int kSymbolsPerReload = 4;
     const uint32_t *words;
     // A fixed-width part is kSyms bytes at a 16-byte aligned offset of at most 16 + 2048 into the stage: always inside it.
     __device__ __forceinline__ void open(const uint8_t *part, uint32_t, uint32_t lane) {

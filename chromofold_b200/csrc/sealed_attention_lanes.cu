@@ -24,7 +24,6 @@
 #include <math_constants.h>
 
 #include <atomic>
-#include <type_traits>
 
 #include "lanes_decoders.cuh"
 
@@ -34,20 +33,23 @@ namespace {
 using namespace lanes;
 
 #ifndef CFB_LANES_WARPS
-#define CFB_LANES_WARPS 16
+#define CFB_LANES_WARPS 24
 #endif
 #ifndef CFB_LANES_WARPS2
 #define CFB_LANES_WARPS2 16
 #endif
-// Warps per CTA (one CTA per SM): the four-head kernel and the kernels whose query rows live in shared memory (they
-// need 2.3 KB more per warp) are sized separately.
-// The kernels for larger blocks (NB = 16 or 8 blocks per stream) keep a 5 KB symbol tile per warp instead of a second
-// record stage: a record is free for the next copy as soon as it has been decoded into the tile.
+#ifndef CFB_LANES_WARPSQ
+#define CFB_LANES_WARPSQ 24
+#endif
 #ifndef CFB_LANES_WARPS_BIG
 #define CFB_LANES_WARPS_BIG 16
 #endif
-template <int NG, int NB = 32> constexpr int kWarpsOf = NB != 32 ? (NG == 1 ? CFB_LANES_WARPS_BIG : 14) : NG == 1 ? CFB_LANES_WARPS : CFB_LANES_WARPS2;
-template <int NG, int NB = 32> constexpr int kThreadsOf = kWarpsOf<NG, NB> * 32;
+#ifndef CFB_LANES_WARPS_BIG2
+#define CFB_LANES_WARPS_BIG2 14
+#endif
+template <int NG, int NB = 32, bool kSplitQ = false> constexpr int kWarpsOf = NB != 32 ? (NG == 1 ? CFB_LANES_WARPS_BIG : CFB_LANES_WARPS_BIG2)
+                                                                              : kSplitQ ? CFB_LANES_WARPSQ : NG == 1 ? CFB_LANES_WARPS : CFB_LANES_WARPS2;
+template <int NG, int NB = 32, bool kSplitQ = false> constexpr int kThreadsOf = kWarpsOf<NG, NB, kSplitQ> * 32;
 // Per-warp running state of one unit; NG = number of four-head query groups served by one decode pass.
 // kDim = head_dim: a lane holds kDim / 8 quads of each stream (K: kDim / 2 channels of one token; V: kDim / 32 channels,
 // every token).
@@ -67,21 +69,10 @@ constexpr int kAttend = 0, kFold = 1, kDump = 2;
 constexpr float kWeightScale = 32768.0f;
 
 // Where a lane finds its B fragments of S = K * Q^T (column n = parity*4 + head; zero where the lane's slice of the
-// contraction belongs to the other token of the pair).
-//   QRegs: held in registers, one group of four heads.
-//   QSmem: the query rows of up to eight heads sit in the warp's shared memory as [head][half][64 channels] with a
-//   row stride of 36 words, which puts the eight rows one load touches into different banks; a lane reads two words
-//   of row (head g&3 of the group, half t&1), or of a zero row when the column is not its own.
-template <int kQuads>
-struct QRegsT {
-    uint32_t bq[kQuads][2];
-    template <int GRP>
-    __device__ __forceinline__ void get(int q, uint32_t &b0, uint32_t &b1) const {
-        b0 = bq[q][0];
-        b1 = bq[q][1];
-    }
-};
-using QRegs = QRegsT<16>;
+// contraction belongs to the other token of the pair): the query rows of up to eight heads sit in the warp's shared memory as
+// [head][half][64 channels] with a row stride of 36 words, which puts the eight rows one load touches into different banks; a
+// lane reads two words of row (head g&3 of the group, half t&1), or of a zero row when the column is not its own. (Held in
+// registers instead, a group of four heads took 32 of them, and with that room for eight warps more per SM.)
 struct QSmem {
     uint32_t addr, group_stride;  // byte address of the lane's row for group 0; distance to the row for group 1 (0 on the zero row)
     template <int GRP>
@@ -121,15 +112,16 @@ __device__ __forceinline__ void decode_fused(KLane &k, VLane &v, UnitState<NG> &
             }
         }
     } else {
-        // two independent decoder chains, interleaved symbol by symbol; each window is refilled as rarely as its
-        // coder's worst case allows, four symbols make one packed register
+        // two independent decoder chains, interleaved symbol by symbol; four symbols make one packed register
         uint32_t ke[4], ve[4];
 #pragma unroll
         for (int i = 0; i < 64; ++i) {
-            if (i % KLane::kSymbolsPerReload == 0) k.reload();
-            if (i % VLane::kSymbolsPerReload == 0) v.reload();
-            ke[i & 3] = k.symbol();
-            ve[i & 3] = v.symbol();
+            ke[i & 3] = k.symbol(i & 1);
+            ve[i & 3] = v.symbol(i & 1);
+            if (i & 1) {
+                k.advance();
+                v.advance();
+            }
             if ((i & 3) == 3) {
                 if constexpr (kMode == kFold) {
                     u.vq[0] ^= pack_low_bytes(ve[0], ve[1], ve[2], ve[3]) ^ pack_low_bytes(ke[0], ke[1], ke[2], ke[3]);
@@ -151,13 +143,11 @@ __device__ __forceinline__ void decode_fused_split(Lane &k, Lane &v, UnitState<N
     uint32_t ke[2], ve[2], kw = 0u, vw = 0u;
 #pragma unroll
     for (int i = 0; i < 32; ++i) {
-        if (i % 4 == 0) {
-            k.reload();
-            v.reload();
-        }
-        ke[i & 1] = k.symbol();
-        ve[i & 1] = v.symbol();
+        ke[i & 1] = k.symbol(i & 1);
+        ve[i & 1] = v.symbol(i & 1);
         if (i & 1) {
+            k.advance();
+            v.advance();
             const int q = i >> 1;
             if ((q & 1) == 0) {
                 kw = k.lo_word(q >> 1);
@@ -260,38 +250,39 @@ __device__ __forceinline__ void stage_blocks(const uint8_t *part, uint32_t part_
     }
 }
 
-// Shared memory of one warp: two record stages, the softmax scratch, two mbarriers and (NG = 2) the query rows.
-//   scratch: P rows fp16 high halves [4 NG][16] | low halves [4 NG][16] | 128 zero bytes | alpha[4 NG]
-template <int NG, int NB = 32>
+// Shared memory of one warp: one record, the softmax scratch, an mbarrier and the query rows. A record is decoded before anything
+// else happens to its page, so its place is free for the next one while the scores and weights are worked out; a second place
+// would cost eight warps per SM.
+//   scratch: P rows fp16 high halves [4 NG][16] | low halves [4 NG][16] | 128 zero bytes
+template <int NG, int NB = 32, bool kSplitQ = false>
 struct WarpLayout {
-    static constexpr uint32_t kPBytes = 4 * NG * 16 * 2;
-    static constexpr uint32_t kStages = NB == 32 ? 2 : 1;
-    static constexpr uint32_t kPLo = kStages * kStageBytes + kPBytes;
+    static constexpr uint32_t kPRows = kStageBytes;
+    static constexpr uint32_t kPBytes = (kSplitQ ? 4 : 4 * NG) * 16 * 2;
+    static constexpr uint32_t kPLo = kPRows + kPBytes;
     static constexpr uint32_t kZero = kPLo + kPBytes;
-    static constexpr uint32_t kAlpha = kZero + 128;
-    static constexpr uint32_t kBars = kAlpha + 4 * NG * 4;
-    static constexpr uint32_t kQRows = kBars + 32;
+    static constexpr uint32_t kBar = kZero + 128;
+    static constexpr uint32_t kQRows = kBar + 16;
     static constexpr uint32_t kQRowWords = 36;
-    static constexpr uint32_t kTile = (kQRows + (NG == 2 ? 16 * kQRowWords * 4 : 0) + 15u) / 16u * 16u;   // NB != 32 only
+    static constexpr uint32_t kTile = (kQRows + 8 * NG * kQRowWords * 4 + 15u) / 16u * 16u;   // NB != 32 only
     static constexpr uint32_t kBytes = kTile + (NB != 32 ? kTileBytes : 0u);
-    static constexpr uint32_t kSmem = kTableBytes + kWarpsOf<NG, NB> * kBytes;
+    static constexpr uint32_t kSmem = kTableBytes + kWarpsOf<NG, NB, kSplitQ> * kBytes;
 };
-static_assert(WarpLayout<1>::kSmem <= 232448 && WarpLayout<2>::kSmem <= 232448 && WarpLayout<1, 16>::kSmem <= 232448 &&
-              WarpLayout<2, 16>::kSmem <= 232448, "a CTA has 227 KB of shared memory");
+static_assert(WarpLayout<1>::kSmem <= 232448 && WarpLayout<2>::kSmem <= 232448 && WarpLayout<2, 32, true>::kSmem <= 232448 &&
+              WarpLayout<1, 16>::kSmem <= 232448 && WarpLayout<2, 16>::kSmem <= 232448 && WarpLayout<2, 16, true>::kSmem <= 232448,
+              "a CTA has 227 KB of shared memory");
 
 // kSplitQ (with NG = 2): the queries are fp32. A pass serves four heads; their rows are split into binary16(q) and
 // binary16(q - binary16(q)), stored as the rows of group 0 and group 1, the two score fragments are added, and one
 // softmax / P V follows: the scores equal fp32-query scores to 2^-22 relative, at the cost of a second score mma.
 template <int NG, int kMode = kAttend, bool kSplitQ = false, int NB = 32, int kDim = 128>
-__global__ void __launch_bounds__(kThreadsOf<NG, NB>, 1) lanes_attention_kernel(AttentionParams p, uint32_t after_prefix) {
+__global__ void __launch_bounds__(kThreadsOf<NG, NB, kSplitQ>, 1) lanes_attention_kernel(AttentionParams p, uint32_t after_prefix) {
     constexpr bool kProbe = kMode != kAttend;
     static_assert(!kSplitQ || NG == 2, "split queries use the two-group query layout");
     static_assert(NB == 32 || NB == 24 || NB == 16 || NB == 12 || NB == 8 || NB == 4, "blocks per stream");
     static_assert(kDim == 128 || ((kDim == 96 || kDim == 64 || kDim == 32) && NB != 32), "other head_dims go through the staging tile");
     constexpr int kQ = kDim / 8, kVCh = kDim / 32, kSyms = 16 * kDim;   // quads per lane and stream; V channels per lane
     constexpr uint32_t kRowWords = kDim / 4;   // words of half a query row (the channels one lane's K block covers)
-    using L = WarpLayout<NG, NB>;
-    using QSrc = typename std::conditional<NG == 1, QRegsT<kQ>, QSmem>::type;
+    using L = WarpLayout<NG, NB, kSplitQ>;
     constexpr uint32_t kPassHeads = kSplitQ ? 4u : 4u * NG;
     constexpr int NS = kSplitQ ? 1 : NG;   // groups that go through softmax and P V
     extern __shared__ __align__(128) uint8_t smem[];
@@ -302,18 +293,16 @@ __global__ void __launch_bounds__(kThreadsOf<NG, NB>, 1) lanes_attention_kernel(
 
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     uint8_t *warp_mem = smem + kTableBytes + warp * L::kBytes;
-    __half *p_rows = reinterpret_cast<__half *>(warp_mem + L::kStages * kStageBytes);   // [4 NG][16] fp16(p)
-    __half *p_rows_lo = reinterpret_cast<__half *>(warp_mem + L::kPLo);        // [4 NG][16] fp16(p - fp16(p))
+    __half *p_rows = reinterpret_cast<__half *>(warp_mem + L::kPRows);         // [4 NS][16] fp16(p)
+    __half *p_rows_lo = reinterpret_cast<__half *>(warp_mem + L::kPLo);        // [4 NS][16] fp16(p - fp16(p))
     const __half *zero_row = reinterpret_cast<const __half *>(warp_mem + L::kZero);
-    float *alpha_s = reinterpret_cast<float *>(warp_mem + L::kAlpha);          // [4 NG]
-    uint64_t *bars = reinterpret_cast<uint64_t *>(warp_mem + L::kBars);
-    uint32_t *q_rows = reinterpret_cast<uint32_t *>(warp_mem + L::kQRows);     // NG == 2 only
+    uint64_t *bar = reinterpret_cast<uint64_t *>(warp_mem + L::kBar);
+    uint32_t *q_rows = reinterpret_cast<uint32_t *>(warp_mem + L::kQRows);
 
-    load_tables(smem, p, tid, kThreadsOf<NG, NB>);   // coding tables: once per CTA
+    load_tables(smem, p, tid, kThreadsOf<NG, NB, kSplitQ>);   // coding tables: once per CTA
     reinterpret_cast<uint32_t *>(warp_mem + L::kZero)[lane] = 0u;   // the zero row inactive lanes read their fragments from
     if (lane == 0) {
-        mbar_init(&bars[0], 1);
-        mbar_init(&bars[1], 1);
+        mbar_init(bar, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
@@ -324,7 +313,7 @@ __global__ void __launch_bounds__(kThreadsOf<NG, NB>, 1) lanes_attention_kernel(
     allow_dependent_launch();
     const uint32_t subgroups = (p.group + kPassHeads - 1u) / kPassHeads;   // 4 NG query heads per pass
     const uint32_t g = lane >> 2, t = lane & 3u;
-    uint32_t phase_bits = 0u;  // bit s: parity the next wait on stage s expects
+    uint32_t phase = 0u;   // parity the next wait on the record's barrier expects
 
     // fixed lane roles
     const uint32_t q_head_of_col = g & 3u;                 // S columns: n = parity*4 + head
@@ -344,7 +333,7 @@ __global__ void __launch_bounds__(kThreadsOf<NG, NB>, 1) lanes_attention_kernel(
         uint32_t partial, page_begin, n_pages, slot, sealed, qpos, q_row, sub, head_local;
         {
             const PageLine line = plan_line(p);
-            const uint32_t unit_lanes = p.kv_head_span * subgroups, unit_count = line.stretches * unit_lanes, warps = kWarpsOf<NG, NB> * gridDim.x;
+            const uint32_t unit_lanes = p.kv_head_span * subgroups, unit_count = line.stretches * unit_lanes, warps = kWarpsOf<NG, NB, kSplitQ> * gridDim.x;
             uint32_t stretch = unit / unit_lanes;
             if (x != 0u && x == line.begin(stretch + 1u)) {   // the unit is done
                 if (unit_count <= warps) break;
@@ -372,20 +361,8 @@ __global__ void __launch_bounds__(kThreadsOf<NG, NB>, 1) lanes_attention_kernel(
         const uint32_t first_token = window_begin(qpos, p.causal_window);
         const uint32_t *table_row = p.page_table + static_cast<uint64_t>(slot) * p.page_table_stride;
 
-        QSrc qs;
-        if constexpr (NG == 1) {
-            const bool live = q_col_mine && q_head_of_col < G;
-            const __half *qrow = reinterpret_cast<const __half *>(p.queries) +
-                                 (static_cast<uint64_t>(q_row) * p.query_head_count + q_head_base + q_head_of_col) * kDim +
-                                 (kDim / 2) * (t & 1u);
-#pragma unroll
-            for (int s = 0; s < kQ; ++s) {
-                uint2 v = make_uint2(0u, 0u);
-                if (live) v = *reinterpret_cast<const uint2 *>(qrow + 4 * s);
-                qs.bq[s][0] = v.x;
-                qs.bq[s][1] = v.y;
-            }
-        } else if constexpr (kSplitQ) {
+        QSmem qs;
+        if constexpr (kSplitQ) {
             const float2 *qsrc = reinterpret_cast<const float2 *>(
                 reinterpret_cast<const float *>(p.queries) + (static_cast<uint64_t>(q_row) * p.query_head_count + q_head_base) * kDim);
             __syncwarp();  // the previous run's readers are done
@@ -400,21 +377,19 @@ __global__ void __launch_bounds__(kThreadsOf<NG, NB>, 1) lanes_attention_kernel(
                 q_rows[(i / kRowWords + 8u) * L::kQRowWords + i % kRowWords] = *reinterpret_cast<const uint32_t *>(&lo);
             }
             __syncwarp();
-            qs.addr = q_col_mine ? smem_addr(q_rows + (q_head_of_col * 2u + (t & 1u)) * L::kQRowWords) : smem_addr(zero_row);
-            qs.group_stride = q_col_mine ? 8u * L::kQRowWords * 4u : 0u;
         } else {
             const uint32_t *qsrc = reinterpret_cast<const uint32_t *>(
                 reinterpret_cast<const __half *>(p.queries) + (static_cast<uint64_t>(q_row) * p.query_head_count + q_head_base) * kDim);
             __syncwarp();  // the previous run's readers are done
 #pragma unroll
-            for (int j = 0; j < kDim / 8; ++j) {   // 8 heads x kDim / 2 words; row = head*2 + half
+            for (int j = 0; j < NG * kDim / 16; ++j) {   // 4 NG heads x kDim / 2 words; row = head*2 + half
                 const uint32_t i = lane + 32u * j, head = i / (2u * kRowWords);
                 q_rows[(i / kRowWords) * L::kQRowWords + i % kRowWords] = head < G ? qsrc[i] : 0u;
             }
-            __syncwarp();
-            qs.addr = q_col_mine ? smem_addr(q_rows + (q_head_of_col * 2u + (t & 1u)) * L::kQRowWords) : smem_addr(zero_row);
-            qs.group_stride = q_col_mine ? 8u * L::kQRowWords * 4u : 0u;
         }
+        __syncwarp();
+        qs.addr = q_col_mine ? smem_addr(q_rows + (q_head_of_col * 2u + (t & 1u)) * L::kQRowWords) : smem_addr(zero_row);
+        qs.group_stride = q_col_mine ? 8u * L::kQRowWords * 4u : 0u;
 
         UnitState<NG, kDim> u;
         if constexpr (kProbe) u.vq[0] = 0u;
@@ -428,7 +403,9 @@ __global__ void __launch_bounds__(kThreadsOf<NG, NB>, 1) lanes_attention_kernel(
             u.m0[n] = u.m1[n] = -CUDART_INF_F;
             u.l0[n] = u.l1[n] = 0.0f;
         }
-        float v_scale_prev = 1.0f;
+        // O is kept in units of a power of two at or above every V scale met so far; a page's scale relative to it rides on the
+        // weights, together with kWeightScale. v_gain = kWeightScale / unit.
+        float v_unit = 0x1p-25f, v_gain = kWeightScale * 0x1p25f;
 
         // bit 63 of an entry (reserved, 0 in the directory) marks the page of the wait-expiry test: armed, never fetched
         auto load_entry = [&](uint32_t page) -> uint64_t {
@@ -436,12 +413,11 @@ __global__ void __launch_bounds__(kThreadsOf<NG, NB>, 1) lanes_attention_kernel(
             const uint64_t entry = p.page_dir[static_cast<uint64_t>(page_id) * p.kv_head_count + kv_head];
             return page_id == p.skip_copy_page ? entry | (1ull << 63) : entry;
         };
-        auto issue = [&](uint32_t st, uint64_t entry) {
+        auto issue = [&](uint64_t entry) {
             const uint32_t units16 = static_cast<uint32_t>(CF_B200_DIR_LENGTH_UNITS(entry));
             if (lane == 0 && units16 != 0 && units16 * 16u <= kStageBytes - 32u) {
-                mbar_expect_tx(&bars[st], units16 * 16u);
-                if (!(entry >> 63))
-                    bulk_load(warp_mem + st * kStageBytes, p.arena + 16ull * CF_B200_DIR_OFFSET_UNITS(entry), units16 * 16u, &bars[st]);
+                mbar_expect_tx(bar, units16 * 16u);
+                if (!(entry >> 63)) bulk_load(warp_mem, p.arena + 16ull * CF_B200_DIR_OFFSET_UNITS(entry), units16 * 16u, bar);
             }
         };
         auto entry_ok = [&](uint64_t entry) {
@@ -452,30 +428,22 @@ __global__ void __launch_bounds__(kThreadsOf<NG, NB>, 1) lanes_attention_kernel(
         uint64_t entry_cur = n_pages ? load_entry(page_begin) : 0ull;
         uint64_t entry_next = n_pages > 1 ? load_entry(page_begin + 1) : 0ull;
         __syncwarp();
-        issue(0, entry_cur);
+        issue(entry_cur);
         bool alive = true;
 
         for (uint32_t i = 0; i < n_pages; ++i) {
-            const uint32_t st = NB == 32 ? (i & 1u) : 0u;
-            uint64_t entry_after = 0ull;
-            bool next_issued = NB == 32;
-            if (i + 1 < n_pages) {
-                if constexpr (NB == 32) {
-                    __syncwarp();  // every lane is done with the other stage (page i-1)
-                    issue(st ^ 1u, entry_next);
-                }
-                if (i + 2 < n_pages) entry_after = load_entry(page_begin + i + 2);
-            }
+            const uint64_t entry_after = i + 2 < n_pages ? load_entry(page_begin + i + 2) : 0ull;
+            bool next_issued = false;
             if (!entry_ok(entry_cur)) {
                 if (lane == 0) raise_status(p, CF_B200_DEVSTAT_BAD_RECORD);
             } else {
-                if (!mbar_wait(&bars[st], (phase_bits >> st) & 1u, p.wait_polls)) {
+                if (!mbar_wait(bar, phase, p.wait_polls)) {
                     if (lane == 0) raise_status(p, CF_B200_DEVSTAT_WAIT_EXPIRED);
                     alive = false;
                     break;
                 }
-                phase_bits ^= 1u << st;
-                const uint8_t *rec = warp_mem + st * kStageBytes;
+                phase ^= 1u;
+                const uint8_t *rec = warp_mem;
                 const uint4 hv = *reinterpret_cast<const uint4 *>(rec);
                 const uint32_t k_bytes = 16u * (hv.x & 0xffffu), v_bytes = 16u * (hv.x >> 16);
                 const uint32_t k_coder = hv.y & 0xffu, v_coder = (hv.y >> 8) & 0xffu, token_count = hv.y >> 16;
@@ -526,7 +494,7 @@ __global__ void __launch_bounds__(kThreadsOf<NG, NB>, 1) lanes_attention_kernel(
                                 stage_one(gb >= static_cast<uint32_t>(NB), gb >= static_cast<uint32_t>(NB) ? gb - NB : gb);
                         }
                         __syncwarp();
-                        if (i + 1 < n_pages) issue(0u, entry_next);   // the record is decoded: its stage takes the next one
+                        if (i + 1 < n_pages) issue(entry_next);   // the record is decoded: its place takes the next one
                         next_issued = true;
 #pragma unroll
                         for (int c = 0; c < kQ / 4; ++c) {
@@ -586,60 +554,85 @@ __global__ void __launch_bounds__(kThreadsOf<NG, NB>, 1) lanes_attention_kernel(
                         else { FixedLane v; v.open(v_part, v_bytes, lane); decode_v_only<kMode>(v, u); }
                     }
 
+                    if constexpr (NB == 32) {
+                        __syncwarp();   // the record is decoded: its place takes the next one
+                        if (i + 1 < n_pages) issue(entry_next);
+                        next_issued = true;
+                    }
                     if constexpr (kSplitQ) {   // K q = K binary16(q) + K residue
 #pragma unroll
                         for (int c = 0; c < 4; ++c) u.score[0][c] += u.score[1][c];
                     }
                     if constexpr (!kProbe) {
                     // ---- online softmax for this page (fp32), per group of four heads ----
-                    const uint32_t token = (page_begin + i) * 16u + my_token;
-                    const bool visible = my_token < token_count && token >= first_token && token < sealed && token <= qpos;
+                    const uint32_t page_token = (page_begin + i) * 16u;
+                    const uint32_t seen_end = min(min(sealed, qpos + 1u), page_token + token_count);   // tokens [first_token, seen_end)
+                    const bool visible = page_token + my_token >= first_token && page_token + my_token < seen_end;
+                    float s0[NS], s1[NS];
+                    bool higher = false;
+#pragma unroll
+                    for (int n = 0; n < NS; ++n) {
+                        s0[n] = visible ? u.score[n][0] * k_scale : -CUDART_INF_F;
+                        s1[n] = visible ? u.score[n][1] * k_scale : -CUDART_INF_F;
+                        higher = higher || s0[n] > u.m0[n] || s1[n] > u.m1[n];
+                    }
+                    // The maximum moves on few pages (about one in n after n pages of a head): only then is it worked out, and O rescaled.
+                    if (__any_sync(0xffffffffu, higher)) {
+#pragma unroll
+                        for (int n = 0; n < NS; ++n) {
+                            float r0 = s0[n], r1 = s1[n];
+#pragma unroll
+                            for (int o = 2; o <= 16; o <<= 1) {  // lanes that hold the same two heads
+                                r0 = fmaxf(r0, __shfl_xor_sync(0xffffffffu, r0, o));
+                                r1 = fmaxf(r1, __shfl_xor_sync(0xffffffffu, r1, o));
+                            }
+                            const float n0 = fmaxf(u.m0[n], r0), n1 = fmaxf(u.m1[n], r1);
+                            const float a0 = n0 == -CUDART_INF_F ? 0.0f : exp2f(u.m0[n] - n0), a1 = n1 == -CUDART_INF_F ? 0.0f : exp2f(u.m1[n] - n1);
+                            u.l0[n] *= a0;
+                            u.l1[n] *= a1;
+                            u.m0[n] = n0;
+                            u.m1[n] = n1;
+                            const float b0 = __shfl_sync(0xffffffffu, a0, o_head >> 1), b1 = __shfl_sync(0xffffffffu, a1, o_head >> 1);
+                            const float alpha = (o_head & 1u) ? b1 : b0;
+#pragma unroll
+                            for (int dd = 0; dd < kVCh; ++dd)
+#pragma unroll
+                                for (int c = 0; c < 4; ++c) u.acc[n][dd][c] *= alpha;
+                        }
+                    }
+                    if (v_scale > v_unit) {   // the whole warp: O changes its unit
+                        const float unit = __uint_as_float((__float_as_uint(v_scale) & 0x7f800000u) + 0x00800000u);   // next power of two
+                        const float gain = __uint_as_float(((2u * 127u + 15u) << 23) - __float_as_uint(unit));        // 2^15 / unit
+                        const float shrink = gain * v_unit * (1.0f / kWeightScale);
+                        v_unit = unit;
+                        v_gain = gain;
+#pragma unroll
+                        for (int n = 0; n < NS; ++n)
+#pragma unroll
+                            for (int dd = 0; dd < kVCh; ++dd)
+#pragma unroll
+                                for (int c = 0; c < 4; ++c) u.acc[n][dd][c] *= shrink;
+                    }
+                    const float weight_scale = v_scale * v_gain;
                     __syncwarp();  // the previous page's readers of the scratch are done
 #pragma unroll
                     for (int n = 0; n < NS; ++n) {
-                        const float s0 = visible ? u.score[n][0] * k_scale : -CUDART_INF_F;
-                        const float s1 = visible ? u.score[n][1] * k_scale : -CUDART_INF_F;
-                        float r0 = s0, r1 = s1;
-#pragma unroll
-                        for (int o = 2; o <= 16; o <<= 1) {  // lanes that hold the same two heads
-                            r0 = fmaxf(r0, __shfl_xor_sync(0xffffffffu, r0, o));
-                            r1 = fmaxf(r1, __shfl_xor_sync(0xffffffffu, r1, o));
-                        }
-                        const float n0 = fmaxf(u.m0[n], r0), n1 = fmaxf(u.m1[n], r1);
-                        const float z0 = n0 == -CUDART_INF_F ? 0.0f : n0, z1 = n1 == -CUDART_INF_F ? 0.0f : n1;
-                        const float p0 = exp2f(s0 - z0), p1 = exp2f(s1 - z1);
-                        const float a0 = exp2f(u.m0[n] - z0), a1 = exp2f(u.m1[n] - z1);
-                        u.l0[n] = u.l0[n] * a0 + p0;
-                        u.l1[n] = u.l1[n] * a1 + p1;
-                        u.m0[n] = n0;
-                        u.m1[n] = n1;
+                        const float p0 = visible ? exp2f(s0[n] - u.m0[n]) : 0.0f, p1 = visible ? exp2f(s1[n] - u.m1[n]) : 0.0f;
+                        u.l0[n] += p0;
+                        u.l1[n] += p1;
                         // P goes to the tensor cores as fp16; the rounding residue is fed as a second operand so that
                         // P V is accurate to fp32 level whatever the magnitude of V
-                        // The weights (at most 1) are scaled by 2^15 on the way, O by 2^-15 at the unit's end, both exact:
+                        // The weights (at most 1) are scaled by 2^15 on the way, O by 2^-15 at the partial's end, both exact:
                         // binary16 then resolves weights down to 2^-40 of the row maximum instead of 2^-25.
                         const uint32_t h0 = 4u * n + my_head0;
-                        const float w0 = p0 * kWeightScale, w1 = p1 * kWeightScale;
+                        const float w0 = p0 * weight_scale, w1 = p1 * weight_scale;
                         const __half p0h = __float2half_rn(w0), p1h = __float2half_rn(w1);
                         p_rows[h0 * 16u + my_token] = p0h;
                         p_rows[(h0 + 1u) * 16u + my_token] = p1h;
                         p_rows_lo[h0 * 16u + my_token] = __float2half_rn(w0 - __half2float(p0h));
                         p_rows_lo[(h0 + 1u) * 16u + my_token] = __float2half_rn(w1 - __half2float(p1h));
-                        if (g == 0 && t < 2) {
-                            alpha_s[h0] = a0;
-                            alpha_s[h0 + 1u] = a1;
-                        }
                     }
                     __syncwarp();
-                    const float v_ratio = v_scale_prev / v_scale;   // O is kept in units of the current page's V scale
-                    v_scale_prev = v_scale;
-#pragma unroll
-                    for (int n = 0; n < NS; ++n) {
-                        const float beta = alpha_s[4u * n + o_head] * v_ratio;
-#pragma unroll
-                        for (int dd = 0; dd < kVCh; ++dd)
-#pragma unroll
-                            for (int c = 0; c < 4; ++c) u.acc[n][dd][c] *= beta;
-                    }
                     // P rows as A fragments. Rows g / g+8 of the fragment belong to lane tags g>>2 / (g>>2)+2; a lane
                     // feeds the row whose tag is its own t and zeros (read from the zero row) otherwise.
                     uint32_t ra[2][NS][8], rb[2][NS][8];   // [fp16(p) | its rounding residue][group][fragment words]
@@ -677,17 +670,16 @@ __global__ void __launch_bounds__(kThreadsOf<NG, NB>, 1) lanes_attention_kernel(
                     }   // !kProbe
                 }
             }
-            if (!next_issued && i + 1 < n_pages) {   // single stage, page skipped: nobody reads the stage any more
+            if (!next_issued && i + 1 < n_pages) {   // page skipped: nobody reads the record any more
                 __syncwarp();
-                issue(0u, entry_next);
+                issue(entry_next);
             }
             entry_cur = entry_next;
             entry_next = entry_after;
         }
         if (!alive) {
-            // give the copies still in flight a bounded chance to land before this warp's buffers go away
-            mbar_wait(&bars[0], phase_bits & 1u, p.wait_polls);
-            if constexpr (L::kStages == 2) mbar_wait(&bars[1], (phase_bits >> 1) & 1u, p.wait_polls);
+            // give the copy still in flight a bounded chance to land before this warp's buffers go away
+            mbar_wait(bar, phase, p.wait_polls);
             break;
         }
 
@@ -726,7 +718,7 @@ __global__ void __launch_bounds__(kThreadsOf<NG, NB>, 1) lanes_attention_kernel(
 #pragma unroll
                     for (int c = 0; c < 4; ++c) {
                         const uint32_t owner = 4u * (2u * t + (c & 1)) + (g >> 2) + 2u * (c >> 1);  // lane whose V block it is
-                        dst[kVCh * owner + dd] = u.acc[n][dd][c] * (v_scale_prev * (1.0f / kWeightScale));
+                        dst[kVCh * owner + dd] = u.acc[n][dd][c] * (v_unit * (1.0f / kWeightScale));
                     }
                 }
             }
@@ -762,11 +754,11 @@ cudaError_t launch_one(const AttentionParams &p, int sm_count, cudaStream_t stre
     const uint64_t bit = 1ull << (device & 63);
     if (!(configured.load(std::memory_order_acquire) & bit)) {
         e = cudaFuncSetAttribute(lanes_attention_kernel<NG, kMode, kSplitQ, NB, kDim>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(WarpLayout<NG, NB>::kSmem));
+                                 static_cast<int>(WarpLayout<NG, NB, kSplitQ>::kSmem));
         if (e != cudaSuccess) return e;
         configured.fetch_or(bit, std::memory_order_release);
     }
-    return launch_kernel(lanes_attention_kernel<NG, kMode, kSplitQ, NB, kDim>, sm_count, kThreadsOf<NG, NB>, WarpLayout<NG, NB>::kSmem,
+    return launch_kernel(lanes_attention_kernel<NG, kMode, kSplitQ, NB, kDim>, sm_count, kThreadsOf<NG, NB, kSplitQ>, WarpLayout<NG, NB, kSplitQ>::kSmem,
                          stream, dependent, p, static_cast<uint32_t>(after_prefix));
 }
 
@@ -785,7 +777,7 @@ void lanes_plan_shape(const AttentionParams &p, uint32_t sm_count, uint32_t *war
     const bool split_q = p.query_type == CF_B200_F32 && !p.decode_probe;
     const bool eight = !split_q && p.group > 4u && !p.decode_probe;   // query heads per pass: eight, else four
     const bool staged = p.block_size != 64u || p.head_dim != 128u;
-    const int per_sm = staged ? (split_q || eight ? kWarpsOf<2, 16> : kWarpsOf<1, 16>) : split_q || eight ? kWarpsOf<2> : kWarpsOf<1>;
+    const int per_sm = staged ? (split_q || eight ? kWarpsOf<2, 16> : kWarpsOf<1, 16>) : split_q ? kWarpsOf<2, 32, true> : eight ? kWarpsOf<2> : kWarpsOf<1>;
     *warps = sm_count * static_cast<uint32_t>(per_sm);
     *unit_lanes = p.kv_head_span * (eight ? (p.group + 7u) / 8u : (p.group + 3u) / 4u);
 }

@@ -175,13 +175,15 @@ __device__ __forceinline__ void decode_page(KLane &k, VLane &v, uint32_t (&kq)[1
                 kq[q] = k.quad(4 * pass + (q - 12));
                 vq[q] = v.quad(4 * pass + (q - 12));
             } else {   // both entropy coded: the two chains interleave symbol by symbol
-                k.reload();
-                v.reload();
                 uint32_t ke[4], ve[4];
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    ke[i] = k.symbol();
-                    ve[i] = v.symbol();
+                    ke[i] = k.symbol(i & 1);
+                    ve[i] = v.symbol(i & 1);
+                    if (i & 1) {
+                        k.advance();
+                        v.advance();
+                    }
                 }
                 kq[q] = pack_low_bytes(ke[0], ke[1], ke[2], ke[3]);
                 vq[q] = pack_low_bytes(ve[0], ve[1], ve[2], ve[3]);
