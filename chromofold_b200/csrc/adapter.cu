@@ -14,6 +14,7 @@
 
 #include <cuda_runtime.h>
 
+#include "attention_params.cuh"
 #include "chromofold_b200/compat_adapter.h"
 #include "chromofold_b200/compat_kv.h"
 #include "chromofold_b200/sealed_kv.h"
@@ -804,11 +805,11 @@ extern "C" int cf_llama_kv_attention(cf_llama_kv_adapter *adapter, uint32_t laye
         d.output_type = CF_B200_F32;
         d.softmax_scale = softmax_scale;
         d.causal_window = causal_window;
-        // Prefill (llama.cpp evaluates a prompt in batches of query tokens): they all see the layer's sealed records in
-        // full, which the shared-prefix kernel then decodes once per 128 query rows instead of once per query token.
-        // Only a hint (the plan kernel checks it), given where it pays and the workspace has or can get the room.
+        // Prefill (llama.cpp evaluates a prompt in batches of query tokens): they share the layer's sealed records, which the
+        // shared-prefix kernel then decodes once per 128 query rows instead of once per query token, masking what the
+        // earlier tokens must not see. Given where it pays and the workspace has or can get the room.
         if (query_count >= 4 && causal_window == 0) {
-            const uint32_t tiles = std::min(h0.sealed / adapter->tile_tokens, (query_token_begin + 1u) / adapter->tile_tokens);
+            const uint32_t tiles = std::min(h0.sealed / adapter->tile_tokens, (query_token_begin + query_count - 1u) / adapter->tile_tokens + 1u);
             if (tiles >= 8 && tiles <= adapter->stride) {
                 cf_b200_sealed_attention_desc room = d;   // the workspace grows for the extra partials, up to 1 GiB
                 room.shared_prefix_pages = 1;
@@ -824,7 +825,8 @@ extern "C" int cf_llama_kv_attention(cf_llama_kv_adapter *adapter, uint32_t laye
         d.workspace = reinterpret_cast<void *>(aligned);
         d.workspace_bytes = adapter->workspace.count - (aligned - ws);
         d.status = adapter->status.ptr;
-        if (cf_b200_sealed_attention_async(&d, s) != CF_OK) throw std::runtime_error("ChromoFold paged attention launch rejected");
+        constexpr uint32_t kAll = CF_B200_STAGE_PLAN | CF_B200_STAGE_ATTENTION | CF_B200_STAGE_COMBINE;
+        if (cfb::sealed_attention_stages(&d, kAll, s, false, true) != CF_OK) throw std::runtime_error("ChromoFold paged attention launch rejected");
     });
 }
 

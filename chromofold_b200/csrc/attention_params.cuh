@@ -40,6 +40,7 @@ struct AttentionParams {
     uint32_t plan_warps;            // warps (any-geometry kernel: CTAs) that are resident at once in the attention kernel
     uint32_t unit_lanes;            // units that share a stretch: kv heads x passes over a kv head's query group
     uint32_t shared_prefix_pages;   // the caller's hint, already zeroed when the launch cannot use it
+    uint32_t one_slot;              // 1: every entry is a query token of the same sequence
     uint32_t sm_count;
     uint32_t decode_probe;          // 1 = measurement: decode every page, fold the symbols into a checksum, no attention;
                                     // 2 = test: store every decoded symbol to `output` ([page id][kv head][K | V stream])
@@ -131,7 +132,7 @@ __device__ __forceinline__ PageLine plan_line(const AttentionParams &p) {
 #endif
 
 // Implemented in sealed_attention.cu
-cf_status sealed_attention_stages(const cf_b200_sealed_attention_desc *d, uint32_t stages, void *stream, bool output_on_peer);
+cf_status sealed_attention_stages(const cf_b200_sealed_attention_desc *d, uint32_t stages, void *stream, bool output_on_peer, bool one_slot = false);
 // dependent: the kernel before it on the stream belongs to the same call and lets this one start early.
 cudaError_t launch_plan(const AttentionParams &p, cudaStream_t stream);
 cudaError_t launch_combine(const AttentionParams &p, cudaStream_t stream, bool dependent);

@@ -14,7 +14,7 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
-#include "cf_device_common.cuh"
+#include "attention_params.cuh"
 #include "engine_common.cuh"
 
 using namespace cfb_engine;
@@ -314,11 +314,11 @@ void core_attention(Core &c, uint32_t layer, const void *q, uint32_t q_type, flo
     d.output_type = CF_B200_F32;
     d.softmax_scale = softmax_scale;
     d.causal_window = window;
-    // Prefill: the query tokens of one call all see the layer's sealed records in full, so those records are decoded
-    // once per 128 query rows by the shared-prefix kernel instead of once per query token. Only a hint (the plan kernel
-    // checks it), given where it pays and where the workspace has or can get room for the extra partials.
+    // Prefill: the query tokens of one call share the layer's sealed records, which are decoded once per 128 query rows by
+    // the shared-prefix kernel instead of once per query token: all of them up to the last token's position, the kernel masks
+    // what the earlier tokens must not see. Given where it pays and where the workspace has or can get room for the extra partials.
     if (count >= 4 && window == 0) {
-        const uint32_t tiles = std::min(L.sealed_tokens / c.tile, (query_begin + 1u) / c.tile);
+        const uint32_t tiles = std::min(L.sealed_tokens / c.tile, (query_begin + count - 1u) / c.tile + 1u);
         if (tiles >= 8 && tiles <= c.stride && shared_prefix_room(c.workspace, count, c.cfg.kv_heads, c.cfg.query_heads, c.cfg.head_dim, s))
             d.shared_prefix_pages = tiles;
     }
@@ -326,7 +326,8 @@ void core_attention(Core &c, uint32_t layer, const void *q, uint32_t q_type, flo
     d.workspace = reinterpret_cast<void *>(aligned);
     d.workspace_bytes = c.workspace.count - (aligned - ws);
     d.status = c.status.ptr;
-    if (cf_b200_sealed_attention_async(&d, s) != CF_OK) throw std::runtime_error("compressed attention launch rejected");
+    constexpr uint32_t kAll = CF_B200_STAGE_PLAN | CF_B200_STAGE_ATTENTION | CF_B200_STAGE_COMBINE;
+    if (cfb::sealed_attention_stages(&d, kAll, s, false, true) != CF_OK) throw std::runtime_error("compressed attention launch rejected");
 }
 
 void core_clear(Core &c, cudaStream_t s) {

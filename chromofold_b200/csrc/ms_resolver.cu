@@ -10,7 +10,7 @@
 #include <vector>
 
 #include "chromofold_b200/compat_ms.h"
-#include "cf_device_common.cuh"
+#include "attention_params.cuh"
 #include "engine_common.cuh"
 #include "ms_internal.h"
 #include "seal_params.cuh"
@@ -993,7 +993,16 @@ extern "C" int cf_ms_cuda_copy_sequence_async(cf_ms_cuda_resolver *r, int64_t so
 // records are decoded once per 128 query rows by the shared-prefix kernel instead of once per row; the number returned
 // here is only a hint, the plan kernel checks it against the page tables. 0 = not worth it or not applicable.
 static uint32_t shared_leading_tiles(cf_ms_cuda_resolver *r, const cf_ms_batch_item *items, uint32_t item_count, uint32_t layer,
-                                     uint32_t rows, uint32_t window) {
+                                     uint32_t rows, uint32_t window, bool *one_sequence) {
+    const cf_ms_batch_item *lead = nullptr;
+    *one_sequence = true;
+    uint32_t highest_position = 0;
+    for (uint32_t i = 0; i < item_count; ++i) {
+        if (items[i].layer != layer) continue;
+        if (!lead) lead = &items[i];
+        else if (items[i].sequence_id != lead->sequence_id) *one_sequence = false;
+        highest_position = std::max(highest_position, items[i].query_token_begin + items[i].query.token_count - 1u);
+    }
     if (rows < 4 || window != 0) return 0;   // a handful of rows is served faster one by one
     const LayerSeq *first = nullptr;
     size_t common_refs = 0;
@@ -1019,7 +1028,8 @@ static uint32_t shared_leading_tiles(cf_ms_cuda_resolver *r, const cf_ms_batch_i
         if (ref.tokens != ref.tiles * r->tile) break;   // a record that is not full ends the run of whole records
         tiles += ref.tiles;
     }
-    tiles = std::min(tiles, (lowest_position + 1u) / r->tile);   // every query token must see the shared records in full
+    // query tokens of several sequences must see the shared records in full; those of one may see them in part
+    tiles = std::min(tiles, *one_sequence ? highest_position / r->tile + 1u : (lowest_position + 1u) / r->tile);
     return tiles >= 8 ? tiles : 0;
 }
 
@@ -1144,14 +1154,16 @@ extern "C" int cf_ms_cuda_execute_batch_async(cf_ms_cuda_resolver *r, const cf_m
             d.softmax_scale = softmax_scale;
             d.causal_window = window;
             // the shared-prefix partials take their own region of the workspace, which grows for them if it has to
-            d.shared_prefix_pages = shared_leading_tiles(r, items, item_count, layer, count, window);
+            bool one_sequence = false;
+            d.shared_prefix_pages = shared_leading_tiles(r, items, item_count, layer, count, window, &one_sequence);
             if (d.shared_prefix_pages && !shared_prefix_room(r->workspace, count, r->config.kv_head_count, Hq, D, s))
                 d.shared_prefix_pages = 0;
             const uintptr_t ws = reinterpret_cast<uintptr_t>(r->workspace.ptr), aligned = (ws + 255) / 256 * 256;
             d.workspace = reinterpret_cast<void *>(aligned);
             d.workspace_bytes = r->workspace.count - (aligned - ws);
             d.status = r->status.ptr;
-            if (cf_b200_sealed_attention_async(&d, s) != CF_OK) throw std::runtime_error("multi-sequence attention launch rejected");
+            constexpr uint32_t kAll = CF_B200_STAGE_PLAN | CF_B200_STAGE_ATTENTION | CF_B200_STAGE_COMBINE;
+            if (cfb::sealed_attention_stages(&d, kAll, s, false, one_sequence) != CF_OK) throw std::runtime_error("multi-sequence attention launch rejected");
             ++r->counters.sequence_attention_launches;
         }
         if (!dense) {

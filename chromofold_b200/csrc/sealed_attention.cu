@@ -84,7 +84,9 @@ __global__ void __launch_bounds__(kPlanThreads) plan_kernel(AttentionParams p) {
     // same ids as the first sequence's (compared by verify_prefix_kernel, result per entry in prefix[]). The pages are
     // then left to the shared-prefix kernel and taken off the line.
     uint32_t shared = p.shared_prefix_pages;
-    if (shared) {
+    if (p.one_slot) {   // query tokens of one sequence: its pages are shared whatever the positions (the shared-prefix kernel masks)
+        shared = min(shared, p.seq_sealed_tokens[slot_of(p, 0)] / p.page_tokens);
+    } else if (shared) {
         int bad = 0;
         wait_for_previous_kernel();
         for (uint32_t s = begin; s < end; ++s) {   // the pages must be sealed and wholly visible to the entry's query token
@@ -353,14 +355,14 @@ __global__ void __launch_bounds__(kGenericThreads) generic_attention_kernel(Atte
 // ---------------------------------------------------------------------------------------------------------------
 // Combine: merge the partials of every (entry, query head) row with the unsealed tail and write the output.
 //
-// A CTA serves R rows: the query heads of one kv head, for one entry or, in multi-query calls, for several entries of one
-// slot. The tail's K and V rows are then read once per CTA instead of once per row (at 500 rows over a tail of up to 127
-// tokens those reads were all of the 274 us this stage took). A launch with too few rows for that, one or a few
-// sequences, gives each row a CTA of its own (R = 1), whose warps share out the row's partials.
+// Bound by the length of its chain of loads, not by what they carry (a few MB): record -> tail rows -> weights -> partials.
+// So every stage has all of its loads in flight at once, the first V rows are fetched before the scores are worked out, and the
+// tail is done before this kernel waits for the attention kernel. Everything the plan kernel wrote may be read before that wait:
+// the attention kernel lets this one start only after it has seen the plan's end itself.
 //
 // Every sum has an order of its own that the shape of the CTA does not change, so that a row's result depends on nothing
-// but the row: partials are added up in 32 consecutive strands and the strands in order, tail tokens in eight interleaved
-// strands.
+// but the row: partials are added up in 32 consecutive strands, each relative to its own maximum, and the strands in
+// order; tail tokens in eight interleaved strands.
 // ---------------------------------------------------------------------------------------------------------------
 constexpr uint32_t kStrands = 32;
 
@@ -386,293 +388,472 @@ __device__ __forceinline__ float sum_many(float (&v)[V], uint32_t lane) {
     return v[0];
 }
 
+__device__ __forceinline__ SeqInfo load_seq_info(const AttentionParams &p, uint32_t seq) {
+    const uint4 *src = reinterpret_cast<const uint4 *>(seq_info(p) + seq);
+    const uint4 a = __ldcg(src), b = __ldcg(src + 1);
+    SeqInfo info;
+    info.slot = a.x, info.sealed = a.y, info.qpos = a.z, info.tail = a.w;
+    info.first_page = b.x, info.page_end = b.y, info.row = b.z, info.line_begin = b.w;
+    return info;
+}
+
+// The partials of a row: slots [first, first + regular), then the shared prefix's cells.
+struct RowPartials {
+    uint32_t first, regular, cells;
+};
+__device__ __forceinline__ RowPartials row_partials(const AttentionParams &p, const PageLine &line, const SeqInfo &info, uint32_t seq,
+                                                    uint32_t local_q) {
+    RowPartials rp = {};
+    const uint32_t pages = info.page_end - info.first_page;
+    if (pages) {
+        const uint32_t a = info.line_begin, b = a + (line.grain == 1u ? pages : (pages + line.grain - 1u) / line.grain) - 1u;
+        const uint32_t j0 = line.stretch_of(a), j1 = line.stretch_of(b);
+        rp.first = line.slot(j0, line.piece_of(j0, a), a, seq);
+        rp.regular = line.slot(j1, line.piece_of(j1, b), b, seq) + 1u - rp.first;
+    }
+    // one per CTA of the shared-prefix kernel that met the row's head-tile
+    static_assert(sizeof(PageLine) == 28 && offsetof(PlanHeader, shared_pages) == 32 && offsetof(PlanHeader, shared_rounds) == 40, "");
+    const uint4 shared = __ldcg(reinterpret_cast<const uint4 *>(p.workspace) + 2);
+    if (shared.x != 0u && shared.y != 0u) {
+        const uint32_t row_tiles = (p.seq_count * p.group + 127u) / 128u;
+        const SharedSplit split = {shared.z, p.kv_head_span * row_tiles, shared.y};
+        const uint64_t first = static_cast<uint64_t>((local_q / p.group) * row_tiles + (seq * p.group + local_q % p.group) / 128u) * split.rounds;
+        rp.cells = min(split.cta_of(first + split.rounds - 1u) - split.cta_of(first) + 1u, CF_B200_SHARED_CHUNKS_MAX);
+    }
+    return rp;
+}
+__device__ __forceinline__ const float *partial_of(const AttentionParams &p, const RowPartials &rp, uint32_t c, uint32_t seq, uint32_t local_q) {
+    return c < rp.regular ? partial_ptr(p, rp.first + c, local_q) : shared_partial_ptr(p, c - rp.regular, seq, local_q);
+}
+__device__ __forceinline__ void store_output(const AttentionParams &p, uint64_t i, float value) {
+    if (p.output_type == CF_B200_F16) reinterpret_cast<__half *>(p.output)[i] = __float2half_rn(value);
+    else reinterpret_cast<float *>(p.output)[i] = value;
+}
+
+// A CTA serves R query heads of one kv head for one entry; kThreads / 32 / R warps share a row's partials. R = 4 reads a tail's rows
+// once for four heads: on 512 threads while all CTAs are resident at once, on 128 beyond that, where a warp per row
+// needs no strands in shared memory and issues a quarter of the instructions (256 sequences: 23 against 68 us). R = 1 on 1024
+// threads spreads a launch with few rows.
 template <int R, int kThreads>
 struct CombineSmem {   // offsets in floats
-    static constexpr int kGroups = kThreads / 128;          // thread groups of one thread per channel
-    static constexpr int kRowStride = R == 1 ? 1 : R + 4;   // of a tail token's weights: 16-byte aligned, banks spread
-    static constexpr int kQ = 0;                            // [R][128]
-    static constexpr int kTail = kQ + R * 128;              // [groups (2 for one group)][R][128] sums of weighted V rows
-    static constexpr int kTailGroups = kGroups < 2 ? 2 : kGroups;
-    static constexpr int kStrand = kTail + kTailGroups * R * 128;   // R = 1: [strand][128]
-    static constexpr int kWeights = kStrand + (R == 1 ? static_cast<int>(kStrands) * 128 : 0);   // [tail_capacity][kRowStride]
-    static size_t bytes(uint32_t tail_capacity) { return (kWeights + static_cast<size_t>(tail_capacity) * kRowStride) * 4u; }
+    static constexpr int kGroups = kThreads / 128;                     // thread groups of one thread per channel
+    static constexpr int kTail = 0;                                    // [group][R][128] sums of weighted V rows
+    static constexpr int kStrand = kTail + kGroups * R * 128;          // [R][strand][128], where several warps share a row
+    static constexpr int kWeights = kStrand + (kThreads == 32 * R ? 0 : R * static_cast<int>(kStrands) * 128);   // [tail_capacity][R]
+    static size_t bytes(uint32_t tail_capacity) { return (kWeights + static_cast<size_t>(tail_capacity) * R) * 4u; }
 };
 
 template <int R, int kThreads>
-__global__ void __launch_bounds__(kThreads) combine_kernel(AttentionParams p, uint32_t cta_entries, uint32_t cta_heads) {
+__global__ void __launch_bounds__(kThreads, 1024 / kThreads > 8 ? 8 : 1024 / kThreads) combine_kernel(AttentionParams p) {
     using S = CombineSmem<R, kThreads>;
-    constexpr int kWarps = kThreads / 32, kGroups = S::kGroups, kGroupStrands = 8 / kGroups;
+    constexpr int kWarps = kThreads / 32, kGroups = S::kGroups, kBatch = 8;
+    constexpr uint32_t kRowWarps = kWarps / R, kOwn = kStrands / kRowWarps;
     extern __shared__ __align__(16) float smem_f[];
-    float *q = smem_f + S::kQ, *tail_acc = smem_f + S::kTail, *weights = smem_f + S::kWeights;
-    __shared__ uint32_t e_slot[R], e_sealed[R], e_qpos[R], e_tail[R], e_row[R];
-    __shared__ float tail_m[R], tail_l[R];
-    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    float *tail_acc = smem_f + S::kTail, *strands = smem_f + S::kStrand, *weights = smem_f + S::kWeights;
+    __shared__ float tail_m[R], tail_l[R], strand_m[R][kStrands], strand_l[R][kStrands];
+    __shared__ RowPartials r_partials[R];
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, d = tid & 127u, grp = tid >> 7;
     const uint32_t G = p.group, D = p.head_dim, C = p.tail_capacity;   // C: rows per (slot, kv head) in the tails
-    const uint32_t entry0 = blockIdx.x * cta_entries, entries = min(cta_entries, p.seq_count - entry0);
-    const uint32_t head0 = blockIdx.y * cta_heads, rows = entries * cta_heads;   // local query heads; row = entry * heads + head
-    const uint32_t kv_head = p.kv_head_begin + head0 / G;
-    auto q_head_of = [&](uint32_t r) { return p.kv_head_begin * G + head0 + r % cta_heads; };
+    const uint32_t seq = blockIdx.x, subs = (G + R - 1u) / R;
+    const uint32_t head_local = blockIdx.y / subs, in_group = blockIdx.y % subs * R, rows = min(static_cast<uint32_t>(R), G - in_group);
+    const uint32_t kv_head = p.kv_head_begin + head_local, q_head = kv_head * G + in_group, local_q = head_local * G + in_group;
+    const SeqInfo info = load_seq_info(p, seq);
+    const PageLine line = plan_line(p);
+    const uint32_t tail = min(info.tail, C);
+    if (tid < R) r_partials[tid] = row_partials(p, line, info, seq, local_q + min(tid, rows - 1u));
 
-    if (tid < entries) {
-        const uint32_t seq = entry0 + tid, slot = slot_of(p, seq), row = row_of(p, seq);
-        const uint32_t sealed = p.seq_sealed_tokens[slot], tail = p.tail_tokens ? p.tail_tokens[slot] : 0u;
-        e_slot[tid] = slot;
-        e_sealed[tid] = sealed;
-        e_qpos[tid] = query_position(p, seq, sealed, tail);
-        e_tail[tid] = min(tail, C);
-        e_row[tid] = row;
-    }
-    __syncthreads();
-    uint32_t any_tail = 0;
-    for (uint32_t e = 0; e < entries; ++e) any_tail |= e_tail[e];
-
-    if (any_tail) {
-        for (uint32_t i = tid; i < R * 128u; i += kThreads) {
-            const uint32_t r = i >> 7, d = i & 127u;
-            q[i] = r < rows && d < D ? load_query(p, e_row[r / cta_heads], q_head_of(r), d) : 0.0f;
-        }
-        __syncthreads();
-        // Scores. Consecutive entries of one slot share the pass over its rows: two tokens per warp at a time, four channels
-        // per lane, the sums of all rows reduced together.
-        for (uint32_t e0 = 0, e1; e0 < entries; e0 = e1) {
-            for (e1 = e0 + 1u; e1 < entries && e_slot[e1] == e_slot[e0]; ++e1) {}
-            const uint32_t tail = e_tail[e0], sealed = e_sealed[e0];
-            const uint64_t base = (static_cast<uint64_t>(e_slot[e0]) * p.kv_head_count + kv_head) * C;
-            for (uint32_t t0 = 2u * warp; t0 < tail; t0 += 2u * kWarps) {
-                float k0[4], k1[4], sums[2 * R];
+    if (tail) {
+        const uint64_t base = (static_cast<uint64_t>(info.slot) * p.kv_head_count + kv_head) * C;
+        float v[kBatch];
+        auto load_v = [&](uint32_t t0) {
 #pragma unroll
-                for (uint32_t j = 0; j < 4; ++j) {
-                    const uint32_t d = lane + 32u * j;
-                    k0[j] = d < D ? load_tail(p.tail_k, p.tail_type, (base + t0) * D + d) : 0.0f;
-                    k1[j] = d < D && t0 + 1u < tail ? load_tail(p.tail_k, p.tail_type, (base + t0 + 1u) * D + d) : 0.0f;
-                }
+            for (int k = 0; k < kBatch; ++k) {
+                const uint32_t t = t0 + grp + static_cast<uint32_t>(k * kGroups);
+                v[k] = t < tail && d < D ? load_tail(p.tail_v, p.tail_type, (base + t) * D + d) : 0.0f;
+            }
+        };
+        load_v(0u);
+        float q[R][4];
 #pragma unroll
-                for (int r = 0; r < R; ++r) {
-                    float a = 0.0f, b = 0.0f;
+        for (int r = 0; r < R; ++r)
 #pragma unroll
-                    for (uint32_t j = 0; j < 4; ++j) {
-                        const float qv = q[r * 128 + lane + 32u * j];
-                        a = fmaf(qv, k0[j], a);
-                        b = fmaf(qv, k1[j], b);
-                    }
-                    sums[r] = a;
-                    sums[R + r] = b;
+            for (uint32_t j = 0; j < 4; ++j)
+                q[r][j] = r < rows && lane + 32u * j < D ? load_query(p, info.row, q_head + r, lane + 32u * j) : 0.0f;
+        // scores: two tokens per warp at a time, four channels per lane, the sums of all rows reduced together
+        for (uint32_t t0 = 2u * warp; t0 < tail; t0 += 2u * kWarps) {
+            float k0[4], k1[4], sums[2 * R];
+#pragma unroll
+            for (uint32_t j = 0; j < 4; ++j) {
+                const uint32_t c = lane + 32u * j;
+                k0[j] = c < D ? load_tail(p.tail_k, p.tail_type, (base + t0) * D + c) : 0.0f;
+                k1[j] = c < D && t0 + 1u < tail ? load_tail(p.tail_k, p.tail_type, (base + t0 + 1u) * D + c) : 0.0f;
+            }
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                float a = 0.0f, b = 0.0f;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    a = fmaf(q[r][j], k0[j], a);
+                    b = fmaf(q[r][j], k1[j], b);
                 }
-                const float sum = sum_many<2 * R>(sums, lane);
-                const uint32_t value = lane / (16u / R), r = value % R, t = t0 + value / R;
-                if (lane % (16u / R) == 0u && t < tail && r < rows && r / cta_heads >= e0 && r / cta_heads < e1) {
-                    const uint32_t qpos = e_qpos[r / cta_heads], token = sealed + t;
-                    const bool visible = token >= window_begin(qpos, p.causal_window) && token <= qpos;
-                    weights[t * S::kRowStride + r] = visible ? sum * p.softmax_scale * kLog2e : -CUDART_INF_F;
-                }
+                sums[r] = a;
+                sums[R + r] = b;
+            }
+            const float sum = sum_many<2 * R>(sums, lane);
+            const uint32_t value = lane / (16u / R), r = value % R, t = t0 + value / R, token = info.sealed + t;
+            if (lane % (16u / R) == 0u && t < tail) {
+                const bool visible = token >= window_begin(info.qpos, p.causal_window) && token <= info.qpos;
+                weights[t * R + r] = visible ? sum * p.softmax_scale * kLog2e : -CUDART_INF_F;
             }
         }
         __syncthreads();
         // softmax of every row over its tail: scores become weights relative to the row's largest
-        for (uint32_t r = warp; r < R; r += kWarps) {
-            const uint32_t tail = r < rows ? e_tail[r / cta_heads] : 0u;
+        if (warp < R) {
             float m = -CUDART_INF_F, l = 0.0f;
-            for (uint32_t t = lane; t < tail; t += 32u) m = fmaxf(m, weights[t * S::kRowStride + r]);
+            for (uint32_t t = lane; t < tail; t += 32u) m = fmaxf(m, weights[t * R + warp]);
             m = warp_max(m);
             for (uint32_t t = lane; t < tail; t += 32u) {
-                const float s = weights[t * S::kRowStride + r], w = s == -CUDART_INF_F ? 0.0f : exp2f(s - m);
-                weights[t * S::kRowStride + r] = w;
+                const float s = weights[t * R + warp], w = s == -CUDART_INF_F ? 0.0f : exp2f(s - m);
+                weights[t * R + warp] = w;
                 l += w;
             }
             l = warp_sum(l);
             if (lane == 0) {
-                tail_m[r] = m;
-                tail_l[r] = l;
+                tail_m[warp] = m;
+                tail_l[warp] = l;
             }
         }
         __syncthreads();
         // weighted V rows: a thread per channel, thread group g takes the token strands g, g + groups, ... of eight
-        const uint32_t d = tid & 127u, grp = tid >> 7;
-        float acc[kGroupStrands][R];
+        constexpr int kOwnTokens = 8 / kGroups;
+        float acc[kOwnTokens][R];
 #pragma unroll
-        for (int k = 0; k < kGroupStrands; ++k)
+        for (int k = 0; k < kOwnTokens; ++k)
 #pragma unroll
             for (int r = 0; r < R; ++r) acc[k][r] = 0.0f;
-        for (uint32_t e0 = 0, e1; e0 < entries; e0 = e1) {
-            for (e1 = e0 + 1u; e1 < entries && e_slot[e1] == e_slot[e0]; ++e1) {}
-            const uint32_t tail = e_tail[e0];
-            const bool whole = e0 == 0u && e1 == entries;   // one slot: every row takes every token
-            const uint64_t base = (static_cast<uint64_t>(e_slot[e0]) * p.kv_head_count + kv_head) * C;
-            for (uint32_t t0 = 0; t0 < tail; t0 += 8u) {
-                float v[kGroupStrands];
+        for (uint32_t t0 = 0;;) {
 #pragma unroll
-                for (int k = 0; k < kGroupStrands; ++k) {
-                    const uint32_t t = t0 + grp + static_cast<uint32_t>(k * kGroups);
-                    v[k] = t < tail && d < D ? load_tail(p.tail_v, p.tail_type, (base + t) * D + d) : 0.0f;
-                }
+            for (int k = 0; k < kBatch; ++k) {
+                const uint32_t t = t0 + grp + static_cast<uint32_t>(k * kGroups);
+                if (t >= tail) break;
 #pragma unroll
-                for (int k = 0; k < kGroupStrands; ++k) {
-                    const uint32_t t = t0 + grp + static_cast<uint32_t>(k * kGroups);
-                    if (t >= tail) continue;
-#pragma unroll
-                    for (int r = 0; r < R; ++r) {
-                        const float w = whole || (r / cta_heads >= e0 && r / cta_heads < e1) ? weights[t * S::kRowStride + r] : 0.0f;
-                        if (w != 0.0f) acc[k][r] = fmaf(w, v[k], acc[k][r]);   // a token the row does not see may hold anything
-                    }
+                for (int r = 0; r < R; ++r) {
+                    const float w = weights[t * R + r];
+                    if (w != 0.0f) acc[k % kOwnTokens][r] = fmaf(w, v[k], acc[k % kOwnTokens][r]);   // a token the row does not see may hold anything
                 }
             }
+            t0 += kBatch * kGroups;
+            if (t0 >= tail) break;
+            load_v(t0);
         }
-        // ((s0 + s2) + (s4 + s6)) and ((s1 + s3) + (s5 + s7)), added below
+        static_assert(kGroups == 1 || kGroups == 4 || kGroups == 8, "strands g and g + 4 are added first, then 0 + 2 and 1 + 3");
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-            if constexpr (kGroups == 1) {
-                tail_acc[r * 128 + d] = (acc[0][r] + acc[2][r]) + (acc[4][r] + acc[6][r]);
-                tail_acc[(R + r) * 128 + d] = (acc[1][r] + acc[3][r]) + (acc[5][r] + acc[7][r]);
-            } else if constexpr (kGroups == 2) {
-                tail_acc[(grp * R + r) * 128 + d] = (acc[0][r] + acc[1][r]) + (acc[2][r] + acc[3][r]);
-            } else {
-                tail_acc[(grp * R + r) * 128 + d] = acc[0][r];
-            }
+            if constexpr (kGroups == 1)
+                tail_acc[r * 128 + d] = ((acc[0][r] + acc[4][r]) + (acc[2][r] + acc[6][r])) + ((acc[1][r] + acc[5][r]) + (acc[3][r] + acc[7][r]));
+            else
+                tail_acc[(grp * R + r) * 128 + d] = kGroups == 4 ? acc[0][r] + acc[kOwnTokens - 1][r] : acc[0][r];
         }
-    } else if (tid < R) {
-        tail_m[tid] = -CUDART_INF_F;
-        tail_l[tid] = 0.0f;
     }
     __syncthreads();
-    auto tail_sum = [&](uint32_t r, uint32_t d) {
-        if (!any_tail) return 0.0f;
-        float h[2];
-        for (int i = 0; i < 2; ++i) {
-            if constexpr (S::kTailGroups == 2) h[i] = tail_acc[(i * R + r) * 128 + d];
-            else h[i] = (tail_acc[i * 128 + d] + tail_acc[(i + 2) * 128 + d]) + (tail_acc[(i + 4) * 128 + d] + tail_acc[(i + 6) * 128 + d]);
-        }
-        return h[0] + h[1];
-    };
-    auto store = [&](uint32_t r, uint32_t d, float value) {
-        const uint64_t i = (static_cast<uint64_t>(e_row[r / cta_heads]) * p.query_head_count + q_head_of(r)) * D + d;
-        if (p.output_type == CF_B200_F16) reinterpret_cast<__half *>(p.output)[i] = __float2half_rn(value);
-        else reinterpret_cast<float *>(p.output)[i] = value;
-    };
 
     // ---- the partials: what the attention kernels wrote ----
+    const uint32_t my_row = warp / kRowWarps;
+    const RowPartials rp = r_partials[my_row];
+    const uint32_t count = rp.regular + rp.cells, strand = (count + kStrands - 1u) / kStrands;
     wait_for_previous_kernel();
-    const PageLine line = plan_line(p);
-    const uint4 more = __ldcg(reinterpret_cast<const uint4 *>(p.workspace) + 2);   // shared_pages.. of the header, see below
-    static_assert(sizeof(PageLine) == 28 && offsetof(PlanHeader, shared_pages) == 32 && offsetof(PlanHeader, shared_rounds) == 40, "");
-    struct RowPartials { uint32_t first, regular, count, seq, local_q; };
-    auto row_partials = [&](uint32_t r) {
-        RowPartials rp = {};
-        rp.seq = entry0 + r / cta_heads;
-        rp.local_q = head0 + r % cta_heads;
-        const uint32_t a = __ldcg(line_prefix(p) + rp.seq), b = __ldcg(line_prefix(p) + rp.seq + 1u);
-        if (b > a) {
-            const uint32_t j0 = line.stretch_of(a), j1 = line.stretch_of(b - 1u);
-            rp.first = line.slot(j0, line.piece_of(j0, a), a, rp.seq);
-            rp.regular = line.slot(j1, line.piece_of(j1, b - 1u), b - 1u, rp.seq) + 1u - rp.first;
-        }
-        rp.count = rp.regular;
-        if (more.x != 0u && more.y != 0u) {   // the shared prefix's: one per CTA of the shared-prefix kernel that met the row's head-tile
-            const uint32_t row_tiles = (p.seq_count * G + 127u) / 128u;
-            const SharedSplit split = {more.z, p.kv_head_span * row_tiles, more.y};
-            const uint64_t first = static_cast<uint64_t>((rp.local_q / G) * row_tiles + (rp.seq * G + rp.local_q % G) / 128u) * split.rounds;
-            rp.count += min(split.cta_of(first + split.rounds - 1u) - split.cta_of(first) + 1u, CF_B200_SHARED_CHUNKS_MAX);
-        }
-        return rp;
-    };
-    auto partial_of = [&](const RowPartials &rp, uint32_t c) {
-        return c < rp.regular ? partial_ptr(p, rp.first + c, rp.local_q) : shared_partial_ptr(p, c - rp.regular, rp.seq, rp.local_q);
-    };
-    // Adds up the partials [begin, end) of a row, a whole number of strands of `strand` each; `emit` gets every strand's sums
-    // (of l, and of this lane's channels lane + 32 j). Eight partials' loads are in flight at a time.
-    auto add_strands = [&](const RowPartials &rp, uint32_t begin, uint32_t end, uint32_t strand, float m, auto emit) {
-        float part[4] = {0.0f, 0.0f, 0.0f, 0.0f}, part_l = 0.0f;
+    if (my_row < rows) {
+        const uint32_t lq = local_q + my_row;
+        uint32_t j = (warp % kRowWarps) * kOwn;   // strand
+        const uint32_t begin = min(j * strand, count), end = min(begin + kOwn * strand, count);
+        const uint32_t whole = strand && strand <= 32u ? 32u / strand * strand : 0u;   // partials per turn: whole strands, or 32 of a long one
+        float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f}, acc_l = 0.0f, mj = -CUDART_INF_F;
         uint32_t left = strand;
-        for (uint32_t c0 = begin; c0 < end; c0 += 32u) {
-            float w = 0.0f, wl = 0.0f;   // lane i: weight of partial c0 + i, and its l
-            if (c0 + lane < end) {
-                const float *src = partial_of(rp, c0 + lane);
-                const float pm = __ldcg(src);
-                wl = __ldcg(src + 1);
-                w = pm == -CUDART_INF_F ? 0.0f : exp2f(pm - m);
+        float top = tail ? tail_m[my_row] : -CUDART_INF_F, row_acc[4] = {0.0f, 0.0f, 0.0f, 0.0f}, row_l = 0.0f;   // a warp per row only
+        if constexpr (kRowWarps == 1u) {
+            float m = -CUDART_INF_F;
+            for (uint32_t c = lane; c < count; c += 32u) m = fmaxf(m, __ldcg(partial_of(p, rp, c, seq, lq)));
+            top = fmaxf(warp_max(m), top);
+        }
+        for (uint32_t c0 = begin, n; c0 < end; c0 += n) {
+            n = min(whole ? whole : min(32u, left), end - c0);
+            float pm = -CUDART_INF_F, pl = 0.0f;
+            if (lane < n) {
+                const float *src = partial_of(p, rp, c0 + lane, seq, lq);
+                pm = __ldcg(src);
+                pl = __ldcg(src + 1);
             }
-            const uint32_t n = min(32u, end - c0);
+            if (whole) {   // every strand's own maximum
+                mj = pm;
+                const uint32_t first = lane / strand * strand;
+                for (uint32_t i = 0; strand > 1u && i < strand; ++i) mj = fmaxf(mj, __shfl_sync(0xffffffffu, pm, (first + i) & 31u));
+            } else if (left == strand) {
+                mj = -CUDART_INF_F;
+                for (uint32_t c = c0 + lane; c < min(c0 + strand, end); c += 32u) mj = fmaxf(mj, __ldcg(partial_of(p, rp, c, seq, lq)));
+                mj = warp_max(mj);
+            }
+            const float w = pm == -CUDART_INF_F ? 0.0f : exp2f(pm - mj);
             for (uint32_t i0 = 0; i0 < n; i0 += 8u) {
                 float x[8][4];
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
-                    const float *src = i0 + i < n ? partial_of(rp, c0 + i0 + i) + 2 : nullptr;
+                    const float *src = partial_of(p, rp, c0 + min(i0 + i, n - 1u), seq, lq) + 2;
 #pragma unroll
-                    for (uint32_t j = 0; j < 4; ++j) x[i][j] = src && lane + 32u * j < D ? __ldcg(src + lane + 32u * j) : 0.0f;
+                    for (uint32_t c = 0; c < 4; ++c) x[i][c] = i0 + i < n && lane + 32u * c < D ? __ldcg(src + lane + 32u * c) : 0.0f;
                 }
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
                     if (i0 + i >= n) break;
-                    const float wi = __shfl_sync(0xffffffffu, w, i0 + i), li = __shfl_sync(0xffffffffu, wl, i0 + i);
+                    const float wi = __shfl_sync(0xffffffffu, w, i0 + i), li = __shfl_sync(0xffffffffu, pl, i0 + i);
+                    const float mi = __shfl_sync(0xffffffffu, mj, i0 + i);
                     if (wi != 0.0f) {   // a partial without a visible token says nothing
-                        part_l = fmaf(li, wi, part_l);
+                        acc_l = fmaf(li, wi, acc_l);
 #pragma unroll
-                        for (int j = 0; j < 4; ++j) part[j] = fmaf(x[i][j], wi, part[j]);
+                        for (int c = 0; c < 4; ++c) acc[c] = fmaf(x[i][c], wi, acc[c]);
                     }
-                    if (--left == 0u) {
-                        emit(part_l, part);
+                    if (--left == 0u || c0 + i0 + i + 1u == end) {
+                        if constexpr (kRowWarps == 1u) {
+                            const float f = mi == -CUDART_INF_F ? 0.0f : exp2f(mi - top);
+                            if (lane == j) row_l = acc_l * f;
+#pragma unroll
+                            for (int c = 0; c < 4; ++c) row_acc[c] = fmaf(acc[c], f, row_acc[c]);
+                        } else {
+                            if (lane == 0) {
+                                strand_m[my_row][j] = mi;
+                                strand_l[my_row][j] = acc_l;
+                            }
+#pragma unroll
+                            for (int c = 0; c < 4; ++c) strands[(my_row * kStrands + j) * 128u + lane + 32u * c] = acc[c];
+                        }
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) acc[c] = 0.0f;
+                        acc_l = 0.0f;
                         left = strand;
-                        part_l = part[0] = part[1] = part[2] = part[3] = 0.0f;
+                        ++j;
                     }
                 }
             }
         }
-        if (left != strand) emit(part_l, part);
-    };
-    if constexpr (R > 1) {   // a warp per row
-        for (uint32_t r = warp; r < rows; r += kWarps) {
-            const RowPartials rp = row_partials(r);
-            float m = -CUDART_INF_F;
-            for (uint32_t c = lane; c < rp.count; c += 32u) m = fmaxf(m, __ldcg(partial_of(rp, c)));
-            m = warp_max(m);
-            float l = 0.0f, a[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-            add_strands(rp, 0u, rp.count, (rp.count + kStrands - 1u) / kStrands, m, [&](float pl, const float (&pa)[4]) {
-                l += pl;
+        if constexpr (kRowWarps == 1u) {
+            const float tm = tail ? tail_m[my_row] : -CUDART_INF_F, ft = tm == -CUDART_INF_F ? 0.0f : exp2f(tm - top);
+            float l = warp_sum(row_l);
+            if (ft != 0.0f) l = fmaf(tail_l[my_row], ft, l);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) a[j] += pa[j];
-            });
-            const float top = fmaxf(m, tail_m[r]);
-            const float sp = m == -CUDART_INF_F ? 0.0f : exp2f(m - top), st = tail_m[r] == -CUDART_INF_F ? 0.0f : exp2f(tail_m[r] - top);
-            const float total = l * sp + tail_l[r] * st;
-            const float inv = total > 0.0f ? 1.0f / total : 0.0f;   // no visible token: zeros (paged_kv_attention.cu:170-173)
-#pragma unroll
-            for (uint32_t j = 0; j < 4; ++j) {
-                const uint32_t d = lane + 32u * j;
-                if (d < D) store(r, d, (a[j] * sp + tail_sum(r, d) * st) * inv);
+            for (uint32_t c = 0; c < 4; ++c) {
+                const uint32_t ch = lane + 32u * c;
+                const float a = ft != 0.0f ? fmaf(tail_acc[my_row * 128u + ch], ft, row_acc[c]) : row_acc[c];
+                if (ch < D) store_output(p, (static_cast<uint64_t>(info.row) * p.query_head_count + q_head + my_row) * D + ch, l > 0.0f ? a / l : 0.0f);
             }
         }
-    } else {   // the CTA's warps share one row's strands
-        constexpr uint32_t kOwn = kStrands / kWarps;
-        __shared__ float warp_m[kWarps], strand_l[kStrands];
-        float *strands = smem_f + S::kStrand;
-        const RowPartials rp = row_partials(0u);
-        const uint32_t strand = (rp.count + kStrands - 1u) / kStrands;
-        const uint32_t begin = min(warp * kOwn * strand, rp.count), end = min(begin + kOwn * strand, rp.count);
-        float m = -CUDART_INF_F;
-        for (uint32_t c = begin + lane; c < end; c += 32u) m = fmaxf(m, __ldcg(partial_of(rp, c)));
-        m = warp_max(m);
-        if (lane == 0) warp_m[warp] = m;
-        __syncthreads();
-        m = warp_max(lane < kWarps ? warp_m[lane] : -CUDART_INF_F);
-        uint32_t k = warp * kOwn;
-        add_strands(rp, begin, end, strand, m, [&](float pl, const float (&pa)[4]) {
-            if (lane == 0) strand_l[k] = pl;
+    }
+    if constexpr (kRowWarps == 1u) return;
+    __syncthreads();
+    const uint32_t r = grp;   // a thread per row and channel
+    if (r < rows) {
+        const uint32_t n = r_partials[r].regular + r_partials[r].cells, per = (n + kStrands - 1u) / kStrands, used = n ? (n + per - 1u) / per : 0u;
+        const float sm = lane < used ? strand_m[r][lane] : -CUDART_INF_F, tm = tail ? tail_m[r] : -CUDART_INF_F;
+        const float top = fmaxf(warp_max(sm), tm);
+        const float f = sm == -CUDART_INF_F ? 0.0f : exp2f(sm - top), ft = tm == -CUDART_INF_F ? 0.0f : exp2f(tm - top);
+        float l = warp_sum(f != 0.0f ? strand_l[r][lane] * f : 0.0f), a = 0.0f;
+#pragma unroll 4
+        for (uint32_t i = 0; i < used; ++i) a = fmaf(strands[(r * kStrands + i) * 128u + d], __shfl_sync(0xffffffffu, f, i), a);
+        if (tail && ft != 0.0f) {
+            float h[4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) strands[k * 128u + lane + 32u * j] = pa[j];
-            ++k;
-        });
-        __syncthreads();
-        const uint32_t used = strand ? (rp.count + strand - 1u) / strand : 0u;
-        if (tid < D) {
-            float l = 0.0f, a = 0.0f;
-            for (uint32_t i = 0; i < used; ++i) {
-                l += strand_l[i];
-                a += strands[i * 128u + tid];
+            for (int i = 0; i < 4; ++i)
+                h[i] = kGroups == 8 ? tail_acc[(i * R + r) * 128 + d] + tail_acc[((i + kGroups - 4) * R + r) * 128 + d] : tail_acc[(i * R + r) * 128 + d];
+            a = fmaf((h[0] + h[2]) + (h[1] + h[3]), ft, a);
+            l = fmaf(tail_l[r], ft, l);
+        }
+        if (d < D) store_output(p, (static_cast<uint64_t>(info.row) * p.query_head_count + q_head + r) * D + d, l > 0.0f ? a / l : 0.0f);
+        // no visible token: zeros (paged_kv_attention.cu:170-173)
+    }
+}
+
+// Two fp32 multiply-adds in one instruction.
+__device__ __forceinline__ void fma_pair(float2 &acc, float2 a, float2 b) {
+    asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%0, %1};\n\t"
+        "fma.rn.f32x2 z, x, y, z;\n\tmov.b64 {%0, %1}, z;\n\t}"
+        : "+f"(acc.x), "+f"(acc.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+}
+
+// Several query tokens of ONE sequence (prefill): a CTA serves 32 rows, the query heads of a kv head for 32 / group
+// tokens. They all read the same tail of up to a page, so its two contractions are register-tiled: a thread forms 4 rows x 2
+// tokens of the scores from shared memory, and 4 rows x 4 channels of the weighted V rows. (A warp per pair of tokens and a
+// block per 16 rows took 366 us for 500 query tokens of 32 heads over 116 tail tokens, most of it index arithmetic and
+// reductions; the products alone are 13 us of multiply-adds.)
+constexpr uint32_t kTileRows = 32, kTileThreads = 256, kTileTokens = 64, kTileStride = 132, kTileWeights = 36;
+inline size_t combine_tile_smem(uint32_t tail_capacity) {
+    return (kTileRows * 128u + kTileTokens * kTileStride + static_cast<size_t>((tail_capacity + kTileTokens - 1u) / kTileTokens * kTileTokens) * kTileWeights) * 4u;
+}
+__global__ void __launch_bounds__(kTileThreads) combine_tile_kernel(AttentionParams p) {
+    extern __shared__ __align__(16) float smem_f[];
+    float *q = smem_f, *k_tile = q + kTileRows * 128u, *weights = k_tile + kTileTokens * kTileStride;   // weights: [token][36]
+    __shared__ uint32_t e_qpos[kTileRows], e_row[kTileRows];
+    __shared__ RowPartials r_partials[kTileRows];
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    const uint32_t G = p.group, D = p.head_dim, C = p.tail_capacity, quads = D / 4u;
+    const uint32_t cta_entries = kTileRows / G, entry0 = blockIdx.x * cta_entries, head_local = blockIdx.y;
+    const uint32_t rows = min(cta_entries, p.seq_count - entry0) * G, kv_head = p.kv_head_begin + head_local;
+    const SeqInfo info0 = load_seq_info(p, entry0);
+    const PageLine line = plan_line(p);
+    const uint32_t tail = min(info0.tail, C), sealed = info0.sealed;
+    if (tid < kTileRows) {
+        const uint32_t seq = entry0 + min(tid, rows - 1u) / G, lq = head_local * G + min(tid, rows - 1u) % G;
+        const SeqInfo info = load_seq_info(p, seq);
+        e_qpos[tid] = info.qpos;
+        e_row[tid] = info.row;
+        r_partials[tid] = row_partials(p, line, info, seq, lq);
+    }
+    __syncthreads();
+    const uint64_t base = (static_cast<uint64_t>(info0.slot) * p.kv_head_count + kv_head) * C;
+    const uint32_t row0 = 4u * warp;   // this warp's rows
+    float m[4], l[4];
+    float2 acc[4][2];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        m[r] = -CUDART_INF_F;
+        l[r] = 0.0f;
+        acc[r][0] = acc[r][1] = make_float2(0.0f, 0.0f);
+    }
+    if (tail) {
+        for (uint32_t r = warp; r < kTileRows; r += kTileThreads / 32u)
+            for (uint32_t d = lane; d < D; d += 32u) q[r * 128u + d] = r < rows ? load_query(p, e_row[r], kv_head * G + r % G, d) : 0.0f;
+        for (uint32_t t0 = 0; t0 < tail; t0 += kTileTokens) {
+            const float4 *src = reinterpret_cast<const float4 *>(static_cast<const float *>(p.tail_k) + (base + t0) * D);
+            const uint32_t n = min(kTileTokens, tail - t0);
+            if (lane < quads) {
+#pragma unroll
+                for (uint32_t t = warp; t < kTileTokens; t += kTileThreads / 32u)
+                    if (t < n) *reinterpret_cast<float4 *>(k_tile + t * kTileStride + 4u * lane) = src[t * quads + lane];
             }
-            const float top = fmaxf(m, tail_m[0]);
-            const float sp = m == -CUDART_INF_F ? 0.0f : exp2f(m - top), st = tail_m[0] == -CUDART_INF_F ? 0.0f : exp2f(tail_m[0] - top);
-            const float total = l * sp + tail_l[0] * st;
-            const float inv = total > 0.0f ? 1.0f / total : 0.0f;
-            store(0u, tid, (a * sp + tail_sum(0u, tid) * st) * inv);
+            __syncthreads();
+            float2 s[4][2];
+#pragma unroll
+            for (int r = 0; r < 4; ++r) s[r][0] = s[r][1] = make_float2(0.0f, 0.0f);
+#pragma unroll 4
+            for (uint32_t c = 0; c < quads; ++c) {
+                const float4 ka = *reinterpret_cast<const float4 *>(k_tile + lane * kTileStride + 4u * c);
+                const float4 kb = *reinterpret_cast<const float4 *>(k_tile + (lane + 32u) * kTileStride + 4u * c);
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    const float4 qv = *reinterpret_cast<const float4 *>(q + (row0 + r) * 128u + 4u * c);
+                    fma_pair(s[r][0], make_float2(qv.x, qv.y), make_float2(ka.x, ka.y));
+                    fma_pair(s[r][1], make_float2(qv.x, qv.y), make_float2(kb.x, kb.y));
+                    fma_pair(s[r][0], make_float2(qv.z, qv.w), make_float2(ka.z, ka.w));
+                    fma_pair(s[r][1], make_float2(qv.z, qv.w), make_float2(kb.z, kb.w));
+                }
+            }
+            __syncthreads();   // the next tile of K rows may come
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const uint32_t t = t0 + lane + 32u * i, token = sealed + t;
+                float w[4];
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    const uint32_t qpos = e_qpos[row0 + r];
+                    const bool visible = t < tail && token >= window_begin(qpos, p.causal_window) && token <= qpos;
+                    w[r] = visible ? (s[r][i].x + s[r][i].y) * p.softmax_scale * kLog2e : -CUDART_INF_F;
+                    m[r] = fmaxf(m[r], w[r]);
+                }
+                *reinterpret_cast<float4 *>(weights + t * kTileWeights + row0) = make_float4(w[0], w[1], w[2], w[3]);
+            }
+        }
+        // this warp's columns of the weights are its own: no barrier from here on
+#pragma unroll
+        for (int r = 0; r < 4; ++r) m[r] = warp_max(m[r]);
+        __syncwarp();
+        for (uint32_t t = lane; t < tail; t += 32u) {
+            float4 *at = reinterpret_cast<float4 *>(weights + t * kTileWeights + row0);
+            const float4 s = *at;
+            const float4 w = make_float4(s.x == -CUDART_INF_F ? 0.0f : exp2f(s.x - m[0]), s.y == -CUDART_INF_F ? 0.0f : exp2f(s.y - m[1]),
+                                         s.z == -CUDART_INF_F ? 0.0f : exp2f(s.z - m[2]), s.w == -CUDART_INF_F ? 0.0f : exp2f(s.w - m[3]));
+            *at = w;
+            l[0] += w.x, l[1] += w.y, l[2] += w.z, l[3] += w.w;
+        }
+        __syncwarp();
+#pragma unroll
+        for (int r = 0; r < 4; ++r) l[r] = warp_sum(l[r]);
+        const float4 *src = reinterpret_cast<const float4 *>(static_cast<const float *>(p.tail_v) + base * D) + lane;
+        for (uint32_t t0 = 0; t0 < tail; t0 += 8u) {
+            float4 v[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) v[k] = t0 + k < tail && lane < quads ? src[(t0 + k) * quads] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                if (t0 + k >= tail) break;
+                const float4 w4 = *reinterpret_cast<const float4 *>(weights + (t0 + k) * kTileWeights + row0);
+                const float w[4] = {w4.x, w4.y, w4.z, w4.w};
+                const float2 va = make_float2(v[k].x, v[k].y), vb = make_float2(v[k].z, v[k].w);
+                if (w[0] != 0.0f && w[1] != 0.0f && w[2] != 0.0f && w[3] != 0.0f) {
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) {
+                        fma_pair(acc[r][0], make_float2(w[r], w[r]), va);
+                        fma_pair(acc[r][1], make_float2(w[r], w[r]), vb);
+                    }
+                } else {   // a token the row does not see may hold anything
+#pragma unroll
+                    for (int r = 0; r < 4; ++r)
+                        if (w[r] != 0.0f) {
+                            fma_pair(acc[r][0], make_float2(w[r], w[r]), va);
+                            fma_pair(acc[r][1], make_float2(w[r], w[r]), vb);
+                        }
+                }
+            }
+        }
+    }
+    wait_for_previous_kernel();
+#pragma unroll 1
+    for (int r = 0; r < 4; ++r) {
+        if (row0 + r >= rows) break;
+        const RowPartials rp = r_partials[row0 + r];
+        const uint32_t seq = entry0 + (row0 + r) / G, lq = head_local * G + (row0 + r) % G, count = rp.regular + rp.cells;
+        float mr = r == 0 ? m[0] : r == 1 ? m[1] : r == 2 ? m[2] : m[3], lr = r == 0 ? l[0] : r == 1 ? l[1] : r == 2 ? l[2] : l[3];
+        const float2 a01 = r == 0 ? acc[0][0] : r == 1 ? acc[1][0] : r == 2 ? acc[2][0] : acc[3][0];
+        const float2 a23 = r == 0 ? acc[0][1] : r == 1 ? acc[1][1] : r == 2 ? acc[2][1] : acc[3][1];
+        float4 a = make_float4(a01.x, a01.y, a23.x, a23.y);
+        for (uint32_t c0 = 0; c0 < count; c0 += 32u) {
+            float pm = -CUDART_INF_F, pl = 0.0f;
+            if (c0 + lane < count) {
+                const float *src = partial_of(p, rp, c0 + lane, seq, lq);
+                pm = __ldcg(src);
+                pl = __ldcg(src + 1);
+            }
+            const float top = fmaxf(mr, warp_max(pm));
+            if (top == -CUDART_INF_F) continue;
+            const float keep = exp2f(mr - top), w = exp2f(pm - top);   // -inf gives 0
+            mr = top;
+            lr = lr * keep + warp_sum(pl * w);
+            a.x *= keep, a.y *= keep, a.z *= keep, a.w *= keep;
+            const uint32_t n = min(32u, count - c0);
+            for (uint32_t i0 = 0; i0 < n; i0 += 4u) {
+                float2 x[4][2];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float2 *src = reinterpret_cast<const float2 *>(partial_of(p, rp, c0 + min(i0 + i, n - 1u), seq, lq) + 2) + 2u * lane;
+                    x[i][0] = lane < quads ? __ldcg(src) : make_float2(0.0f, 0.0f);
+                    x[i][1] = lane < quads ? __ldcg(src + 1) : make_float2(0.0f, 0.0f);
+                }
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float wi = __shfl_sync(0xffffffffu, w, (i0 + i) & 31u);
+                    if (i0 + i < n && wi != 0.0f) {
+                        a.x = fmaf(x[i][0].x, wi, a.x);
+                        a.y = fmaf(x[i][0].y, wi, a.y);
+                        a.z = fmaf(x[i][1].x, wi, a.z);
+                        a.w = fmaf(x[i][1].y, wi, a.w);
+                    }
+                }
+            }
+        }
+        const float inv = lr > 0.0f ? 1.0f / lr : 0.0f;
+        const uint64_t at = (static_cast<uint64_t>(e_row[row0 + r]) * p.query_head_count + kv_head * G + (row0 + r) % G) * D + 4u * lane;
+        if (lane < quads) {
+            store_output(p, at, a.x * inv);
+            store_output(p, at + 1u, a.y * inv);
+            store_output(p, at + 2u, a.z * inv);
+            store_output(p, at + 3u, a.w * inv);
         }
     }
 }
@@ -753,6 +934,7 @@ bool fill_params(const cf_b200_sealed_attention_desc *d, AttentionParams *p) {
     p->layout = workspace_layout(d->seq_count, p->kv_head_span * p->group, d->head_dim, d->workspace_bytes,
                                  d->shared_prefix_pages != 0);
     p->min_pages_per_unit = d->min_pages_per_unit;
+    p->one_slot = 0;
     p->shared_prefix_pages = 0;   // the launch code sets it when the lanes kernels serve the call
     p->sm_count = 0;
     p->decode_probe = d->kernel == CF_B200_KERNEL_DECODE_PROBE ? 1u : d->kernel == CF_B200_KERNEL_DECODE_DUMP ? 2u : 0u;
@@ -769,43 +951,57 @@ bool fill_params(const cf_b200_sealed_attention_desc *d, AttentionParams *p) {
 }  // namespace
 
 cudaError_t launch_plan(const AttentionParams &p, cudaStream_t stream) {
-    if (p.shared_prefix_pages) verify_prefix_kernel<<<p.seq_count, 256, 0, stream>>>(p);
+    const bool verify = p.shared_prefix_pages != 0u && !p.one_slot;
+    if (verify) verify_prefix_kernel<<<p.seq_count, 256, 0, stream>>>(p);
     const uint32_t threads = p.seq_count <= 128u ? 128u : kPlanThreads;   // small batches: fewer warps to start and to meet
-    return launch_kernel(plan_kernel, 1, threads, 0, stream, p.shared_prefix_pages != 0u, p);
+    return launch_kernel(plan_kernel, 1, threads, 0, stream, verify, p);
 }
 
 namespace {
 
+constexpr size_t kCombineSmemMax = 200u * 1024u;
+
+template <class Kernel>
+cudaError_t allow_shared_memory(Kernel kernel, std::atomic<uint64_t> &configured) {   // once per device
+    int device = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess) return e;
+    const uint64_t bit = 1ull << (device & 63);
+    if (configured.load(std::memory_order_acquire) & bit) return cudaSuccess;
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kCombineSmemMax));
+    if (e == cudaSuccess) configured.fetch_or(bit, std::memory_order_release);
+    return e;
+}
+
 template <int R, int kThreads>
-cudaError_t launch_combine_as(const AttentionParams &p, cudaStream_t stream, bool dependent, uint32_t entries, uint32_t heads) {
-    const dim3 grid((p.seq_count + entries - 1u) / entries, p.kv_head_span * p.group / heads);
-    const size_t smem = CombineSmem<R, kThreads>::bytes(p.tail_capacity);
-    if (smem > 47u * 1024u) {   // tails of thousands of tokens
-        const cudaError_t e = cudaFuncSetAttribute(combine_kernel<R, kThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-        if (e != cudaSuccess) return e;
-    }
-    return launch_kernel(combine_kernel<R, kThreads>, grid, kThreads, smem, stream, dependent, p, entries, heads);
+cudaError_t launch_combine_as(const AttentionParams &p, cudaStream_t stream, bool dependent) {
+    static std::atomic<uint64_t> configured{0};
+    const cudaError_t e = allow_shared_memory(combine_kernel<R, kThreads>, configured);
+    if (e != cudaSuccess) return e;
+    const dim3 grid(p.seq_count, p.kv_head_span * ((p.group + R - 1u) / R));
+    return launch_kernel(combine_kernel<R, kThreads>, grid, kThreads, CombineSmem<R, kThreads>::bytes(p.tail_capacity), stream, dependent, p);
 }
 
 }  // namespace
 
-// Rows per CTA of the combine kernel: a kv head's whole query group where that still makes about a CTA per SM, and in
-// multi-query calls as many entries beside it as make sixteen rows, if their tails are long enough to be worth sharing.
-// Otherwise a CTA per row: of 1024 threads while all of them are resident at once, of 256 beyond that. The tail's weights must
-// fit the 48 KB of shared memory that need no opt-in.
+// Four rows per CTA where that still makes about a CTA per SM, else one; 32 where all entries are query tokens of one sequence
+// (the caller says so), their tail is worth sharing and its rows can be read 16 bytes at a time.
 cudaError_t launch_combine(const AttentionParams &p, cudaStream_t stream, bool dependent) {
-    constexpr uint32_t kEnoughCtas = 120, kSharedBytes = 48 * 1024 - 1024;
-    const uint32_t groups = p.seq_count * p.kv_head_span, G = p.group, C = p.tail_capacity;
-    if (groups >= kEnoughCtas) {
-        const uint32_t entries = p.query_positions && p.seq_slots && C > 16u ? 16u / G : 1u;
-        if (entries > 1u && (groups + entries - 1u) / entries >= kEnoughCtas && CombineSmem<16, 256>::bytes(C) <= kSharedBytes)
-            return launch_combine_as<16, 256>(p, stream, dependent, entries, G);
-        if (G <= 4u && CombineSmem<4, 128>::bytes(C) <= kSharedBytes) return launch_combine_as<4, 128>(p, stream, dependent, 1u, G);
-        if (G <= 8u && CombineSmem<8, 256>::bytes(C) <= kSharedBytes) return launch_combine_as<8, 256>(p, stream, dependent, 1u, G);
-        if (CombineSmem<16, 256>::bytes(C) <= kSharedBytes) return launch_combine_as<16, 256>(p, stream, dependent, 1u, G);
+    constexpr uint32_t kEnoughCtas = 120;
+    const uint32_t G = p.group, C = p.tail_capacity;
+    const uint32_t tiles = (p.seq_count + kTileRows / G - 1u) / (kTileRows / G) * p.kv_head_span;
+    const bool by_16 = p.tail_type == CF_B200_F32 && p.head_dim % 4u == 0u &&
+                       ((reinterpret_cast<uintptr_t>(p.tail_k) | reinterpret_cast<uintptr_t>(p.tail_v)) & 15u) == 0u;
+    if (p.one_slot && C > 16u && by_16 && tiles >= kEnoughCtas / 2u && combine_tile_smem(C) <= kCombineSmemMax) {
+        static std::atomic<uint64_t> configured{0};
+        const cudaError_t e = allow_shared_memory(combine_tile_kernel, configured);
+        if (e != cudaSuccess) return e;
+        return launch_kernel(combine_tile_kernel, dim3(tiles / p.kv_head_span, p.kv_head_span), kTileThreads, combine_tile_smem(C), stream, dependent, p);
     }
-    if (groups * G <= 2u * 148u && CombineSmem<1, 1024>::bytes(C) <= kSharedBytes) return launch_combine_as<1, 1024>(p, stream, dependent, 1u, 1u);
-    return launch_combine_as<1, 256>(p, stream, dependent, 1u, 1u);
+    const uint32_t fours = p.seq_count * p.kv_head_span * ((G + 3u) / 4u);
+    if (fours >= kEnoughCtas && CombineSmem<4, 512>::bytes(C) <= kCombineSmemMax / 2u)
+        return fours <= 2u * 148u ? launch_combine_as<4, 512>(p, stream, dependent) : launch_combine_as<4, 128>(p, stream, dependent);
+    return launch_combine_as<1, 1024>(p, stream, dependent);
 }
 
 cudaError_t launch_generic_attention(const AttentionParams &p, cudaStream_t stream) {
@@ -882,7 +1078,9 @@ extern "C" cf_status cf_b200_sealed_attention_stages_async(const cf_b200_sealed_
 // output_on_peer: the one exception to "every pointer is the current device's" — the multi-GPU scheduler lets the
 // combine kernel store its output rows straight into the root GPU's tensor (plain coalesced stores over a peer mapping
 // the scheduler has enabled and checked). Everything that is READ stays local.
-cf_status cfb::sealed_attention_stages(const cf_b200_sealed_attention_desc *d, uint32_t stages, void *stream, bool output_on_peer) {
+// one_slot: every entry is a query token of the same sequence (seq_slots repeats one slot). The shared-prefix hint may then name
+// pages that the earlier tokens see in part or not at all.
+cf_status cfb::sealed_attention_stages(const cf_b200_sealed_attention_desc *d, uint32_t stages, void *stream, bool output_on_peer, bool one_slot) {
     const cf_status valid = cf_b200_sealed_attention_validate(d);
     if (valid != CF_OK) return valid;
     if (stages == 0 || stages > 7u) return CF_ERR_INVALID_ARGUMENT;
@@ -891,6 +1089,7 @@ cf_status cfb::sealed_attention_stages(const cf_b200_sealed_attention_desc *d, u
         return CF_ERR_INVALID_ARGUMENT;   // memory of another GPU: the call must be made with that GPU current
     AttentionParams p;
     cfb::fill_params(d, &p);
+    p.one_slot = one_slot ? 1u : 0u;
     const bool lanes_ok = cfb::lanes_kernel_supports(p);
     const bool probe = d->kernel == CF_B200_KERNEL_DECODE_PROBE || d->kernel == CF_B200_KERNEL_DECODE_DUMP;
     if ((d->kernel == CF_B200_KERNEL_LANES || probe) && !lanes_ok) return CF_ERR_UNSUPPORTED;

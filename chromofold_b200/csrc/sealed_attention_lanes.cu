@@ -299,6 +299,11 @@ __global__ void __launch_bounds__(kThreadsOf<NG, NB, kSplitQ>, 1) lanes_attentio
     uint64_t *bar = reinterpret_cast<uint64_t *>(warp_mem + L::kBar);
     uint32_t *q_rows = reinterpret_cast<uint32_t *>(warp_mem + L::kQRows);
 
+    if (after_prefix && __ldcg(&plan_header(p)->line.stretches) == 0u) {   // the shared-prefix kernel has taken every page
+        allow_dependent_launch();
+        wait_for_previous_kernel();
+        return;
+    }
     load_tables(smem, p, tid, kThreadsOf<NG, NB, kSplitQ>);   // coding tables: once per CTA
     reinterpret_cast<uint32_t *>(warp_mem + L::kZero)[lane] = 0u;   // the zero row inactive lanes read their fragments from
     if (lane == 0) {

@@ -491,6 +491,11 @@ __device__ __forceinline__ void softmax_role(const AttentionParams &p, uint8_t *
     float m_run = -CUDART_INF_F, l_run = 0.0f;   // the row's running maximum; this thread's half of its running sum
     float v_unit = 0.0f;                          // largest V scale met so far in the unit: the unit of O
     bool o_started = false;
+    int32_t seen = 0;   // tokens from the round's first on that the row's query token sees (16 per page and more: all of it)
+    auto seen_of = [&](uint32_t pg, uint32_t count) {   // of page pg of the round, which holds `count`
+        const int32_t left = seen - 16 * static_cast<int32_t>(pg);
+        return left >= 16 ? count : min(count, static_cast<uint32_t>(max(left, 0)));
+    };
 
     for (uint32_t it = 0;; ++it) {
         const uint32_t pair = it & 1u;
@@ -513,6 +518,9 @@ __device__ __forceinline__ void softmax_role(const AttentionParams &p, uint8_t *
             v_unit = 0.0f;
             o_started = false;
             const uint32_t row = u.tile_index * 128u + row_in_tile;
+            // entries of one sequence see its pages up to their own position; entries of several see every shared page
+            seen = p.one_slot ? static_cast<int32_t>(__ldcg(&seq_info(p)[min(row, rows_total - 1u) / G].qpos)) + 1 - static_cast<int32_t>(16u * u.page_begin)
+                              : 0x40000000;
             if constexpr (kSplitQ) {
                 const float4 *src = reinterpret_cast<const float4 *>(
                     reinterpret_cast<const float *>(p.queries) +
@@ -593,7 +601,7 @@ __device__ __forceinline__ void softmax_role(const AttentionParams &p, uint8_t *
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             const uint32_t pg = 4u * half + q;
-            const uint32_t count = __float_as_uint(meta[4 * pg + 2]);
+            const uint32_t count = seen_of(pg, __float_as_uint(meta[4 * pg + 2]));
             const float ks = meta[4 * pg];
             if (count == 16u) {   // a full page (the usual case): the scale is applied to the extreme, not to every score
                 float hi = __uint_as_float(s_raw[q >> 1][16 * (q & 1)]), lo = hi;
@@ -646,7 +654,7 @@ __device__ __forceinline__ void softmax_role(const AttentionParams &p, uint8_t *
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 const uint32_t pg = 4u * half + q;
-                const uint32_t count = __float_as_uint(meta[4 * pg + 2]);
+                const uint32_t count = seen_of(pg, __float_as_uint(meta[4 * pg + 2]));
                 const float ks = meta[4 * pg];
                 // the weights (at most 1) also carry 2^15, exactly, which O sheds at the unit's end: binary16 then resolves
                 // weights down to 2^-40 of the row maximum instead of 2^-25
@@ -656,7 +664,7 @@ __device__ __forceinline__ void softmax_role(const AttentionParams &p, uint8_t *
                 for (int j = 0; j < 16; j += 2) {
                     float w0 = fast_exp2(fmaf(__uint_as_float(s_raw[q >> 1][16 * (q & 1) + j]), ks, -z));
                     float w1 = fast_exp2(fmaf(__uint_as_float(s_raw[q >> 1][16 * (q & 1) + j + 1]), ks, -z));
-                    if (count != 16u) {   // tokens past the page's count weigh nothing
+                    if (count != 16u) {   // tokens past the page's count, or past the row's position, weigh nothing
                         w0 = static_cast<uint32_t>(j) < count ? w0 : 0.0f;
                         w1 = static_cast<uint32_t>(j + 1) < count ? w1 : 0.0f;
                     }
@@ -690,6 +698,7 @@ __device__ __forceinline__ void softmax_role(const AttentionParams &p, uint8_t *
         }
         o_started = true;
         o_pending = true;
+        if (p.one_slot) seen -= 16 * static_cast<int32_t>(kRoundPages);
 
         // ---- last round of the unit: one (max, sum, weighted[128]) per row; each thread writes its 64 channels ----
         if (flags & kLastRound) {
