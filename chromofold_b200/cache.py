@@ -7,6 +7,8 @@ sealing and attention are the library's CUDA entry points (include/chromofold_b2
 used for device memory and streams only.
 """
 import ctypes as C
+import functools
+import math
 
 import numpy as np
 import torch
@@ -18,20 +20,31 @@ def _ptr(t):
     return C.c_void_p(t.data_ptr()) if t is not None else None
 
 
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)   # the stream handle without a Stream object around it
+_current_device = getattr(torch._C, "_cuda_getDevice", torch.cuda.current_device)
+
+
 def _stream_ptr():
+    if _raw_stream is not None:
+        return C.c_void_p(_raw_stream(_current_device()))
     return C.c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
 def _on_own_device(method):
     """Runs a method with the layer's GPU as the current CUDA device: the library launches on the current device, and a
-    kernel must only ever be given memory of the GPU it runs on."""
-    import functools
+    kernel must only ever be given memory of the GPU it runs on. (Where it is current already, the usual case, a switch
+    there and back would cost a decode step of one sequence a tenth of its time.)"""
 
     @functools.wraps(method)
     def wrapper(self, *args, **kw):
+        if self.device.index is not None and _current_device() == self.device.index:
+            return method(self, *args, **kw)
         with torch.cuda.device(self.device):
             return method(self, *args, **kw)
     return wrapper
+
+
+_DESC_BYTES = C.sizeof(N.SealedAttentionDesc)
 
 
 class SealedKvLayer:
@@ -322,12 +335,12 @@ class SealedKvLayer:
         if out is None:
             out = torch.zeros((n, self.query_heads, self.head_dim), dtype=torch.float32, device=self.device)
         d = self._attention_desc(queries, out, n, slots)
-        d.softmax_scale = softmax_scale if softmax_scale is not None else 1.0 / float(np.sqrt(self.head_dim))
-        d.causal_window = causal_window
-        d.kernel = kernel
-        d.kv_head_begin, d.kv_head_span = kv_head_begin, kv_head_span
-        d.min_pages_per_unit = min_pages_per_unit
-        d.shared_prefix_pages = shared_prefix_pages
+        d.softmax_scale = softmax_scale if softmax_scale is not None else 1.0 / math.sqrt(self.head_dim)
+        if causal_window: d.causal_window = causal_window
+        if kernel: d.kernel = kernel
+        if kv_head_begin or kv_head_span: d.kv_head_begin, d.kv_head_span = kv_head_begin, kv_head_span
+        if min_pages_per_unit: d.min_pages_per_unit = min_pages_per_unit
+        if shared_prefix_pages: d.shared_prefix_pages = shared_prefix_pages
         if query_positions is not None:
             d.query_positions = query_positions.data_ptr()
         if row_map is not None:
@@ -411,27 +424,24 @@ class SealedKvLayer:
         return torch.as_tensor(np.asarray(slots, np.int32), device=self.device)
 
     def _attention_desc(self, queries, out, n, slots):
-        d = N.SealedAttentionDesc()
-        d.struct_size, d.abi_version = C.sizeof(N.SealedAttentionDesc), N.ABI_VERSION
-        d.kv_head_count, d.query_head_count, d.head_dim = self.kv_heads, self.query_heads, self.head_dim
-        d.page_tokens, d.block_size, d.codebook_id = self.page_tokens, self.block_size, self.codebook_id
-        d.arena, d.page_dir = self.arena.data_ptr(), self.page_dir.data_ptr()
-        d.page_table, d.seq_sealed_tokens = self.page_table.data_ptr(), self.sealed_tokens.data_ptr()
+        d = N.SealedAttentionDesc(
+            _DESC_BYTES, N.ABI_VERSION, self.kv_heads, self.query_heads, self.head_dim, self.page_tokens, self.block_size, 0, 0,
+            self.codebook_id, self.arena.data_ptr(), self.page_dir.data_ptr(), self.page_table.data_ptr(),
+            self.sealed_tokens.data_ptr(), None, self.max_pages_per_sequence, n, self.k_tables.data_ptr(), self.v_tables.data_ptr(),
+            self.tail_k.data_ptr(), self.tail_v.data_ptr(), self.tail_tokens.data_ptr())
         if slots is not None:
             self._slots_keepalive = self._slots_tensor(slots)
             d.seq_slots = self._slots_keepalive.data_ptr()
-        d.page_table_stride, d.seq_count = self.max_pages_per_sequence, n
-        d.k_tables, d.v_tables = self.k_tables.data_ptr(), self.v_tables.data_ptr()
-        d.tail_k, d.tail_v, d.tail_tokens = self.tail_k.data_ptr(), self.tail_v.data_ptr(), self.tail_tokens.data_ptr()
         if queries is not None:
             d.queries = queries.data_ptr()
             d.query_type = N.F16 if queries.dtype == torch.float16 else N.F32
             d.output = out.data_ptr()
             d.output_type = N.F16 if out.dtype == torch.float16 else N.F32
-        ws = self.workspace.data_ptr() if hasattr(self, "workspace") else 0
-        aligned = (ws + 255) // 256 * 256
-        d.workspace = aligned
-        d.workspace_bytes = (self.workspace.numel() - (aligned - ws)) if hasattr(self, "workspace") else 0
+        workspace = getattr(self, "workspace", None)
+        if workspace is not None:
+            ws = workspace.data_ptr()
+            aligned = (ws + 255) // 256 * 256
+            d.workspace, d.workspace_bytes = aligned, workspace.numel() - (aligned - ws)
         d.status = self.status.data_ptr()
         return d
 
