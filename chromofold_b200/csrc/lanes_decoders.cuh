@@ -288,21 +288,30 @@ struct FixedLaneT {
 using FixedLane = FixedLaneT<32>;
 
 // Coding tables into shared memory, once per CTA: [k rANS slots | v rANS slots | k Huffman LUT | v Huffman LUT].
-// Slot entries are re-packed for RansLane::symbol(): sym | (slot - cum) << 8 | freq << 20.
-__device__ __forceinline__ void load_tables(uint8_t *smem, const AttentionParams &p, uint32_t tid, uint32_t threads) {
-    uint32_t *k_slot = reinterpret_cast<uint32_t *>(smem);
-    uint32_t *v_slot = k_slot + 4096;
-    auto repack = [](uint32_t e) { return (e & 0xffu) | ((e >> 20) << 8) | (((e >> 8) & 0xfffu) << 20); };
-    for (uint32_t i = tid; i < 4096; i += threads) {
-        k_slot[i] = repack(p.k_tables->rans_slot[i]);
-        v_slot[i] = repack(p.v_tables->rans_slot[i]);
+// Slot entries are re-packed for RansLane::symbol(): sym | (slot - cum) << 8 | freq << 20. All of a thread's loads are issued
+// before the first store: a launch that reads a page per warp would otherwise spend a third of its time here, one L2
+// latency after the other.
+template <uint32_t kThreads>
+__device__ __forceinline__ void load_tables(uint8_t *smem, const AttentionParams &p, uint32_t tid) {
+    constexpr uint32_t kWords = kTableBytes / 16u, kEach = (kWords + kThreads - 1u) / kThreads;   // 1024 | 1024 | 512 | 512 words
+    uint4 *dst = reinterpret_cast<uint4 *>(smem);
+    uint4 w[kEach];
+#pragma unroll
+    for (uint32_t j = 0; j < kEach; ++j) {
+        const uint32_t i = tid + j * kThreads;
+        const bool v_side = i < 2048u ? i >= 1024u : i >= 2560u;
+        const cf_b200_codebook_tables *tables = v_side ? p.v_tables : p.k_tables;
+        const uint4 *src = i < 2048u ? reinterpret_cast<const uint4 *>(tables->rans_slot) + (i & 1023u)
+                                     : reinterpret_cast<const uint4 *>(tables->huff_lut) + (i & 511u);
+        if (i < kWords) w[j] = *src;
     }
-    const uint4 *src = reinterpret_cast<const uint4 *>(p.k_tables->huff_lut);
-    uint4 *dst = reinterpret_cast<uint4 *>(v_slot + 4096);
-    for (uint32_t i = tid; i < 512; i += threads) dst[i] = src[i];
-    src = reinterpret_cast<const uint4 *>(p.v_tables->huff_lut);
-    dst += 512;
-    for (uint32_t i = tid; i < 512; i += threads) dst[i] = src[i];
+    auto repack = [](uint32_t e) { return (e & 0xffu) | ((e >> 20) << 8) | (((e >> 8) & 0xfffu) << 20); };
+#pragma unroll
+    for (uint32_t j = 0; j < kEach; ++j) {
+        const uint32_t i = tid + j * kThreads;
+        if (i < 2048u) w[j] = make_uint4(repack(w[j].x), repack(w[j].y), repack(w[j].z), repack(w[j].w));
+        if (i < kWords) dst[i] = w[j];
+    }
 }
 
 // Header checks of a staged record against its directory entry; false = the page is to be skipped.

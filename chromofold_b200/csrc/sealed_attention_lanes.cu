@@ -32,24 +32,18 @@ namespace {
 
 using namespace lanes;
 
-#ifndef CFB_LANES_WARPS
-#define CFB_LANES_WARPS 24
-#endif
-#ifndef CFB_LANES_WARPS2
-#define CFB_LANES_WARPS2 16
-#endif
-#ifndef CFB_LANES_WARPSQ
-#define CFB_LANES_WARPSQ 24
-#endif
-#ifndef CFB_LANES_WARPS_BIG
-#define CFB_LANES_WARPS_BIG 16
-#endif
-#ifndef CFB_LANES_WARPS_BIG2
-#define CFB_LANES_WARPS_BIG2 14
-#endif
-template <int NG, int NB = 32, bool kSplitQ = false> constexpr int kWarpsOf = NB != 32 ? (NG == 1 ? CFB_LANES_WARPS_BIG : CFB_LANES_WARPS_BIG2)
-                                                                              : kSplitQ ? CFB_LANES_WARPSQ : NG == 1 ? CFB_LANES_WARPS : CFB_LANES_WARPS2;
-template <int NG, int NB = 32, bool kSplitQ = false> constexpr int kThreadsOf = kWarpsOf<NG, NB, kSplitQ> * 32;
+// NG = groups of four query rows that one decode serves: 1 or 2 for up to four or eight heads of binary16 queries; fp32 queries
+// (kSplitQ) take two groups for four heads, value and residue, and four for eight. NS = groups that go through softmax and P V.
+template <int NG, bool kSplitQ> constexpr int kHeadGroups = kSplitQ ? NG / 2 : NG;
+// Warps per CTA, one CTA per SM: what registers (65536, no spill worth the name) and shared memory (227 KB) leave. The
+// decoders want as many warps as they can get: 16 -> 24 of them took 8 % off a launch, 24 -> 28 do not fit.
+template <int NG, int NB, bool kSplitQ, int kDim>
+constexpr int kWarpsOf = NB == 32                ? (kHeadGroups<NG, kSplitQ> == 1 ? 24 : 16)
+                         : kDim <= 64            ? 20
+                         : NG == 4               ? (kDim == 96 ? 14 : 12)
+                         : NG == 2               ? 14
+                                                 : 16;
+template <int NG, int NB, bool kSplitQ, int kDim> constexpr int kThreadsOf = kWarpsOf<NG, NB, kSplitQ, kDim> * 32;
 // Per-warp running state of one unit; NG = number of four-head query groups served by one decode pass.
 // kDim = head_dim: a lane holds kDim / 8 quads of each stream (K: kDim / 2 channels of one token; V: kDim / 32 channels,
 // every token).
@@ -87,9 +81,15 @@ __device__ __forceinline__ void score_quad(UnitState<NG, kDim> &u, const QSrc &q
     quad_to_half2(kq, lo, hi);
     qs.template get<0>(q, b0, b1);
     mma_16816(u.score[0], lo, 0u, hi, 0u, b0, b1);
-    if constexpr (NG == 2) {
+    if constexpr (NG >= 2) {
         qs.template get<1>(q, b0, b1);
         mma_16816(u.score[1], lo, 0u, hi, 0u, b0, b1);
+    }
+    if constexpr (NG == 4) {
+        qs.template get<2>(q, b0, b1);
+        mma_16816(u.score[2], lo, 0u, hi, 0u, b0, b1);
+        qs.template get<3>(q, b0, b1);
+        mma_16816(u.score[3], lo, 0u, hi, 0u, b0, b1);
     }
 }
 
@@ -208,7 +208,6 @@ __device__ __forceinline__ void decode_v_only(VLane &v, UnitState<NG> &u) {
 // one lane's kDim / 2 symbols + padding that keeps the row stride off multiples of 64 bytes
 template <int kDim> constexpr uint32_t kTileRowOf = kDim / 2u + ((kDim / 2u + 16u) % 64u == 0 ? 32u : 16u);
 template <int kDim> constexpr uint32_t kTileStreamOf = 32u * kTileRowOf<kDim>;
-constexpr uint32_t kTileBytes = 2u * kTileStreamOf<128> + 32u;
 
 template <int NB, int kDim, class Lane>
 __device__ __forceinline__ void stage_with(Lane &d, uint32_t block, uint8_t *tile) {
@@ -254,37 +253,36 @@ __device__ __forceinline__ void stage_blocks(const uint8_t *part, uint32_t part_
 // else happens to its page, so its place is free for the next one while the scores and weights are worked out; a second place
 // would cost eight warps per SM.
 //   scratch: P rows fp16 high halves [4 NG][16] | low halves [4 NG][16] | 128 zero bytes
-template <int NG, int NB = 32, bool kSplitQ = false>
+template <int NG, int NB, bool kSplitQ, int kDim>
 struct WarpLayout {
-    static constexpr uint32_t kPRows = kStageBytes;
-    static constexpr uint32_t kPBytes = (kSplitQ ? 4 : 4 * NG) * 16 * 2;
+    static constexpr uint32_t kStage = kDim == 128 ? kStageBytes : 16u + 32u * kDim + 48u;   // header, two streams, read-ahead
+    static constexpr uint32_t kPRows = kStage;
+    static constexpr uint32_t kPBytes = 4 * kHeadGroups<NG, kSplitQ> * 16 * 2;
     static constexpr uint32_t kPLo = kPRows + kPBytes;
     static constexpr uint32_t kZero = kPLo + kPBytes;
     static constexpr uint32_t kBar = kZero + 128;
     static constexpr uint32_t kQRows = kBar + 16;
-    static constexpr uint32_t kQRowWords = 36;
+    static constexpr uint32_t kQRowWords = kDim / 4 + 4;
     static constexpr uint32_t kTile = (kQRows + 8 * NG * kQRowWords * 4 + 15u) / 16u * 16u;   // NB != 32 only
-    static constexpr uint32_t kBytes = kTile + (NB != 32 ? kTileBytes : 0u);
-    static constexpr uint32_t kSmem = kTableBytes + kWarpsOf<NG, NB, kSplitQ> * kBytes;
+    static constexpr uint32_t kBytes = kTile + (NB != 32 ? 2u * kTileStreamOf<kDim> + 32u : 0u);
+    static constexpr uint32_t kSmem = kTableBytes + kWarpsOf<NG, NB, kSplitQ, kDim> * kBytes;
+    static_assert(kSmem <= 232448, "a CTA has 227 KB of shared memory");
 };
-static_assert(WarpLayout<1>::kSmem <= 232448 && WarpLayout<2>::kSmem <= 232448 && WarpLayout<2, 32, true>::kSmem <= 232448 &&
-              WarpLayout<1, 16>::kSmem <= 232448 && WarpLayout<2, 16>::kSmem <= 232448 && WarpLayout<2, 16, true>::kSmem <= 232448,
-              "a CTA has 227 KB of shared memory");
 
-// kSplitQ (with NG = 2): the queries are fp32. A pass serves four heads; their rows are split into binary16(q) and
-// binary16(q - binary16(q)), stored as the rows of group 0 and group 1, the two score fragments are added, and one
-// softmax / P V follows: the scores equal fp32-query scores to 2^-22 relative, at the cost of a second score mma.
-template <int NG, int kMode = kAttend, bool kSplitQ = false, int NB = 32, int kDim = 128>
-__global__ void __launch_bounds__(kThreadsOf<NG, NB, kSplitQ>, 1) lanes_attention_kernel(AttentionParams p, uint32_t after_prefix) {
+// kSplitQ: the queries are fp32. Their rows are split into binary16(q) and binary16(q - binary16(q)), stored as the rows of the
+// first and of the last NS groups, the two score fragments of a head are added, and one softmax / P V follows: the scores
+// equal fp32-query scores to 2^-22 relative, at the cost of a second score mma.
+template <int NG, int kMode, bool kSplitQ, int NB, int kDim>
+__global__ void __launch_bounds__(kThreadsOf<NG, NB, kSplitQ, kDim>, 1) lanes_attention_kernel(AttentionParams p, uint32_t after_prefix) {
     constexpr bool kProbe = kMode != kAttend;
-    static_assert(!kSplitQ || NG == 2, "split queries use the two-group query layout");
+    static_assert(!kSplitQ || NG != 1, "split queries take two groups for four heads");
     static_assert(NB == 32 || NB == 24 || NB == 16 || NB == 12 || NB == 8 || NB == 4, "blocks per stream");
     static_assert(kDim == 128 || ((kDim == 96 || kDim == 64 || kDim == 32) && NB != 32), "other head_dims go through the staging tile");
     constexpr int kQ = kDim / 8, kVCh = kDim / 32, kSyms = 16 * kDim;   // quads per lane and stream; V channels per lane
     constexpr uint32_t kRowWords = kDim / 4;   // words of half a query row (the channels one lane's K block covers)
-    using L = WarpLayout<NG, NB, kSplitQ>;
-    constexpr uint32_t kPassHeads = kSplitQ ? 4u : 4u * NG;
-    constexpr int NS = kSplitQ ? 1 : NG;   // groups that go through softmax and P V
+    using L = WarpLayout<NG, NB, kSplitQ, kDim>;
+    constexpr int NS = kHeadGroups<NG, kSplitQ>;
+    constexpr uint32_t kPassHeads = 4u * NS;
     extern __shared__ __align__(128) uint8_t smem[];
     uint32_t *k_slot = reinterpret_cast<uint32_t *>(smem);
     uint32_t *v_slot = k_slot + 4096;
@@ -304,7 +302,7 @@ __global__ void __launch_bounds__(kThreadsOf<NG, NB, kSplitQ>, 1) lanes_attentio
         wait_for_previous_kernel();
         return;
     }
-    load_tables(smem, p, tid, kThreadsOf<NG, NB, kSplitQ>);   // coding tables: once per CTA
+    load_tables<kThreadsOf<NG, NB, kSplitQ, kDim>>(smem, p, tid);   // coding tables: once per CTA
     reinterpret_cast<uint32_t *>(warp_mem + L::kZero)[lane] = 0u;   // the zero row inactive lanes read their fragments from
     if (lane == 0) {
         mbar_init(bar, 1);
@@ -338,7 +336,7 @@ __global__ void __launch_bounds__(kThreadsOf<NG, NB, kSplitQ>, 1) lanes_attentio
         uint32_t partial, page_begin, n_pages, slot, sealed, qpos, q_row, sub, head_local;
         {
             const PageLine line = plan_line(p);
-            const uint32_t unit_lanes = p.kv_head_span * subgroups, unit_count = line.stretches * unit_lanes, warps = kWarpsOf<NG, NB, kSplitQ> * gridDim.x;
+            const uint32_t unit_lanes = p.kv_head_span * subgroups, unit_count = line.stretches * unit_lanes, warps = kWarpsOf<NG, NB, kSplitQ, kDim> * gridDim.x;
             uint32_t stretch = unit / unit_lanes;
             if (x != 0u && x == line.begin(stretch + 1u)) {   // the unit is done
                 if (unit_count <= warps) break;
@@ -366,26 +364,48 @@ __global__ void __launch_bounds__(kThreadsOf<NG, NB, kSplitQ>, 1) lanes_attentio
         const uint32_t first_token = window_begin(qpos, p.causal_window);
         const uint32_t *table_row = p.page_table + static_cast<uint64_t>(slot) * p.page_table_stride;
 
+        // bit 63 of an entry (reserved, 0 in the directory) marks the page of the wait-expiry test: armed, never fetched
+        auto load_entry = [&](uint32_t page) -> uint64_t {
+            const uint32_t page_id = table_row[page];
+            const uint64_t entry = p.page_dir[static_cast<uint64_t>(page_id) * p.kv_head_count + kv_head];
+            return page_id == p.skip_copy_page ? entry | (1ull << 63) : entry;
+        };
+        auto issue = [&](uint64_t entry) {
+            const uint32_t units16 = static_cast<uint32_t>(CF_B200_DIR_LENGTH_UNITS(entry));
+            if (lane == 0 && units16 != 0 && units16 * 16u <= L::kStage - 32u) {
+                mbar_expect_tx(bar, units16 * 16u);
+                if (!(entry >> 63)) bulk_load(warp_mem, p.arena + 16ull * CF_B200_DIR_OFFSET_UNITS(entry), units16 * 16u, bar);
+            }
+        };
+        auto entry_ok = [&](uint64_t entry) {
+            const uint32_t units16 = static_cast<uint32_t>(CF_B200_DIR_LENGTH_UNITS(entry));
+            return units16 != 0 && units16 * 16u <= L::kStage - 32u;
+        };
+
+        // the first record is on its way while the queries are fetched
+        uint64_t entry_cur = load_entry(page_begin);
+        uint64_t entry_next = n_pages > 1 ? load_entry(page_begin + 1) : 0ull;
+        __syncwarp();   // the previous run's readers of the record and of the query rows are done
+        issue(entry_cur);
+
         QSmem qs;
         if constexpr (kSplitQ) {
             const float2 *qsrc = reinterpret_cast<const float2 *>(
                 reinterpret_cast<const float *>(p.queries) + (static_cast<uint64_t>(q_row) * p.query_head_count + q_head_base) * kDim);
-            __syncwarp();  // the previous run's readers are done
 #pragma unroll
-            for (int j = 0; j < kDim / 16; ++j) {    // 4 heads x kDim / 2 channel pairs; row = head*2 + half, residues 8 rows further
+            for (int j = 0; j < NS * kDim / 16; ++j) {    // 4 NS heads x kDim / 2 channel pairs; row = head*2 + half, residues 8 NS rows further
                 const uint32_t i = lane + 32u * j, head = i / (2u * kRowWords);
                 const float2 x = head < G ? qsrc[i] : make_float2(0.0f, 0.0f);
                 const __half2 hi = __floats2half2_rn(x.x, x.y);
                 const float2 back = __half22float2(hi);
                 const __half2 lo = __floats2half2_rn(x.x - back.x, x.y - back.y);
                 q_rows[(i / kRowWords) * L::kQRowWords + i % kRowWords] = *reinterpret_cast<const uint32_t *>(&hi);
-                q_rows[(i / kRowWords + 8u) * L::kQRowWords + i % kRowWords] = *reinterpret_cast<const uint32_t *>(&lo);
+                q_rows[(i / kRowWords + 8u * NS) * L::kQRowWords + i % kRowWords] = *reinterpret_cast<const uint32_t *>(&lo);
             }
             __syncwarp();
         } else {
             const uint32_t *qsrc = reinterpret_cast<const uint32_t *>(
                 reinterpret_cast<const __half *>(p.queries) + (static_cast<uint64_t>(q_row) * p.query_head_count + q_head_base) * kDim);
-            __syncwarp();  // the previous run's readers are done
 #pragma unroll
             for (int j = 0; j < NG * kDim / 16; ++j) {   // 4 NG heads x kDim / 2 words; row = head*2 + half
                 const uint32_t i = lane + 32u * j, head = i / (2u * kRowWords);
@@ -412,28 +432,6 @@ __global__ void __launch_bounds__(kThreadsOf<NG, NB, kSplitQ>, 1) lanes_attentio
         // weights, together with kWeightScale. v_gain = kWeightScale / unit.
         float v_unit = 0x1p-25f, v_gain = kWeightScale * 0x1p25f;
 
-        // bit 63 of an entry (reserved, 0 in the directory) marks the page of the wait-expiry test: armed, never fetched
-        auto load_entry = [&](uint32_t page) -> uint64_t {
-            const uint32_t page_id = table_row[page];
-            const uint64_t entry = p.page_dir[static_cast<uint64_t>(page_id) * p.kv_head_count + kv_head];
-            return page_id == p.skip_copy_page ? entry | (1ull << 63) : entry;
-        };
-        auto issue = [&](uint64_t entry) {
-            const uint32_t units16 = static_cast<uint32_t>(CF_B200_DIR_LENGTH_UNITS(entry));
-            if (lane == 0 && units16 != 0 && units16 * 16u <= kStageBytes - 32u) {
-                mbar_expect_tx(bar, units16 * 16u);
-                if (!(entry >> 63)) bulk_load(warp_mem, p.arena + 16ull * CF_B200_DIR_OFFSET_UNITS(entry), units16 * 16u, bar);
-            }
-        };
-        auto entry_ok = [&](uint64_t entry) {
-            const uint32_t units16 = static_cast<uint32_t>(CF_B200_DIR_LENGTH_UNITS(entry));
-            return units16 != 0 && units16 * 16u <= kStageBytes - 32u;
-        };
-
-        uint64_t entry_cur = n_pages ? load_entry(page_begin) : 0ull;
-        uint64_t entry_next = n_pages > 1 ? load_entry(page_begin + 1) : 0ull;
-        __syncwarp();
-        issue(entry_cur);
         bool alive = true;
 
         for (uint32_t i = 0; i < n_pages; ++i) {
@@ -566,7 +564,9 @@ __global__ void __launch_bounds__(kThreadsOf<NG, NB, kSplitQ>, 1) lanes_attentio
                     }
                     if constexpr (kSplitQ) {   // K q = K binary16(q) + K residue
 #pragma unroll
-                        for (int c = 0; c < 4; ++c) u.score[0][c] += u.score[1][c];
+                        for (int n = 0; n < NS; ++n)
+#pragma unroll
+                            for (int c = 0; c < 4; ++c) u.score[n][c] += u.score[n + NS][c];
                     }
                     if constexpr (!kProbe) {
                     // ---- online softmax for this page (fp32), per group of four heads ----
@@ -745,13 +745,33 @@ bool lanes_kernel_supports(const AttentionParams &p) {
            (p.query_type == CF_B200_F16 || p.query_type == CF_B200_F32);
 }
 
-// Query groups of up to four heads per kv head run the four-head kernel; larger groups run the eight-head one, which
-// decodes a page once for eight query heads (its query operands live in shared memory instead of registers). fp32
-// queries (the reference's own ABIs pass nothing else) run the split-query kernel, four heads per pass.
 namespace {
+
+// Calls f with the kernel's template arguments for a launch. Query groups of up to four heads per kv head run the four-head kernel;
+// larger groups the eight-head one, which decodes a page once for eight query heads (a group of 16 in two passes). fp32
+// queries (the reference's own ABIs pass nothing else) take the forms with split queries.
+template <int NB, int kDim, class F>
+cudaError_t with_heads(const AttentionParams &p, F f) {
+    if (p.decode_probe == 2u) return f.template operator()<1, kDump, false, NB, kDim>();
+    if (p.decode_probe) return f.template operator()<1, kFold, false, NB, kDim>();
+    if (p.query_type == CF_B200_F32)
+        return p.group <= 4 ? f.template operator()<2, kAttend, true, NB, kDim>() : f.template operator()<4, kAttend, true, NB, kDim>();
+    return p.group <= 4 ? f.template operator()<1, kAttend, false, NB, kDim>() : f.template operator()<2, kAttend, false, NB, kDim>();
+}
+template <class F>
+cudaError_t with_variant(const AttentionParams &p, F f) {
+    // 16 x 64 pages have 16 (or 8) blocks per stream, 16 x 96 pages 24 (or 12), 16 x 32 pages 8: always staged
+    if (p.head_dim == 64) return p.block_size == 64 ? with_heads<16, 64>(p, f) : with_heads<8, 64>(p, f);
+    if (p.head_dim == 96) return p.block_size == 64 ? with_heads<24, 96>(p, f) : with_heads<12, 96>(p, f);
+    if (p.head_dim == 32) return with_heads<8, 32>(p, f);
+    if (p.block_size == 128) return with_heads<16, 128>(p, f);
+    if (p.block_size == 256) return with_heads<8, 128>(p, f);
+    return with_heads<32, 128>(p, f);
+}
 
 template <int NG, int kMode, bool kSplitQ, int NB, int kDim>
 cudaError_t launch_one(const AttentionParams &p, int sm_count, cudaStream_t stream, bool dependent, bool after_prefix) {
+    using L = WarpLayout<NG, NB, kSplitQ, kDim>;
     static std::atomic<uint64_t> configured{0};   // bit = device ordinal
     int device = 0;
     cudaError_t e = cudaGetDevice(&device);
@@ -759,32 +779,23 @@ cudaError_t launch_one(const AttentionParams &p, int sm_count, cudaStream_t stre
     const uint64_t bit = 1ull << (device & 63);
     if (!(configured.load(std::memory_order_acquire) & bit)) {
         e = cudaFuncSetAttribute(lanes_attention_kernel<NG, kMode, kSplitQ, NB, kDim>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(WarpLayout<NG, NB, kSplitQ>::kSmem));
+                                 static_cast<int>(L::kSmem));
         if (e != cudaSuccess) return e;
         configured.fetch_or(bit, std::memory_order_release);
     }
-    return launch_kernel(lanes_attention_kernel<NG, kMode, kSplitQ, NB, kDim>, sm_count, kThreadsOf<NG, NB, kSplitQ>, WarpLayout<NG, NB, kSplitQ>::kSmem,
+    return launch_kernel(lanes_attention_kernel<NG, kMode, kSplitQ, NB, kDim>, sm_count, kThreadsOf<NG, NB, kSplitQ, kDim>, L::kSmem,
                          stream, dependent, p, static_cast<uint32_t>(after_prefix));
-}
-
-template <int NB, int kDim = 128>
-cudaError_t launch_for_blocks(const AttentionParams &p, int sm_count, cudaStream_t stream, bool dependent, bool after_prefix) {
-    if (p.decode_probe == 2u) return launch_one<1, kDump, false, NB, kDim>(p, sm_count, stream, dependent, after_prefix);
-    if (p.decode_probe) return launch_one<1, kFold, false, NB, kDim>(p, sm_count, stream, dependent, after_prefix);
-    if (p.query_type == CF_B200_F32) return launch_one<2, kAttend, true, NB, kDim>(p, sm_count, stream, dependent, after_prefix);
-    if (p.group <= 4) return launch_one<1, kAttend, false, NB, kDim>(p, sm_count, stream, dependent, after_prefix);
-    return launch_one<2, kAttend, false, NB, kDim>(p, sm_count, stream, dependent, after_prefix);
 }
 
 }  // namespace
 
 void lanes_plan_shape(const AttentionParams &p, uint32_t sm_count, uint32_t *warps, uint32_t *unit_lanes) {
-    const bool split_q = p.query_type == CF_B200_F32 && !p.decode_probe;
-    const bool eight = !split_q && p.group > 4u && !p.decode_probe;   // query heads per pass: eight, else four
-    const bool staged = p.block_size != 64u || p.head_dim != 128u;
-    const int per_sm = staged ? (split_q || eight ? kWarpsOf<2, 16> : kWarpsOf<1, 16>) : split_q ? kWarpsOf<2, 32, true> : eight ? kWarpsOf<2> : kWarpsOf<1>;
-    *warps = sm_count * static_cast<uint32_t>(per_sm);
-    *unit_lanes = p.kv_head_span * (eight ? (p.group + 7u) / 8u : (p.group + 3u) / 4u);
+    with_variant(p, [&]<int NG, int kMode, bool kSplitQ, int NB, int kDim>() {
+        constexpr uint32_t kHeads = 4u * kHeadGroups<NG, kSplitQ>;
+        *warps = sm_count * kWarpsOf<NG, NB, kSplitQ, kDim>;
+        *unit_lanes = p.kv_head_span * ((p.group + kHeads - 1u) / kHeads);
+        return cudaSuccess;
+    });
 }
 
 cudaError_t launch_lanes_attention(const AttentionParams &p, cudaStream_t stream, bool dependent, bool after_prefix) {
@@ -792,18 +803,10 @@ cudaError_t launch_lanes_attention(const AttentionParams &p, cudaStream_t stream
     cudaError_t e;
     LauncherState *state = launcher_state(table, &e);
     if (!state) return e;
-    if (p.head_dim == 64) {   // 16 x 64 pages: 16 (or 8) blocks per stream, always staged
-        return p.block_size == 64 ? launch_for_blocks<16, 64>(p, state->sm_count, stream, dependent, after_prefix)
-                                  : launch_for_blocks<8, 64>(p, state->sm_count, stream, dependent, after_prefix);
-    }
-    if (p.head_dim == 96) {
-        return p.block_size == 64 ? launch_for_blocks<24, 96>(p, state->sm_count, stream, dependent, after_prefix)
-                                  : launch_for_blocks<12, 96>(p, state->sm_count, stream, dependent, after_prefix);
-    }
-    if (p.head_dim == 32) return launch_for_blocks<8, 32>(p, state->sm_count, stream, dependent, after_prefix);
-    if (p.block_size == 128) return launch_for_blocks<16>(p, state->sm_count, stream, dependent, after_prefix);
-    if (p.block_size == 256) return launch_for_blocks<8>(p, state->sm_count, stream, dependent, after_prefix);
-    return launch_for_blocks<32>(p, state->sm_count, stream, dependent, after_prefix);
+    const int sm_count = state->sm_count;
+    return with_variant(p, [&]<int NG, int kMode, bool kSplitQ, int NB, int kDim>() {
+        return launch_one<NG, kMode, kSplitQ, NB, kDim>(p, sm_count, stream, dependent, after_prefix);
+    });
 }
 
 }  // namespace cfb

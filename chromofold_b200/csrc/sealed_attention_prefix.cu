@@ -743,7 +743,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) prefix_attention_kernel(Attenti
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + kOffBars);
     uint32_t *misc = reinterpret_cast<uint32_t *>(smem + kOffMisc);
 
-    load_tables(smem, p, tid, kTcThreads);   // the caller's: needs nothing of the plan kernel
+    load_tables<kTcThreads>(smem, p, tid);   // the caller's: needs nothing of the plan kernel
     wait_for_previous_kernel();
     // From here on the plan is complete, so the per-sequence kernel may take over every SM this kernel leaves.
     allow_dependent_launch();
