@@ -90,6 +90,14 @@ __host__ __device__ inline uint32_t shared_split_ctas(uint32_t rounds, uint32_t 
     return head_tiles * (cells - 1u);
 }
 
+// The row tiles of a launch: tiles of 128 (entry, query head) rows, taken by single CTAs, or, from two on, in groups of two by
+// pairs of CTAs that share what they decode. The split above is then one of pairs over (kv head, group of tiles).
+__host__ __device__ inline uint32_t shared_cluster(uint32_t rows) { return rows > 128u ? 2u : 1u; }
+__host__ __device__ inline uint32_t shared_tile_groups(uint32_t rows) {
+    const uint32_t per_group = 128u * shared_cluster(rows);
+    return (rows + per_group - 1u) / per_group;
+}
+
 // What is known of a batch entry, written by the plan kernel so that later kernels read two 16-byte words instead of chasing
 // slot -> counts -> position.
 struct SeqInfo {
@@ -188,18 +196,30 @@ __device__ __forceinline__ void wait_for_previous_kernel() { asm volatile("gridd
 __device__ __forceinline__ void allow_dependent_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 template <class... KernelArgs, class... Args>
-inline cudaError_t launch_kernel(void (*kernel)(KernelArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, bool dependent, Args... args) {
+inline cudaError_t launch_in_clusters(uint32_t cluster, void (*kernel)(KernelArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                                      bool dependent, Args... args) {
     cudaLaunchConfig_t config = {};
     config.gridDim = grid;
     config.blockDim = block;
     config.dynamicSmemBytes = smem;
     config.stream = stream;
-    cudaLaunchAttribute attribute;
-    attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attribute.val.programmaticStreamSerializationAllowed = 1;
-    config.attrs = &attribute;
-    config.numAttrs = dependent ? 1 : 0;
+    cudaLaunchAttribute attributes[2];
+    config.attrs = attributes;
+    if (dependent) {
+        attributes[config.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attributes[config.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1u) {
+        attributes[config.numAttrs].id = cudaLaunchAttributeClusterDimension;
+        attributes[config.numAttrs].val.clusterDim.x = cluster;
+        attributes[config.numAttrs].val.clusterDim.y = attributes[config.numAttrs].val.clusterDim.z = 1;
+        ++config.numAttrs;
+    }
     return cudaLaunchKernelEx(&config, kernel, static_cast<KernelArgs>(args)...);
+}
+template <class... KernelArgs, class... Args>
+inline cudaError_t launch_kernel(void (*kernel)(KernelArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, bool dependent, Args... args) {
+    return launch_in_clusters(1u, kernel, grid, block, smem, stream, dependent, args...);
 }
 
 __device__ __forceinline__ float warp_sum(float v) {

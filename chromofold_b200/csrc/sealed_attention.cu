@@ -101,9 +101,9 @@ __global__ void __launch_bounds__(kPlanThreads) plan_kernel(AttentionParams p) {
     }
     uint32_t shared_ctas = 0, shared_rounds = 0;
     if (shared) {   // an even split of the prefix's rounds over the CTAs of the shared-prefix kernel (SharedSplit)
-        const uint32_t row_tiles = (p.seq_count * p.group + 127u) / 128u;
+        const uint32_t rows = p.seq_count * p.group;
         shared_rounds = (shared + 7u) / 8u;
-        shared_ctas = shared_split_ctas(shared_rounds, p.kv_head_span * row_tiles, p.sm_count, CF_B200_SHARED_CHUNKS_MAX);
+        shared_ctas = shared_split_ctas(shared_rounds, p.kv_head_span * shared_tile_groups(rows), p.sm_count / shared_cluster(rows), CF_B200_SHARED_CHUNKS_MAX);
         if (shared_ctas == 0u) shared = 0;   // no CTA to take it: the pages stay on the line
     }
 
@@ -415,9 +415,10 @@ __device__ __forceinline__ RowPartials row_partials(const AttentionParams &p, co
     static_assert(sizeof(PageLine) == 28 && offsetof(PlanHeader, shared_pages) == 32 && offsetof(PlanHeader, shared_rounds) == 40, "");
     const uint4 shared = __ldcg(reinterpret_cast<const uint4 *>(p.workspace) + 2);
     if (shared.x != 0u && shared.y != 0u) {
-        const uint32_t row_tiles = (p.seq_count * p.group + 127u) / 128u;
-        const SharedSplit split = {shared.z, p.kv_head_span * row_tiles, shared.y};
-        const uint64_t first = static_cast<uint64_t>((local_q / p.group) * row_tiles + (seq * p.group + local_q % p.group) / 128u) * split.rounds;
+        const uint32_t rows = p.seq_count * p.group, groups = shared_tile_groups(rows);
+        const SharedSplit split = {shared.z, p.kv_head_span * groups, shared.y};
+        const uint64_t first =
+            static_cast<uint64_t>((local_q / p.group) * groups + (seq * p.group + local_q % p.group) / (128u * shared_cluster(rows))) * split.rounds;
         rp.cells = min(split.cta_of(first + split.rounds - 1u) - split.cta_of(first) + 1u, CF_B200_SHARED_CHUNKS_MAX);
     }
     return rp;
@@ -1108,8 +1109,8 @@ cf_status cfb::sealed_attention_stages(const cf_b200_sealed_attention_desc *d, u
         p.plan_warps = p.sm_count * cfb::kGenericCtasPerSm;
         p.unit_lanes = p.kv_head_span;
     }
-    // the shared-prefix kernel works on rows of 128 = whole query groups and on pages every query token sees in full
-    if (use_lanes && p.block_size == 64 && p.head_dim == 128 && d->row_map == nullptr && p.decode_probe != 1u && d->shared_prefix_pages && d->causal_window == 0 && 128u % p.group == 0)
+    // the shared-prefix kernel works on whole records of 16 x 128 or 16 x 64 symbols in blocks of 64, and on pages without a window
+    if (use_lanes && p.block_size == 64 && (p.head_dim == 128 || p.head_dim == 64) && d->row_map == nullptr && p.decode_probe != 1u && d->shared_prefix_pages && d->causal_window == 0)
         p.shared_prefix_pages = d->shared_prefix_pages;
     const bool plan = (stages & CF_B200_STAGE_PLAN) != 0, attention = (stages & CF_B200_STAGE_ATTENTION) != 0;
     if (plan && cfb::launch_plan(p, s) != cudaSuccess) return CF_ERR_CUDA;

@@ -1,14 +1,17 @@
 // sealed_attention_prefix.cu — attention over a SHARED sealed prefix: pages that every sequence of the batch
 // references (one copy in the arena, the same page ids at the head of every page-table row; the reference's
-// shared-page semantics, src/multisequence_cache.cpp:235-292), on the 5th-generation tensor cores (tcgen05.mma with
-// accumulators and the A operands in tensor memory). Geometry: head_dim 128, page_tokens 16, block 64.
+// shared-page semantics, src/multisequence_cache.cpp:235-292), or that the query tokens of one sequence share, on the
+// 5th-generation tensor cores (tcgen05.mma with accumulators and the A operands in tensor memory). Geometry: head_dim 128 or
+// 64, page_tokens 16, block 64.
 //
 // The per-sequence kernel would decode such a page once per sequence. Here a page is decoded once per tile of 128
 // query rows (rows = sequence x query head of the kv head's group) and contracted with all those rows at once.
 //
 // One CTA of 20 warps per SM. The work is cut evenly (SharedSplit): the rounds (8 pages = 128 tokens) of every
 // (kv head, row tile) pair form one line and each CTA takes an equal stretch of it; the part of a stretch inside one
-// pair is a unit, which ends in one partial per row. The warps are specialised:
+// pair is a unit, which ends in one partial per row. From two row tiles on, two CTAs (a cluster) take a stretch together, a row
+// tile each: each decodes half of every round's pages and stores them in both, so that a page is decoded once per 256 rows.
+// The warps are specialised:
 //   decoder warps 0..11  the page slots of the CTA's units form one sequence; warp w takes slots w, w + 12, ... It
 //                        receives the record by one bulk async copy (mbarrier, bounded wait), decodes it with the
 //                        lane-per-block decoders INTO REGISTERS (32 packed quads per lane), starts the copy of its next
@@ -16,31 +19,30 @@
 //                        are written as exact binary16 codes into one of TWO tile pairs in shared memory: K tile
 //                        [token][channel] (B of S = Q K^T), V tile [channel][token] (B of O = P V); then the warp
 //                        arrives on the pair's "full" barrier (8 arrivals = one round). A pair is free when the tensor
-//                        core's commit for the round that read it has arrived on its "free" barrier. Twelve warps keep
-//                        decoding while the other group works on the previous round.
+//                        core's commit for the round that read it has arrived on its "free" barrier.
 //   softmax warps 12..19 a thread owns one row (= tensor-memory lane, in its warp's quarter) and half of the round's
-//                        128 score columns. Thread 0 of the group issues the tensor-core work:
-//                          S     8 tcgen05.mma (M 128, N 128, K 16): Q from tensor memory x K tile -> columns 0..127
-//                          O    16 tcgen05.mma: P (binary16, then its rounding residue) from tensor memory x V tile
-//                                -> columns 128..255, then commits to the "O" barrier and the pair's "free" barrier
-//                        All threads: one tcgen05.ld of their 64 scores (kept in registers), page K scales and masks,
+//                        128 score columns: one tcgen05.ld of its 64 scores (kept in registers), page K scales and masks,
 //                        the row's two threads share their maxima through shared memory, running max / sum updated,
 //                        O rescaled in tensor memory (tcgen05.ld / .st) only when some row of the warp moved its max,
-//                        P and its residue written to tensor memory (tcgen05.st) as the next A operands.
+//                        P and its residue written over the scores (tcgen05.st) as the next A operands.
+//                        Thread 0 of the group issues the tensor-core work (M 128, K 16 per instruction):
+//                          S     Q from tensor memory x K tile -> one of two sets of 128 score columns
+//                          O     16 tcgen05.mma: P (binary16, then its rounding residue) from tensor memory x V tile
 //                        Unit start: the Q rows go from global memory straight to tensor memory. Unit end: O read back,
 //                        scaled, written with (max, sum) to the shared-prefix partials; the combine kernel merges
 //                        them with the per-sequence partials of the private pages and the tail.
 // Registers: the kernel starts at 96 per thread; the decoders drop to 80 and the softmax warps rise to 120 (setmaxnreg).
-// Tensor memory (512 columns): S 0..127, O 128..255, Q 256..319, P 320..383, P residue 384..447, Q residue 448..511 (fp32
-// queries only: the row is split into binary16(q) and its rounding residue, S = Q K^T + Q residue K^T) (binary16 pairs per
-// column, row = lane). B tiles use the no-swizzle K-major canonical layout: 8 rows x 16 bytes core matrices, element
-// (row r, 16-byte chunk c) at (r % 8) * 16 + (r / 8) * 2048 + c * 128 bytes.
+// Tensor memory (512 columns): scores and weights of even rounds 0..127, of odd rounds 128..255 (P 64 columns of binary16 pairs, then
+// its residue), O 256..383, Q 384..447, Q residue 448..511 (fp32 queries only: the row is split into binary16(q) and its
+// rounding residue, S = Q K^T + Q residue K^T). Row = lane. B tiles use the no-swizzle K-major canonical layout: 8 rows x 16
+// bytes core matrices, element (row r, 16-byte chunk c) at (r % 8) * 16 + (r / 8) * 2048 + c * 128 bytes.
+// Head_dim 64 runs the same kernel on the left half of the K tile and the upper half of the V tile.
 // The page's V scale relative to the largest one met so far in the unit rides on P (never above 1, so the binary16
 // weights cannot overflow); O is kept in units of that scale and rescaled when a larger one arrives.
 // Every mbarrier wait is bounded. A warp whose wait ran out raises CF_B200_DEVSTAT_WAIT_EXPIRED and skips all later
-// waits and work; a decoder warp still arrives for each of its slots, a softmax warp still takes part in its group's
-// barriers, which OR-reduce the failure so that the whole group leaves its loop at the same point; the CTA then frees
-// its tensor memory.
+// waits and work; a decoder warp still arrives for each of its slots, a softmax warp still takes part in the barrier with its
+// partner, which OR-reduces the failure so that both leave their loops at the same point, and the roles that wait for
+// them run out of their own waits; the CTA then frees its tensor memory.
 
 #include "lanes_decoders.cuh"
 
@@ -52,25 +54,26 @@ using namespace lanes;
 constexpr int kDecodeWarps = 12;     // warps 0..11 (three warpgroups)
 constexpr int kSoftmaxWarps = 8;     // warps 12..19 (two warpgroups)
 constexpr int kRoundPages = 8;
-constexpr int kGroupThreads = kSoftmaxWarps * 32;
 constexpr int kTcThreads = (kDecodeWarps + kSoftmaxWarps) * 32;
 constexpr uint32_t kTileBytes = 128 * 128 * 2;   // one operand tile: 128 rows x 128 binary16
+// A stage takes the largest record. The decoders look up to two words past a part's end: there the next stage begins, or the tiles,
+// and what they find is not used.
+constexpr uint32_t kRecordBytes = 16 + 2 * 2048;
 constexpr uint32_t kOffStages = kTableBytes;
-constexpr uint32_t kOffTiles = (kOffStages + kDecodeWarps * kStageBytes + 127u) / 128u * 128u;   // K[0] V[0] K[1] V[1]
+constexpr uint32_t kOffTiles = (kOffStages + kDecodeWarps * kRecordBytes + 127u) / 128u * 128u;   // K[0] V[0] K[1] V[1]
 constexpr uint32_t kOffMeta = kOffTiles + 4 * kTileBytes;      // [pair][page of the round]: k scale, v scale, token count, -
 constexpr uint32_t kOffRound = kOffMeta + 2 * kRoundPages * 16;    // [pair]: unit, flags, -, -
-constexpr uint32_t kOffBars = kOffRound + 2 * 16;              // 12 copy barriers, full[2], free[2], S, O
-constexpr uint32_t kBarFull = kDecodeWarps, kBarFree = kBarFull + 2, kBarS = kBarFree + 2, kBarO = kBarS + 1, kBarCount = kBarO + 1;
+constexpr uint32_t kOffBars = kOffRound + 2 * 16;              // 12 copy barriers, full[2], free[4], S[2], O[2]
+constexpr uint32_t kBarFull = kDecodeWarps, kBarFree = kBarFull + 2, kBarS = kBarFree + 4, kBarO = kBarS + 2, kBarCount = kBarO + 2;
 constexpr uint32_t kOffMisc = kOffBars + kBarCount * 8;        // [0] tmem base
-constexpr uint32_t kOffRowMax = kOffMisc + 32;                 // [2 column halves][128 rows]
-constexpr uint32_t kTcSmem = kOffRowMax + 2 * 128 * 4;
+constexpr uint32_t kOffRowMax = kOffMisc + 32;                 // [round parity][2 column halves][128 rows]
+constexpr uint32_t kTcSmem = kOffRowMax + 4 * 128 * 4;
 static_assert(kTcSmem <= 232448, "the shared-prefix kernel must fit the 227 KB of one CTA");
 constexpr uint32_t kTmemColumns = 512;
-constexpr uint32_t kColS = 0, kColO = 128, kColQ = 256, kColP = 320, kColPResidue = 384, kColQResidue = 448;
+constexpr uint32_t kColS = 0, kColO = 256, kColQ = 384, kColQResidue = 448;
 constexpr uint32_t kStopUnit = 0xffffffffu;
 constexpr float kWeightScale = 32768.0f;   // power of two the binary16 weights are scaled by (O sheds it at a unit's end)
 constexpr uint32_t kFirstRound = 1u, kLastRound = 2u;   // round flags
-constexpr uint32_t kSoftmaxBarrier = 1;   // named barrier (0 is __syncthreads)
 // Register split (setmaxnreg). A CTA can only redistribute the registers it was launched with: kLaunchRegs per thread,
 // the most that 640 threads can have. What the softmax warps ask for must not exceed what the decoders give back, or
 // the request would wait forever; the launch function checks kLaunchRegs against the compiled kernel.
@@ -78,8 +81,9 @@ constexpr int kLaunchRegs = 96, kDecoderRegs = 80, kSoftmaxRegs = 120;
 static_assert(kLaunchRegs * kTcThreads <= 65536 && kDecoderRegs % 8 == 0 && kSoftmaxRegs % 8 == 0 &&
                   kDecodeWarps * 32 * kDecoderRegs + kSoftmaxWarps * 32 * kSoftmaxRegs <= kLaunchRegs * kTcThreads,
               "the register split must fit the CTA's own registers");
-// instruction descriptor: f32 accumulate, f16 x f16, both operands K-major, N = 128, M = 128
-constexpr uint32_t kIdesc = (1u << 4) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
+// instruction descriptors: f32 accumulate, f16 x f16, both operands K-major, M = 128; N = 128 tokens (S) or kDim channels (O)
+constexpr uint32_t kIdescS = (1u << 4) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
+template <int kDim> constexpr uint32_t kIdescO = (1u << 4) | ((static_cast<uint32_t>(kDim) >> 3) << 17) | ((128u >> 4) << 24);
 
 __device__ __forceinline__ uint32_t tile_offset(uint32_t row, uint32_t chunk) {
     return (row & 7u) * 16u + (row >> 3) * 2048u + chunk * 128u;
@@ -96,20 +100,67 @@ __device__ __forceinline__ uint64_t tile_desc(uint32_t smem_address) {
            (static_cast<uint64_t>(2048u >> 4) << 32) | (1ull << 46);
 }
 // D[tmem_d] (+)= A[tmem_a: 128 lanes x 8 columns of binary16 pairs] x B[shared-memory tile]^T, one K step of 16
-__device__ __forceinline__ void umma(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t accumulate) {
+__device__ __forceinline__ void umma(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t accumulate, uint32_t idesc) {
     asm volatile(
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d),
-        "r"(tmem_a), "l"(desc_b), "r"(kIdesc), "r"(accumulate)
+        "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
         : "memory");
 }
 __device__ __forceinline__ void umma_commit(uint64_t *bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_addr(bar)) : "memory");
 }
+// A pair of CTAs (a cluster of two) shares the decoded pages: each decodes every other half round and stores it in both.
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ uint32_t peer_address(uint32_t smem_address, uint32_t rank) {   // the same place in CTA `rank` of the pair
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_address), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void store_peer(uint32_t address, uint4 v) {
+    asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(address), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive_peer(uint32_t address) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(address) : "memory");
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// Waits and polls that also see what the other CTA of the pair stored before it arrived.
+__device__ __forceinline__ bool mbar_wait_pair(uint64_t *bar, uint32_t parity, uint32_t polls) {
+    for (uint32_t i = 0; i < polls; ++i) {
+        uint32_t ok;
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                     : "=r"(ok)
+                     : "r"(smem_addr(bar)), "r"(parity), "r"(1000u)
+                     : "memory");
+        if (ok) return true;
+    }
+    return false;
+}
+__device__ __forceinline__ bool mbar_test_pair(uint64_t *bar, uint32_t parity) {   // one poll that does not wait
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok)
+                 : "r"(smem_addr(bar)), "r"(parity)
+                 : "memory");
+    return ok != 0;
+}
 __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
 }
-// Barrier over one group (whole warps) that also ORs a predicate: every thread of the group gets the same answer.
+// The same, for both CTAs of the pair.
+__device__ __forceinline__ void umma_commit_pair(uint64_t *bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_addr(bar)),
+                 "h"(static_cast<uint16_t>(3))
+                 : "memory");
+}
+// Barrier over whole warps that also ORs a predicate: every thread of them gets the same answer.
+template <uint32_t kThreads>
 __device__ __forceinline__ bool group_any(uint32_t barrier_id, bool pred) {
     uint32_t r;
     asm volatile(
@@ -117,7 +168,7 @@ __device__ __forceinline__ bool group_any(uint32_t barrier_id, bool pred) {
         "bar.red.or.pred q, %2, %3, p;\n\t"
         "selp.u32 %0, 1, 0, q;\n\t}"
         : "=r"(r)
-        : "r"(static_cast<uint32_t>(pred)), "r"(barrier_id), "r"(static_cast<uint32_t>(kGroupThreads))
+        : "r"(static_cast<uint32_t>(pred)), "r"(barrier_id), "r"(kThreads)
         : "memory");
     return r != 0;
 }
@@ -144,7 +195,11 @@ __device__ __forceinline__ void tmem_store32(uint32_t taddr, const uint32_t (&v)
         "r"(v[31])
         : "memory");
 }
-__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+template <int kCluster>
+__device__ __forceinline__ void fence_async_smem() {
+    if constexpr (kCluster == 1) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    else asm volatile("fence.proxy.async;" ::: "memory");
+}
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
@@ -171,7 +226,19 @@ __device__ __forceinline__ void decode_page(KLane &k, VLane &v, uint32_t (&kq)[1
         }
 #pragma unroll
         for (int q = 12; q < 16; ++q) {
-            if constexpr (KLane::kWholeQuads || VLane::kWholeQuads) {   // fixed width or nibble-split: a quad per call
+            if constexpr (requires { k.lo_word(0); v.lo_word(0); }) {   // both nibble-split: two steps per quad, the chains interleave
+                uint32_t ke[2], ve[2];
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    ke[i] = k.symbol(i);
+                    ve[i] = v.symbol(i);
+                }
+                k.advance();
+                v.advance();
+                const int j = 2 * pass + ((q - 12) >> 1), shift = 4 * (q & 1);
+                kq[q] = merge_split_quad(ke[0], ke[1], k.lo_word(j) >> shift);
+                vq[q] = merge_split_quad(ve[0], ve[1], v.lo_word(j) >> shift);
+            } else if constexpr (KLane::kWholeQuads || VLane::kWholeQuads) {   // fixed width: a quad per call
                 kq[q] = k.quad(4 * pass + (q - 12));
                 vq[q] = v.quad(4 * pass + (q - 12));
             } else {   // both entropy coded: the two chains interleave symbol by symbol
@@ -199,29 +266,62 @@ __device__ __forceinline__ void decode_stream(Lane &s, uint32_t (&quads)[16]) {
 // The decoded page goes into slot `slot` of the round's tiles as exact binary16 codes. K quad q of lane l = token l/2,
 // channels 64(l&1)+4q..+3 -> K tile row 16*slot + l/2; V quad q of lane l = channel 4l + q/4, tokens 4(q%4)..+3 -> V tile
 // row v_tile_row(l, q/4), token chunks 2*slot and 2*slot+1.
-__device__ __forceinline__ void store_tiles(const uint32_t (&kq)[16], const uint32_t (&vq)[16], uint8_t *k_tile, uint8_t *v_tile,
-                                            uint32_t slot, uint32_t lane) {
+template <int kCluster>
+__device__ __forceinline__ void store_codes(uint8_t *at, uint4 codes, uint32_t peer_delta) {
+    *reinterpret_cast<uint4 *>(at) = codes;
+    if constexpr (kCluster == 2) store_peer(smem_addr(at) + peer_delta, codes);
+}
+// A page that is absent (past the unit's end, or refused) leaves zeros in its slot of both tiles.
+template <int kCluster>
+__device__ __forceinline__ void store_tiles(const uint32_t (&kq)[16], const uint32_t (&vq)[16], bool present, uint8_t *k_tile, uint8_t *v_tile,
+                                            uint32_t slot, uint32_t lane, uint32_t peer_delta) {
     const uint32_t k_row = 16u * slot + (lane >> 1);
+    auto put = [&](uint8_t *at, uint32_t qa, uint32_t qb) { store_codes<kCluster>(at, present ? codes8(qa, qb) : make_uint4(0u, 0u, 0u, 0u), peer_delta); };
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
         const uint32_t k_chunk = 8u * (lane & 1u) + 2u * c;
-        *reinterpret_cast<uint4 *>(k_tile + tile_offset(k_row, k_chunk)) = codes8(kq[4 * c], kq[4 * c + 1]);
-        *reinterpret_cast<uint4 *>(k_tile + tile_offset(k_row, k_chunk + 1u)) = codes8(kq[4 * c + 2], kq[4 * c + 3]);
+        put(k_tile + tile_offset(k_row, k_chunk), kq[4 * c], kq[4 * c + 1]);
+        put(k_tile + tile_offset(k_row, k_chunk + 1u), kq[4 * c + 2], kq[4 * c + 3]);
         const uint32_t v_row = v_tile_row(lane, c);
-        *reinterpret_cast<uint4 *>(v_tile + tile_offset(v_row, 2u * slot)) = codes8(vq[4 * c], vq[4 * c + 1]);
-        *reinterpret_cast<uint4 *>(v_tile + tile_offset(v_row, 2u * slot + 1u)) = codes8(vq[4 * c + 2], vq[4 * c + 3]);
+        put(v_tile + tile_offset(v_row, 2u * slot), vq[4 * c], vq[4 * c + 1]);
+        put(v_tile + tile_offset(v_row, 2u * slot + 1u), vq[4 * c + 2], vq[4 * c + 3]);
     }
 }
-// A page that is absent (past the chunk's end, or refused) leaves zeros in its slot of both tiles.
-__device__ __forceinline__ void zero_slot(uint8_t *k_tile, uint8_t *v_tile, uint32_t slot, uint32_t lane) {
-    const uint4 z = make_uint4(0u, 0u, 0u, 0u);
-    const uint32_t k_row = 16u * slot + (lane >> 1);
+// Head_dim 64: a stream has sixteen blocks, a lane decodes one block of one stream. K block l = token l, V block l = channels
+// 4 l .. 4 l + 3 of every token.
+__device__ __forceinline__ void decode_half(const uint8_t *part, uint32_t part_bytes, uint32_t coder, uint32_t block, const uint32_t *slot_table,
+                                            const uint16_t *lut, uint32_t (&quads)[16]) {
+    if (coder == CF_B200_CODER_RANS_SPLIT4) {
+        RansSplitLaneT<16, 1024> d;
+        d.open(part, part_bytes, block, slot_table);
+        decode_stream(d, quads);
+    } else if (coder == CF_B200_CODER_HUFFMAN_SPLIT4) {
+        HuffSplitLaneT<16, 1024> d;
+        d.open(part, part_bytes, block, lut);
+        decode_stream(d, quads);
+    } else if (coder == CF_B200_CODER_RANS) {
+        RansLaneT<16> d;
+        d.open(part, part_bytes, block, slot_table);
+        decode_stream(d, quads);
+    } else if (coder == CF_B200_CODER_HUFFMAN) {
+        HuffLaneT<16> d;
+        d.open(part, part_bytes, block, lut);
+        decode_stream(d, quads);
+    } else {
+        FixedLaneT<16, 1024> d;
+        d.open(part, part_bytes, block);
+        decode_stream(d, quads);
+    }
+}
+template <int kCluster>
+__device__ __forceinline__ void store_half(const uint32_t (&quads)[16], bool present, uint8_t *k_tile, uint8_t *v_tile, uint32_t slot, uint32_t lane,
+                                           uint32_t peer_delta) {
+    const uint32_t l = lane & 15u;
 #pragma unroll
-    for (int c = 0; c < 8; ++c) *reinterpret_cast<uint4 *>(k_tile + tile_offset(k_row, 8u * (lane & 1u) + c)) = z;
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-        *reinterpret_cast<uint4 *>(v_tile + tile_offset(v_tile_row(lane, c), 2u * slot)) = z;
-        *reinterpret_cast<uint4 *>(v_tile + tile_offset(v_tile_row(lane, c), 2u * slot + 1u)) = z;
+    for (int c = 0; c < 8; ++c) {   // K: chunk c of token l's row; V: half c & 1 of channel 4 l + c / 2's sixteen tokens
+        const uint4 codes = present ? codes8(quads[2 * c], quads[2 * c + 1]) : make_uint4(0u, 0u, 0u, 0u);
+        uint8_t *at = lane < 16u ? k_tile + tile_offset(16u * slot + l, c) : v_tile + tile_offset(v_tile_row(l, c >> 1), 2u * slot + (c & 1));
+        store_codes<kCluster>(at, codes, peer_delta);
     }
 }
 
@@ -244,7 +344,7 @@ struct UnitShape {
     uint32_t tile_index, head_local, chunk, kv_head, page_begin, page_end, valid;
 };
 __device__ __forceinline__ UnitShape unit_shape(const AttentionParams &p, const SharedSplit &split, uint32_t cta, uint32_t unit,
-                                                uint32_t row_tiles, uint32_t shared_pages) {
+                                                uint32_t tile_groups, uint32_t shared_pages) {
     UnitShape u = {};
     const uint64_t lo = split.first_round(cta), hi = split.first_round(cta + 1u);
     const uint64_t head_tile = lo / split.rounds + unit, base = head_tile * split.rounds;
@@ -252,8 +352,8 @@ __device__ __forceinline__ UnitShape unit_shape(const AttentionParams &p, const 
     if (!u.valid) return u;
     const uint32_t r0 = static_cast<uint32_t>((lo > base ? lo : base) - base);
     const uint32_t r1 = static_cast<uint32_t>((hi < base + split.rounds ? hi : base + split.rounds) - base);
-    u.tile_index = static_cast<uint32_t>(head_tile % row_tiles);
-    u.head_local = static_cast<uint32_t>(head_tile / row_tiles);
+    u.tile_index = static_cast<uint32_t>(head_tile % tile_groups);   // of groups of kCluster tiles
+    u.head_local = static_cast<uint32_t>(head_tile / tile_groups);
     u.chunk = cta - split.cta_of(base);
     u.kv_head = p.kv_head_begin + u.head_local;
     u.page_begin = 8u * r0;
@@ -269,13 +369,18 @@ struct SlotCursor {
     UnitShape u;
 };
 
+template <int kDim, int kCluster>
 __device__ __forceinline__ void decoder_role(const AttentionParams &p, uint8_t *smem, PlanHeader *hdr, uint32_t warp, uint32_t lane,
-                                             uint32_t row_tiles, const SharedSplit &split) {
+                                             uint32_t tile_groups, const SharedSplit &split) {
+    const uint32_t worker = blockIdx.x / kCluster, rank = kCluster == 1 ? 0u : cluster_rank();
+    const uint32_t peer_delta = kCluster == 1 ? 0u : peer_address(smem_addr(smem), rank ^ 1u) - smem_addr(smem);   // own place -> the peer's
+    // this CTA's m-th slot: all of them, or its half of every round
+    auto slot_number = [&](uint32_t m) { return kCluster == 1 ? m : (m >> 2) * 8u + 4u * rank + (m & 3u); };
     const uint32_t *k_slot = reinterpret_cast<const uint32_t *>(smem);
     const uint32_t *v_slot = k_slot + 4096;
     const uint16_t *k_lut = reinterpret_cast<const uint16_t *>(v_slot + 4096);
     const uint16_t *v_lut = k_lut + 4096;
-    uint8_t *stage = smem + kOffStages + warp * kStageBytes;
+    uint8_t *stage = smem + kOffStages + warp * kRecordBytes;
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + kOffBars);
     uint64_t *bar = bars + warp, *bar_full = bars + kBarFull, *bar_free = bars + kBarFree;
     uint32_t *round_desc = reinterpret_cast<uint32_t *>(smem + kOffRound);
@@ -283,7 +388,7 @@ __device__ __forceinline__ void decoder_role(const AttentionParams &p, uint8_t *
     const uint32_t *table_row = p.page_table + static_cast<uint64_t>(slot_of(p, 0)) * p.page_table_stride;
 
     auto load_unit = [&](SlotCursor &c) {
-        c.u = unit_shape(p, split, blockIdx.x, c.unit, row_tiles, shared_pages);
+        c.u = unit_shape(p, split, worker, c.unit, tile_groups, shared_pages);
         c.valid = c.u.valid;
         if (c.valid) c.slots = (c.u.page_end - c.u.page_begin + 7u) / 8u * 8u;
     };
@@ -306,7 +411,7 @@ __device__ __forceinline__ void decoder_role(const AttentionParams &p, uint8_t *
     };
     auto entry_ok = [&](uint64_t entry) {
         const uint32_t units16 = static_cast<uint32_t>(CF_B200_DIR_LENGTH_UNITS(entry));
-        return units16 != 0 && units16 * 16u <= kStageBytes - 32u;
+        return units16 != 0 && units16 * 16u <= kRecordBytes;
     };
     auto issue = [&](uint64_t entry) {
         if (lane == 0 && entry_ok(entry)) {
@@ -317,13 +422,23 @@ __device__ __forceinline__ void decoder_role(const AttentionParams &p, uint8_t *
     };
     uint32_t copy_phase = 0;
     bool failed = false;   // warp-uniform; once set, the warp waits for nothing and decodes nothing, but keeps arriving
-    // The pair of round `it` is free once the tensor core has finished round it - 2. The parity wait is sound because a
-    // warp's slots are 12 apart, less than two rounds: it has always seen the completion before the one it waits for.
+    // The pair of round `it` is free once the tensor core (of both CTAs) has finished round it - 2, which the barrier of that round's
+    // number modulo four tells. The parity wait is sound because a warp's slots are at most three rounds apart, so that it has
+    // seen the end of a round later than it - 6, the barrier's previous one.
     auto wait_pair_free = [&](uint32_t it) {
-        if (it >= 2u && !failed && !__all_sync(0xffffffffu, mbar_wait(&bar_free[it & 1u], ((it >> 1) - 1u) & 1u, p.wait_polls))) {
+        if (it >= 2u && !failed && !__all_sync(0xffffffffu, mbar_wait_pair(&bar_free[(it - 2u) & 3u], ((it - 2u) >> 2) & 1u, p.wait_polls))) {
             failed = true;
             if (lane == 0) raise_status(p, CF_B200_DEVSTAT_WAIT_EXPIRED);
         }
+    };
+    auto arrive_full = [&](uint32_t pair) {
+        mbar_arrive(&bar_full[pair]);
+        if constexpr (kCluster == 2) mbar_arrive_peer(smem_addr(&bar_full[pair]) + peer_delta);
+    };
+    auto describe_round = [&](uint32_t pair, uint32_t unit, uint32_t flags) {
+        round_desc[4 * pair] = unit;
+        round_desc[4 * pair + 1] = flags;
+        if constexpr (kCluster == 2) store_peer(smem_addr(round_desc + 4 * pair) + peer_delta, make_uint4(unit, flags, 0u, 0u));
     };
 
     SlotCursor cur;
@@ -332,18 +447,18 @@ __device__ __forceinline__ void decoder_role(const AttentionParams &p, uint8_t *
     cur.first_round = 0;
     cur.slots = 0;
     load_unit(cur);
-    uint32_t n = warp;
+    uint32_t m = warp, n = slot_number(m);
     seek(cur, n);
     uint64_t entry = slot_entry(cur, n);
     issue(entry);
 
-    for (;; n += kDecodeWarps) {
+    for (;; m += kDecodeWarps, n = slot_number(m)) {
         if (!cur.valid) {   // past the last unit: the eight slots after it make the round that tells the softmax group to stop
             if (n < cur.first_slot + 8u) {
                 wait_pair_free(cur.first_round);
                 if (lane == 0) {
-                    if (n == cur.first_slot) round_desc[4 * (cur.first_round & 1u)] = kStopUnit;
-                    mbar_arrive(&bar_full[cur.first_round & 1u]);
+                    if (n == cur.first_slot) describe_round(cur.first_round & 1u, kStopUnit, 0u);
+                    arrive_full(cur.first_round & 1u);
                 }
             }
             break;
@@ -351,8 +466,9 @@ __device__ __forceinline__ void decoder_role(const AttentionParams &p, uint8_t *
         const uint32_t in_unit = n - cur.first_slot, slot = in_unit & 7u, it = cur.first_round + (in_unit >> 3), pair = it & 1u;
         // the warp's next slot: its directory entry is fetched now (dependent loads), needed only after this decode
         SlotCursor next = cur;
-        seek(next, n + kDecodeWarps);
-        const uint64_t next_entry = slot_entry(next, n + kDecodeWarps);
+        const uint32_t next_n = slot_number(m + kDecodeWarps);
+        seek(next, next_n);
+        const uint64_t next_entry = slot_entry(next, next_n);
 
         float k_scale = 0.0f, v_scale = 0.0f;
         uint32_t token_count = 0;
@@ -369,15 +485,20 @@ __device__ __forceinline__ void decoder_role(const AttentionParams &p, uint8_t *
                 const uint32_t k_bytes = 16u * (hv.x & 0xffffu), v_bytes = 16u * (hv.x >> 16);
                 const uint32_t k_coder = hv.y & 0xffu, v_coder = (hv.y >> 8) & 0xffu;
                 const uint8_t *k_part = stage + 16, *v_part = k_part + k_bytes;
-                if (!record_header_ok(hv, entry, p.codebook_id) ||
-                    !__all_sync(0xffffffffu, part_offsets_ok(k_part, k_coder, k_bytes, lane) &&
-                                                 part_offsets_ok(v_part, v_coder, v_bytes, lane))) {
+                bool tables_ok;
+                if constexpr (kDim == 128) tables_ok = part_offsets_ok(k_part, k_coder, k_bytes, lane) && part_offsets_ok(v_part, v_coder, v_bytes, lane);
+                else tables_ok = lane < 16u ? part_offsets_ok<16, 1024>(k_part, k_coder, k_bytes, lane) : part_offsets_ok<16, 1024>(v_part, v_coder, v_bytes, lane - 16u);
+                if (!record_header_ok(hv, entry, p.codebook_id) || !__all_sync(0xffffffffu, tables_ok)) {
                     if (lane == 0) raise_status(p, CF_B200_DEVSTAT_BAD_RECORD);
                 } else {
                     token_count = hv.y >> 16;
                     k_scale = __half2float(__ushort_as_half(static_cast<unsigned short>(hv.z & 0xffffu))) * (p.softmax_scale * kLog2e);
                     v_scale = __half2float(__ushort_as_half(static_cast<unsigned short>(hv.z >> 16)));
-                    if (k_coder == CF_B200_CODER_RANS && v_coder == CF_B200_CODER_RANS) {
+                    if constexpr (kDim == 64) {   // lanes 0..15: the K blocks, lanes 16..31: the V blocks
+                        const bool is_v = lane >= 16u;
+                        decode_half(is_v ? v_part : k_part, is_v ? v_bytes : k_bytes, is_v ? v_coder : k_coder, lane & 15u, is_v ? v_slot : k_slot,
+                                    is_v ? v_lut : k_lut, kq);
+                    } else if (k_coder == CF_B200_CODER_RANS && v_coder == CF_B200_CODER_RANS) {
                         RansLane k, v;
                         k.open(k_part, k_bytes, lane, k_slot);
                         v.open(v_part, v_bytes, lane, v_slot);
@@ -418,11 +539,11 @@ __device__ __forceinline__ void decoder_role(const AttentionParams &p, uint8_t *
                         const uint32_t page_id = table_row[cur.u.page_begin + in_unit];
                         if (page_id < p.dump_pages) {
                             uint32_t *dump = reinterpret_cast<uint32_t *>(p.output) +
-                                             (static_cast<uint64_t>(page_id) * p.kv_head_count + cur.u.kv_head) * 1024u + 16u * lane;
+                                             (static_cast<uint64_t>(page_id) * p.kv_head_count + cur.u.kv_head) * (8u * kDim) + 16u * lane;
 #pragma unroll
                             for (int q = 0; q < 16; ++q) {
                                 dump[q] = kq[q];
-                                dump[512 + q] = vq[q];
+                                if constexpr (kDim == 128) dump[512 + q] = vq[q];
                             }
                         }
                     }
@@ -434,21 +555,18 @@ __device__ __forceinline__ void decoder_role(const AttentionParams &p, uint8_t *
 
         wait_pair_free(it);
         uint8_t *k_tile = smem + kOffTiles + pair * 2u * kTileBytes, *v_tile = k_tile + kTileBytes;
-        if (token_count != 0u) store_tiles(kq, vq, k_tile, v_tile, slot, lane);
-        else zero_slot(k_tile, v_tile, slot, lane);
+        if constexpr (kDim == 128) store_tiles<kCluster>(kq, vq, token_count != 0u, k_tile, v_tile, slot, lane, peer_delta);
+        else store_half<kCluster>(kq, token_count != 0u, k_tile, v_tile, slot, lane, peer_delta);
         if (lane == 0) {
-            float *meta = reinterpret_cast<float *>(smem + kOffMeta) + pair * 32u + 4u * slot;
-            meta[0] = k_scale;
-            meta[1] = v_scale;
-            meta[2] = __uint_as_float(token_count);   // 0: the page contributes nothing
-            if (slot == 0) {
-                round_desc[4 * pair] = cur.unit;
-                round_desc[4 * pair + 1] = (in_unit < 8u ? kFirstRound : 0u) | (in_unit + 8u >= cur.slots ? kLastRound : 0u);
-            }
+            uint4 *meta = reinterpret_cast<uint4 *>(smem + kOffMeta) + pair * 8u + slot;   // token count 0: the page contributes nothing
+            const uint4 about = make_uint4(__float_as_uint(k_scale), __float_as_uint(v_scale), token_count, 0u);
+            *meta = about;
+            if constexpr (kCluster == 2) store_peer(smem_addr(meta) + peer_delta, about);
+            if (slot == 0) describe_round(pair, cur.unit, (in_unit < 8u ? kFirstRound : 0u) | (in_unit + 8u >= cur.slots ? kLastRound : 0u));
         }
-        fence_async_smem();   // the tiles were written through the generic proxy; the tensor core reads through the async one
+        fence_async_smem<kCluster>();   // the tiles were written through the generic proxy; the tensor core reads through the async one
         __syncwarp();
-        if (lane == 0) mbar_arrive(&bar_full[pair]);
+        if (lane == 0) arrive_full(pair);
         cur = next;
         entry = next_entry;
     }
@@ -456,272 +574,281 @@ __device__ __forceinline__ void decoder_role(const AttentionParams &p, uint8_t *
     if (failed) mbar_wait(bar, copy_phase & 1u, p.wait_polls);
 }
 
-// ---- softmax group: warps 12..19; its thread 0 also issues the tensor-core work ---------------------------------------
+// ---- softmax group: warps 12..19; its thread 0 also issues the tensor-core work -------------------------------------------------------------------------------------------
 // kSplitQ: the queries are fp32; a row goes to tensor memory as binary16(q) and as binary16(q - binary16(q)), and S is the
 // sum of two products, which equals the fp32-query product to 2^-22 relative.
-template <bool kSplitQ>
+//
+// S of the next round goes out in the middle of a round, if its tiles are there, into the other half of the score columns: its
+// result is then ready when the round's weights have been stored. (Issued when the round's turn came, the chain S -> softmax -> O
+// was serial and alone took 80 % of the kernel: 492 of 618 us with the page decoders switched off.) Products issued by
+// one thread run in order, so S may overwrite the weights of the round before once their O has been issued.
+template <int kDim, bool kSplitQ, int kCluster>
 __device__ __forceinline__ void softmax_role(const AttentionParams &p, uint8_t *smem, PlanHeader *hdr, uint32_t tmem, uint32_t warp,
-                                             uint32_t lane, uint32_t row_tiles, const SharedSplit &split) {
+                                             uint32_t lane, uint32_t tile_groups, const SharedSplit &split) {
+    constexpr uint32_t kHalfDim = kDim / 2;   // channels of a thread
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + kOffBars);
     uint64_t *bar_full = bars + kBarFull, *bar_free = bars + kBarFree, *bar_s = bars + kBarS, *bar_o = bars + kBarO;
+    const uint32_t worker = blockIdx.x / kCluster, rank = kCluster == 1 ? 0u : cluster_rank();
     const uint32_t *round_desc = reinterpret_cast<const uint32_t *>(smem + kOffRound);
-    float *row_max = reinterpret_cast<float *>(smem + kOffRowMax);
     const uint32_t shared_pages = hdr->shared_pages;
     const uint32_t G = p.group, rows_total = p.seq_count * G;
     // Thread (warp w, lane) owns row 32 (w & 3) + lane — its warp's quarter of the tensor-memory lanes — and the 64 score
-    // columns (4 pages) of half (w - 12) >> 2; the two threads of a row meet through row_max[].
-    const uint32_t half = (warp - kDecodeWarps) >> 2, row_in_tile = (warp & 3u) * 32u + lane;
+    // columns (4 pages) of half (w - 12) >> 2; the two threads of a row meet through row_max[], their warps at a barrier of
+    // their own.
+    const uint32_t half = (warp - kDecodeWarps) >> 2, row_in_tile = (warp & 3u) * 32u + lane, pair_barrier = 2u + (warp & 3u);
     const uint32_t tmem_row = tmem + (((warp & 3u) * 32u) << 16);
     const bool issuer = warp == kDecodeWarps && lane == 0;
 
-    uint32_t s_phase = 0, o_phase = 0;
-    bool failed = false;      // warp-uniform
-    bool o_pending = false;   // a P V commit whose arrival on the O barrier has not been waited for yet
-    auto wait_o = [&]() {     // O and P in tensor memory may be touched again once the last P V has completed
-        if (!o_pending) return;
-        o_pending = false;
-        if (!failed && !__all_sync(0xffffffffu, mbar_wait(bar_o, o_phase & 1u, p.wait_polls))) {
+    bool failed = false;   // warp-uniform
+    auto wait = [&](uint64_t *bar, uint32_t parity) {
+        if (!failed && !__all_sync(0xffffffffu, mbar_wait(bar, parity, p.wait_polls))) {
             failed = true;
             if (lane == 0) raise_status(p, CF_B200_DEVSTAT_WAIT_EXPIRED);
         }
-        o_phase ^= 1u;
-        tc_fence_after();
     };
-    UnitShape u = {};
+    // Q rows of a unit: global memory -> tensor memory (binary16 pairs)
+    auto load_queries = [&](const UnitShape &u) {
+        const uint32_t row = (u.tile_index * kCluster + rank) * 128u + row_in_tile, r = min(row, rows_total - 1u);
+        const uint64_t first = (static_cast<uint64_t>(r / G) * p.query_head_count + u.kv_head * G + r % G) * kDim + kHalfDim * half;
+        const uint32_t column = kHalfDim / 2u * half;
+        if constexpr (kSplitQ) {
+            const float4 *src = reinterpret_cast<const float4 *>(reinterpret_cast<const float *>(p.queries) + first);
+#pragma unroll
+            for (uint32_t c = 0; c < kHalfDim / 16; ++c) {   // 16 channels = 8 columns of pairs at a time
+                uint32_t hi[8], lo[8];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    float4 x = src[4 * c + j];
+                    if (row >= rows_total) x = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    const __half2 h0 = __floats2half2_rn(x.x, x.y), h1 = __floats2half2_rn(x.z, x.w);
+                    const float2 b0 = __half22float2(h0), b1 = __half22float2(h1);
+                    const __half2 l0 = __floats2half2_rn(x.x - b0.x, x.y - b0.y), l1 = __floats2half2_rn(x.z - b1.x, x.w - b1.y);
+                    hi[2 * j] = *reinterpret_cast<const uint32_t *>(&h0);
+                    hi[2 * j + 1] = *reinterpret_cast<const uint32_t *>(&h1);
+                    lo[2 * j] = *reinterpret_cast<const uint32_t *>(&l0);
+                    lo[2 * j + 1] = *reinterpret_cast<const uint32_t *>(&l1);
+                }
+                tmem_store8(tmem_row + kColQ + column + 8u * c, hi);
+                tmem_store8(tmem_row + kColQResidue + column + 8u * c, lo);
+            }
+        } else {
+            const uint4 *src = reinterpret_cast<const uint4 *>(reinterpret_cast<const __half *>(p.queries) + first);
+#pragma unroll
+            for (uint32_t c = 0; c < kHalfDim / 16; ++c) {
+                uint4 a = src[2 * c], b = src[2 * c + 1];
+                if (row >= rows_total) a = b = make_uint4(0u, 0u, 0u, 0u);
+                const uint32_t q_raw[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+                tmem_store8(tmem_row + kColQ + column + 8u * c, q_raw);
+            }
+        }
+        tmem_store_wait();
+        tc_fence_before();
+    };
+    // Issuer only: S of round r, whose tiles are there.
+    auto issue_s = [&](uint32_t r) {
+        fence_async_smem<kCluster>();
+        tc_fence_after();
+        const uint32_t k_tile = smem_addr(smem + kOffTiles + (r & 1u) * 2u * kTileBytes), s_to = tmem + kColS + 128u * (r & 1u);
+#pragma unroll
+        for (uint32_t s = 0; s < kDim / 16; ++s) umma(s_to, tmem + kColQ + 8u * s, tile_desc(k_tile + 256u * s), s, kIdescS);
+        if constexpr (kSplitQ) {
+#pragma unroll
+            for (uint32_t s = 0; s < kDim / 16; ++s) umma(s_to, tmem + kColQResidue + 8u * s, tile_desc(k_tile + 256u * s), 1u, kIdescS);
+        }
+        umma_commit(&bar_s[r & 1u]);
+    };
+    uint32_t rounds = 0;    // whose O has been issued
+    uint32_t s_round = 0;   // issuer: the next round whose S is due
+    // Issuer only: S of round r ahead of its turn, unless its tiles are not there yet or its queries are another unit's.
+    auto issue_s_early = [&](uint32_t r) {
+        if (s_round != r || !mbar_test_pair(&bar_full[r & 1u], (r >> 1) & 1u)) return;
+        if (round_desc[4 * (r & 1u)] == kStopUnit || (round_desc[4 * (r & 1u) + 1] & kFirstRound)) return;
+        issue_s(r);
+        s_round = r + 1u;
+    };
+
+    UnitShape u = unit_shape(p, split, worker, 0u, tile_groups, shared_pages);
+    if (u.valid) load_queries(u);
+    group_any<kSoftmaxWarps * 32>(1u, false);
     float m_run = -CUDART_INF_F, l_run = 0.0f;   // the row's running maximum; this thread's half of its running sum
     float v_unit = 0.0f;                          // largest V scale met so far in the unit: the unit of O
-    bool o_started = false;
     int32_t seen = 0;   // tokens from the round's first on that the row's query token sees (16 per page and more: all of it)
     auto seen_of = [&](uint32_t pg, uint32_t count) {   // of page pg of the round, which holds `count`
         const int32_t left = seen - 16 * static_cast<int32_t>(pg);
         return left >= 16 ? count : min(count, static_cast<uint32_t>(max(left, 0)));
     };
+    const bool descending = p.softmax_scale < 0.0f;   // the largest score then comes from the smallest product
 
     for (uint32_t it = 0;; ++it) {
         const uint32_t pair = it & 1u;
-        uint8_t *k_tile = smem + kOffTiles + pair * 2u * kTileBytes, *v_tile = k_tile + kTileBytes;
         const float *meta = reinterpret_cast<const float *>(smem + kOffMeta) + pair * 4u * kRoundPages;
-        // ---- the round's tiles are decoded (one thread waits, the barrier passes the news on) ----
-        if (issuer && !failed && !mbar_wait(&bar_full[pair], (it >> 1) & 1u, p.wait_polls)) {
-            failed = true;
-            raise_status(p, CF_B200_DEVSTAT_WAIT_EXPIRED);
+        float *row_max = reinterpret_cast<float *>(smem + kOffRowMax) + 256u * pair;
+        const uint32_t s_cols = tmem_row + kColS + 128u * pair;   // scores, then weights [0, 64) and their residues [64, 128)
+        if (issuer && s_round == it) {   // one thread polls, the others sleep at the barrier
+            if (!failed && !mbar_wait_pair(&bar_full[pair], (it >> 1) & 1u, p.wait_polls)) {
+                failed = true;
+                raise_status(p, CF_B200_DEVSTAT_WAIT_EXPIRED);
+            }
+            if (!failed && round_desc[4 * pair] != kStopUnit) issue_s(it);
+            s_round = it + 1u;
         }
         failed = __any_sync(0xffffffffu, failed);
-        if (group_any(kSoftmaxBarrier, failed)) break;
+        if (group_any<kSoftmaxWarps * 32>(1u, failed)) break;
         const uint32_t unit = round_desc[4 * pair], flags = round_desc[4 * pair + 1];
         if (unit == kStopUnit) break;
-
-        if (flags & kFirstRound) {   // Q rows of the unit: global memory -> tensor memory (binary16 pairs, 64 columns)
-            u = unit_shape(p, split, blockIdx.x, unit, row_tiles, shared_pages);
-            m_run = -CUDART_INF_F;
-            l_run = 0.0f;
-            v_unit = 0.0f;
-            o_started = false;
-            const uint32_t row = u.tile_index * 128u + row_in_tile;
-            // entries of one sequence see its pages up to their own position; entries of several see every shared page
-            seen = p.one_slot ? static_cast<int32_t>(__ldcg(&seq_info(p)[min(row, rows_total - 1u) / G].qpos)) + 1 - static_cast<int32_t>(16u * u.page_begin)
-                              : 0x40000000;
-            if constexpr (kSplitQ) {
-                const float4 *src = reinterpret_cast<const float4 *>(
-                    reinterpret_cast<const float *>(p.queries) +
-                    (static_cast<uint64_t>(min(row, rows_total - 1u) / G) * p.query_head_count + u.kv_head * G + min(row, rows_total - 1u) % G) * 128u +
-                    64u * half);
-#pragma unroll
-                for (int c = 0; c < 4; ++c) {   // 16 channels = 8 columns of pairs at a time
-                    uint32_t hi[8], lo[8];
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        float4 x = src[4 * c + j];
-                        if (row >= rows_total) x = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                        const __half2 h0 = __floats2half2_rn(x.x, x.y), h1 = __floats2half2_rn(x.z, x.w);
-                        const float2 b0 = __half22float2(h0), b1 = __half22float2(h1);
-                        const __half2 l0 = __floats2half2_rn(x.x - b0.x, x.y - b0.y), l1 = __floats2half2_rn(x.z - b1.x, x.w - b1.y);
-                        hi[2 * j] = *reinterpret_cast<const uint32_t *>(&h0);
-                        hi[2 * j + 1] = *reinterpret_cast<const uint32_t *>(&h1);
-                        lo[2 * j] = *reinterpret_cast<const uint32_t *>(&l0);
-                        lo[2 * j + 1] = *reinterpret_cast<const uint32_t *>(&l1);
-                    }
-                    tmem_store8(tmem_row + kColQ + 32u * half + 8u * c, hi);
-                    tmem_store8(tmem_row + kColQResidue + 32u * half + 8u * c, lo);
-                }
-            } else {
-            uint32_t q_raw[32];
-            if (row < rows_total) {
-                const uint4 *src = reinterpret_cast<const uint4 *>(
-                    reinterpret_cast<const __half *>(p.queries) +
-                    (static_cast<uint64_t>(row / G) * p.query_head_count + u.kv_head * G + row % G) * 128u + 64u * half);
-#pragma unroll
-                for (int c = 0; c < 8; ++c) {
-                    const uint4 x = src[c];
-                    q_raw[4 * c] = x.x;
-                    q_raw[4 * c + 1] = x.y;
-                    q_raw[4 * c + 2] = x.z;
-                    q_raw[4 * c + 3] = x.w;
-                }
-            } else {
-#pragma unroll
-                for (int j = 0; j < 32; ++j) q_raw[j] = 0u;
-            }
-            tmem_store32(tmem_row + kColQ + 32u * half, q_raw);
-            }
-            tmem_store_wait();
-            tc_fence_before();
-            if (group_any(kSoftmaxBarrier, false)) break;
-        }
-
-        // ---- S = Q K^T ----
-        if (issuer) {
-            tc_fence_after();
-#pragma unroll
-            for (uint32_t s = 0; s < 8; ++s) umma(tmem + kColS, tmem + kColQ + 8u * s, tile_desc(smem_addr(k_tile) + 256u * s), s);
-            if constexpr (kSplitQ) {
-#pragma unroll
-                for (uint32_t s = 0; s < 8; ++s) umma(tmem + kColS, tmem + kColQResidue + 8u * s, tile_desc(smem_addr(k_tile) + 256u * s), 1u);
-            }
-            umma_commit(bar_s);
-        }
-        float round_scale = 0.0f;   // largest V scale among the round's present pages
-#pragma unroll
-        for (uint32_t pg = 0; pg < kRoundPages; ++pg)
-            if (__float_as_uint(meta[4 * pg + 2]) != 0u) round_scale = fmaxf(round_scale, meta[4 * pg + 1]);
-        if (!failed && !__all_sync(0xffffffffu, mbar_wait(bar_s, s_phase & 1u, p.wait_polls))) {
-            failed = true;
-            if (lane == 0) raise_status(p, CF_B200_DEVSTAT_WAIT_EXPIRED);
-        }
-        s_phase ^= 1u;
+        wait(&bar_s[pair], (it >> 1) & 1u);
         tc_fence_after();
         uint32_t s_raw[2][32];
         if (!failed) {
-            tmem_load32(tmem_row + kColS + 64u * half, s_raw[0]);
-            tmem_load32(tmem_row + kColS + 64u * half + 32u, s_raw[1]);
+            tmem_load32(s_cols + 64u * half, s_raw[0]);
+            tmem_load32(s_cols + 64u * half + 32u, s_raw[1]);
+            if (flags & kFirstRound) {
+                m_run = -CUDART_INF_F;
+                l_run = 0.0f;
+                v_unit = 0.0f;
+                // entries of one sequence see its pages up to their own position; entries of several see every shared page
+                const uint32_t row = min((u.tile_index * kCluster + rank) * 128u + row_in_tile, rows_total - 1u);
+                seen = p.one_slot ? static_cast<int32_t>(__ldcg(&seq_info(p)[row / G].qpos)) + 1 - static_cast<int32_t>(16u * u.page_begin)
+                                  : 0x40000000;
+            }
             tmem_load_wait();
-        }
-        // maximum of the scaled, masked scores of this thread's 4 pages; the raw scores stay in the registers
-        float part_max = -CUDART_INF_F;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const uint32_t pg = 4u * half + q;
-            const uint32_t count = seen_of(pg, __float_as_uint(meta[4 * pg + 2]));
-            const float ks = meta[4 * pg];
-            if (count == 16u) {   // a full page (the usual case): the scale is applied to the extreme, not to every score
-                float hi = __uint_as_float(s_raw[q >> 1][16 * (q & 1)]), lo = hi;
-#pragma unroll
-                for (int j = 1; j < 16; ++j) {
-                    hi = fmaxf(hi, __uint_as_float(s_raw[q >> 1][16 * (q & 1) + j]));
-                    lo = fminf(lo, __uint_as_float(s_raw[q >> 1][16 * (q & 1) + j]));
-                }
-                part_max = fmaxf(part_max, fmaxf(hi * ks, lo * ks));
-            } else {
-#pragma unroll
-                for (int j = 0; j < 16; ++j)
-                    if (static_cast<uint32_t>(j) < count)
-                        part_max = fmaxf(part_max, __uint_as_float(s_raw[q >> 1][16 * (q & 1) + j]) * ks);
-            }
-        }
-        row_max[half * 128u + row_in_tile] = part_max;
-        tc_fence_before();   // this thread's reads of S are complete: the next round's S may overwrite it
-        if (group_any(kSoftmaxBarrier, failed)) break;
-
-        wait_o();   // the previous round's P V is done with O and P
-        if (!failed) {
-            const float m_new = fmaxf(m_run, fmaxf(row_max[row_in_tile], row_max[128u + row_in_tile]));
-            const float z = m_new == -CUDART_INF_F ? 0.0f : m_new;
-            const float alpha = fast_exp2(m_run - z);   // m_run = -inf gives 0
-            m_run = m_new;
-            // The unit of O is the largest V scale met so far in the unit, so that a page's scale relative to it (which
-            // rides on the binary16 weights) never exceeds 1; when a round brings a larger one, O changes unit with it.
-            float o_scale = alpha;
-            if (round_scale > v_unit) {
-                o_scale *= v_unit / round_scale;   // v_unit = 0: nothing accumulated yet
-                v_unit = round_scale;
-            }
-            // O in tensor memory follows the new maximum and unit (this thread's 64 channels); skipped when no row of the
-            // warp moved
-            if (o_started && !__all_sync(0xffffffffu, o_scale == 1.0f)) {
-#pragma unroll 1
-                for (uint32_t c0 = 0; c0 < 64u; c0 += 32u) {
-                    uint32_t o_raw[32];
-                    tmem_load32(tmem_row + kColO + 64u * half + c0, o_raw);
-                    tmem_load_wait();
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) o_raw[j] = __float_as_uint(__uint_as_float(o_raw[j]) * o_scale);
-                    tmem_store32(tmem_row + kColO + 64u * half + c0, o_raw);
-                }
-            }
-            // weights as binary16 plus their rounding residue (two A operands), so that P V is accurate to fp32 level
-            // whatever the spread of the V scales
-            float sum = 0.0f;
+            // maximum of the scaled, masked scores of this thread's 4 pages; the raw scores stay in the registers
+            float part_max = -CUDART_INF_F;
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 const uint32_t pg = 4u * half + q;
                 const uint32_t count = seen_of(pg, __float_as_uint(meta[4 * pg + 2]));
                 const float ks = meta[4 * pg];
-                // the weights (at most 1) also carry 2^15, exactly, which O sheds at the unit's end: binary16 then resolves
-                // weights down to 2^-40 of the row maximum instead of 2^-25
-                const float ratio = count ? __fdividef(meta[4 * pg + 1], v_unit) * kWeightScale : 0.0f;
-                uint32_t hi[8], lo[8];
+                if (count == 16u && !descending) {   // a full page (the usual case): the scale is applied to the extreme, not to every score
+                    float hi = __uint_as_float(s_raw[q >> 1][16 * (q & 1)]);
 #pragma unroll
-                for (int j = 0; j < 16; j += 2) {
-                    float w0 = fast_exp2(fmaf(__uint_as_float(s_raw[q >> 1][16 * (q & 1) + j]), ks, -z));
-                    float w1 = fast_exp2(fmaf(__uint_as_float(s_raw[q >> 1][16 * (q & 1) + j + 1]), ks, -z));
-                    if (count != 16u) {   // tokens past the page's count, or past the row's position, weigh nothing
-                        w0 = static_cast<uint32_t>(j) < count ? w0 : 0.0f;
-                        w1 = static_cast<uint32_t>(j + 1) < count ? w1 : 0.0f;
-                    }
-                    sum += w0 + w1;
-                    const float a0 = w0 * ratio, a1 = w1 * ratio;
-                    const __half2 h = __floats2half2_rn(a0, a1);
-                    const float2 back = __half22float2(h);
-                    const __half2 l = __floats2half2_rn(a0 - back.x, a1 - back.y);
-                    hi[j >> 1] = *reinterpret_cast<const uint32_t *>(&h);
-                    lo[j >> 1] = *reinterpret_cast<const uint32_t *>(&l);
+                    for (int j = 1; j < 16; ++j) hi = fmaxf(hi, __uint_as_float(s_raw[q >> 1][16 * (q & 1) + j]));
+                    part_max = fmaxf(part_max, hi * ks);
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 16; ++j)
+                        if (static_cast<uint32_t>(j) < count)
+                            part_max = fmaxf(part_max, __uint_as_float(s_raw[q >> 1][16 * (q & 1) + j]) * ks);
                 }
-                tmem_store8(tmem_row + kColP + 8u * pg, hi);          // 16 tokens = 8 columns of pairs
-                tmem_store8(tmem_row + kColPResidue + 8u * pg, lo);
             }
-            tmem_store_wait();
-            l_run = l_run * alpha + sum;   // this thread's half of the row's sum; the halves are added at the unit's end
+            row_max[half * 128u + row_in_tile] = part_max;
         }
-        tc_fence_before();
-        if (group_any(kSoftmaxBarrier, failed)) break;
+        tc_fence_before();   // both threads of a row have read their scores: the weights may overwrite them
+        group_any<64>(pair_barrier, false);
+        tc_fence_after();
+        if (issuer && !failed) issue_s_early(it + 1u);
 
-        // ---- O += P V ----
-        if (issuer) {
-            tc_fence_after();
+        float round_scale = 0.0f;   // largest V scale among the round's present pages
 #pragma unroll
-            for (uint32_t s = 0; s < 8; ++s)
-                umma(tmem + kColO, tmem + kColP + 8u * s, tile_desc(smem_addr(v_tile) + 256u * s), (o_started || s) ? 1u : 0u);
-#pragma unroll
-            for (uint32_t s = 0; s < 8; ++s) umma(tmem + kColO, tmem + kColPResidue + 8u * s, tile_desc(smem_addr(v_tile) + 256u * s), 1u);
-            umma_commit(bar_o);
-            umma_commit(&bar_free[pair]);   // the decoders may refill this pair of tiles
+        for (uint32_t pg = 0; pg < kRoundPages; ++pg)
+            if (__float_as_uint(meta[4 * pg + 2]) != 0u) round_scale = fmaxf(round_scale, meta[4 * pg + 1]);
+        const float m_new = fmaxf(m_run, fmaxf(row_max[row_in_tile], row_max[128u + row_in_tile]));
+        const float z = m_new == -CUDART_INF_F ? 0.0f : m_new;
+        const float alpha = fast_exp2(m_run - z);   // m_run = -inf gives 0
+        m_run = m_new;
+        // The unit of O is the largest V scale met so far in the unit, so that a page's scale relative to it (which
+        // rides on the binary16 weights) never exceeds 1; when a round brings a larger one, O changes unit with it.
+        float o_scale = alpha;
+        if (round_scale > v_unit) {
+            o_scale *= v_unit / round_scale;   // v_unit = 0: nothing accumulated yet
+            v_unit = round_scale;
         }
-        o_started = true;
-        o_pending = true;
+        // weights as binary16 plus their rounding residue (two A operands), so that P V is accurate to fp32 level
+        // whatever the spread of the V scales
+        float sum = 0.0f;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const uint32_t pg = 4u * half + q;
+            const uint32_t count = seen_of(pg, __float_as_uint(meta[4 * pg + 2]));
+            const float ks = meta[4 * pg];
+            // the weights (at most 1) also carry 2^15, exactly, which O sheds at the unit's end: binary16 then resolves
+            // weights down to 2^-40 of the row maximum instead of 2^-25
+            const float ratio = count ? __fdividef(meta[4 * pg + 1], v_unit) * kWeightScale : 0.0f;
+            uint32_t hi[8], lo[8];
+#pragma unroll
+            for (int j = 0; j < 16; j += 2) {
+                float w0 = fast_exp2(fmaf(__uint_as_float(s_raw[q >> 1][16 * (q & 1) + j]), ks, -z));
+                float w1 = fast_exp2(fmaf(__uint_as_float(s_raw[q >> 1][16 * (q & 1) + j + 1]), ks, -z));
+                if (count != 16u) {   // tokens past the page's count, or past the row's position, weigh nothing
+                    w0 = static_cast<uint32_t>(j) < count ? w0 : 0.0f;
+                    w1 = static_cast<uint32_t>(j + 1) < count ? w1 : 0.0f;
+                }
+                sum += w0 + w1;
+                const float a0 = w0 * ratio, a1 = w1 * ratio;
+                const __half2 h = __floats2half2_rn(a0, a1);
+                const float2 back = __half22float2(h);
+                const __half2 l = __floats2half2_rn(a0 - back.x, a1 - back.y);
+                hi[j >> 1] = *reinterpret_cast<const uint32_t *>(&h);
+                lo[j >> 1] = *reinterpret_cast<const uint32_t *>(&l);
+            }
+            tmem_store8(s_cols + 8u * pg, hi);          // 16 tokens = 8 columns of pairs
+            tmem_store8(s_cols + 64u + 8u * pg, lo);
+        }
+        l_run = l_run * alpha + sum;   // this thread's half of the row's sum; the halves are added at the unit's end
+        // O in tensor memory follows the new maximum and unit (this thread's channels), once the previous round's product has
+        // reached it; skipped when no row of the warp moved
+        if (!(flags & kFirstRound) && !__all_sync(0xffffffffu, o_scale == 1.0f)) {
+            wait(&bar_o[pair ^ 1u], ((it - 1u) >> 1) & 1u);
+            tc_fence_after();
+            if (!failed) {
+#pragma unroll 1
+                for (uint32_t c0 = 0; c0 < kHalfDim; c0 += 32u) {
+                    uint32_t o_raw[32];
+                    tmem_load32(tmem_row + kColO + kHalfDim * half + c0, o_raw);
+                    tmem_load_wait();
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) o_raw[j] = __float_as_uint(__uint_as_float(o_raw[j]) * o_scale);
+                    tmem_store32(tmem_row + kColO + kHalfDim * half + c0, o_raw);
+                }
+            }
+        }
+        tmem_store_wait();
+        tc_fence_before();
+        if (group_any<kSoftmaxWarps * 32>(1u, failed)) break;
+        if (issuer) {   // O += P V
+            tc_fence_after();
+            const uint32_t v_tile = smem_addr(smem + kOffTiles + pair * 2u * kTileBytes + kTileBytes), p_from = tmem + kColS + 128u * pair;
+#pragma unroll
+            for (uint32_t s = 0; s < 8; ++s) umma(tmem + kColO, p_from + 8u * s, tile_desc(v_tile + 256u * s), (flags & kFirstRound) && !s ? 0u : 1u, kIdescO<kDim>);
+#pragma unroll
+            for (uint32_t s = 0; s < 8; ++s) umma(tmem + kColO, p_from + 64u + 8u * s, tile_desc(v_tile + 256u * s), 1u, kIdescO<kDim>);
+            if constexpr (kCluster == 1) umma_commit(&bar_free[it & 3u]);   // the decoders may refill this pair of tiles
+            else umma_commit_pair(&bar_free[it & 3u]);
+            umma_commit(&bar_o[pair]);
+            issue_s_early(it + 1u);
+        }
+        __syncwarp();
+        rounds = it + 1u;
         if (p.one_slot) seen -= 16 * static_cast<int32_t>(kRoundPages);
 
-        // ---- last round of the unit: one (max, sum, weighted[128]) per row; each thread writes its 64 channels ----
+        // ---- last round of the unit: one (max, sum, weighted[kDim]) per row; each thread writes its channels ----
         if (flags & kLastRound) {
-            wait_o();
-            row_max[half * 128u + row_in_tile] = l_run;   // reused: the two halves of the row's sum
-            if (group_any(kSoftmaxBarrier, failed)) break;
-            const uint32_t row = u.tile_index * 128u + row_in_tile;
+            const UnitShape done = u;
+            u = unit_shape(p, split, worker, unit + 1u, tile_groups, shared_pages);
+            if (u.valid) load_queries(u);   // this unit's last scores have been read: its queries may go
+            wait(&bar_o[pair], (it >> 1) & 1u);
+            tc_fence_after();
+            // the two halves of the row's sum take the places of the maxima: O of this round is complete, so every warp has stored
+            // its weights, and read the maxima before
+            row_max[half * 128u + row_in_tile] = l_run;
+            if (group_any<kSoftmaxWarps * 32>(1u, failed)) break;   // the next unit's queries are stored, too
+            const uint32_t row = (done.tile_index * kCluster + rank) * 128u + row_in_tile;
             const bool live = row < rows_total;   // whole warps go on: the tensor-memory loads are warp-wide
-            float *dst = live ? shared_partial_ptr(p, u.chunk, row / G, u.head_local * G + row % G) : nullptr;
+            float *dst = live ? shared_partial_ptr(p, done.chunk, row / G, done.head_local * G + row % G) : nullptr;
             const float o_unit = v_unit * (1.0f / kWeightScale);
             if (live && half == 0) {
                 dst[0] = m_run;
                 dst[1] = row_max[row_in_tile] + row_max[128u + row_in_tile];
             }
 #pragma unroll 1
-            for (uint32_t c0 = 0; c0 < 64u; c0 += 32u) {
+            for (uint32_t c0 = 0; c0 < kHalfDim; c0 += 32u) {
                 uint32_t o_raw[32];
-                tmem_load32(tmem_row + kColO + 64u * half + c0, o_raw);
+                tmem_load32(tmem_row + kColO + kHalfDim * half + c0, o_raw);
                 tmem_load_wait();
                 if (live) {
 #pragma unroll
                     for (int t = 0; t < 8; ++t) {   // columns t, t + 8, t + 16, t + 24 of the 32 are 4 consecutive channels
-                        float *out = dst + 2 + 64u * half + c0 + 4 * t;
+                        float *out = dst + 2 + kHalfDim * half + c0 + 4 * t;
                         *reinterpret_cast<float2 *>(out) =
                             make_float2(__uint_as_float(o_raw[t]) * o_unit, __uint_as_float(o_raw[t + 8]) * o_unit);
                         *reinterpret_cast<float2 *>(out + 2) =
@@ -732,11 +859,16 @@ __device__ __forceinline__ void softmax_role(const AttentionParams &p, uint8_t *
             tc_fence_before();
         }
     }
-    // leaving early: give the tensor core's last commit a bounded chance to arrive before tensor memory is freed
-    if (o_pending && !failed) mbar_wait(bar_o, o_phase & 1u, p.wait_polls);
+    // What the other CTA of the pair still signals here has to land before this one leaves; leaving early, the last product of
+    // this one as well. Bounded, whatever happened.
+    if (issuer && rounds) {
+        if (kCluster == 2 && !failed)
+            for (uint32_t r = rounds < 2u ? 0u : rounds - 2u; r < rounds; ++r) mbar_wait_pair(&bar_free[r & 3u], (r >> 2) & 1u, p.wait_polls);
+        if (failed) mbar_wait(&bar_o[(rounds - 1u) & 1u], ((rounds - 1u) >> 1) & 1u, p.wait_polls);
+    }
 }
 
-template <bool kSplitQ>
+template <int kDim, bool kSplitQ, int kCluster>
 __global__ void __launch_bounds__(kTcThreads, 1) prefix_attention_kernel(AttentionParams p) {
     extern __shared__ __align__(1024) uint8_t smem[];
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
@@ -749,13 +881,14 @@ __global__ void __launch_bounds__(kTcThreads, 1) prefix_attention_kernel(Attenti
     allow_dependent_launch();
     PlanHeader *hdr = plan_header(p);
     // uniform: nothing shared, the plan refused the hint, or the split leaves this CTA without a share
-    if (hdr->shared_pages == 0 || blockIdx.x >= hdr->shared_ctas) return;
+    if (hdr->shared_pages == 0 || blockIdx.x / kCluster >= hdr->shared_ctas) return;   // both CTAs of a pair alike
 
     if (tid == 0) {
         for (uint32_t w = 0; w < kDecodeWarps; ++w) mbar_init(bars + w, 1);   // copies
         mbar_init(bars + kBarFull, kRoundPages);                    // full[0], full[1]: one arrival per page slot of the round
         mbar_init(bars + kBarFull + 1, kRoundPages);
-        for (uint32_t i = kBarFree; i < kBarCount; ++i) mbar_init(bars + i, 1);   // free[0], free[1], S, O: tensor-core commits
+        for (uint32_t i = 0; i < 4u; ++i) mbar_init(bars + kBarFree + i, kCluster);   // tensor-core commits, of both CTAs
+        for (uint32_t i = kBarS; i < kBarCount; ++i) mbar_init(bars + i, 1);          // tensor-core commits
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncwarp();
@@ -768,18 +901,23 @@ __global__ void __launch_bounds__(kTcThreads, 1) prefix_attention_kernel(Attenti
     tc_fence_after();
     const uint32_t tmem = misc[0];
 
-    const uint32_t rows_total = p.seq_count * p.group;
-    const uint32_t row_tiles = (rows_total + 127u) / 128u;
-    const SharedSplit split = {hdr->shared_rounds, p.kv_head_span * row_tiles, hdr->shared_ctas};
+    if constexpr (kCluster == 2) cluster_sync();   // the peer's barriers are set up
+
+    const uint32_t tile_groups = shared_tile_groups(p.seq_count * p.group);
+    const SharedSplit split = {hdr->shared_rounds, p.kv_head_span * tile_groups, hdr->shared_ctas};
 
     if (warp < kDecodeWarps) {   // whole warpgroups on either side: the register split is per warpgroup
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kDecoderRegs));
-        decoder_role(p, smem, hdr, warp, lane, row_tiles, split);
+        decoder_role<kDim, kCluster>(p, smem, hdr, warp, lane, tile_groups, split);
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSoftmaxRegs));
-        softmax_role<kSplitQ>(p, smem, hdr, tmem, warp, lane, row_tiles, split);
+        softmax_role<kDim, kSplitQ, kCluster>(p, smem, hdr, tmem, warp, lane, tile_groups, split);
     }
 
+    if constexpr (kCluster == 2) {   // the peer may still store into this CTA's tiles
+        __syncwarp();
+        cluster_sync();
+    }
     tc_fence_before();
     __syncthreads();
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemColumns));
@@ -792,22 +930,27 @@ cudaError_t launch_prefix_attention(const AttentionParams &p, cudaStream_t strea
     cudaError_t e;
     LauncherState *state = launcher_state(table, &e);
     if (!state) return e;
-    const int sm_count = state->sm_count;
+    using Kernel = void (*)(AttentionParams);
+    const Kernel kernels[2][2][2] = {   // [pair of CTAs][head_dim 64][fp32 queries]
+        {{prefix_attention_kernel<128, false, 1>, prefix_attention_kernel<128, true, 1>},
+         {prefix_attention_kernel<64, false, 1>, prefix_attention_kernel<64, true, 1>}},
+        {{prefix_attention_kernel<128, false, 2>, prefix_attention_kernel<128, true, 2>},
+         {prefix_attention_kernel<64, false, 2>, prefix_attention_kernel<64, true, 2>}}};
     if (!state->configured) {
-        for (int split = 0; split < 2; ++split) {
-            const void *kernel = split ? reinterpret_cast<const void *>(prefix_attention_kernel<true>)
-                                       : reinterpret_cast<const void *>(prefix_attention_kernel<false>);
+        for (int i = 0; i < 8; ++i) {
+            const Kernel kernel = kernels[i >> 2][i >> 1 & 1][i & 1];
             e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kTcSmem));
             if (e != cudaSuccess) return e;
             cudaFuncAttributes attr;
             e = cudaFuncGetAttributes(&attr, kernel);
             if (e != cudaSuccess) return e;
-            if (attr.numRegs != kLaunchRegs) return cudaErrorLaunchOutOfResources;   // the register split assumes this count
+            if ((attr.numRegs + 7) / 8 * 8 != kLaunchRegs) return cudaErrorLaunchOutOfResources;   // the register split assumes this count
         }
         state->configured = true;
     }
-    return launch_kernel(p.query_type == CF_B200_F32 ? prefix_attention_kernel<true> : prefix_attention_kernel<false>, sm_count, kTcThreads,
-                         kTcSmem, stream, dependent, p);
+    const uint32_t cluster = shared_cluster(p.seq_count * p.group);
+    return launch_in_clusters(cluster, kernels[cluster - 1u][p.head_dim == 64 ? 1 : 0][p.query_type == CF_B200_F32 ? 1 : 0],
+                              static_cast<uint32_t>(state->sm_count) / cluster * cluster, kTcThreads, kTcSmem, stream, dependent, p);
 }
 
 }  // namespace cfb

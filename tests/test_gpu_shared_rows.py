@@ -1,0 +1,74 @@
+"""The shared-prefix kernel and the combine forms at the edges of their ranges: query groups that do not divide a row tile, both
+head_dims, a chunk of query tokens that sees its own pages in part, groups of more than four heads of fp32 queries."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from compat_types import DeviceKvConfig, TensorView
+from helpers import attention_close
+from test_gpu_device_engine import _expected
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("heads,dim,coder,pages,seqs,f32", [
+    ((14, 2), 128, "rans4", 8, 9, False), ((12, 4), 64, "huffman4", 33, 7, True), ((8, 8), 64, "rans", 17, 130, False),
+    ((14, 2), 64, "huffman", 24, 19, True), ((32, 8), 64, "fixed8", 9, 40, False), ((48, 4), 128, "rans4", 16, 11, True)])
+def test_shared_pages_give_what_each_sequence_alone_gives(native, heads, dim, coder, pages, seqs, f32):
+    import torch
+    from chromofold_b200.workloads import build_sealed_layer
+    hq, hkv = heads
+    layer, _ = build_sealed_layer(np.array([16 * pages] + [0] * (seqs - 1)), query_heads=hq, kv_heads=hkv, head_dim=dim, coder=coder, seed=5,
+                                  extra_pages_per_sequence=pages + 2, reserve_pages=4 * seqs)
+    for s in range(1, seqs):
+        layer.copy_sequence(0, s)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(6)
+    for _ in range(19):     # a private page and a tail for every sequence
+        k, v = ((torch.randn((seqs, hkv, dim), generator=g, device="cuda") * 0.7).half() for _ in range(2))
+        layer.append(list(range(seqs)), k, v)
+        layer.seal_full_pages()
+    q = torch.randn((seqs, hq, dim), generator=g, device="cuda")
+    q = q if f32 else q.half()
+    before = native.lib().cf_b200_shared_prefix_launches()
+    shared = layer.attention(q, shared_prefix_pages=pages).cpu().numpy()
+    assert native.lib().cf_b200_shared_prefix_launches() == before + 1
+    alone = layer.attention(q).cpu().numpy()
+    assert layer.device_status() == 0
+    ok, err = attention_close(shared, alone, rel=2e-5, abs_=2e-5)
+    assert ok, err
+
+
+@pytest.mark.parametrize("heads,dim,page,history,rows", [
+    ((8, 2), 128, 128, 0, 150), ((32, 8), 128, 16, 130, 301), ((14, 2), 64, 64, 300, 70), ((12, 4), 128, 256, 1, 255), ((8, 8), 64, 32, 515, 129)])
+def test_a_chunk_of_query_tokens_sees_each_token_up_to_its_own(native, oracle, heads, dim, page, history, rows):
+    import torch
+    lib = native.lib()
+    lib.cf_device_kv_create.restype = C.c_void_p
+    lib.cf_device_kv_last_error.restype = C.c_char_p
+    hq, hkv = heads
+    cfg = DeviceKvConfig(1, hkv, hq, dim, page, hq // hkv, 0)
+    kv = C.c_void_p(lib.cf_device_kv_create(C.byref(cfg)))
+    rng = np.random.default_rng(rows)
+    tokens = history + rows
+    k, v = (rng.standard_normal((tokens, hkv, dim)).astype(np.float32) for _ in range(2))
+    q = rng.standard_normal((rows, hq, dim)).astype(np.float32)
+    dk, dv, dq = (torch.from_numpy(x).cuda() for x in (k, v, q))
+    def view(t):
+        return TensorView(t.data_ptr(), native.F32, *t.shape, hkv * dim * 4, dim * 4, 4, 0)
+
+    for begin in range(0, tokens, page):
+        end = min(begin + page, tokens)
+        assert lib.cf_device_kv_append_async(kv, 0, begin, C.byref(view(dk[begin:end])), C.byref(view(dv[begin:end])), None) == 0
+        assert lib.cf_device_kv_seal_full_pages_async(kv, None) == 0, lib.cf_device_kv_last_error(kv)
+    out = torch.full((rows, hq, dim), 7.0, device="cuda")
+    scale = dim ** -0.5
+    assert lib.cf_device_kv_attention_async(kv, 0, C.c_void_p(dq.data_ptr()), C.c_void_p(out.data_ptr()), rows, history, C.c_float(scale), 0,
+                                            None) == 0, lib.cf_device_kv_last_error(kv)
+    torch.cuda.synchronize()
+    some = sorted({0, 1, 15, 16, rows // 2, rows - 2, rows - 1})
+    want = _expected(oracle, k, v, tokens // page * page, 16, q[some], [history + i for i in some], 0, scale, hq // hkv)
+    ok, err = attention_close(out.cpu().numpy()[some], want)
+    assert ok, err
+    lib.cf_device_kv_destroy(kv, None)
