@@ -25,7 +25,7 @@
 //                        the row's two threads share their maxima through shared memory, running max / sum updated,
 //                        O rescaled in tensor memory (tcgen05.ld / .st) only when some row of the warp moved its max,
 //                        P and its residue written over the scores (tcgen05.st) as the next A operands.
-//                        Thread 0 of the group issues the tensor-core work (M 128, K 16 per instruction):
+//                        Thread 0 of the group (in a pair of CTAs: warp 11) issues the tensor-core work (M 128, K 16):
 //                          S     Q from tensor memory x K tile -> one of two sets of 128 score columns
 //                          O     16 tcgen05.mma: P (binary16, then its rounding residue) from tensor memory x V tile
 //                        Unit start: the Q rows go from global memory straight to tensor memory. Unit end: O read back,
@@ -52,6 +52,9 @@ namespace {
 using namespace lanes;
 
 constexpr int kDecodeWarps = 12;     // warps 0..11 (three warpgroups)
+// In a pair of CTAs warp 11 issues the tensor-core work: decoding half of the pages needs no twelfth warp. A CTA on its own
+// decodes them all, and thread 0 of the softmax group issues.
+template <int kCluster> constexpr int kDecoders = kCluster == 2 ? kDecodeWarps - 1 : kDecodeWarps;
 constexpr int kSoftmaxWarps = 8;     // warps 12..19 (two warpgroups)
 constexpr int kRoundPages = 8;
 constexpr int kTcThreads = (kDecodeWarps + kSoftmaxWarps) * 32;
@@ -63,8 +66,9 @@ constexpr uint32_t kOffStages = kTableBytes;
 constexpr uint32_t kOffTiles = (kOffStages + kDecodeWarps * kRecordBytes + 127u) / 128u * 128u;   // K[0] V[0] K[1] V[1]
 constexpr uint32_t kOffMeta = kOffTiles + 4 * kTileBytes;      // [pair][page of the round]: k scale, v scale, token count, -
 constexpr uint32_t kOffRound = kOffMeta + 2 * kRoundPages * 16;    // [pair]: unit, flags, -, -
-constexpr uint32_t kOffBars = kOffRound + 2 * 16;              // 12 copy barriers, full[2], free[4], S[2], O[2]
-constexpr uint32_t kBarFull = kDecodeWarps, kBarFree = kBarFull + 2, kBarS = kBarFree + 4, kBarO = kBarS + 2, kBarCount = kBarO + 2;
+constexpr uint32_t kOffBars = kOffRound + 2 * 16;              // 12 copy barriers, full[2], free[4], S[2], O[2], P, Q
+constexpr uint32_t kBarFull = kDecodeWarps, kBarFree = kBarFull + 2, kBarS = kBarFree + 4, kBarO = kBarS + 2, kBarP = kBarO + 2, kBarQ = kBarP + 1,
+                   kBarCount = kBarQ + 1;
 constexpr uint32_t kOffMisc = kOffBars + kBarCount * 8;        // [0] tmem base
 constexpr uint32_t kOffRowMax = kOffMisc + 32;                 // [round parity][2 column halves][128 rows]
 constexpr uint32_t kTcSmem = kOffRowMax + 4 * 128 * 4;
@@ -452,7 +456,7 @@ __device__ __forceinline__ void decoder_role(const AttentionParams &p, uint8_t *
     uint64_t entry = slot_entry(cur, n);
     issue(entry);
 
-    for (;; m += kDecodeWarps, n = slot_number(m)) {
+    for (;; m += kDecoders<kCluster>, n = slot_number(m)) {
         if (!cur.valid) {   // past the last unit: the eight slots after it make the round that tells the softmax group to stop
             if (n < cur.first_slot + 8u) {
                 wait_pair_free(cur.first_round);
@@ -466,7 +470,7 @@ __device__ __forceinline__ void decoder_role(const AttentionParams &p, uint8_t *
         const uint32_t in_unit = n - cur.first_slot, slot = in_unit & 7u, it = cur.first_round + (in_unit >> 3), pair = it & 1u;
         // the warp's next slot: its directory entry is fetched now (dependent loads), needed only after this decode
         SlotCursor next = cur;
-        const uint32_t next_n = slot_number(m + kDecodeWarps);
+        const uint32_t next_n = slot_number(m + kDecoders<kCluster>);
         seek(next, next_n);
         const uint64_t next_entry = slot_entry(next, next_n);
 
@@ -574,7 +578,74 @@ __device__ __forceinline__ void decoder_role(const AttentionParams &p, uint8_t *
     if (failed) mbar_wait(bar, copy_phase & 1u, p.wait_polls);
 }
 
-// ---- softmax group: warps 12..19; its thread 0 also issues the tensor-core work -------------------------------------------------------------------------------------------
+// ---- tensor-core work, issued by one thread ----------------------------------------------------------------------------------
+// S of round r, whose tiles are there.
+template <int kDim, bool kSplitQ, int kCluster>
+__device__ __forceinline__ void issue_scores(uint8_t *smem, uint32_t tmem, uint64_t *bars, uint32_t r) {
+    fence_async_smem<kCluster>();
+    tc_fence_after();
+    const uint32_t k_tile = smem_addr(smem + kOffTiles + (r & 1u) * 2u * kTileBytes), s_to = tmem + kColS + 128u * (r & 1u);
+#pragma unroll
+    for (uint32_t s = 0; s < kDim / 16; ++s) umma(s_to, tmem + kColQ + 8u * s, tile_desc(k_tile + 256u * s), s, kIdescS);
+    if constexpr (kSplitQ) {
+#pragma unroll
+        for (uint32_t s = 0; s < kDim / 16; ++s) umma(s_to, tmem + kColQResidue + 8u * s, tile_desc(k_tile + 256u * s), 1u, kIdescS);
+    }
+    umma_commit(bars + kBarS + (r & 1u));
+}
+// O (+)= P V of round r, whose weights are stored.
+template <int kDim, int kCluster>
+__device__ __forceinline__ void issue_output(uint8_t *smem, uint32_t tmem, uint64_t *bars, uint32_t r, bool first) {
+    tc_fence_after();
+    const uint32_t v_tile = smem_addr(smem + kOffTiles + (r & 1u) * 2u * kTileBytes + kTileBytes), p_from = tmem + kColS + 128u * (r & 1u);
+#pragma unroll
+    for (uint32_t s = 0; s < 8; ++s) umma(tmem + kColO, p_from + 8u * s, tile_desc(v_tile + 256u * s), first && !s ? 0u : 1u, kIdescO<kDim>);
+#pragma unroll
+    for (uint32_t s = 0; s < 8; ++s) umma(tmem + kColO, p_from + 64u + 8u * s, tile_desc(v_tile + 256u * s), 1u, kIdescO<kDim>);
+    if constexpr (kCluster == 1) umma_commit(bars + kBarFree + (r & 3u));   // the decoders may refill this pair of tiles
+    else umma_commit_pair(bars + kBarFree + (r & 3u));
+    umma_commit(bars + kBarO + (r & 1u));
+}
+// The issuing thread of a pair's CTA (warp 11). Issuing a product takes some 70 clocks whatever its size, 24 to 32 of them a round
+// (1700 to 2200 clocks): in the softmax group they are part of its serial chain, here they run beside it. Whichever comes first,
+// the tiles of the next round or the weights of the last: O frees its tiles for the decoders, S is what the softmax warps wait
+// for. S of a round two ahead would land on weights that are still to be read.
+template <int kDim, bool kSplitQ, int kCluster>
+__device__ __forceinline__ void issuer_role(const AttentionParams &p, uint8_t *smem, uint32_t tmem) {
+    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + kOffBars);
+    const uint32_t *round_desc = reinterpret_cast<const uint32_t *>(smem + kOffRound);
+    bool ok = true, stop = false;
+    uint32_t units = 0, s_round = 0, o_round = 0;   // units begun; the next round whose S, whose O, is due
+    uint32_t fresh = 0;                             // bit: the round (by parity) is its unit's first
+    for (uint32_t polls = 0; ok && !(stop && o_round == s_round);) {
+        if (!stop && s_round < o_round + 2u && mbar_test_pair(bars + kBarFull + (s_round & 1u), (s_round >> 1) & 1u)) {
+            const uint32_t pair = s_round & 1u;
+            polls = 0;
+            if (round_desc[4 * pair] == kStopUnit) {
+                stop = true;
+                mbar_arrive(bars + kBarS + pair);   // the softmax warps read the stop mark
+                continue;
+            }
+            const bool first = (round_desc[4 * pair + 1] & kFirstRound) != 0u;
+            fresh = first ? fresh | 1u << pair : fresh & ~(1u << pair);
+            if (first) ok = mbar_wait(bars + kBarQ, units++ & 1u, p.wait_polls);   // the unit's queries are in tensor memory
+            if (ok) issue_scores<kDim, kSplitQ, kCluster>(smem, tmem, bars, s_round++);
+        } else if (o_round < s_round && mbar_test_pair(bars + kBarP, o_round & 1u)) {
+            polls = 0;
+            issue_output<kDim, kCluster>(smem, tmem, bars, o_round, (fresh >> (o_round & 1u) & 1u) != 0u);
+            ++o_round;
+        } else if (++polls / 16u >= p.wait_polls) {   // these polls do not suspend the thread
+            ok = false;
+        }
+    }
+    if (!ok) raise_status(p, CF_B200_DEVSTAT_WAIT_EXPIRED);
+    // What the other CTA of the pair still signals here has to land before this one leaves; leaving early, the last product of
+    // this one as well. Bounded, whatever happened.
+    for (uint32_t r = o_round < 2u ? 0u : o_round - 2u; ok && r < o_round; ++r) mbar_wait_pair(bars + kBarFree + (r & 3u), (r >> 2) & 1u, p.wait_polls);
+    if (!ok && o_round) mbar_wait(bars + kBarO + ((o_round - 1u) & 1u), ((o_round - 1u) >> 1) & 1u, p.wait_polls);
+}
+
+// ---- softmax group: warps 12..19; in a CTA on its own its thread 0 also issues the tensor-core work -------------------------------------------------------------------------------------------
 // kSplitQ: the queries are fp32; a row goes to tensor memory as binary16(q) and as binary16(q - binary16(q)), and S is the
 // sum of two products, which equals the fp32-query product to 2^-22 relative.
 //
@@ -587,7 +658,7 @@ __device__ __forceinline__ void softmax_role(const AttentionParams &p, uint8_t *
                                              uint32_t lane, uint32_t tile_groups, const SharedSplit &split) {
     constexpr uint32_t kHalfDim = kDim / 2;   // channels of a thread
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + kOffBars);
-    uint64_t *bar_full = bars + kBarFull, *bar_free = bars + kBarFree, *bar_s = bars + kBarS, *bar_o = bars + kBarO;
+    uint64_t *bar_full = bars + kBarFull, *bar_s = bars + kBarS, *bar_o = bars + kBarO;
     const uint32_t worker = blockIdx.x / kCluster, rank = kCluster == 1 ? 0u : cluster_rank();
     const uint32_t *round_desc = reinterpret_cast<const uint32_t *>(smem + kOffRound);
     const uint32_t shared_pages = hdr->shared_pages;
@@ -597,7 +668,8 @@ __device__ __forceinline__ void softmax_role(const AttentionParams &p, uint8_t *
     // their own.
     const uint32_t half = (warp - kDecodeWarps) >> 2, row_in_tile = (warp & 3u) * 32u + lane, pair_barrier = 2u + (warp & 3u);
     const uint32_t tmem_row = tmem + (((warp & 3u) * 32u) << 16);
-    const bool issuer = warp == kDecodeWarps && lane == 0;
+    constexpr bool kIssuerWarp = kCluster == 2;
+    const bool issuer = !kIssuerWarp && warp == kDecodeWarps && lane == 0;
 
     bool failed = false;   // warp-uniform
     auto wait = [&](uint64_t *bar, uint32_t parity) {
@@ -643,20 +715,12 @@ __device__ __forceinline__ void softmax_role(const AttentionParams &p, uint8_t *
         }
         tmem_store_wait();
         tc_fence_before();
-    };
-    // Issuer only: S of round r, whose tiles are there.
-    auto issue_s = [&](uint32_t r) {
-        fence_async_smem<kCluster>();
-        tc_fence_after();
-        const uint32_t k_tile = smem_addr(smem + kOffTiles + (r & 1u) * 2u * kTileBytes), s_to = tmem + kColS + 128u * (r & 1u);
-#pragma unroll
-        for (uint32_t s = 0; s < kDim / 16; ++s) umma(s_to, tmem + kColQ + 8u * s, tile_desc(k_tile + 256u * s), s, kIdescS);
-        if constexpr (kSplitQ) {
-#pragma unroll
-            for (uint32_t s = 0; s < kDim / 16; ++s) umma(s_to, tmem + kColQResidue + 8u * s, tile_desc(k_tile + 256u * s), 1u, kIdescS);
+        if constexpr (kIssuerWarp) {
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bars + kBarQ);
         }
-        umma_commit(&bar_s[r & 1u]);
     };
+    auto issue_s = [&](uint32_t r) { issue_scores<kDim, kSplitQ, kCluster>(smem, tmem, bars, r); };   // issuer only
     uint32_t rounds = 0;    // whose O has been issued
     uint32_t s_round = 0;   // issuer: the next round whose S is due
     // Issuer only: S of round r ahead of its turn, unless its tiles are not there yet or its queries are another unit's.
@@ -669,7 +733,7 @@ __device__ __forceinline__ void softmax_role(const AttentionParams &p, uint8_t *
 
     UnitShape u = unit_shape(p, split, worker, 0u, tile_groups, shared_pages);
     if (u.valid) load_queries(u);
-    group_any<kSoftmaxWarps * 32>(1u, false);
+    if constexpr (!kIssuerWarp) group_any<kSoftmaxWarps * 32>(1u, false);
     float m_run = -CUDART_INF_F, l_run = 0.0f;   // the row's running maximum; this thread's half of its running sum
     float v_unit = 0.0f;                          // largest V scale met so far in the unit: the unit of O
     int32_t seen = 0;   // tokens from the round's first on that the row's query token sees (16 per page and more: all of it)
@@ -684,22 +748,24 @@ __device__ __forceinline__ void softmax_role(const AttentionParams &p, uint8_t *
         const float *meta = reinterpret_cast<const float *>(smem + kOffMeta) + pair * 4u * kRoundPages;
         float *row_max = reinterpret_cast<float *>(smem + kOffRowMax) + 256u * pair;
         const uint32_t s_cols = tmem_row + kColS + 128u * pair;   // scores, then weights [0, 64) and their residues [64, 128)
-        if (issuer && s_round == it) {   // one thread polls, the others sleep at the barrier
-            if (!failed && !mbar_wait_pair(&bar_full[pair], (it >> 1) & 1u, p.wait_polls)) {
-                failed = true;
-                raise_status(p, CF_B200_DEVSTAT_WAIT_EXPIRED);
+        if constexpr (!kIssuerWarp) {
+            if (issuer && s_round == it) {   // one thread polls, the others sleep at the barrier
+                if (!failed && !mbar_wait_pair(&bar_full[pair], (it >> 1) & 1u, p.wait_polls)) {
+                    failed = true;
+                    raise_status(p, CF_B200_DEVSTAT_WAIT_EXPIRED);
+                }
+                if (!failed && round_desc[4 * pair] != kStopUnit) issue_s(it);
+                s_round = it + 1u;
             }
-            if (!failed && round_desc[4 * pair] != kStopUnit) issue_s(it);
-            s_round = it + 1u;
+            failed = __any_sync(0xffffffffu, failed);
+            if (group_any<kSoftmaxWarps * 32>(1u, failed) || round_desc[4 * pair] == kStopUnit) break;
         }
-        failed = __any_sync(0xffffffffu, failed);
-        if (group_any<kSoftmaxWarps * 32>(1u, failed)) break;
-        const uint32_t unit = round_desc[4 * pair], flags = round_desc[4 * pair + 1];
-        if (unit == kStopUnit) break;
         wait(&bar_s[pair], (it >> 1) & 1u);
         tc_fence_after();
+        const uint32_t unit = round_desc[4 * pair], flags = round_desc[4 * pair + 1];
+        const bool stop = failed || unit == kStopUnit;
         uint32_t s_raw[2][32];
-        if (!failed) {
+        if (!stop) {
             tmem_load32(s_cols + 64u * half, s_raw[0]);
             tmem_load32(s_cols + 64u * half + 32u, s_raw[1]);
             if (flags & kFirstRound) {
@@ -734,7 +800,7 @@ __device__ __forceinline__ void softmax_role(const AttentionParams &p, uint8_t *
             row_max[half * 128u + row_in_tile] = part_max;
         }
         tc_fence_before();   // both threads of a row have read their scores: the weights may overwrite them
-        group_any<64>(pair_barrier, false);
+        if (group_any<64>(pair_barrier, kIssuerWarp && failed) || (kIssuerWarp && stop)) break;
         tc_fence_after();
         if (issuer && !failed) issue_s_early(it + 1u);
 
@@ -804,20 +870,17 @@ __device__ __forceinline__ void softmax_role(const AttentionParams &p, uint8_t *
         }
         tmem_store_wait();
         tc_fence_before();
-        if (group_any<kSoftmaxWarps * 32>(1u, failed)) break;
-        if (issuer) {   // O += P V
-            tc_fence_after();
-            const uint32_t v_tile = smem_addr(smem + kOffTiles + pair * 2u * kTileBytes + kTileBytes), p_from = tmem + kColS + 128u * pair;
-#pragma unroll
-            for (uint32_t s = 0; s < 8; ++s) umma(tmem + kColO, p_from + 8u * s, tile_desc(v_tile + 256u * s), (flags & kFirstRound) && !s ? 0u : 1u, kIdescO<kDim>);
-#pragma unroll
-            for (uint32_t s = 0; s < 8; ++s) umma(tmem + kColO, p_from + 64u + 8u * s, tile_desc(v_tile + 256u * s), 1u, kIdescO<kDim>);
-            if constexpr (kCluster == 1) umma_commit(&bar_free[it & 3u]);   // the decoders may refill this pair of tiles
-            else umma_commit_pair(&bar_free[it & 3u]);
-            umma_commit(&bar_o[pair]);
-            issue_s_early(it + 1u);
+        if constexpr (kIssuerWarp) {
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bars + kBarP);
+        } else {
+            if (group_any<kSoftmaxWarps * 32>(1u, failed)) break;
+            if (issuer) {
+                issue_output<kDim, kCluster>(smem, tmem, bars, it, (flags & kFirstRound) != 0u);
+                issue_s_early(it + 1u);
+            }
+            __syncwarp();
         }
-        __syncwarp();
         rounds = it + 1u;
         if (p.one_slot) seen -= 16 * static_cast<int32_t>(kRoundPages);
 
@@ -831,7 +894,8 @@ __device__ __forceinline__ void softmax_role(const AttentionParams &p, uint8_t *
             // the two halves of the row's sum take the places of the maxima: O of this round is complete, so every warp has stored
             // its weights, and read the maxima before
             row_max[half * 128u + row_in_tile] = l_run;
-            if (group_any<kSoftmaxWarps * 32>(1u, failed)) break;   // the next unit's queries are stored, too
+            // for a CTA on its own the next unit's queries are stored, too
+            if (kIssuerWarp ? group_any<64>(pair_barrier, failed) : group_any<kSoftmaxWarps * 32>(1u, failed)) break;
             const uint32_t row = (done.tile_index * kCluster + rank) * 128u + row_in_tile;
             const bool live = row < rows_total;   // whole warps go on: the tensor-memory loads are warp-wide
             float *dst = live ? shared_partial_ptr(p, done.chunk, row / G, done.head_local * G + row % G) : nullptr;
@@ -859,13 +923,8 @@ __device__ __forceinline__ void softmax_role(const AttentionParams &p, uint8_t *
             tc_fence_before();
         }
     }
-    // What the other CTA of the pair still signals here has to land before this one leaves; leaving early, the last product of
-    // this one as well. Bounded, whatever happened.
-    if (issuer && rounds) {
-        if (kCluster == 2 && !failed)
-            for (uint32_t r = rounds < 2u ? 0u : rounds - 2u; r < rounds; ++r) mbar_wait_pair(&bar_free[r & 3u], (r >> 2) & 1u, p.wait_polls);
-        if (failed) mbar_wait(&bar_o[(rounds - 1u) & 1u], ((rounds - 1u) >> 1) & 1u, p.wait_polls);
-    }
+    // leaving early: give the tensor core's last commit a bounded chance to arrive before tensor memory is freed
+    if (issuer && rounds && failed) mbar_wait(&bar_o[(rounds - 1u) & 1u], ((rounds - 1u) >> 1) & 1u, p.wait_polls);
 }
 
 template <int kDim, bool kSplitQ, int kCluster>
@@ -888,7 +947,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) prefix_attention_kernel(Attenti
         mbar_init(bars + kBarFull, kRoundPages);                    // full[0], full[1]: one arrival per page slot of the round
         mbar_init(bars + kBarFull + 1, kRoundPages);
         for (uint32_t i = 0; i < 4u; ++i) mbar_init(bars + kBarFree + i, kCluster);   // tensor-core commits, of both CTAs
-        for (uint32_t i = kBarS; i < kBarCount; ++i) mbar_init(bars + i, 1);          // tensor-core commits
+        for (uint32_t i = kBarS; i < kBarP; ++i) mbar_init(bars + i, 1);          // tensor-core commits
+        mbar_init(bars + kBarP, kSoftmaxWarps);   // weights stored, queries stored (where a warp of its own issues)
+        mbar_init(bars + kBarQ, kSoftmaxWarps);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncwarp();
@@ -908,7 +969,12 @@ __global__ void __launch_bounds__(kTcThreads, 1) prefix_attention_kernel(Attenti
 
     if (warp < kDecodeWarps) {   // whole warpgroups on either side: the register split is per warpgroup
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kDecoderRegs));
-        decoder_role<kDim, kCluster>(p, smem, hdr, warp, lane, tile_groups, split);
+        if (warp < kDecoders<kCluster>) {
+            decoder_role<kDim, kCluster>(p, smem, hdr, warp, lane, tile_groups, split);
+        } else {
+            if (lane == 0) issuer_role<kDim, kSplitQ, kCluster>(p, smem, tmem);
+            __syncwarp();
+        }
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSoftmaxRegs));
         softmax_role<kDim, kSplitQ, kCluster>(p, smem, hdr, tmem, warp, lane, tile_groups, split);
