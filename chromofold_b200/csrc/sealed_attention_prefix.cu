@@ -334,6 +334,30 @@ __device__ __forceinline__ void tmem_store8(uint32_t taddr, const uint32_t (&v)[
                  "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
                  : "memory");
 }
+// Two fp32 operations in one instruction, and the largest of three.
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    float2 r;
+    asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%6, %7};\n\tfma.rn.f32x2 x, x, y, z;\n\tmov.b64 {%0, %1}, x;\n\t}"
+        : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return r;
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+    float2 r;
+    asm("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmul.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;\n\t}"
+        : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    float2 r;
+    asm("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tadd.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;\n\t}"
+        : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
+}
+__device__ __forceinline__ float max3(uint32_t a, uint32_t b, uint32_t c) {
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(__uint_as_float(a)), "f"(__uint_as_float(b)), "f"(__uint_as_float(c)));
+    return r;
+}
 // 2^x by the special-function unit (inputs below -126 give 0, -inf gives 0)
 __device__ __forceinline__ float fast_exp2(float x) {
     float r;
@@ -786,10 +810,15 @@ __device__ __forceinline__ void softmax_role(const AttentionParams &p, uint8_t *
                 const uint32_t count = seen_of(pg, __float_as_uint(meta[4 * pg + 2]));
                 const float ks = meta[4 * pg];
                 if (count == 16u && !descending) {   // a full page (the usual case): the scale is applied to the extreme, not to every score
-                    float hi = __uint_as_float(s_raw[q >> 1][16 * (q & 1)]);
+                    const uint32_t *sc = &s_raw[q >> 1][16 * (q & 1)];
+                    float a = max3(sc[0], sc[1], sc[2]), b = max3(sc[3], sc[4], sc[5]);
 #pragma unroll
-                    for (int j = 1; j < 16; ++j) hi = fmaxf(hi, __uint_as_float(s_raw[q >> 1][16 * (q & 1) + j]));
-                    part_max = fmaxf(part_max, hi * ks);
+                    for (int j = 6; j < 14; j += 4) {
+                        a = max3(__float_as_uint(a), sc[j], sc[j + 1]);
+                        b = max3(__float_as_uint(b), sc[j + 2], sc[j + 3]);
+                    }
+                    a = max3(__float_as_uint(a), sc[14], sc[15]);
+                    part_max = fmaxf(part_max, fmaxf(a, b) * ks);
                 } else {
 #pragma unroll
                     for (int j = 0; j < 16; ++j)
@@ -821,7 +850,7 @@ __device__ __forceinline__ void softmax_role(const AttentionParams &p, uint8_t *
         }
         // weights as binary16 plus their rounding residue (two A operands), so that P V is accurate to fp32 level
         // whatever the spread of the V scales
-        float sum = 0.0f;
+        float2 sums = make_float2(0.0f, 0.0f);
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             const uint32_t pg = 4u * half + q;
@@ -833,24 +862,25 @@ __device__ __forceinline__ void softmax_role(const AttentionParams &p, uint8_t *
             uint32_t hi[8], lo[8];
 #pragma unroll
             for (int j = 0; j < 16; j += 2) {
-                float w0 = fast_exp2(fmaf(__uint_as_float(s_raw[q >> 1][16 * (q & 1) + j]), ks, -z));
-                float w1 = fast_exp2(fmaf(__uint_as_float(s_raw[q >> 1][16 * (q & 1) + j + 1]), ks, -z));
+                const float2 x = fma2(make_float2(__uint_as_float(s_raw[q >> 1][16 * (q & 1) + j]), __uint_as_float(s_raw[q >> 1][16 * (q & 1) + j + 1])),
+                                      make_float2(ks, ks), make_float2(-z, -z));
+                float2 w = make_float2(fast_exp2(x.x), fast_exp2(x.y));
                 if (count != 16u) {   // tokens past the page's count, or past the row's position, weigh nothing
-                    w0 = static_cast<uint32_t>(j) < count ? w0 : 0.0f;
-                    w1 = static_cast<uint32_t>(j + 1) < count ? w1 : 0.0f;
+                    w.x = static_cast<uint32_t>(j) < count ? w.x : 0.0f;
+                    w.y = static_cast<uint32_t>(j + 1) < count ? w.y : 0.0f;
                 }
-                sum += w0 + w1;
-                const float a0 = w0 * ratio, a1 = w1 * ratio;
-                const __half2 h = __floats2half2_rn(a0, a1);
-                const float2 back = __half22float2(h);
-                const __half2 l = __floats2half2_rn(a0 - back.x, a1 - back.y);
+                sums = add2(sums, w);
+                const float2 scaled = mul2(w, make_float2(ratio, ratio));
+                const __half2 h = __floats2half2_rn(scaled.x, scaled.y);
+                const float2 rest = fma2(__half22float2(h), make_float2(-1.0f, -1.0f), scaled);   // exact
+                const __half2 l = __floats2half2_rn(rest.x, rest.y);
                 hi[j >> 1] = *reinterpret_cast<const uint32_t *>(&h);
                 lo[j >> 1] = *reinterpret_cast<const uint32_t *>(&l);
             }
             tmem_store8(s_cols + 8u * pg, hi);          // 16 tokens = 8 columns of pairs
             tmem_store8(s_cols + 64u + 8u * pg, lo);
         }
-        l_run = l_run * alpha + sum;   // this thread's half of the row's sum; the halves are added at the unit's end
+        l_run = l_run * alpha + (sums.x + sums.y);   // this thread's half of the row's sum; the halves are added at the unit's end
         // O in tensor memory follows the new maximum and unit (this thread's channels), once the previous round's product has
         // reached it; skipped when no row of the warp moved
         if (!(flags & kFirstRound) && !__all_sync(0xffffffffu, o_scale == 1.0f)) {
