@@ -40,7 +40,7 @@ template <int NG, bool kSplitQ> constexpr int kHeadGroups = kSplitQ ? NG / 2 : N
 template <int NG, int NB, bool kSplitQ, int kDim>
 constexpr int kWarpsOf = NB == 32                ? (kHeadGroups<NG, kSplitQ> == 1 ? 24 : 16)
                          : kDim <= 64            ? 20
-                         : NG == 4               ? (kDim == 96 ? 14 : 12)
+                         : NG == 4               ? (kDim < 128 ? 14 : 12)
                          : NG == 2               ? 14
                                                  : 16;
 template <int NG, int NB, bool kSplitQ, int kDim> constexpr int kThreadsOf = kWarpsOf<NG, NB, kSplitQ, kDim> * 32;
@@ -50,8 +50,8 @@ template <int NG, int NB, bool kSplitQ, int kDim> constexpr int kThreadsOf = kWa
 template <int NG, int kDim = 128>
 struct UnitState {
     float score[NG][4];      // S fragments of the current page
-    float acc[NG][kDim / 32][4];   // O fragments: [group][channel of the lane's V block][fragment register]
-    uint32_t vq[kDim / 8];   // V symbols of the current page, [channel*4 + token quad]
+    float acc[NG][(kDim + 31) / 32][4];   // O fragments: [group][channel of the lane's V block][fragment register]
+    uint32_t vq[4 * ((kDim + 31) / 32)];   // V symbols of the current page, [channel*4 + token quad]
     float m0[NG], m1[NG], l0[NG], l1[NG];  // running max / partial sum of the lane's two heads of each group
     uint32_t *dump;          // kDump only: where this lane's quads of the current record go (K at +0, V at +512 words)
 };
@@ -206,8 +206,13 @@ __device__ __forceinline__ void decode_v_only(VLane &v, UnitState<NG> &u) {
 // 96 with 64-symbol blocks there are 48 blocks for 32 lanes: every lane takes block `lane`, the first sixteen
 // lanes also block `lane + 32`.
 // one lane's kDim / 2 symbols + padding that keeps the row stride off multiples of 64 bytes
+// Head_dim 80 (1280 symbols, 20 blocks): a lane's K share is 40 symbols, and three V channels, of which lanes 27..31 have none and
+// lane 26 two; what they read instead goes to channels that are never stored. Its tile has no padding: rows of 40 and 48
+// bytes are off each other's banks as they are.
+template <int kDim> constexpr int kVChannelsOf = (kDim + 31) / 32;
 template <int kDim> constexpr uint32_t kTileRowOf = kDim / 2u + ((kDim / 2u + 16u) % 64u == 0 ? 32u : 16u);
-template <int kDim> constexpr uint32_t kTileStreamOf = 32u * kTileRowOf<kDim>;
+template <int kDim> constexpr uint32_t kTileStreamOf = kDim == 80 ? 1280u : 32u * kTileRowOf<kDim>;   // bytes of the K part
+template <int kDim> constexpr uint32_t kTileBytesOf = kDim == 80 ? 1280u + 32u * 48u + 32u : 2u * kTileStreamOf<kDim> + 32u;
 
 template <int NB, int kDim, class Lane>
 __device__ __forceinline__ void stage_with(Lane &d, uint32_t block, uint8_t *tile) {
@@ -217,7 +222,8 @@ __device__ __forceinline__ void stage_with(Lane &d, uint32_t block, uint8_t *til
     for (int q = 0; q < kQuads; q += 4) {
         const uint32_t a = d.quad(q), b = d.quad(q + 1), c = d.quad(q + 2), e = d.quad(q + 3);
         const uint32_t at = block * kQuads + q;   // quad index in the stream: row = at / kRowQuads, column = at % kRowQuads
-        *reinterpret_cast<uint4 *>(tile + (at / kRowQuads) * kTileRowOf<kDim> + (at % kRowQuads) * 4u) = make_uint4(a, b, c, e);
+        const uint32_t to = kDim == 80 ? 4u * at : (at / kRowQuads) * kTileRowOf<kDim> + (at % kRowQuads) * 4u;
+        *reinterpret_cast<uint4 *>(tile + to) = make_uint4(a, b, c, e);
     }
 }
 
@@ -262,9 +268,9 @@ struct WarpLayout {
     static constexpr uint32_t kZero = kPLo + kPBytes;
     static constexpr uint32_t kBar = kZero + 128;
     static constexpr uint32_t kQRows = kBar + 16;
-    static constexpr uint32_t kQRowWords = kDim / 4 + 4;
+    static constexpr uint32_t kQRowWords = kDim / 4 + (kDim == 80 ? 8 : 4);
     static constexpr uint32_t kTile = (kQRows + 8 * NG * kQRowWords * 4 + 15u) / 16u * 16u;   // NB != 32 only
-    static constexpr uint32_t kBytes = kTile + (NB != 32 ? 2u * kTileStreamOf<kDim> + 32u : 0u);
+    static constexpr uint32_t kBytes = kTile + (NB != 32 ? kTileBytesOf<kDim> : 0u);
     static constexpr uint32_t kSmem = kTableBytes + kWarpsOf<NG, NB, kSplitQ, kDim> * kBytes;
     static_assert(kSmem <= 232448, "a CTA has 227 KB of shared memory");
 };
@@ -276,9 +282,9 @@ template <int NG, int kMode, bool kSplitQ, int NB, int kDim>
 __global__ void __launch_bounds__(kThreadsOf<NG, NB, kSplitQ, kDim>, 1) lanes_attention_kernel(AttentionParams p, uint32_t after_prefix) {
     constexpr bool kProbe = kMode != kAttend;
     static_assert(!kSplitQ || NG != 1, "split queries take two groups for four heads");
-    static_assert(NB == 32 || NB == 24 || NB == 16 || NB == 12 || NB == 8 || NB == 4, "blocks per stream");
-    static_assert(kDim == 128 || ((kDim == 96 || kDim == 64 || kDim == 32) && NB != 32), "other head_dims go through the staging tile");
-    constexpr int kQ = kDim / 8, kVCh = kDim / 32, kSyms = 16 * kDim;   // quads per lane and stream; V channels per lane
+    static_assert(NB == 32 || NB == 24 || NB == 20 || NB == 16 || NB == 12 || NB == 8 || NB == 4, "blocks per stream");
+    static_assert(kDim == 128 || ((kDim == 96 || kDim == 80 || kDim == 64 || kDim == 32) && NB != 32), "other head_dims go through the staging tile");
+    constexpr int kQ = kDim / 8, kVCh = kVChannelsOf<kDim>, kSyms = 16 * kDim;   // K quads per lane; V channels per lane
     constexpr uint32_t kRowWords = kDim / 4;   // words of half a query row (the channels one lane's K block covers)
     using L = WarpLayout<NG, NB, kSplitQ, kDim>;
     constexpr int NS = kHeadGroups<NG, kSplitQ>;
@@ -474,7 +480,7 @@ __global__ void __launch_bounds__(kThreadsOf<NG, NB, kSplitQ, kDim>, 1) lanes_at
                 } else {
                     if constexpr (kMode == kDump)   // [page id][kv head][K stream | V stream], one byte per symbol
                         u.dump = reinterpret_cast<uint32_t *>(p.output) +
-                                 (static_cast<uint64_t>(dump_page) * p.kv_head_count + kv_head) * (kSyms / 2) + kQ * lane;
+                                 (static_cast<uint64_t>(dump_page) * p.kv_head_count + kv_head) * (kSyms / 2) + (kDim == 80 ? 0u : kQ * lane);
                     const float k_scale = __half2float(__ushort_as_half(static_cast<unsigned short>(hv.z & 0xffffu))) *
                                           (p.softmax_scale * kLog2e);
                     const float v_scale = __half2float(__ushort_as_half(static_cast<unsigned short>(hv.z >> 16)));
@@ -499,6 +505,34 @@ __global__ void __launch_bounds__(kThreadsOf<NG, NB, kSplitQ, kDim>, 1) lanes_at
                         __syncwarp();
                         if (i + 1 < n_pages) issue(entry_next);   // the record is decoded: its place takes the next one
                         next_issued = true;
+                        if constexpr (kDim == 80) {
+                            const uint8_t *k_row = tile + 40u * lane, *v_row = tile + kTileStreamOf<kDim> + 16u + 48u * lane;
+#pragma unroll
+                            for (int c = 0; c < 3; ++c) {
+                                const uint4 vv = *reinterpret_cast<const uint4 *>(v_row + 16u * c);
+                                const uint32_t vq[4] = {vv.x, vv.y, vv.z, vv.w};
+#pragma unroll
+                                for (int j = 0; j < 4; ++j) {
+                                    const uint32_t at = 12u * lane + 4u * c + j;   // of the stream's 320 quads
+                                    if constexpr (kMode == kFold) u.vq[0] ^= at < 320u ? vq[j] : 0u;
+                                    else if constexpr (kMode == kAttend) u.vq[4 * c + j] = vq[j];
+                                    else if (at < 320u) u.dump[320u + at] = vq[j];
+                                }
+                            }
+#pragma unroll
+                            for (int q = 0; q < kQ; q += 2) {
+                                const uint2 kk = *reinterpret_cast<const uint2 *>(k_row + 4u * q);
+                                if constexpr (kMode == kFold) {
+                                    u.vq[0] ^= kk.x ^ kk.y;
+                                } else if constexpr (kMode == kDump) {
+                                    u.dump[kQ * lane + q] = kk.x;
+                                    u.dump[kQ * lane + q + 1] = kk.y;
+                                } else {
+                                    score_quad(u, qs, q, kk.x);
+                                    score_quad(u, qs, q + 1, kk.y);
+                                }
+                            }
+                        } else {
 #pragma unroll
                         for (int c = 0; c < kQ / 4; ++c) {
                             const uint4 kk = *reinterpret_cast<const uint4 *>(tile + lane * kTileRowOf<kDim> + 16u * c);
@@ -517,6 +551,7 @@ __global__ void __launch_bounds__(kThreadsOf<NG, NB, kSplitQ, kDim>, 1) lanes_at
                                     score_quad(u, qs, q, kq[j]);
                                 }
                             }
+                        }
                         }
                         if constexpr (kProbe) __syncwarp();   // the tile is rewritten for the next page
                     } else if (k_coder == CF_B200_CODER_RANS_SPLIT4 && v_coder == CF_B200_CODER_RANS_SPLIT4) {
@@ -723,7 +758,7 @@ __global__ void __launch_bounds__(kThreadsOf<NG, NB, kSplitQ, kDim>, 1) lanes_at
 #pragma unroll
                     for (int c = 0; c < 4; ++c) {
                         const uint32_t owner = 4u * (2u * t + (c & 1)) + (g >> 2) + 2u * (c >> 1);  // lane whose V block it is
-                        dst[kVCh * owner + dd] = u.acc[n][dd][c] * (v_unit * (1.0f / kWeightScale));
+                        if (kDim != 80 || kVCh * owner + dd < 80u) dst[kVCh * owner + dd] = u.acc[n][dd][c] * (v_unit * (1.0f / kWeightScale));
                     }
                 }
             }
@@ -740,7 +775,7 @@ bool lanes_kernel_supports(const AttentionParams &p) {
     const bool geometry = p.page_tokens == 16 &&
                           ((p.head_dim == 128 && (p.block_size == 64 || p.block_size == 128 || p.block_size == 256)) ||
                            ((p.head_dim == 96 || p.head_dim == 64) && (p.block_size == 64 || p.block_size == 128)) ||
-                           (p.head_dim == 32 && p.block_size == 64));
+                           ((p.head_dim == 80 || p.head_dim == 32) && p.block_size == 64));
     return geometry && p.group >= 1 && p.group <= 16 &&
            (p.query_type == CF_B200_F16 || p.query_type == CF_B200_F32);
 }
@@ -760,9 +795,11 @@ cudaError_t with_heads(const AttentionParams &p, F f) {
 }
 template <class F>
 cudaError_t with_variant(const AttentionParams &p, F f) {
-    // 16 x 64 pages have 16 (or 8) blocks per stream, 16 x 96 pages 24 (or 12), 16 x 32 pages 8: always staged
+    // 16 x 64 pages have 16 (or 8) blocks per stream, 16 x 96 pages 24 (or 12), 16 x 80 pages 20, 16 x 32
+    // pages 8: always staged
     if (p.head_dim == 64) return p.block_size == 64 ? with_heads<16, 64>(p, f) : with_heads<8, 64>(p, f);
     if (p.head_dim == 96) return p.block_size == 64 ? with_heads<24, 96>(p, f) : with_heads<12, 96>(p, f);
+    if (p.head_dim == 80) return with_heads<20, 80>(p, f);
     if (p.head_dim == 32) return with_heads<8, 32>(p, f);
     if (p.block_size == 128) return with_heads<16, 128>(p, f);
     if (p.block_size == 256) return with_heads<8, 128>(p, f);

@@ -72,3 +72,24 @@ def test_a_chunk_of_query_tokens_sees_each_token_up_to_its_own(native, oracle, h
     ok, err = attention_close(out.cpu().numpy()[some], want)
     assert ok, err
     lib.cf_device_kv_destroy(kv, None)
+
+
+@pytest.mark.parametrize("heads,dim,coder,f32,window", [
+    ((8, 8), 80, "rans4", False, 0), ((32, 8), 80, "huffman4", True, 200), ((14, 2), 80, "rans", True, 0), ((40, 4), 80, "huffman", False, 0),
+    ((6, 1), 80, "fixed8", True, 0), ((64, 8), 128, "rans4", True, 0), ((16, 1), 64, "rans", True, 77), ((24, 4), 96, "huffman4", True, 0)])
+def test_lane_kernels_agree_with_the_any_geometry_kernel(native, heads, dim, coder, f32, window):
+    import torch
+    from chromofold_b200.workloads import build_sealed_layer
+    hq, hkv = heads
+    layer, _ = build_sealed_layer(np.array([16, 16 * 70, 16 * 9, 16 * 33]), query_heads=hq, kv_heads=hkv, head_dim=dim, coder=coder, seed=9)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(10)
+    tails = torch.randn((4, hkv, 16, dim), generator=g, device="cuda").half()
+    layer.fill_tails([0, 1, 2, 3], tails, tails.flip(0).contiguous(), 5)
+    q = torch.randn((4, hq, dim), generator=g, device="cuda")
+    q = q if f32 else q.half()
+    fast = layer.attention(q, kernel=native.KERNEL_LANES, causal_window=window).cpu().numpy()
+    slow = layer.attention(q, kernel=native.KERNEL_GENERIC, causal_window=window).cpu().numpy()
+    assert layer.device_status() == 0
+    ok, err = attention_close(fast, slow, rel=2e-5, abs_=2e-5)
+    assert ok, err
