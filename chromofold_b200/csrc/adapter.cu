@@ -15,6 +15,7 @@
 #include <cuda_runtime.h>
 
 #include "attention_params.cuh"
+#include "host_rows.h"
 #include "chromofold_b200/compat_adapter.h"
 #include "chromofold_b200/compat_kv.h"
 #include "chromofold_b200/sealed_kv.h"
@@ -81,7 +82,8 @@ struct KiviJob {
     const float *stage_k, *stage_v;
     float *tail_k, *tail_v;
     uint32_t row_stride, tail_rows, tokens, dim, bits, pages, rest_rows;
-    uint32_t *first_bad;                       // host-mapped: lowest page that holds a non-finite value (its page is not to be used)
+    cf_kv_device_page *pages_out;              // descriptor of page p goes to pages_out[p]
+    cf_kv_device_page page;                    // what those of all pages have in common; token_begin is page 0's
     uint8_t *block[kKiviPagesPerLaunch];
 };
 
@@ -133,17 +135,12 @@ __global__ void __launch_bounds__(1024) kivi_quantise_kernel(const __grid_consta
         }
     }
     __syncthreads();
-    int bad = 0;
     for (uint32_t i = threadIdx.x; i < dim + tokens; i += blockDim.x) {   // dim K channels, then tokens V rows
         const uint32_t m = magnitudes[i];
-        bad |= m >= 0x7f800000u;   // inf and NaN lie above every finite magnitude
         const float scale = m == 0u ? 1.0f : __fdiv_rn(__uint_as_float(m), static_cast<float>(qmax));
         magnitudes[i] = __float_as_uint(scale);
     }
-    if (__syncthreads_or(bad)) {   // kv_gpu_fixture.cpp:13: a non-finite value is an error; nothing of the page is used
-        if (threadIdx.x == 0) atomicMin_system(job.first_bad, page);
-        return;
-    }
+    __syncthreads();
     const float *k_scale = reinterpret_cast<const float *>(k_mag), *v_scale = reinterpret_cast<const float *>(v_mag);
     const uint32_t per_word = 32u / bits;
     uint8_t *block = job.block[page];
@@ -196,6 +193,17 @@ __global__ void __launch_bounds__(1024) kivi_quantise_kernel(const __grid_consta
         reinterpret_cast<int32_t *>(block + lay.k_offsets)[b] = static_cast<int32_t>(b * 64u * bits);
         reinterpret_cast<int32_t *>(block + lay.v_offsets)[b] = static_cast<int32_t>(b * 64u * bits);
     }
+    if (threadIdx.x == 0) {
+        cf_kv_device_page d = job.page;
+        d.k_words = kw;
+        d.v_words = vw;
+        d.k_scales = reinterpret_cast<const float *>(block + lay.k_scales);
+        d.v_scales = reinterpret_cast<const float *>(block + lay.v_scales);
+        d.k_block_offsets = reinterpret_cast<const int32_t *>(block + lay.k_offsets);
+        d.v_block_offsets = reinterpret_cast<const int32_t *>(block + lay.v_offsets);
+        d.token_begin += page * tokens;
+        job.pages_out[page] = d;
+    }
     if (page != 0) return;
     __syncthreads();   // the tail's old rows have been read: the rows after the last page take their place
     const uint32_t from = job.pages * tokens - job.tail_rows;
@@ -206,11 +214,27 @@ __global__ void __launch_bounds__(1024) kivi_quantise_kernel(const __grid_consta
     }
 }
 
+// Copies `rows` rows of `dim` floats and returns the first that holds NaN or Inf, or `rows`.
+uint32_t copy_rows_checked(float *dst, const float *src, uint32_t rows, uint32_t dim) {
+    const size_t n = static_cast<size_t>(rows) * dim;
+    if (chromofold_copy_max_magnitude(dst, src, n) < 0x7f800000u) return rows;   // inf and NaN lie above every finite magnitude
+    uint32_t r = 0;
+    while (chromofold_copy_max_magnitude(dst + static_cast<size_t>(r) * dim, src + static_cast<size_t>(r) * dim, dim) < 0x7f800000u) ++r;
+    return r;
+}
+
+uint32_t first_bad_row(const float *src, uint32_t rows, uint32_t dim) {
+    uint32_t r = 0;
+    while (r < rows && chromofold_max_magnitude(src + static_cast<size_t>(r) * dim, dim) < 0x7f800000u) ++r;
+    return r;
+}
+
 struct HeadState {   // per (layer, kv head), in tokens
     uint64_t appended = 0;      // everything ever appended
     uint32_t sealed = 0;        // tokens in sealed tiles
     uint32_t tail = 0;          // tokens in the device tail
     uint32_t next_token = 0;    // position the next append must start at
+    uint32_t bad_row = 0xffffffffu;   // first row of the tail that holds NaN or Inf
     bool started = false;
     bool flushed_partial = false;
 };
@@ -261,15 +285,22 @@ struct cf_llama_kv_adapter {
     std::vector<std::vector<cf_kv_device_page>> kivi_host_descs;                // per layer, the same on the host
     uint64_t kivi_resident_bytes = 0;
     DeviceBuffer<float> kivi_stage;          // rows of an append that fills pages: [K rows | V rows]
-    float *kivi_pinned = nullptr;            // the same on their way from the caller's pageable memory
+    float *kivi_pinned = nullptr;            // the same on their way from the caller's pageable memory, twice: appends take turns
     size_t kivi_stage_floats = 0;            // of one of the two streams
-    uint32_t *kivi_first_bad = nullptr;      // host-mapped word the quantiser reports to
+    cudaEvent_t kivi_done[2] = {};           // the append that used pinned half i has ended
+    uint32_t kivi_turn = 0;                  // pinned half of the next append
+    cudaStream_t kivi_stream = nullptr;      // of the last append, and
+    bool kivi_pending = false;               // whether it may still be under way
     static constexpr size_t kKiviStageBytes = 4u << 20;   // rows staged at a time (at least one page)
 
     ~cf_llama_kv_adapter() {
         for (uint8_t *c : kivi_chunks) cudaFree(c);
+        for (cudaEvent_t e : kivi_done)
+            if (e) {
+                cudaEventSynchronize(e);
+                cudaEventDestroy(e);
+            }
         if (kivi_pinned) cudaFreeHost(kivi_pinned);
-        if (kivi_first_bad) cudaFreeHost(kivi_first_bad);
     }
     size_t kivi_row_floats() const { return static_cast<size_t>(opt.kv_head_count) * opt.head_dim; }
     float *kivi_tail(DeviceBuffer<float> &buffer, uint32_t layer) const {
@@ -301,7 +332,7 @@ struct cf_llama_kv_adapter {
         for (uint32_t v = 0; v < levels; ++v) lut[v] = static_cast<int32_t>(v | (kivi_bits << 8));
         kivi_lut.ensure(levels, s);
         cuda_check(cudaMemcpy(kivi_lut.ptr, lut.data(), levels * 4, cudaMemcpyHostToDevice), "upload lut");
-        cuda_check(cudaHostAlloc(reinterpret_cast<void **>(&kivi_first_bad), sizeof(uint32_t), cudaHostAllocMapped), "cudaHostAlloc");
+        for (cudaEvent_t &e : kivi_done) cuda_check(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "create append event");
         kivi_descs.clear();
         for (uint32_t l = 0; l < opt.layer_count; ++l) {
             kivi_descs.push_back(std::make_unique<DeviceBuffer<cf_kv_device_page>>());
@@ -329,10 +360,24 @@ struct cf_llama_kv_adapter {
         kivi_resident_bytes = 0;
         for (auto &d : kivi_host_descs) d.clear();
     }
+    // Work on stream s comes after the last append, which may have used another stream and still be under way.
+    void kivi_join(cudaStream_t s) {
+        if (!kivi_pending || s == kivi_stream) return;
+        const cudaEvent_t last = kivi_done[(kivi_turn ^ 1u) & 1u];
+        if (cudaEventQuery(last) == cudaSuccess) kivi_pending = false;
+        else cuda_check(cudaStreamWaitEvent(s, last, 0), "wait for the last append");
+    }
+    void kivi_mark(cudaStream_t s) {   // an append's work has been issued on s
+        cuda_check(cudaEventRecord(kivi_done[kivi_turn], s), "record append event");
+        kivi_turn ^= 1u;
+        kivi_stream = s;
+        kivi_pending = true;
+    }
     // Quantise `pages` pages of `tokens` rows of (layer, kv_head): the rows of the tail, then the staged ones; `rest` staged rows
-    // after them become the tail. One launch and one synchronisation: the reference quantises on the host and throws at
-    // once, and so does this front. Returns the pages that were sealed: fewer than asked if the next one holds NaN or Inf.
-    uint32_t kivi_seal(uint32_t layer, uint32_t kv_head, uint32_t pages, uint32_t tokens, uint32_t rest, cudaStream_t s) {
+    // after them become the tail. One launch, which also publishes the descriptors. The rows are known to be finite: they were
+    // checked while they were copied, so that a refusal is thrown at once (the reference quantises on the host and does the
+    // same) and no append waits for the GPU: one of 512 x 128 rows took 85 us, of which 40 are the copy.
+    void kivi_seal(uint32_t layer, uint32_t kv_head, uint32_t pages, uint32_t tokens, uint32_t rest, cudaStream_t s) {
         HeadState &h = head(layer, kv_head);
         const uint32_t D = opt.head_dim;
         const KiviLayout lay = kivi_layout(tokens, D, kivi_bits);
@@ -348,61 +393,57 @@ struct cf_llama_kv_adapter {
         job.bits = kivi_bits;
         job.pages = pages;
         job.rest_rows = rest;
-        job.first_bad = kivi_first_bad;
-        const size_t chunk_index = kivi_chunk_index, chunk_used = kivi_chunk_used;
-        for (uint32_t p = 0; p < pages; ++p) job.block[p] = kivi_take(lay.total);
-        *kivi_first_bad = pages;
-        kivi_quantise_kernel<<<pages, 1024, (static_cast<size_t>(D) + tokens) * sizeof(float), s>>>(job, lay);
-        cuda_check(cudaGetLastError(), "page quantise launch");
+        cf_kv_device_page &common = job.page;
+        common.k_lut = common.v_lut = kivi_lut.ptr;
+        common.token_begin = h.next_token - h.tail;
+        common.token_count = tokens;
+        common.head_dim = D;
+        common.block_size = 64;
+        common.k_max_code_length = common.v_max_code_length = common.fixed_code_length = kivi_bits;
+        common.zero_point = 1u << (kivi_bits - 1);
+        common.kv_head = kv_head;
         std::vector<cf_kv_device_page> &host = kivi_host_descs[layer];
         const size_t first = host.size();
         for (uint32_t p = 0; p < pages; ++p) {
-            const uint8_t *block = job.block[p];
-            cf_kv_device_page page{};
+            const uint8_t *block = job.block[p] = kivi_take(lay.total);
+            cf_kv_device_page page = common;
             page.k_words = reinterpret_cast<const uint32_t *>(block + lay.k_words);
             page.v_words = reinterpret_cast<const uint32_t *>(block + lay.v_words);
             page.k_scales = reinterpret_cast<const float *>(block + lay.k_scales);
             page.v_scales = reinterpret_cast<const float *>(block + lay.v_scales);
             page.k_block_offsets = reinterpret_cast<const int32_t *>(block + lay.k_offsets);
             page.v_block_offsets = reinterpret_cast<const int32_t *>(block + lay.v_offsets);
-            page.k_lut = page.v_lut = kivi_lut.ptr;
-            page.token_begin = h.next_token - h.tail + p * tokens;
-            page.token_count = tokens;
-            page.head_dim = D;
-            page.block_size = 64;
-            page.k_max_code_length = page.v_max_code_length = page.fixed_code_length = kivi_bits;
-            page.zero_point = 1u << (kivi_bits - 1);
-            page.kv_head = kv_head;
+            page.token_begin += p * tokens;
             host.push_back(page);
         }
         DeviceBuffer<cf_kv_device_page> &dev = *kivi_descs[layer];
-        dev.ensure(host.size(), s);   // (entries past the list's length are never read: a refused page's is overwritten later)
-        cuda_check(cudaMemcpyAsync(dev.ptr + first, host.data() + first, pages * sizeof(cf_kv_device_page), cudaMemcpyHostToDevice, s), "publish pages");
-        cuda_check(cudaStreamSynchronize(s), "cudaStreamSynchronize");
-        const uint32_t first_bad = *static_cast<volatile uint32_t *>(kivi_first_bad), sealed = std::min(pages, first_bad);
-        if (sealed < pages) {   // the page blocks after the last good page are handed out again
-            host.resize(first + sealed);
-            kivi_chunk_index = chunk_index;
-            kivi_chunk_used = chunk_used;
-            for (uint32_t p = 0; p < sealed; ++p) kivi_take(lay.total);
-        }
+        dev.ensure(host.size(), s);
+        job.pages_out = dev.ptr + first;
+        kivi_quantise_kernel<<<pages, 1024, (static_cast<size_t>(D) + tokens) * sizeof(float), s>>>(job, lay);
+        cuda_check(cudaGetLastError(), "page quantise launch");
         // EncodedKvPage::resident_bytes: words, offsets, both LUTs, scales
-        kivi_resident_bytes += sealed * (8ull * lay.word_count + 8ull * lay.block_count + 8ull * (1u << kivi_bits) + 4ull * (D + tokens));
-        if (sealed && tokens < opt.page_size) h.flushed_partial = true;
-        h.sealed += sealed * tokens;
-        sealed_tiles += sealed;
-        return sealed;
+        kivi_resident_bytes += pages * (8ull * lay.word_count + 8ull * lay.block_count + 8ull * (1u << kivi_bits) + 4ull * (D + tokens));
+        if (tokens < opt.page_size) h.flushed_partial = true;
+        h.sealed += pages * tokens;
+        sealed_tiles += pages;
     }
     void kivi_flush(uint32_t layer, uint32_t kv_head, cudaStream_t s) {
         HeadState &h = head(layer, kv_head);
         if (h.tail == 0) return;
-        if (kivi_seal(layer, kv_head, 1, h.tail, 0, s) == 0) throw std::invalid_argument("invalid quantization input");
+        if (h.bad_row < h.tail) throw std::invalid_argument("invalid quantization input");   // kv_gpu_fixture.cpp:13
+        kivi_join(s);
+        kivi_seal(layer, kv_head, 1, h.tail, 0, s);
+        kivi_mark(s);
         h.tail = 0;
     }
     // `take` host rows into the tail ([token][kv head][dim]: the layout the attention reads).
     void kivi_rows_to_tail(uint32_t layer, uint32_t kv_head, const float *keys, const float *values, uint32_t take, cudaStream_t s) {
         if (take == 0) return;
         HeadState &h = head(layer, kv_head);
+        if (h.bad_row >= h.tail) {
+            const uint32_t bad = std::min(first_bad_row(keys, take, opt.head_dim), first_bad_row(values, take, opt.head_dim));
+            h.bad_row = bad < take ? h.tail + bad : 0xffffffffu;
+        }
         const size_t row = kivi_row_floats(), D = opt.head_dim, at = static_cast<size_t>(h.tail) * row + static_cast<size_t>(kv_head) * D;
         cuda_check(cudaMemcpy2DAsync(kivi_tail(kivi_tail_k, layer) + at, row * 4, keys, D * 4, D * 4, take, cudaMemcpyHostToDevice, s), "append keys");
         cuda_check(cudaMemcpy2DAsync(kivi_tail(kivi_tail_v, layer) + at, row * 4, values, D * 4, D * 4, take, cudaMemcpyHostToDevice, s), "append values");
@@ -415,6 +456,7 @@ struct cf_llama_kv_adapter {
         HeadState &h = head(layer, kv_head);
         const uint32_t T = tile_tokens, D = opt.head_dim;
         uint32_t done = 0;
+        kivi_join(s);
         while (done < token_count) {
             const uint32_t left = token_count - done;
             if (h.tail + left < T) {
@@ -428,27 +470,37 @@ struct cf_llama_kv_adapter {
             const size_t floats = static_cast<size_t>(rows) * D;
             if (floats > kivi_stage_floats) {
                 const size_t wanted = std::max(floats, kivi_stage_floats * 2);
-                if (kivi_pinned) cudaFreeHost(kivi_pinned);   // every launch that read it has been waited for
+                for (cudaEvent_t e : kivi_done) cuda_check(cudaEventSynchronize(e), "wait for earlier appends");
+                if (kivi_pinned) cudaFreeHost(kivi_pinned);
                 kivi_pinned = nullptr;
                 kivi_stage_floats = 0;
-                cuda_check(cudaHostAlloc(reinterpret_cast<void **>(&kivi_pinned), 2 * wanted * sizeof(float), cudaHostAllocDefault), "cudaHostAlloc");
+                cuda_check(cudaHostAlloc(reinterpret_cast<void **>(&kivi_pinned), 4 * wanted * sizeof(float), cudaHostAllocDefault), "cudaHostAlloc");
                 kivi_stage.ensure(2 * wanted, s);
                 kivi_stage_floats = wanted;
             }
+            cuda_check(cudaEventSynchronize(kivi_done[kivi_turn]), "wait for an earlier append");   // its half of the pinned memory
             const float *source[2] = {keys + static_cast<size_t>(done) * D, values + static_cast<size_t>(done) * D};
+            uint32_t bad = rows;   // first staged row with NaN or Inf
             for (int stream = 0; stream < 2; ++stream) {   // the copy of K crosses the bus while V is gathered
-                std::memcpy(kivi_pinned + stream * kivi_stage_floats, source[stream], floats * sizeof(float));
-                cuda_check(cudaMemcpyAsync(kivi_stage.ptr + stream * kivi_stage_floats, kivi_pinned + stream * kivi_stage_floats, floats * sizeof(float),
-                                           cudaMemcpyHostToDevice, s), "stage rows");
+                float *half = kivi_pinned + (2u * kivi_turn + stream) * kivi_stage_floats;
+                bad = std::min(bad, copy_rows_checked(half, source[stream], rows, D));
+                cuda_check(cudaMemcpyAsync(kivi_stage.ptr + stream * kivi_stage_floats, half, floats * sizeof(float), cudaMemcpyHostToDevice, s), "stage rows");
             }
-            const uint32_t sealed = kivi_seal(layer, kv_head, pages, T, rest, s);
+            const uint32_t sealed = h.bad_row < h.tail ? 0u : std::min(pages, (h.tail + bad) / T);
+            if (sealed) kivi_seal(layer, kv_head, sealed, T, sealed == pages ? rest : 0u, s);
+            kivi_mark(s);
             if (sealed < pages) {   // pages before the refused one stay; its rows become the (full) tail, as if appended page by page
                 const uint32_t skip = sealed ? sealed * T - h.tail : 0u, keep = sealed ? 0u : h.tail;
-                if (sealed) h.next_token += skip;
+                if (sealed) {
+                    h.next_token += skip;
+                    h.bad_row = 0xffffffffu;
+                }
                 h.tail = keep;
                 kivi_rows_to_tail(layer, kv_head, source[0] + static_cast<size_t>(skip) * D, source[1] + static_cast<size_t>(skip) * D, T - keep, s);
+                cuda_check(cudaStreamSynchronize(s), "cudaStreamSynchronize");
                 throw std::invalid_argument("invalid quantization input");
             }
+            h.bad_row = bad < rows ? h.tail + bad - pages * T : 0xffffffffu;   // in the rest
             h.tail = rest;
             h.next_token += rows;
             done += rows;
@@ -744,6 +796,7 @@ extern "C" int cf_llama_kv_attention(cf_llama_kv_adapter *adapter, uint32_t laye
             if (h.sealed != h0.sealed || h.tail != h0.tail) throw std::runtime_error("KV active tails are not aligned across heads");
         }
         if (adapter->kivi) {   // the reference's own call over the reference's own page descriptors (its adapter, :107-131)
+            adapter->kivi_join(s);
             cf_kv_paged_attention_desc desc{};
             desc.struct_size = sizeof desc;
             desc.abi_version = CF_KV_CUDA_ABI_VERSION;
@@ -940,6 +993,7 @@ extern "C" int cf_b200_llama_kv_reference_page(const cf_llama_kv_adapter *adapte
     if (adapter == nullptr || out_page == nullptr || !adapter->kivi || layer >= adapter->kivi_host_descs.size() ||
         page_index >= adapter->kivi_host_descs[layer].size())
         return -1;
+    for (cudaEvent_t e : adapter->kivi_done) cudaEventSynchronize(e);   // the caller reads the page by ways of its own
     *out_page = adapter->kivi_host_descs[layer][page_index];
     return 0;
 }

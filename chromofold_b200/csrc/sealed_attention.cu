@@ -985,7 +985,7 @@ cudaError_t launch_combine_as(const AttentionParams &p, cudaStream_t stream, boo
 
 }  // namespace
 
-// Four rows per CTA where that still makes about a CTA per SM, else one; 32 where all entries are query tokens of one sequence
+// Four rows per CTA where that still makes about a CTA per SM, or where a CTA per row would not find room for all at once, else one; 32 where all entries are query tokens of one sequence
 // (the caller says so), their tail is worth sharing and its rows can be read 16 bytes at a time.
 cudaError_t launch_combine(const AttentionParams &p, cudaStream_t stream, bool dependent) {
     constexpr uint32_t kEnoughCtas = 120;
@@ -1000,7 +1000,7 @@ cudaError_t launch_combine(const AttentionParams &p, cudaStream_t stream, bool d
         return launch_kernel(combine_tile_kernel, dim3(tiles / p.kv_head_span, p.kv_head_span), kTileThreads, combine_tile_smem(C), stream, dependent, p);
     }
     const uint32_t fours = p.seq_count * p.kv_head_span * ((G + 3u) / 4u);
-    if (fours >= kEnoughCtas && CombineSmem<4, 512>::bytes(C) <= kCombineSmemMax / 2u)
+    if ((fours >= kEnoughCtas || p.seq_count * p.kv_head_span * G > 2u * 148u) && CombineSmem<4, 512>::bytes(C) <= kCombineSmemMax / 2u)
         return fours <= 2u * 148u ? launch_combine_as<4, 512>(p, stream, dependent) : launch_combine_as<4, 128>(p, stream, dependent);
     return launch_combine_as<1, 1024>(p, stream, dependent);
 }
