@@ -98,12 +98,12 @@ typedef struct cf_b200_sealed_attention_desc {
 
     void *workspace;                     /* split-KV partials; see cf_b200_sealed_attention_workspace_bytes */
     uint64_t workspace_bytes;
-    uint32_t min_pages_per_unit;         /* pages per split-KV unit; 0 = the library chooses (4 to 35) on the device, from the
-                                            pages the launch will read: the size whose rounds over the GPU's resident
-                                            warps cost least, among those whose partials fit the workspace. A unit's
-                                            weighted sum is kept by the tensor cores in fp32; its rounding drifts by
-                                            about 1e-7 of the output's scale per page, so units of hundreds of pages
-                                            are a few 1e-5 off where the library's own sizes stay below 4e-6 */
+    uint32_t min_pages_per_unit;         /* pages per split-KV unit; 0 = the library cuts the pages the launch will read
+                                            evenly over the GPU's resident warps, on the device, with a partial result
+                                            per 32 pages (more where the workspace has no room for that many). A
+                                            partial's weighted sum is kept by the tensor cores in fp32; its rounding
+                                            drifts by about 1e-7 of the output's scale per page, so units of hundreds of
+                                            pages are a few 1e-5 off where the library's own stay below 4e-6 */
     uint32_t kernel;                     /* CF_B200_KERNEL_* */
     uint32_t *status;                    /* optional device word; a kernel ORs CF_B200_DEVSTAT_* into it */
     uint32_t tail_type;                  /* CF_B200_F16 (0 means F16 too) or CF_B200_F32: element type of the tails */
@@ -167,15 +167,15 @@ cf_status cf_b200_test_wait_expiry(uint32_t skip_copy_page_id, uint32_t wait_pol
 cf_status cf_b200_sealed_attention_validate(const cf_b200_sealed_attention_desc *desc);
 
 /* Workspace needed so that a batch with at most total_pages sealed pages (summed over sequences) never
- * has to grow its units beyond min_pages_per_unit (or, with 0, beyond 16 pages, 4 for small batches). A smaller
- * workspace is legal: units grow to fit. */
+ * has to grow its units beyond min_pages_per_unit (with 0: has a warp without a page while there are pages, or a partial
+ * over more than 32 pages). A smaller workspace is legal: units grow to fit. */
 cf_status cf_b200_sealed_attention_workspace_bytes(const cf_b200_sealed_attention_desc *desc,
                                                    uint64_t total_pages, uint64_t *out_bytes);
 
 cf_status cf_b200_sealed_attention_async(const cf_b200_sealed_attention_desc *desc, void *stream);
 
 /* The same launch cut into its three kernels, so that a profiler or a benchmark can put events between them:
- * plan (chunk layout, one block), attention (the kernel that reads the pages), combine (merge + tail + output).
+ * plan (the cut of the pages, one block), attention (the kernel that reads the pages), combine (merge + tail + output).
  * `stages` is a mask; running all three in order equals cf_b200_sealed_attention_async. */
 #define CF_B200_STAGE_PLAN 1u
 #define CF_B200_STAGE_ATTENTION 2u
@@ -189,9 +189,9 @@ cf_status cf_b200_sealed_attention_stages_async(const cf_b200_sealed_attention_d
  * cf_b200_sealed_attention_async, ignores `workspace` / `workspace_bytes`, and uses a fixed array inside the
  * library image instead: CF_B200_STATIC_WORKSPACE_BYTES per GPU that loads the library, held until exit.
  *   - It calls no cudaMalloc, cudaFree or allocating library routine.
- *   - A batch whose partials cannot fit (seq_count x local query heads x (head_dim + 2) floats, one chunk per
+ *   - A batch whose partials cannot fit (seq_count x local query heads x (head_dim + 2) floats, one per
  *     sequence at least) is rejected with CF_ERR_UNSUPPORTED; cf_b200_sealed_attention_static_error() says why and
- *     how many bytes were needed. Larger contexts are fine: chunks grow to fit the array. A shared_prefix_pages hint
+ *     how many bytes were needed. Larger contexts are fine: units grow to fit the array. A shared_prefix_pages hint
  *     needs CF_B200_SHARED_CHUNKS_MAX more partials per sequence and query head; when only those do not fit, the
  *     call is served without the hint (every page then handled per sequence) instead of refused.
  *   - The first call on a device looks up the array's device address; make that call outside any stream capture.
