@@ -291,7 +291,7 @@ struct cf_llama_kv_adapter {
     uint32_t kivi_turn = 0;                  // pinned half of the next append
     cudaStream_t kivi_stream = nullptr;      // of the last append, and
     bool kivi_pending = false;               // whether it may still be under way
-    static constexpr size_t kKiviStageBytes = 4u << 20;   // rows staged at a time (at least one page)
+    static constexpr size_t kKiviStageBytes = 1u << 20;   // of one stream, staged at a time (at least one page): the next turn copies meanwhile
 
     ~cf_llama_kv_adapter() {
         for (uint8_t *c : kivi_chunks) cudaFree(c);
