@@ -578,12 +578,21 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads > 8 ? 8 : 1024 / kTh
         }
         for (uint32_t c0 = begin, n; c0 < end; c0 += n) {
             n = min(whole ? whole : min(32u, left), end - c0);
-            float pm = -CUDART_INF_F, pl = 0.0f;
+            float pm = -CUDART_INF_F, pl = 0.0f, x[8][4];
             if (lane < n) {
                 const float *src = partial_of(p, rp, c0 + lane, seq, lq);
                 pm = __ldcg(src);
                 pl = __ldcg(src + 1);
             }
+            auto load_batch = [&](uint32_t i0) {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const float *src = partial_of(p, rp, c0 + min(i0 + i, n - 1u), seq, lq) + 2;
+#pragma unroll
+                    for (uint32_t c = 0; c < 4; ++c) x[i][c] = i0 + i < n && lane + 32u * c < D ? __ldcg(src + lane + 32u * c) : 0.0f;
+                }
+            };
+            load_batch(0u);   // on its way before its weights are known
             if (whole) {   // every strand's own maximum
                 mj = pm;
                 const uint32_t first = lane / strand * strand;
@@ -595,13 +604,7 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads > 8 ? 8 : 1024 / kTh
             }
             const float w = pm == -CUDART_INF_F ? 0.0f : exp2f(pm - mj);
             for (uint32_t i0 = 0; i0 < n; i0 += 8u) {
-                float x[8][4];
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const float *src = partial_of(p, rp, c0 + min(i0 + i, n - 1u), seq, lq) + 2;
-#pragma unroll
-                    for (uint32_t c = 0; c < 4; ++c) x[i][c] = i0 + i < n && lane + 32u * c < D ? __ldcg(src + lane + 32u * c) : 0.0f;
-                }
+                if (i0) load_batch(i0);
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
                     if (i0 + i >= n) break;
