@@ -95,7 +95,17 @@ __device__ __forceinline__ void score_quad(UnitState<NG, kDim> &u, const QSrc &q
 
 // kFold: the symbols are only folded into a checksum (u.vq[0]) — the decode work of the kernel without its attention.
 // kDump: lane l's quad q of a stream holds the symbols 64 l + 4 q .. + 3 of that stream, first symbol in byte 0.
-template <int kMode = kAttend, class KLane, class VLane, int NG, class QSrc>
+// kRolled: the page in four passes of four quads, a quarter of the code, so that more of it stays in the instruction cache; the V
+// quads shift down, so that quad q ends in element q. Taken by the eight-head kernel of binary16 queries, whose 16 warps hide
+// less of the fetches: 64 sequences of rANS pages 1403 -> 1335 us, of Huffman pages 1098 -> 1022. Half as many steps, as
+// nibble-split pages have, gain nothing by it, and neither the 24 warps of the four-head kernels nor eight heads of split
+// queries have registers to spare for it (821 -> 901, 1102 -> 1202 us).
+template <int kEach>
+__device__ __forceinline__ void shift_quads(uint32_t (&vq)[16]) {
+#pragma unroll
+    for (int i = 0; i < 16 - kEach; ++i) vq[i] = vq[i + kEach];
+}
+template <int kMode = kAttend, bool kRolled = false, class KLane, class VLane, int NG, class QSrc>
 __device__ __forceinline__ void decode_fused(KLane &k, VLane &v, UnitState<NG> &u, const QSrc &qs) {
     if constexpr (KLane::kWholeQuads || VLane::kWholeQuads) {
 #pragma unroll
@@ -113,24 +123,30 @@ __device__ __forceinline__ void decode_fused(KLane &k, VLane &v, UnitState<NG> &
         }
     } else {
         // two independent decoder chains, interleaved symbol by symbol; four symbols make one packed register
-        uint32_t ke[4], ve[4];
+        constexpr int kPasses = kRolled ? 4 : 1, kEach = 16 / kPasses;   // quads of a pass
+#pragma unroll 1
+        for (int pass = 0; pass < kPasses; ++pass) {
+            if constexpr (kRolled) shift_quads<kEach>(u.vq);
+            uint32_t ke[4], ve[4];
 #pragma unroll
-        for (int i = 0; i < 64; ++i) {
-            ke[i & 3] = k.symbol(i & 1);
-            ve[i & 3] = v.symbol(i & 1);
-            if (i & 1) {
-                k.advance();
-                v.advance();
-            }
-            if ((i & 3) == 3) {
-                if constexpr (kMode == kFold) {
-                    u.vq[0] ^= pack_low_bytes(ve[0], ve[1], ve[2], ve[3]) ^ pack_low_bytes(ke[0], ke[1], ke[2], ke[3]);
-                } else if constexpr (kMode == kDump) {
-                    u.dump[i >> 2] = pack_low_bytes(ke[0], ke[1], ke[2], ke[3]);
-                    u.dump[512 + (i >> 2)] = pack_low_bytes(ve[0], ve[1], ve[2], ve[3]);
-                } else {
-                    u.vq[i >> 2] = pack_low_bytes(ve[0], ve[1], ve[2], ve[3]);
-                    score_quad(u, qs, i >> 2, pack_low_bytes(ke[0], ke[1], ke[2], ke[3]));
+            for (int i = 0; i < 4 * kEach; ++i) {
+                ke[i & 3] = k.symbol(i & 1);
+                ve[i & 3] = v.symbol(i & 1);
+                if (i & 1) {
+                    k.advance();
+                    v.advance();
+                }
+                if ((i & 3) == 3) {
+                    const int q = kEach * pass + (i >> 2);
+                    if constexpr (kMode == kFold) {
+                        u.vq[0] ^= pack_low_bytes(ve[0], ve[1], ve[2], ve[3]) ^ pack_low_bytes(ke[0], ke[1], ke[2], ke[3]);
+                    } else if constexpr (kMode == kDump) {
+                        u.dump[q] = pack_low_bytes(ke[0], ke[1], ke[2], ke[3]);
+                        u.dump[512 + q] = pack_low_bytes(ve[0], ve[1], ve[2], ve[3]);
+                    } else {
+                        u.vq[16 - kEach + (i >> 2)] = pack_low_bytes(ve[0], ve[1], ve[2], ve[3]);
+                        score_quad(u, qs, q, pack_low_bytes(ke[0], ke[1], ke[2], ke[3]));
+                    }
                 }
             }
         }
@@ -289,6 +305,7 @@ __global__ void __launch_bounds__(kThreadsOf<NG, NB, kSplitQ, kDim>, 1) lanes_at
     using L = WarpLayout<NG, NB, kSplitQ, kDim>;
     constexpr int NS = kHeadGroups<NG, kSplitQ>;
     constexpr uint32_t kPassHeads = 4u * NS;
+    constexpr bool kRolled = NS == 2 && !kSplitQ && kMode == kAttend;
     extern __shared__ __align__(128) uint8_t smem[];
     uint32_t *k_slot = reinterpret_cast<uint32_t *>(smem);
     uint32_t *v_slot = k_slot + 4096;
@@ -568,17 +585,17 @@ __global__ void __launch_bounds__(kThreadsOf<NG, NB, kSplitQ, kDim>, 1) lanes_at
                         RansLane k, v;
                         k.open(k_part, k_bytes, lane, k_slot);
                         v.open(v_part, v_bytes, lane, v_slot);
-                        decode_fused<kMode>(k, v, u, qs);
+                        decode_fused<kMode, kRolled>(k, v, u, qs);
                     } else if (k_coder == CF_B200_CODER_HUFFMAN && v_coder == CF_B200_CODER_HUFFMAN) {
                         HuffLane k, v;
                         k.open(k_part, k_bytes, lane, k_lut);
                         v.open(v_part, v_bytes, lane, v_lut);
-                        decode_fused<kMode>(k, v, u, qs);
+                        decode_fused<kMode, kRolled>(k, v, u, qs);
                     } else if (k_coder == CF_B200_CODER_FIXED8 && v_coder == CF_B200_CODER_FIXED8) {
                         FixedLane k, v;
                         k.open(k_part, k_bytes, lane);
                         v.open(v_part, v_bytes, lane);
-                        decode_fused<kMode>(k, v, u, qs);
+                        decode_fused<kMode, kRolled>(k, v, u, qs);
                     } else {  // mixed coders (one stream fell back to fixed width): one stream after the other
                         if (k_coder == CF_B200_CODER_RANS) { RansLane k; k.open(k_part, k_bytes, lane, k_slot); decode_k_only<kMode>(k, u, qs); }
                         else if (k_coder == CF_B200_CODER_HUFFMAN) { HuffLane k; k.open(k_part, k_bytes, lane, k_lut); decode_k_only<kMode>(k, u, qs); }
