@@ -98,6 +98,17 @@ __host__ __device__ inline uint32_t shared_tile_groups(uint32_t rows) {
     return (rows + per_group - 1u) / per_group;
 }
 
+// The barrier on which a pair's CTA of the shared-prefix kernel is told that the weights of round r are stored, and the parity of
+// that arrival. The issuing thread sends the scores of round r + 1 before the output of round r, so the softmax warps can have
+// arrived for both before it looks: on one barrier the second arrival hides the first (the phase is back at the parity it waits
+// for). With two by turns they get no further: the weights of round r + 2 need its scores, which go out after the output of
+// round r, and that once the weights of round r were seen.
+constexpr uint32_t kWeightBarriers = 2;
+struct RoundBarrier {
+    uint32_t index, parity;
+};
+__host__ __device__ inline RoundBarrier weights_barrier(uint32_t round) { return {round % kWeightBarriers, round / kWeightBarriers & 1u}; }
+
 // What is known of a batch entry, written by the plan kernel so that later kernels read two 16-byte words instead of chasing
 // slot -> counts -> position.
 struct SeqInfo {

@@ -66,8 +66,8 @@ constexpr uint32_t kOffStages = kTableBytes;
 constexpr uint32_t kOffTiles = (kOffStages + kDecodeWarps * kRecordBytes + 127u) / 128u * 128u;   // K[0] V[0] K[1] V[1]
 constexpr uint32_t kOffMeta = kOffTiles + 4 * kTileBytes;      // [pair][page of the round]: k scale, v scale, token count, -
 constexpr uint32_t kOffRound = kOffMeta + 2 * kRoundPages * 16;    // [pair]: unit, flags, -, -
-constexpr uint32_t kOffBars = kOffRound + 2 * 16;              // 12 copy barriers, full[2], free[4], S[2], O[2], P, Q
-constexpr uint32_t kBarFull = kDecodeWarps, kBarFree = kBarFull + 2, kBarS = kBarFree + 4, kBarO = kBarS + 2, kBarP = kBarO + 2, kBarQ = kBarP + 1,
+constexpr uint32_t kOffBars = kOffRound + 2 * 16;              // 12 copy barriers, full[2], free[4], S[2], O[2], P[2], Q
+constexpr uint32_t kBarFull = kDecodeWarps, kBarFree = kBarFull + 2, kBarS = kBarFree + 4, kBarO = kBarS + 2, kBarP = kBarO + 2, kBarQ = kBarP + kWeightBarriers,
                    kBarCount = kBarQ + 1;
 constexpr uint32_t kOffMisc = kOffBars + kBarCount * 8;        // [0] tmem base
 constexpr uint32_t kOffRowMax = kOffMisc + 32;                 // [round parity][2 column halves][128 rows]
@@ -654,7 +654,7 @@ __device__ __forceinline__ void issuer_role(const AttentionParams &p, uint8_t *s
             fresh = first ? fresh | 1u << pair : fresh & ~(1u << pair);
             if (first) ok = mbar_wait(bars + kBarQ, units++ & 1u, p.wait_polls);   // the unit's queries are in tensor memory
             if (ok) issue_scores<kDim, kSplitQ, kCluster>(smem, tmem, bars, s_round++);
-        } else if (o_round < s_round && mbar_test_pair(bars + kBarP, o_round & 1u)) {
+        } else if (o_round < s_round && mbar_test_pair(bars + kBarP + weights_barrier(o_round).index, weights_barrier(o_round).parity)) {
             polls = 0;
             issue_output<kDim, kCluster>(smem, tmem, bars, o_round, (fresh >> (o_round & 1u) & 1u) != 0u);
             ++o_round;
@@ -902,7 +902,7 @@ __device__ __forceinline__ void softmax_role(const AttentionParams &p, uint8_t *
         tc_fence_before();
         if constexpr (kIssuerWarp) {
             __syncwarp();
-            if (lane == 0) mbar_arrive(bars + kBarP);
+            if (lane == 0) mbar_arrive(bars + kBarP + weights_barrier(it).index);
         } else {
             if (group_any<kSoftmaxWarps * 32>(1u, failed)) break;
             if (issuer) {
@@ -978,8 +978,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) prefix_attention_kernel(Attenti
         mbar_init(bars + kBarFull + 1, kRoundPages);
         for (uint32_t i = 0; i < 4u; ++i) mbar_init(bars + kBarFree + i, kCluster);   // tensor-core commits, of both CTAs
         for (uint32_t i = kBarS; i < kBarP; ++i) mbar_init(bars + i, 1);          // tensor-core commits
-        mbar_init(bars + kBarP, kSoftmaxWarps);   // weights stored, queries stored (where a warp of its own issues)
-        mbar_init(bars + kBarQ, kSoftmaxWarps);
+        for (uint32_t i = kBarP; i < kBarCount; ++i) mbar_init(bars + i, kSoftmaxWarps);   // weights stored, queries stored (where a warp of its own issues)
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncwarp();
