@@ -6,13 +6,13 @@
 // V per-token fp32 scales), so this path keeps their cost; it is split over the pages of a kv head to fill the GPU
 // and runs faster than the reference's kernels on the same descriptors, but the sealed-KV entry points are the fast path.
 
-#include <mutex>
 #include <algorithm>
 #include <math_constants.h>
 
 #include "cf_device_common.cuh"
 #include "chromofold_b200/compat_kv.h"
 #include "compat_paged_mma.cuh"
+#include "slot_ring.h"
 
 namespace cfb {
 // Implemented in flat_rans_decode.cu
@@ -88,7 +88,7 @@ __host__ __device__ inline Smem smem_layout(uint32_t group, uint32_t head_dim, u
 constexpr uint32_t kCompatSlots = 4;
 constexpr uint32_t kCompatSlotFloats = 512u * 1024u;   // 2 MiB per slot
 constexpr uint32_t kCompatMaxSplits = 64;
-__device__ float g_compat_partials[kCompatSlots * kCompatSlotFloats];
+__device__ __align__(256) float g_compat_partials[kCompatSlots * kCompatSlotFloats];   // read four floats at a time
 __device__ uint32_t g_compat_arrived[kCompatSlots * kPagedMmaCounters];   // zero between calls
 
 __global__ void __launch_bounds__(kThreads) compat_paged_attention_kernel(cf_kv_paged_attention_desc desc,
@@ -493,12 +493,11 @@ extern "C" cf_status cf_kv_validate_paged_attention_desc(const cf_kv_paged_atten
 namespace {
 // Slots of the partials array, per device: whose turn it is and when the slot's last user is done.
 struct CompatSlots {
-    std::mutex lock;
+    cfb::SlotRing<cfb::kCompatSlots> ring;
     bool made = false;
     cudaEvent_t done[cfb::kCompatSlots] = {};
     float *base = nullptr;
     uint32_t *arrived = nullptr;
-    uint32_t next = 0;
     int sm_count = 0;
 };
 CompatSlots g_compat_slots[64];
@@ -514,49 +513,51 @@ extern "C" cf_status cf_kv_paged_attention_async(const cf_kv_paged_attention_des
     const bool mma = cfb::paged_mma_supports(*d);
     int device = 0;
     if (cudaGetDevice(&device) != cudaSuccess) return CF_ERR_CUDA;
-    uint32_t splits = 1, slot = 0;
+    uint32_t splits = 1;
     CompatSlots *slots = device >= 0 && device < 64 ? &g_compat_slots[device] : nullptr;
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &capture) != cudaSuccess) return CF_ERR_CUDA;
     if (capture != cudaStreamCaptureStatusNone) slots = nullptr;   // a captured call keeps to one launch and no events
     if (slots) {
-        std::lock_guard<std::mutex> guard(slots->lock);
-        if (!slots->made) {   // first call on this device: events, the arrays' addresses, the SM count
+        const bool ready = slots->ring.locked([&] {
+            if (slots->made) return true;   // else the first call on this device: events, the arrays' addresses, the SM count
             for (cudaEvent_t &e : slots->done)
-                if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) return CF_ERR_CUDA;
+                if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) return false;
             if (cudaGetSymbolAddress(reinterpret_cast<void **>(&slots->base), cfb::g_compat_partials) != cudaSuccess ||
                 cudaGetSymbolAddress(reinterpret_cast<void **>(&slots->arrived), cfb::g_compat_arrived) != cudaSuccess ||
                 cudaDeviceGetAttribute(&slots->sm_count, cudaDevAttrMultiProcessorCount, device) != cudaSuccess)
-                return CF_ERR_CUDA;
+                return false;
             slots->made = true;
-        }
+            return true;
+        });
+        if (!ready) return CF_ERR_CUDA;
         const uint64_t pairs = static_cast<uint64_t>(d->query_count) * d->kv_head_count;
         const uint64_t room = cfb::kCompatSlotFloats / (static_cast<uint64_t>(d->query_count) * d->query_head_count * (d->head_dim + 2u));
         const uint64_t wanted = mma ? cfb::paged_mma_splits(*d, slots->sm_count) : (2ull * slots->sm_count + pairs - 1) / pairs;
         splits = static_cast<uint32_t>(std::max<uint64_t>(1, std::min({wanted, room, static_cast<uint64_t>(cfb::kCompatMaxSplits)})));
-        if (splits > 1) {
-            slot = slots->next++ % cfb::kCompatSlots;
-            if (cudaStreamWaitEvent(s, slots->done[slot], 0) != cudaSuccess) return CF_ERR_CUDA;   // the slot's last user
-        }
     }
-    float *partials = splits > 1 ? slots->base + static_cast<size_t>(slot) * cfb::kCompatSlotFloats : nullptr;
-    if (mma) {   // head_dim 128 and 64; the splits are merged by the kernel itself
-        uint32_t *arrived = splits > 1 ? slots->arrived + slot * cfb::kPagedMmaCounters : nullptr;
-        if (cfb::launch_paged_mma(*d, splits, partials, arrived, s) != cudaSuccess) return CF_ERR_CUDA;
-    } else {
+    auto launch = [&](float *partials, uint32_t *arrived) {
+        if (mma)   // head_dim 128 and 64; the splits are merged by the kernel itself
+            return cfb::launch_paged_mma(*d, splits, partials, arrived, s);
         const uint32_t batch_tokens = cfb::kBatchSymbols / d->head_dim;
         const cfb::Smem lay = cfb::smem_layout(d->gqa_group_size, d->head_dim, batch_tokens);
-        if (cudaFuncSetAttribute(cfb::compat_paged_attention_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(lay.total)) != cudaSuccess)
-            return CF_ERR_CUDA;
+        const cudaError_t e = cudaFuncSetAttribute(cfb::compat_paged_attention_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   static_cast<int>(lay.total));
+        if (e != cudaSuccess) return e;
         cfb::compat_paged_attention_kernel<<<dim3(d->query_count, d->kv_head_count, splits), cfb::kThreads, lay.total, s>>>(
             *d, batch_tokens, splits, partials);
         if (splits > 1)
             cfb::compat_combine_kernel<<<dim3(d->query_count, d->query_head_count), 128, 0, s>>>(d->output, partials, d->query_head_count,
                                                                                               d->head_dim, splits);
-    }
-    if (splits > 1 && cudaEventRecord(slots->done[slot], s) != cudaSuccess) return CF_ERR_CUDA;
-    return cudaPeekAtLastError() == cudaSuccess ? CF_OK : CF_ERR_CUDA;
+        return cudaPeekAtLastError();
+    };
+    if (splits == 1) return launch(nullptr, nullptr) == cudaSuccess ? CF_OK : CF_ERR_CUDA;
+    return slots->ring.take([&](uint32_t slot) {
+        const bool ok = cudaStreamWaitEvent(s, slots->done[slot], 0) == cudaSuccess &&   // the slot's last user
+                        launch(slots->base + static_cast<size_t>(slot) * cfb::kCompatSlotFloats, slots->arrived + slot * cfb::kPagedMmaCounters) == cudaSuccess &&
+                        cudaEventRecord(slots->done[slot], s) == cudaSuccess;
+        return ok ? CF_OK : CF_ERR_CUDA;
+    });
 }
 
 extern "C" cf_status cf_rans_decode_async(const uint8_t *data, const int32_t *byte_off, const uint32_t *state0,

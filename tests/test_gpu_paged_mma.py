@@ -107,6 +107,65 @@ def test_paged_attention_on_the_tensor_cores(native, oracle, case):
     assert np.abs(got - want).max() <= 1e-5 * np.abs(want).max(), np.abs(got - want).max() / np.abs(want).max()
 
 
+def test_paged_attention_from_several_threads(native):
+    """Callers on streams of their own share the slots in which splits leave their partials: every call, whatever its number of
+    splits, gives what it gives alone."""
+    import threading
+    import torch
+    lib, d, hq, hkv, page, threads, calls = native.lib(), 128, 8, 2, 32, 12, 250
+    rng = np.random.default_rng(11)
+    dev = lambda a: torch.from_numpy(np.array(a, copy=True)).cuda()
+    most = 40
+    held = [dev(rng.integers(0, 1 << 32, page * d // 8, dtype=np.uint32).view(np.int32)) for _ in range(2 * hkv * most)]
+    scales = dev(rng.uniform(0.005, 0.02, max(d, page)).astype(np.float32))
+    spare = dev(np.zeros(page * d // 64, np.int32))
+    jobs = []
+    for i in range(threads):
+        pages = (DevicePage * ((3 + 3 * i) * hkv))()
+        for n, pg in enumerate(pages):
+            pg.k_words, pg.v_words = held[2 * (n % (hkv * most))].data_ptr(), held[2 * (n % (hkv * most)) + 1].data_ptr()
+            pg.k_block_offsets = pg.v_block_offsets = pg.k_lut = pg.v_lut = spare.data_ptr()
+            pg.k_scales = pg.v_scales = scales.data_ptr()
+            pg.token_begin, pg.token_count, pg.head_dim, pg.block_size = n // hkv * page, page, d, 64
+            pg.k_max_code_length = pg.v_max_code_length = pg.fixed_code_length = 4
+            pg.zero_point, pg.kv_head = 8, n % hkv
+        table = dev(np.frombuffer(bytes(pages), np.uint8))
+        q = dev(rng.standard_normal((1 + i % 3, hq, d)).astype(np.float32))
+        out = torch.zeros((calls, *q.shape), device="cuda")
+        desc = PagedAttentionDesc()
+        desc.struct_size, desc.abi_version = C.sizeof(desc), 0
+        desc.pages, desc.page_count = table.data_ptr(), len(pages)
+        desc.kv_head_count, desc.query_head_count, desc.gqa_group_size = hkv, hq, hq // hkv
+        desc.queries, desc.query_token_begin, desc.query_count = q.data_ptr(), page * len(pages) // hkv, q.shape[0]
+        desc.head_dim, desc.softmax_scale = d, d ** -0.5
+        jobs.append((desc, out, torch.cuda.Stream(), table, q))
+    alone = []
+    for desc, out, *_ in jobs:
+        desc.output = out[0].data_ptr()
+        assert lib.cf_kv_paged_attention_async(C.byref(desc), None) == 0
+        torch.cuda.synchronize()
+        alone.append(out[0].clone())
+        out.zero_()
+    torch.cuda.synchronize()
+    failed = []
+
+    def work(desc, out, stream):
+        for n in range(calls):
+            desc.output = out.data_ptr() + n * out[0].numel() * 4
+            if lib.cf_kv_paged_attention_async(C.byref(desc), C.c_void_p(stream.cuda_stream)) != 0:
+                failed.append(n)
+
+    runners = [threading.Thread(target=work, args=job[:3]) for job in jobs]
+    for t in runners:
+        t.start()
+    for t in runners:
+        t.join()
+    torch.cuda.synchronize()
+    assert not failed
+    for want, (_, out, *_) in zip(alone, jobs):   # the same splits, merged in the same order
+        assert torch.equal(out, want.expand_as(out))
+
+
 # ---- the adapter's page quantiser (csrc/adapter.cu): several pages per launch --------------------------------------------
 def _quantised(x, axis, bits):
     """The reference fixture's rule (src/runtime/kv_gpu_fixture.cpp:12-16, 46-95) in fp32: one scale along `axis`."""
