@@ -279,6 +279,7 @@ struct cf_llama_kv_adapter {
     static constexpr size_t kKiviChunk = 32u << 20;
     std::vector<uint8_t *> kivi_chunks;      // page blocks never move: descriptors hold their addresses
     size_t kivi_chunk_index = 0, kivi_chunk_used = 0;
+    uint32_t kivi_chunk_limit = 0xffffffffu; // test hook: no further chunk is to be had
     DeviceBuffer<float> kivi_tail_k, kivi_tail_v;   // [layer][page_size][kv_head][head_dim]: the layout the attention reads
     DeviceBuffer<int32_t> kivi_lut;
     std::vector<std::unique_ptr<DeviceBuffer<cf_kv_device_page>>> kivi_descs;   // per layer, device
@@ -314,7 +315,7 @@ struct cf_llama_kv_adapter {
         }
         if (kivi_chunk_index >= kivi_chunks.size()) {
             uint8_t *fresh = nullptr;
-            cuda_check(cudaMalloc(reinterpret_cast<void **>(&fresh), kKiviChunk), "cudaMalloc");
+            cuda_check(kivi_chunks.size() < kivi_chunk_limit ? cudaMalloc(reinterpret_cast<void **>(&fresh), kKiviChunk) : cudaErrorMemoryAllocation, "cudaMalloc");
             kivi_chunks.push_back(fresh);
             kivi_chunk_used = 0;
         }
@@ -367,11 +368,13 @@ struct cf_llama_kv_adapter {
         if (cudaEventQuery(last) == cudaSuccess) kivi_pending = false;
         else cuda_check(cudaStreamWaitEvent(s, last, 0), "wait for the last append");
     }
-    void kivi_mark(cudaStream_t s) {   // an append's work has been issued on s
-        cuda_check(cudaEventRecord(kivi_done[kivi_turn], s), "record append event");
+    cudaError_t kivi_mark(cudaStream_t s) {   // an append's work has been issued on s
+        const cudaError_t e = cudaEventRecord(kivi_done[kivi_turn], s);
+        if (e != cudaSuccess) return e;
         kivi_turn ^= 1u;
         kivi_stream = s;
         kivi_pending = true;
+        return cudaSuccess;
     }
     // Quantise `pages` pages of `tokens` rows of (layer, kv_head): the rows of the tail, then the staged ones; `rest` staged rows
     // after them become the tail. One launch, which also publishes the descriptors. The rows are known to be finite: they were
@@ -402,10 +405,24 @@ struct cf_llama_kv_adapter {
         common.k_max_code_length = common.v_max_code_length = common.fixed_code_length = kivi_bits;
         common.zero_point = 1u << (kivi_bits - 1);
         common.kv_head = kv_head;
+        // Everything that can fail comes first: the host's list names no page that the launch below does not write.
         std::vector<cf_kv_device_page> &host = kivi_host_descs[layer];
-        const size_t first = host.size();
+        const size_t first = host.size(), chunk_index = kivi_chunk_index, chunk_used = kivi_chunk_used;
+        try {
+            if (host.capacity() < first + pages) host.reserve(2 * first + pages);
+            for (uint32_t p = 0; p < pages; ++p) job.block[p] = kivi_take(lay.total);
+            DeviceBuffer<cf_kv_device_page> &dev = *kivi_descs[layer];
+            dev.ensure(first + pages, s);
+            job.pages_out = dev.ptr + first;
+            kivi_quantise_kernel<<<pages, 1024, (static_cast<size_t>(D) + tokens) * sizeof(float), s>>>(job, lay);
+            cuda_check(cudaGetLastError(), "page quantise launch");
+        } catch (...) {
+            kivi_chunk_index = chunk_index;
+            kivi_chunk_used = chunk_used;
+            throw;
+        }
         for (uint32_t p = 0; p < pages; ++p) {
-            const uint8_t *block = job.block[p] = kivi_take(lay.total);
+            const uint8_t *block = job.block[p];
             cf_kv_device_page page = common;
             page.k_words = reinterpret_cast<const uint32_t *>(block + lay.k_words);
             page.v_words = reinterpret_cast<const uint32_t *>(block + lay.v_words);
@@ -416,11 +433,6 @@ struct cf_llama_kv_adapter {
             page.token_begin += p * tokens;
             host.push_back(page);
         }
-        DeviceBuffer<cf_kv_device_page> &dev = *kivi_descs[layer];
-        dev.ensure(host.size(), s);
-        job.pages_out = dev.ptr + first;
-        kivi_quantise_kernel<<<pages, 1024, (static_cast<size_t>(D) + tokens) * sizeof(float), s>>>(job, lay);
-        cuda_check(cudaGetLastError(), "page quantise launch");
         // EncodedKvPage::resident_bytes: words, offsets, both LUTs, scales
         kivi_resident_bytes += pages * (8ull * lay.word_count + 8ull * lay.block_count + 8ull * (1u << kivi_bits) + 4ull * (D + tokens));
         if (tokens < opt.page_size) h.flushed_partial = true;
@@ -433,7 +445,7 @@ struct cf_llama_kv_adapter {
         if (h.bad_row < h.tail) throw std::invalid_argument("invalid quantization input");   // kv_gpu_fixture.cpp:13
         kivi_join(s);
         kivi_seal(layer, kv_head, 1, h.tail, 0, s);
-        kivi_mark(s);
+        cuda_check(kivi_mark(s), "record append event");
         h.tail = 0;
     }
     // `take` host rows into the tail ([token][kv head][dim]: the layout the attention reads).
@@ -480,15 +492,20 @@ struct cf_llama_kv_adapter {
             }
             cuda_check(cudaEventSynchronize(kivi_done[kivi_turn]), "wait for an earlier append");   // its half of the pinned memory
             const float *source[2] = {keys + static_cast<size_t>(done) * D, values + static_cast<size_t>(done) * D};
-            uint32_t bad = rows;   // first staged row with NaN or Inf
-            for (int stream = 0; stream < 2; ++stream) {   // the copy of K crosses the bus while V is gathered
-                float *half = kivi_pinned + (2u * kivi_turn + stream) * kivi_stage_floats;
-                bad = std::min(bad, copy_rows_checked(half, source[stream], rows, D));
-                cuda_check(cudaMemcpyAsync(kivi_stage.ptr + stream * kivi_stage_floats, half, floats * sizeof(float), cudaMemcpyHostToDevice, s), "stage rows");
+            uint32_t bad = rows, sealed = 0;   // first staged row with NaN or Inf; pages in front of it
+            try {
+                for (int stream = 0; stream < 2; ++stream) {   // the copy of K crosses the bus while V is gathered
+                    float *half = kivi_pinned + (2u * kivi_turn + stream) * kivi_stage_floats;
+                    bad = std::min(bad, copy_rows_checked(half, source[stream], rows, D));
+                    cuda_check(cudaMemcpyAsync(kivi_stage.ptr + stream * kivi_stage_floats, half, floats * sizeof(float), cudaMemcpyHostToDevice, s), "stage rows");
+                }
+                sealed = h.bad_row < h.tail ? 0u : std::min(pages, (h.tail + bad) / T);
+                if (sealed) kivi_seal(layer, kv_head, sealed, T, sealed == pages ? rest : 0u, s);
+            } catch (...) {   // the pinned half may still be on its way
+                kivi_mark(s);
+                throw;
             }
-            const uint32_t sealed = h.bad_row < h.tail ? 0u : std::min(pages, (h.tail + bad) / T);
-            if (sealed) kivi_seal(layer, kv_head, sealed, T, sealed == pages ? rest : 0u, s);
-            kivi_mark(s);
+            cuda_check(kivi_mark(s), "record append event");
             if (sealed < pages) {   // pages before the refused one stay; its rows become the (full) tail, as if appended page by page
                 const uint32_t skip = sealed ? sealed * T - h.tail : 0u, keep = sealed ? 0u : h.tail;
                 if (sealed) {
@@ -986,6 +1003,12 @@ extern "C" const char *cf_llama_kv_last_error(const cf_llama_kv_adapter *adapter
 // page_index counts the pages of `layer` in the order they were sealed, over all kv heads. Returns -1 in format-v1 mode.
 extern "C" uint64_t cf_b200_llama_kv_reserved_bytes(const cf_llama_kv_adapter *adapter) {
     return adapter ? static_cast<uint64_t>(adapter->kivi_chunks.size()) * cf_llama_kv_adapter::kKiviChunk : 0;
+}
+
+extern "C" int cf_b200_test_llama_kv_chunk_limit(cf_llama_kv_adapter *adapter, uint32_t chunks) {
+    if (adapter == nullptr) return -1;
+    adapter->kivi_chunk_limit = chunks;
+    return 0;
 }
 
 extern "C" int cf_b200_llama_kv_reference_page(const cf_llama_kv_adapter *adapter, uint32_t layer, uint32_t page_index,

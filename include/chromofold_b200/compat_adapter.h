@@ -96,6 +96,8 @@ int cf_b200_llama_kv_reference_page(const cf_llama_kv_adapter *adapter, uint32_t
  * sequence position, i.e. context length> in the environment makes cf_llama_kv_create take the chunks and the
  * descriptor arrays for that many tokens of every layer and kv head up front, so that no append allocates. */
 uint64_t cf_b200_llama_kv_reserved_bytes(const cf_llama_kv_adapter *adapter);
+/* Test hook: an append that would need more than `chunks` chunks of page memory fails as it does when the GPU has none left. */
+int cf_b200_test_llama_kv_chunk_limit(cf_llama_kv_adapter *adapter, uint32_t chunks);
 
 #ifdef __cplusplus
 }

@@ -244,3 +244,42 @@ def test_adapter_append_keeps_the_pages_before_a_refused_one(native):
     ks, _ = _quantised(k[32:48], 0, 4)
     assert np.array_equal(_read_device(pg.k_words, 128, np.uint32), _pack(ks, 4)[:128])
     lib.cf_llama_kv_destroy(handle)
+
+
+def _attend(lib, handle, q, begin, stream=None):
+    import torch
+    out = torch.full(q.shape, 5.0, device="cuda")
+    hq = q.shape[1]
+    assert lib.cf_llama_kv_attention(handle, 0, C.c_void_p(q.data_ptr()), C.c_void_p(out.data_ptr()), q.shape[0], hq, 1, begin,
+                                     C.c_float(q.shape[2] ** -0.5), 0, C.c_void_p(stream.cuda_stream) if stream else None) == 0
+    return out
+
+
+def test_adapter_append_that_runs_out_of_memory_leaves_no_page_behind(native):
+    """The page memory ends in the middle of a launch's pages: the pages before that launch stay, none of its own is named, and the
+    same rows go in once there is memory again."""
+    import torch
+    lib, handle = _adapter(native, 1, 128, 128, 8)
+    rng = np.random.default_rng(5)
+    block = 2 * 128 * 128 + 4 * 256 + 2 * 4 * 256
+    pages = (32 << 20) // ((block + 255) // 256 * 256)       # of the first chunk
+    rows = np.tile(rng.standard_normal((128 * 16, 128)).astype(np.float32), ((pages + 40) // 16 + 1, 1))[:128 * (pages + 40)]
+    k, v = rows, np.ascontiguousarray(rows[::-1])
+    assert lib.cf_b200_test_llama_kv_chunk_limit(handle, 1) == 0
+    assert _append(lib, handle, 0, 0, k, v) == -1 and lib.cf_b200_llama_kv_reserved_bytes(handle) == 32 << 20
+    named = 0
+    while lib.cf_b200_llama_kv_reference_page(handle, 0, named, C.byref(DevicePage())) == 0:
+        named += 1
+    launch = (1 << 20) // (4 * 128 * 128)                    # pages of a launch
+    assert pages % launch != 0 and named == pages // launch * launch
+    q = torch.from_numpy(rng.standard_normal((2, 1, 128)).astype(np.float32)).cuda()
+    few = _attend(lib, handle, q, 128 * named - 1)
+    other_lib, other = _adapter(native, 1, 128, 128, 8)
+    assert _append(lib, other, 0, 0, k[:128 * named], v[:128 * named]) == 0
+    assert torch.equal(few, _attend(lib, other, q, 128 * named - 1))
+    assert lib.cf_b200_test_llama_kv_chunk_limit(handle, 2) == 0
+    for h in (handle, other):
+        assert _append(lib, h, 0, 128 * named, k[128 * named:], v[128 * named:]) == 0
+    assert torch.equal(_attend(lib, handle, q, len(k) - 1), _attend(lib, other, q, len(k) - 1))
+    for h in (handle, other):
+        lib.cf_llama_kv_destroy(h)
