@@ -229,6 +229,59 @@ uint32_t first_bad_row(const float *src, uint32_t rows, uint32_t dim) {
     return r;
 }
 
+// Work on the GPU that later calls on other streams have to come after: an event per stream, recorded anew by every call on it.
+// Streams go by their id, which unlike the handle is never used again; the event of a stream whose work has ended serves the next.
+class StreamMarks {
+    struct Mark {
+        unsigned long long stream_id;
+        cudaEvent_t event;
+        bool pending;
+    };
+    std::vector<Mark> marks;
+
+public:
+    StreamMarks() = default;
+    StreamMarks(const StreamMarks &) = delete;
+    StreamMarks &operator=(const StreamMarks &) = delete;
+    ~StreamMarks() {
+        for (const Mark &m : marks) cudaEventDestroy(m.event);
+    }
+    void mark(cudaStream_t s) {   // everything issued on s so far (what a graph will run later is the graph's caller's to order)
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        cuda_check(cudaStreamIsCapturing(s, &capture), "cudaStreamIsCapturing");
+        if (capture != cudaStreamCaptureStatusNone) return;
+        unsigned long long id = 0;
+        cuda_check(cudaStreamGetId(s, &id), "cudaStreamGetId");
+        Mark *mine = nullptr;
+        for (Mark &m : marks)
+            if (m.stream_id == id) mine = &m;
+        for (size_t i = 0; !mine && i < marks.size(); ++i)
+            if (!marks[i].pending || cudaEventQuery(marks[i].event) == cudaSuccess) mine = &marks[i];
+        if (!mine) {
+            Mark fresh{id, nullptr, false};
+            cuda_check(cudaEventCreateWithFlags(&fresh.event, cudaEventDisableTiming), "create adapter event");
+            marks.push_back(fresh);
+            mine = &marks.back();
+        }
+        mine->stream_id = id;
+        cuda_check(cudaEventRecord(mine->event, s), "record adapter event");
+        mine->pending = true;
+    }
+    void join(cudaStream_t s) {   // what is issued on s from now on comes after all that was marked
+        unsigned long long id = 0;
+        cuda_check(cudaStreamGetId(s, &id), "cudaStreamGetId");
+        for (Mark &m : marks) {
+            if (!m.pending || m.stream_id == id) continue;
+            if (cudaEventQuery(m.event) == cudaSuccess) m.pending = false;
+            else cuda_check(cudaStreamWaitEvent(s, m.event, 0), "wait for another stream's work");
+        }
+    }
+    void wait() const {   // on the host
+        for (const Mark &m : marks)
+            if (m.pending) cudaEventSynchronize(m.event);
+    }
+};
+
 struct HeadState {   // per (layer, kv head), in tokens
     uint64_t appended = 0;      // everything ever appended
     uint32_t sealed = 0;        // tokens in sealed tiles
@@ -290,8 +343,7 @@ struct cf_llama_kv_adapter {
     size_t kivi_stage_floats = 0;            // of one of the two streams
     cudaEvent_t kivi_done[2] = {};           // the append that used pinned half i has ended
     uint32_t kivi_turn = 0;                  // pinned half of the next append
-    cudaStream_t kivi_stream = nullptr;      // of the last append, and
-    bool kivi_pending = false;               // whether it may still be under way
+    StreamMarks kivi_written, kivi_read;     // appends and flushes, attention calls
     static constexpr size_t kKiviStageBytes = 1u << 20;   // of one stream, staged at a time (at least one page): the next turn copies meanwhile
 
     ~cf_llama_kv_adapter() {
@@ -303,6 +355,23 @@ struct cf_llama_kv_adapter {
             }
         if (kivi_pinned) cudaFreeHost(kivi_pinned);
     }
+    // A call that writes pages or tails on stream s: after all earlier writes and attention calls, whatever streams they were on; its
+    // own work is marked on every way out.
+    struct WriteCall {
+        cf_llama_kv_adapter &adapter;
+        cudaStream_t s;
+        WriteCall(cf_llama_kv_adapter &a, cudaStream_t stream) : adapter(a), s(stream) {
+            adapter.kivi_written.join(s);
+            adapter.kivi_read.join(s);
+        }
+        ~WriteCall() {
+            try {
+                adapter.kivi_written.mark(s);
+            } catch (...) {   // no event to be had: the work ends before the call does
+                cudaStreamSynchronize(s);
+            }
+        }
+    };
     size_t kivi_row_floats() const { return static_cast<size_t>(opt.kv_head_count) * opt.head_dim; }
     float *kivi_tail(DeviceBuffer<float> &buffer, uint32_t layer) const {
         return buffer.ptr + static_cast<size_t>(layer) * opt.page_size * kivi_row_floats();
@@ -361,20 +430,10 @@ struct cf_llama_kv_adapter {
         kivi_resident_bytes = 0;
         for (auto &d : kivi_host_descs) d.clear();
     }
-    // Work on stream s comes after the last append, which may have used another stream and still be under way.
-    void kivi_join(cudaStream_t s) {
-        if (!kivi_pending || s == kivi_stream) return;
-        const cudaEvent_t last = kivi_done[(kivi_turn ^ 1u) & 1u];
-        if (cudaEventQuery(last) == cudaSuccess) kivi_pending = false;
-        else cuda_check(cudaStreamWaitEvent(s, last, 0), "wait for the last append");
-    }
-    cudaError_t kivi_mark(cudaStream_t s) {   // an append's work has been issued on s
+    cudaError_t kivi_mark(cudaStream_t s) {   // the copies out of a pinned half have been issued on s
         const cudaError_t e = cudaEventRecord(kivi_done[kivi_turn], s);
-        if (e != cudaSuccess) return e;
-        kivi_turn ^= 1u;
-        kivi_stream = s;
-        kivi_pending = true;
-        return cudaSuccess;
+        if (e == cudaSuccess) kivi_turn ^= 1u;
+        return e;
     }
     // Quantise `pages` pages of `tokens` rows of (layer, kv_head): the rows of the tail, then the staged ones; `rest` staged rows
     // after them become the tail. One launch, which also publishes the descriptors. The rows are known to be finite: they were
@@ -443,9 +502,7 @@ struct cf_llama_kv_adapter {
         HeadState &h = head(layer, kv_head);
         if (h.tail == 0) return;
         if (h.bad_row < h.tail) throw std::invalid_argument("invalid quantization input");   // kv_gpu_fixture.cpp:13
-        kivi_join(s);
         kivi_seal(layer, kv_head, 1, h.tail, 0, s);
-        cuda_check(kivi_mark(s), "record append event");
         h.tail = 0;
     }
     // `take` host rows into the tail ([token][kv head][dim]: the layout the attention reads).
@@ -468,7 +525,6 @@ struct cf_llama_kv_adapter {
         HeadState &h = head(layer, kv_head);
         const uint32_t T = tile_tokens, D = opt.head_dim;
         uint32_t done = 0;
-        kivi_join(s);
         while (done < token_count) {
             const uint32_t left = token_count - done;
             if (h.tail + left < T) {
@@ -772,6 +828,7 @@ extern "C" int cf_llama_kv_append(cf_llama_kv_adapter *adapter, uint32_t layer, 
         }
         const uint32_t D = adapter->opt.head_dim, T = adapter->tile_tokens;
         if (adapter->kivi) {
+            const cf_llama_kv_adapter::WriteCall call(*adapter, s);
             adapter->kivi_append(layer, kv_head, keys, values, token_count, s);
             h.appended += token_count;
             return;
@@ -813,7 +870,7 @@ extern "C" int cf_llama_kv_attention(cf_llama_kv_adapter *adapter, uint32_t laye
             if (h.sealed != h0.sealed || h.tail != h0.tail) throw std::runtime_error("KV active tails are not aligned across heads");
         }
         if (adapter->kivi) {   // the reference's own call over the reference's own page descriptors (its adapter, :107-131)
-            adapter->kivi_join(s);
+            adapter->kivi_written.join(s);
             cf_kv_paged_attention_desc desc{};
             desc.struct_size = sizeof desc;
             desc.abi_version = CF_KV_CUDA_ABI_VERSION;
@@ -834,6 +891,7 @@ extern "C" int cf_llama_kv_attention(cf_llama_kv_adapter *adapter, uint32_t laye
             desc.causal_window = causal_window;
             desc.softmax_scale = softmax_scale;
             if (cf_kv_paged_attention_async(&desc, s) != CF_OK) throw std::runtime_error("ChromoFold paged attention launch rejected");
+            adapter->kivi_read.mark(s);
             return;
         }
         LayerState &ls = adapter->layers[layer];
@@ -930,6 +988,8 @@ extern "C" int cf_llama_kv_attention_host(cf_llama_kv_adapter *adapter, uint32_t
 
 extern "C" int cf_llama_kv_flush(cf_llama_kv_adapter *adapter, void *stream) {
     return guarded(adapter, [&] {
+        std::unique_ptr<cf_llama_kv_adapter::WriteCall> call;
+        if (adapter->kivi) call = std::make_unique<cf_llama_kv_adapter::WriteCall>(*adapter, static_cast<cudaStream_t>(stream));
         for (uint32_t layer = 0; layer < adapter->opt.layer_count; ++layer)
             for (uint32_t h = 0; h < adapter->opt.kv_head_count; ++h) {
                 if (adapter->kivi) adapter->kivi_flush(layer, h, static_cast<cudaStream_t>(stream));
@@ -1016,7 +1076,7 @@ extern "C" int cf_b200_llama_kv_reference_page(const cf_llama_kv_adapter *adapte
     if (adapter == nullptr || out_page == nullptr || !adapter->kivi || layer >= adapter->kivi_host_descs.size() ||
         page_index >= adapter->kivi_host_descs[layer].size())
         return -1;
-    for (cudaEvent_t e : adapter->kivi_done) cudaEventSynchronize(e);   // the caller reads the page by ways of its own
+    adapter->kivi_written.wait();   // the caller reads the page by ways of its own
     *out_page = adapter->kivi_host_descs[layer][page_index];
     return 0;
 }

@@ -5,6 +5,8 @@
  * the reference's name, argument list and return convention (0 / -1 and a last_error string owned by the handle,
  * exceptions never cross the boundary — chromofold_kv_adapter.cpp:35-49).
  *
+ * Streams: a call comes after the appends and flushes before it, an append or flush also after the attention calls before it, on
+ * whatever streams they were; a captured attention call keeps its place by the caller's own ordering of the graph.
  * What is kept: one sequence (id 0) per adapter (src/runtime/compressed_kv_cache.cu:180-193); append takes HOST fp32
  * rows per (layer, kv head) and must be logically contiguous (:78-80); full pages seal on append (:87), flush seals
  * the partial tail (:111-125); attention takes DEVICE fp32 queries [query_count][Hq][head_dim], query row i sits at

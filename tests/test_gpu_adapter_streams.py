@@ -1,0 +1,76 @@
+"""The llama.cpp adapter called on several streams: whatever stream a call names, it comes after the appends before it, and an append
+after the attention calls before it."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from test_gpu_paged_mma import _adapter
+
+pytestmark = pytest.mark.gpu
+HEADS, D, PAGE = 2, 64, 16
+
+
+class _Calls:
+    """One adapter and a fixed sequence of rows; `late` puts 40 ms of other work in front of the calls that ask for it, and then
+    nothing waits for the GPU; otherwise every call ends before the next."""
+
+    def __init__(self, native, late):
+        import torch
+        self.torch, self.late = torch, late
+        self.lib, self.handle = _adapter(native, HEADS, D, PAGE, 8)
+        self.streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+        rng = np.random.default_rng(2)
+        self.k, self.v = (rng.standard_normal((HEADS, 400, D)).astype(np.float32) for _ in range(2))
+        self.q = torch.from_numpy(rng.standard_normal((1, HEADS, D)).astype(np.float32)).cuda()
+        self.outs, self.at = [], 0
+        torch.cuda.synchronize()
+
+    def _delay(self, stream, late):
+        if self.late and late:
+            with self.torch.cuda.stream(stream):
+                self.torch.cuda._sleep(80_000_000)
+
+    def append(self, on, rows, late=False):
+        s = self.streams[on]
+        self._delay(s, late)
+        for h in range(HEADS):
+            kk, vv = self.k[h, self.at:], self.v[h, self.at:]
+            assert self.lib.cf_llama_kv_append(self.handle, 0, h, self.at, C.c_void_p(kk.ctypes.data), C.c_void_p(vv.ctypes.data), rows,
+                                               C.c_void_p(s.cuda_stream)) == 0
+        self.at += rows
+        if not self.late:
+            self.torch.cuda.synchronize()
+
+    def attend(self, on, late=False):
+        s = self.streams[on]
+        out = self.torch.zeros_like(self.q)
+        s.wait_stream(self.torch.cuda.current_stream())   # for the zeros
+        self._delay(s, late)
+        assert self.lib.cf_llama_kv_attention(self.handle, 0, C.c_void_p(self.q.data_ptr()), C.c_void_p(out.data_ptr()), 1, HEADS, 1, self.at - 1,
+                                              C.c_float(D ** -0.5), 0, C.c_void_p(s.cuda_stream)) == 0
+        self.outs.append(out)
+        if not self.late:
+            self.torch.cuda.synchronize()
+
+
+STORIES = {
+    "a tail row on one stream, attention on the other": [("append", 0, 20), ("append", 0, 1, True), ("attend", 1)],
+    "a tail row on one stream, the page it belongs to filled on the other": [("append", 0, 20), ("append", 0, 3, True), ("append", 1, 12), ("attend", 1)],
+    "pages on one stream, attention on the other": [("append", 0, 5), ("append", 0, 90, True), ("attend", 1)],
+    "attention on one stream, the tail it reads replaced on the other": [("append", 0, 20), ("attend", 0, True), ("append", 1, 30), ("attend", 1)],
+    "two readers, then a writer on neither's turn": [("append", 0, 9), ("attend", 1, True), ("attend", 0), ("append", 0, 39), ("attend", 1)],
+}
+
+
+@pytest.mark.parametrize("story", STORIES)
+def test_calls_on_two_streams_take_effect_in_their_order(native, story):
+    import torch
+    got, want = _Calls(native, True), _Calls(native, False)
+    for calls in (want, got):
+        for name, *args in STORIES[story]:
+            getattr(calls, name)(*args)
+        torch.cuda.synchronize()
+        calls.lib.cf_llama_kv_destroy(calls.handle)
+    for a, b in zip(got.outs, want.outs):
+        assert torch.equal(a, b)
