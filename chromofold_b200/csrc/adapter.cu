@@ -268,6 +268,19 @@ public:
         mine->pending = true;
     }
     void join(cudaStream_t s) {   // what is issued on s from now on comes after all that was marked
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        cuda_check(cudaStreamIsCapturing(s, &capture), "cudaStreamIsCapturing");
+        if (capture != cudaStreamCaptureStatusNone) {   // a graph cannot wait for what is outside of it: it ends before the call goes on
+            cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;   // and only so may a capturing thread wait
+            cuda_check(cudaThreadExchangeStreamCaptureMode(&mode), "cudaThreadExchangeStreamCaptureMode");
+            cudaError_t e = cudaSuccess;
+            for (Mark &m : marks)
+                if (m.pending && (e = cudaEventSynchronize(m.event)) == cudaSuccess) m.pending = false;
+                else if (e != cudaSuccess) break;
+            cuda_check(cudaThreadExchangeStreamCaptureMode(&mode), "cudaThreadExchangeStreamCaptureMode");
+            cuda_check(e, "wait for another stream's work");
+            return;
+        }
         unsigned long long id = 0;
         cuda_check(cudaStreamGetId(s, &id), "cudaStreamGetId");
         for (Mark &m : marks) {

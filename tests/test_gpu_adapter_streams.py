@@ -74,3 +74,28 @@ def test_calls_on_two_streams_take_effect_in_their_order(native, story):
         calls.lib.cf_llama_kv_destroy(calls.handle)
     for a, b in zip(got.outs, want.outs):
         assert torch.equal(a, b)
+
+
+def test_attention_after_an_append_on_another_stream_can_be_captured(native):
+    import torch
+    calls = _Calls(native, True)
+    calls.append(0, 20, late=True)
+    out = torch.zeros_like(calls.q)
+    graph, side = torch.cuda.CUDAGraph(), calls.streams[1]
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        graph.capture_begin()
+        rc = calls.lib.cf_llama_kv_attention(calls.handle, 0, C.c_void_p(calls.q.data_ptr()), C.c_void_p(out.data_ptr()), 1, HEADS, 1, 19,
+                                             C.c_float(D ** -0.5), 0, C.c_void_p(side.cuda_stream))
+        graph.capture_end()
+    assert rc == 0
+    graph.replay()
+    torch.cuda.synchronize()
+    calls.attend(1)
+    torch.cuda.synchronize()
+    # one launch under capture, splits outside of it: the same sums in another order
+    assert torch.allclose(out, calls.outs[0], rtol=1e-5, atol=1e-6) and float(out.abs().max()) > 0
+    calls.append(0, 30)      # the captured call left nothing behind that a later one would trip over
+    calls.attend(0)
+    torch.cuda.synchronize()
+    calls.lib.cf_llama_kv_destroy(calls.handle)
