@@ -214,6 +214,27 @@ __global__ void __launch_bounds__(1024) kivi_quantise_kernel(const __grid_consta
     }
 }
 
+// *first_bad = the smallest of itself and the numbers (from `first` on) of the rows that hold NaN or Inf. A warp per row.
+__global__ void __launch_bounds__(256) first_bad_row_kernel(const float *k, const float *v, size_t row_stride, uint32_t dim, uint32_t rows, uint32_t first,
+                                                            uint32_t *first_bad) {
+    const uint32_t row = blockIdx.x * (blockDim.x / 32u) + threadIdx.x / 32u;
+    if (row >= rows) return;
+    bool bad = false;
+    for (uint32_t d = threadIdx.x % 32u; d < dim; d += 32u) bad = bad || !isfinite(k[row * row_stride + d]) || !isfinite(v[row * row_stride + d]);
+    if (__any_sync(0xffffffffu, bad) && threadIdx.x % 32u == 0) atomicMin(first_bad, first + row);
+}
+
+// Whether a copy reads this memory in stream order (pinned, managed and device memory): what it holds when the call is
+// made need not be what the stream's earlier work will have put there, and the host may not be able to look at it.
+bool in_stream_order(const void *ptr) {
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, ptr) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return a.type != cudaMemoryTypeUnregistered;
+}
+
 // Copies `rows` rows of `dim` floats and returns the first that holds NaN or Inf, or `rows`.
 uint32_t copy_rows_checked(float *dst, const float *src, uint32_t rows, uint32_t dim) {
     const size_t n = static_cast<size_t>(rows) * dim;
@@ -300,7 +321,8 @@ struct HeadState {   // per (layer, kv head), in tokens
     uint32_t sealed = 0;        // tokens in sealed tiles
     uint32_t tail = 0;          // tokens in the device tail
     uint32_t next_token = 0;    // position the next append must start at
-    uint32_t bad_row = 0xffffffffu;   // first row of the tail that holds NaN or Inf
+    uint32_t bad_row = 0xffffffffu;   // first row of the tail that holds NaN or Inf, as far as it has been looked at
+    bool unchecked = false;           // rows of the tail came in stream order: the GPU looks at them when they become a page
     bool started = false;
     bool flushed_partial = false;
 };
@@ -351,6 +373,7 @@ struct cf_llama_kv_adapter {
     std::vector<std::unique_ptr<DeviceBuffer<cf_kv_device_page>>> kivi_descs;   // per layer, device
     std::vector<std::vector<cf_kv_device_page>> kivi_host_descs;                // per layer, the same on the host
     uint64_t kivi_resident_bytes = 0;
+    DeviceBuffer<uint32_t> kivi_first_bad;   // result of first_bad_row_kernel
     DeviceBuffer<float> kivi_stage;          // rows of an append that fills pages: [K rows | V rows]
     float *kivi_pinned = nullptr;            // the same on their way from the caller's pageable memory, twice: appends take turns
     size_t kivi_stage_floats = 0;            // of one of the two streams
@@ -511,18 +534,41 @@ struct cf_llama_kv_adapter {
         h.sealed += pages * tokens;
         sealed_tiles += pages;
     }
+    // The first row with NaN or Inf among the tail's rows that have not been looked at, and `staged` rows behind them.
+    uint32_t kivi_look(uint32_t layer, uint32_t kv_head, uint32_t staged, cudaStream_t s) {
+        HeadState &h = head(layer, kv_head);
+        const uint32_t D = opt.head_dim;
+        uint32_t first = 0xffffffffu;
+        kivi_first_bad.ensure(1, s);
+        cuda_check(cudaMemsetAsync(kivi_first_bad.ptr, 0xff, 4, s), "clear row check");
+        if (h.unchecked)
+            first_bad_row_kernel<<<(h.tail + 7u) / 8u, 256, 0, s>>>(kivi_tail(kivi_tail_k, layer) + static_cast<size_t>(kv_head) * D,
+                                                                   kivi_tail(kivi_tail_v, layer) + static_cast<size_t>(kv_head) * D, kivi_row_floats(), D,
+                                                                   h.tail, 0u, kivi_first_bad.ptr);
+        if (staged)
+            first_bad_row_kernel<<<(staged + 7u) / 8u, 256, 0, s>>>(kivi_stage.ptr, kivi_stage.ptr + kivi_stage_floats, D, D, staged, h.tail, kivi_first_bad.ptr);
+        cuda_check(cudaGetLastError(), "row check launch");
+        cuda_check(cudaMemcpyAsync(&first, kivi_first_bad.ptr, 4, cudaMemcpyDeviceToHost, s), "read row check");
+        cuda_check(cudaStreamSynchronize(s), "cudaStreamSynchronize");   // a page is refused by the call that brings it
+        if (first < h.tail) h.bad_row = std::min(h.bad_row, first);
+        h.unchecked = false;
+        return first;
+    }
     void kivi_flush(uint32_t layer, uint32_t kv_head, cudaStream_t s) {
         HeadState &h = head(layer, kv_head);
         if (h.tail == 0) return;
+        if (h.unchecked) kivi_look(layer, kv_head, 0, s);
         if (h.bad_row < h.tail) throw std::invalid_argument("invalid quantization input");   // kv_gpu_fixture.cpp:13
         kivi_seal(layer, kv_head, 1, h.tail, 0, s);
         h.tail = 0;
     }
     // `take` host rows into the tail ([token][kv head][dim]: the layout the attention reads).
-    void kivi_rows_to_tail(uint32_t layer, uint32_t kv_head, const float *keys, const float *values, uint32_t take, cudaStream_t s) {
+    void kivi_rows_to_tail(uint32_t layer, uint32_t kv_head, const float *keys, const float *values, uint32_t take, bool ordered, cudaStream_t s) {
         if (take == 0) return;
         HeadState &h = head(layer, kv_head);
-        if (h.bad_row >= h.tail) {
+        if (ordered) {
+            h.unchecked = true;
+        } else if (h.bad_row >= h.tail) {
             const uint32_t bad = std::min(first_bad_row(keys, take, opt.head_dim), first_bad_row(values, take, opt.head_dim));
             h.bad_row = bad < take ? h.tail + bad : 0xffffffffu;
         }
@@ -537,11 +583,12 @@ struct cf_llama_kv_adapter {
     void kivi_append(uint32_t layer, uint32_t kv_head, const float *keys, const float *values, uint32_t token_count, cudaStream_t s) {
         HeadState &h = head(layer, kv_head);
         const uint32_t T = tile_tokens, D = opt.head_dim;
+        const bool ordered = in_stream_order(keys) || in_stream_order(values);
         uint32_t done = 0;
         while (done < token_count) {
             const uint32_t left = token_count - done;
             if (h.tail + left < T) {
-                kivi_rows_to_tail(layer, kv_head, keys + static_cast<size_t>(done) * D, values + static_cast<size_t>(done) * D, left, s);
+                kivi_rows_to_tail(layer, kv_head, keys + static_cast<size_t>(done) * D, values + static_cast<size_t>(done) * D, left, ordered, s);
                 return;
             }
             const uint32_t room = std::max<uint32_t>(1u, std::min<uint32_t>(kKiviPagesPerLaunch, static_cast<uint32_t>(kKiviStageBytes / (4ull * T * D))));
@@ -564,9 +611,17 @@ struct cf_llama_kv_adapter {
             uint32_t bad = rows, sealed = 0;   // first staged row with NaN or Inf; pages in front of it
             try {
                 for (int stream = 0; stream < 2; ++stream) {   // the copy of K crosses the bus while V is gathered
-                    float *half = kivi_pinned + (2u * kivi_turn + stream) * kivi_stage_floats;
-                    bad = std::min(bad, copy_rows_checked(half, source[stream], rows, D));
+                    const float *half = source[stream];
+                    if (!ordered) {
+                        float *pinned = kivi_pinned + (2u * kivi_turn + stream) * kivi_stage_floats;
+                        bad = std::min(bad, copy_rows_checked(pinned, half, rows, D));
+                        half = pinned;
+                    }
                     cuda_check(cudaMemcpyAsync(kivi_stage.ptr + stream * kivi_stage_floats, half, floats * sizeof(float), cudaMemcpyHostToDevice, s), "stage rows");
+                }
+                if (ordered || h.unchecked) {
+                    const uint32_t first = kivi_look(layer, kv_head, ordered ? rows : 0u, s);
+                    if (first >= h.tail) bad = std::min(bad, first - h.tail);
                 }
                 sealed = h.bad_row < h.tail ? 0u : std::min(pages, (h.tail + bad) / T);
                 if (sealed) kivi_seal(layer, kv_head, sealed, T, sealed == pages ? rest : 0u, s);
@@ -582,7 +637,7 @@ struct cf_llama_kv_adapter {
                     h.bad_row = 0xffffffffu;
                 }
                 h.tail = keep;
-                kivi_rows_to_tail(layer, kv_head, source[0] + static_cast<size_t>(skip) * D, source[1] + static_cast<size_t>(skip) * D, T - keep, s);
+                kivi_rows_to_tail(layer, kv_head, source[0] + static_cast<size_t>(skip) * D, source[1] + static_cast<size_t>(skip) * D, T - keep, ordered, s);
                 cuda_check(cudaStreamSynchronize(s), "cudaStreamSynchronize");
                 throw std::invalid_argument("invalid quantization input");
             }

@@ -99,3 +99,59 @@ def test_attention_after_an_append_on_another_stream_can_be_captured(native):
     calls.attend(0)
     torch.cuda.synchronize()
     calls.lib.cf_llama_kv_destroy(calls.handle)
+
+
+@pytest.mark.parametrize("rows", [[1, 14, 1], [3, 45], [70], [5, 2]], ids=str)
+def test_rows_in_pinned_memory_are_read_in_stream_order(native, rows):
+    """Rows that the stream's earlier work is still to put into pinned memory (a copy from the GPU, as a model's projections come)."""
+    import torch
+    calls, want = _Calls(native, True), _Calls(native, False)
+    stream, held = calls.streams[0], []
+    for n in rows:
+        want.append(0, n)
+        for h in range(HEADS):
+            source = [torch.from_numpy(x[h, calls.at:calls.at + n]).cuda() for x in (calls.k, calls.v)]
+            pinned = [torch.full((n, D), float("nan")).pin_memory() for _ in source]
+            torch.cuda.synchronize()
+            with torch.cuda.stream(stream):
+                torch.cuda._sleep(20_000_000)
+                for a, b in zip(pinned, source):
+                    a.copy_(b, non_blocking=True)
+            held.append((source, pinned))
+            assert calls.lib.cf_llama_kv_append(calls.handle, 0, h, calls.at, C.c_void_p(pinned[0].data_ptr()), C.c_void_p(pinned[1].data_ptr()), n,
+                                                C.c_void_p(stream.cuda_stream)) == 0
+        calls.at += n
+    for c in (calls, want):
+        c.attend(0)
+        assert c.lib.cf_llama_kv_flush(c.handle, C.c_void_p(c.streams[0].cuda_stream)) == 0
+        c.attend(0)
+        torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(calls.outs, want.outs))
+    bad = torch.zeros((40, D)).pin_memory()          # pages before a refused one stay, as with rows in pageable memory
+    bad[25, 3] = float("inf")
+    for c, rows in ((calls, bad.data_ptr()), (want, bad.numpy().copy())):
+        ptr = C.c_void_p(rows if c is calls else rows.ctypes.data)
+        begin = c.at
+        assert c.lib.cf_llama_kv_append(c.handle, 0, 0, begin, ptr, ptr, 40, C.c_void_p(c.streams[0].cuda_stream)) == -1
+    from compat_types import LlamaKvStats
+    stats = [LlamaKvStats() for _ in range(2)]
+    assert calls.lib.cf_llama_kv_get_stats(calls.handle, C.byref(stats[0])) == 0 and calls.lib.cf_llama_kv_get_stats(want.handle, C.byref(stats[1])) == 0
+    assert bytes(stats[0]) == bytes(stats[1])
+    for c in (calls, want):
+        c.lib.cf_llama_kv_destroy(c.handle)
+
+
+def test_rows_in_device_memory_are_taken_too(native):
+    import torch
+    calls, want = _Calls(native, False), _Calls(native, False)
+    k, v = (torch.from_numpy(x).cuda() for x in (calls.k, calls.v))
+    for n in (3, 40):
+        want.append(0, n)
+        for h in range(HEADS):
+            assert calls.lib.cf_llama_kv_append(calls.handle, 0, h, calls.at, C.c_void_p(k[h, calls.at:].data_ptr()), C.c_void_p(v[h, calls.at:].data_ptr()),
+                                                n, C.c_void_p(calls.streams[0].cuda_stream)) == 0
+        calls.at += n
+    for c in (calls, want):
+        c.attend(0)
+        c.lib.cf_llama_kv_destroy(c.handle)
+    assert torch.equal(calls.outs[0], want.outs[0])
