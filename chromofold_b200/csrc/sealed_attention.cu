@@ -1112,8 +1112,10 @@ cf_status cfb::sealed_attention_stages(const cf_b200_sealed_attention_desc *d, u
         p.plan_warps = p.sm_count * cfb::kGenericCtasPerSm;
         p.unit_lanes = p.kv_head_span;
     }
-    // the shared-prefix kernel works on whole records of 16 x 128 or 16 x 64 symbols in blocks of 64, and on pages without a window
-    if (use_lanes && p.block_size == 64 && (p.head_dim == 128 || p.head_dim == 64) && d->row_map == nullptr && p.decode_probe != 1u && d->shared_prefix_pages && d->causal_window == 0)
+    // the shared-prefix kernel works on whole records of 16 x 128 or 16 x 64 symbols in blocks of 64, on pages without a window, and
+    // reads query rows 16 bytes at a time
+    if (use_lanes && p.block_size == 64 && (p.head_dim == 128 || p.head_dim == 64) && d->row_map == nullptr && p.decode_probe != 1u && d->shared_prefix_pages &&
+        d->causal_window == 0 && reinterpret_cast<uintptr_t>(d->queries) % 16u == 0)
         p.shared_prefix_pages = d->shared_prefix_pages;
     const bool plan = (stages & CF_B200_STAGE_PLAN) != 0, attention = (stages & CF_B200_STAGE_ATTENTION) != 0;
     if (plan && cfb::launch_plan(p, s) != cudaSuccess) return CF_ERR_CUDA;

@@ -793,7 +793,9 @@ bool lanes_kernel_supports(const AttentionParams &p) {
                           ((p.head_dim == 128 && (p.block_size == 64 || p.block_size == 128 || p.block_size == 256)) ||
                            ((p.head_dim == 96 || p.head_dim == 64) && (p.block_size == 64 || p.block_size == 128)) ||
                            ((p.head_dim == 80 || p.head_dim == 32) && p.block_size == 64));
-    return geometry && p.group >= 1 && p.group <= 16 &&
+    // queries are read two channels at a time; others go to the any-geometry kernel, which reads them one by one
+    const uint32_t query_bytes = p.query_type == CF_B200_F32 ? 8u : 4u;
+    return geometry && p.group >= 1 && p.group <= 16 && reinterpret_cast<uintptr_t>(p.queries) % query_bytes == 0 &&
            (p.query_type == CF_B200_F16 || p.query_type == CF_B200_F32);
 }
 

@@ -93,3 +93,29 @@ def test_lane_kernels_agree_with_the_any_geometry_kernel(native, heads, dim, cod
     assert layer.device_status() == 0
     ok, err = attention_close(fast, slow, rel=2e-5, abs_=2e-5)
     assert ok, err
+
+
+@pytest.mark.parametrize("heads,dim,f32,shift,shared", [
+    ((8, 2), 80, True, 4, 0), ((8, 2), 80, False, 2, 0), ((14, 2), 64, True, 8, 12), ((14, 2), 64, False, 2, 12), ((8, 8), 128, True, 4, 9),
+    ((32, 8), 128, False, 8, 9), ((6, 2), 96, True, 12, 0)])
+def test_queries_that_begin_anywhere(native, heads, dim, f32, shift, shared):
+    """The kernels that read queries 4, 8 or 16 bytes at a time are only given rows that lie so."""
+    import torch
+    from chromofold_b200.workloads import build_sealed_layer
+    hq, hkv = heads
+    layer, _ = build_sealed_layer(np.array([16 * 13, 0, 0, 0, 0]), query_heads=hq, kv_heads=hkv, head_dim=dim, seed=3, extra_pages_per_sequence=2)
+    for s in range(1, 5):
+        layer.copy_sequence(0, s)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(4)
+    q = torch.randn((5, hq, dim), generator=g, device="cuda")
+    q = q if f32 else q.half()
+    offset = shift // q.element_size()
+    room = torch.zeros(q.numel() + offset, dtype=q.dtype, device="cuda")
+    moved = room[offset:].view_as(q)
+    moved.copy_(q)
+    assert moved.data_ptr() % 16 == shift
+    a, b = (layer.attention(x, shared_prefix_pages=shared).cpu().numpy() for x in (q, moved))
+    assert layer.device_status() == 0
+    ok, err = attention_close(b, a, rel=2e-5, abs_=2e-5)
+    assert ok, err
