@@ -250,8 +250,21 @@ uint32_t first_bad_row(const float *src, uint32_t rows, uint32_t dim) {
     return r;
 }
 
-// Work on the GPU that later calls on other streams have to come after: an event per stream, recorded anew by every call on it.
-// Streams go by their id, which unlike the handle is never used again; the event of a stream whose work has ended serves the next.
+// The stream of a call. Streams go by their id, which unlike the handle is never used again.
+struct CallStream {
+    cudaStream_t handle;
+    unsigned long long id = 0;
+    bool capturing = false;
+    explicit CallStream(cudaStream_t s) : handle(s) {
+        cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+        cuda_check(cudaStreamIsCapturing(s, &status), "cudaStreamIsCapturing");
+        capturing = status != cudaStreamCaptureStatusNone;
+        if (!capturing) cuda_check(cudaStreamGetId(s, &id), "cudaStreamGetId");   // (ends a capture)
+    }
+};
+
+// Work on the GPU that later calls on other streams have to come after: an event per stream, recorded anew by every call on it. The
+// event of a stream whose work has ended serves the next stream.
 class StreamMarks {
     struct Mark {
         unsigned long long stream_id;
@@ -267,52 +280,44 @@ public:
     ~StreamMarks() {
         for (const Mark &m : marks) cudaEventDestroy(m.event);
     }
-    void mark(cudaStream_t s) {   // everything issued on s so far (what a graph will run later is the graph's caller's to order)
-        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-        cuda_check(cudaStreamIsCapturing(s, &capture), "cudaStreamIsCapturing");
-        if (capture != cudaStreamCaptureStatusNone) return;
-        unsigned long long id = 0;
-        cuda_check(cudaStreamGetId(s, &id), "cudaStreamGetId");
+    void mark(const CallStream &s) {   // everything issued on s so far (what a graph will run later is the graph's caller's to order)
+        if (s.capturing) return;
         Mark *mine = nullptr;
         for (Mark &m : marks)
-            if (m.stream_id == id) mine = &m;
+            if (m.stream_id == s.id) mine = &m;
         for (size_t i = 0; !mine && i < marks.size(); ++i)
             if (!marks[i].pending || cudaEventQuery(marks[i].event) == cudaSuccess) mine = &marks[i];
         if (!mine) {
-            Mark fresh{id, nullptr, false};
+            Mark fresh{s.id, nullptr, false};
             cuda_check(cudaEventCreateWithFlags(&fresh.event, cudaEventDisableTiming), "create adapter event");
             marks.push_back(fresh);
             mine = &marks.back();
         }
-        mine->stream_id = id;
-        cuda_check(cudaEventRecord(mine->event, s), "record adapter event");
+        mine->stream_id = s.id;
+        cuda_check(cudaEventRecord(mine->event, s.handle), "record adapter event");
         mine->pending = true;
     }
-    void join(cudaStream_t s) {   // what is issued on s from now on comes after all that was marked
-        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-        cuda_check(cudaStreamIsCapturing(s, &capture), "cudaStreamIsCapturing");
-        if (capture != cudaStreamCaptureStatusNone) {   // a graph cannot wait for what is outside of it: it ends before the call goes on
+    void join(const CallStream &s) {   // what is issued on s from now on comes after all that was marked
+        if (s.capturing) {   // a graph cannot wait for what is outside of it: it ends before the call goes on
             cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;   // and only so may a capturing thread wait
             cuda_check(cudaThreadExchangeStreamCaptureMode(&mode), "cudaThreadExchangeStreamCaptureMode");
-            cudaError_t e = cudaSuccess;
-            for (Mark &m : marks)
-                if (m.pending && (e = cudaEventSynchronize(m.event)) == cudaSuccess) m.pending = false;
-                else if (e != cudaSuccess) break;
+            const cudaError_t e = wait();
             cuda_check(cudaThreadExchangeStreamCaptureMode(&mode), "cudaThreadExchangeStreamCaptureMode");
             cuda_check(e, "wait for another stream's work");
             return;
         }
-        unsigned long long id = 0;
-        cuda_check(cudaStreamGetId(s, &id), "cudaStreamGetId");
         for (Mark &m : marks) {
-            if (!m.pending || m.stream_id == id) continue;
+            if (!m.pending || m.stream_id == s.id) continue;
             if (cudaEventQuery(m.event) == cudaSuccess) m.pending = false;
-            else cuda_check(cudaStreamWaitEvent(s, m.event, 0), "wait for another stream's work");
+            else cuda_check(cudaStreamWaitEvent(s.handle, m.event, 0), "wait for another stream's work");
         }
     }
-    void wait() const {   // on the host
-        for (const Mark &m : marks)
-            if (m.pending) cudaEventSynchronize(m.event);
+    cudaError_t wait() const {   // on the host
+        for (const Mark &m : marks) {
+            const cudaError_t e = m.pending ? cudaEventSynchronize(m.event) : cudaSuccess;
+            if (e != cudaSuccess) return e;
+        }
+        return cudaSuccess;
     }
 };
 
@@ -395,7 +400,7 @@ struct cf_llama_kv_adapter {
     // own work is marked on every way out.
     struct WriteCall {
         cf_llama_kv_adapter &adapter;
-        cudaStream_t s;
+        const CallStream s;
         WriteCall(cf_llama_kv_adapter &a, cudaStream_t stream) : adapter(a), s(stream) {
             adapter.kivi_written.join(s);
             adapter.kivi_read.join(s);
@@ -404,7 +409,7 @@ struct cf_llama_kv_adapter {
             try {
                 adapter.kivi_written.mark(s);
             } catch (...) {   // no event to be had: the work ends before the call does
-                cudaStreamSynchronize(s);
+                cudaStreamSynchronize(s.handle);
             }
         }
     };
@@ -938,7 +943,8 @@ extern "C" int cf_llama_kv_attention(cf_llama_kv_adapter *adapter, uint32_t laye
             if (h.sealed != h0.sealed || h.tail != h0.tail) throw std::runtime_error("KV active tails are not aligned across heads");
         }
         if (adapter->kivi) {   // the reference's own call over the reference's own page descriptors (its adapter, :107-131)
-            adapter->kivi_written.join(s);
+            const CallStream call(s);
+            adapter->kivi_written.join(call);
             cf_kv_paged_attention_desc desc{};
             desc.struct_size = sizeof desc;
             desc.abi_version = CF_KV_CUDA_ABI_VERSION;
@@ -959,7 +965,7 @@ extern "C" int cf_llama_kv_attention(cf_llama_kv_adapter *adapter, uint32_t laye
             desc.causal_window = causal_window;
             desc.softmax_scale = softmax_scale;
             if (cf_kv_paged_attention_async(&desc, s) != CF_OK) throw std::runtime_error("ChromoFold paged attention launch rejected");
-            adapter->kivi_read.mark(s);
+            adapter->kivi_read.mark(call);
             return;
         }
         LayerState &ls = adapter->layers[layer];
