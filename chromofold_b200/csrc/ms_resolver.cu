@@ -1072,8 +1072,9 @@ extern "C" int cf_ms_cuda_execute_batch_async(cf_ms_cuda_resolver *r, const cf_m
         std::vector<ItemIo> io(item_count);
         std::vector<uint32_t> rows(2 * total_rows);   // slots, then positions
         std::vector<std::pair<uint32_t, uint32_t>> layer_rows(r->config.layer_count, {0u, 0u});  // first row, count
-        // Usually the items' queries are the rows of one dense fp32 tensor and their outputs those of another: the kernels
-        // then read and write those directly; otherwise the rows are gathered into and scattered from dense copies.
+        // Usually the items' queries are the rows of one dense fp32 tensor and their outputs those of another on this GPU: the kernels
+        // then read and write those directly; otherwise the rows are gathered into and scattered from dense copies. (So are
+        // tensors that overlap: a layer's outputs would be written before another layer's queries are read.)
         const void *q_base = nullptr, *o_base = nullptr;
         bool dense = true;
         uint32_t at = 0;
@@ -1101,7 +1102,9 @@ extern "C" int cf_ms_cuda_execute_batch_async(cf_ms_cuda_resolver *r, const cf_m
             }
             layer_rows[layer].second = at - layer_rows[layer].first;
         }
-        dense = dense && ((reinterpret_cast<uintptr_t>(q_base) | reinterpret_cast<uintptr_t>(o_base)) & 15u) == 0;
+        const uintptr_t q_at = reinterpret_cast<uintptr_t>(q_base), o_at = reinterpret_cast<uintptr_t>(o_base), bytes = 4ull * row_values * total_rows;
+        dense = dense && ((q_at | o_at) & 15u) == 0 && (q_at + bytes <= o_at || o_at + bytes <= q_at) && cfb::on_current_device(q_base) &&
+                cfb::on_current_device(o_base);
         if (!dense) {   // (taken when a batch first needs them)
             r->item_io.ensure(1024, s);
             r->q_dense.ensure(static_cast<size_t>(kMaxBatchTokens) * row_values, s);

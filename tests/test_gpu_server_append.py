@@ -107,3 +107,33 @@ def test_reset_slots_are_reused_without_a_reclaim_call(native):
             free = torch.cuda.mem_get_info()[0]
     assert torch.cuda.mem_get_info()[0] >= free - (4 << 20)
     server.lib.cf_llama_server_runtime_destroy(server.rt, None)
+
+
+@pytest.mark.parametrize("shift", [1, 2, 0])
+def test_outputs_may_overlap_the_queries_of_the_batch(native, shift):
+    """Queries and outputs in one buffer, `shift` rows apart: every query is read before any output is written."""
+    import torch
+    hq, hkv, d, page, layers = 8, 2, 128, 16, 4
+    server = Server(native, hq, hkv, d, page, layers)
+    assert server.lib.cf_llama_server_slot_create(server.rt, i64(1)) == 0
+    for layer in range(layers):
+        k, v = _rows(40, hkv, d, 20 + layer)
+        assert server.append(1, k, v, 0, layer) == 0, server.error()
+    g = torch.Generator(device="cuda")
+    g.manual_seed(6)
+    q = torch.randn((layers, hq, d), generator=g, device="cuda")
+    alone = torch.cat([server.attend(1, q[layer:layer + 1].contiguous(), 40, layer) for layer in range(layers)])
+    room = torch.zeros((layers + shift, hq, d), device="cuda")
+    room[:layers] = q
+    items = (MsBatchItem * layers)()
+    for i, it in enumerate(items):
+        it.sequence_id, it.layer = 1, i
+        it.query = TensorView(room[i].data_ptr(), 3, 1, hq, d, hq * d * 4, d * 4, 4, 0)
+        it.output, it.output_type = room[i + shift].data_ptr(), 3
+        it.output_token_stride_bytes, it.output_head_stride_bytes, it.output_element_stride_bytes = hq * d * 4, d * 4, 4
+        it.query_token_begin, it.softmax_scale, it.causal_window = 40, 1.0 / np.sqrt(d), 0
+    batch = LlamaServerBatch(None, 0, C.cast(items, C.c_void_p), layers)
+    assert server.lib.cf_llama_server_execute_batch_async(server.rt, C.byref(batch), None) == 0, server.error()
+    torch.cuda.synchronize()
+    assert torch.equal(room[shift:], alone)
+    server.lib.cf_llama_server_runtime_destroy(server.rt, None)
