@@ -349,7 +349,17 @@ __device__ __forceinline__ void page_group(Rows<D, NR> &st, const cf_kv_device_p
         }
 }
 
-// One 16-token group of the fp32 tail ([token][kv head][D]; paged_kv_attention.cu:154-166).
+// Largest magnitude of four values and m; NaN wins.
+__device__ __forceinline__ float top4(float m, const float4 &x) {
+    asm("max.NaN.f32 %0, %0, %1, %2;" : "+f"(m) : "f"(fabsf(x.x)), "f"(fabsf(x.y)));
+    asm("max.NaN.f32 %0, %0, %1, %2;" : "+f"(m) : "f"(fabsf(x.z)), "f"(fabsf(x.w)));
+    return m;
+}
+
+// One 16-token group of the fp32 tail ([token][kv head][D]; paged_kv_attention.cu:154-166). Unlike a page's values the tail's are
+// whatever the caller has, and products by value and residue spread NaN and infinities (0 * inf, inf - inf). A group with some among
+// its K takes its scores one by one in fp32; so do four channels of V with some among them their products: they end where fp32
+// arithmetic puts them, and a token that a row does not see adds nothing.
 template <int D, int NR>
 __device__ __forceinline__ void tail_group(Rows<D, NR> &st, const cf_kv_paged_attention_desc &desc, uint32_t kv_head, uint32_t t0, const float *q_rows,
                                            const uint32_t (&qtok)[NR], const uint32_t (&first)[NR], uint32_t lane) {
@@ -374,6 +384,29 @@ __device__ __forceinline__ void tail_group(Rows<D, NR> &st, const cf_kv_paged_at
             mma_3xtf32(s[tile], ah[1], al[1], k.z, k.w);
         }
     }
+    bool odd = false;   // an infinity's residue is NaN, so its token's scores are
+#pragma unroll
+    for (int tile = 0; tile < 2; ++tile)
+#pragma unroll
+        for (int i = 0; i < 2 * NR; ++i) odd = odd || isnan(s[tile][i]);
+    if (__any_sync(0xffffffffu, odd)) {
+#pragma unroll
+        for (int tile = 0; tile < 2; ++tile)
+#pragma unroll
+            for (int c = 0; c < 2; ++c)
+#pragma unroll
+                for (int r = 0; r < NR; ++r) {
+                    const uint32_t tok = t0 + 8u * tile + 2u * t + c;
+                    float dot = 0.0f;
+#pragma unroll 1
+                    for (uint32_t i = 0; i < (tok < count ? D / 4u : 0u); ++i) {   // four channels: (step, lane & 3) of the row's order
+                        const float4 q = *reinterpret_cast<const float4 *>(q_rows + (((i >> 2) * 16u + g + 8u * r) * 4u + (i & 3u)) * 4u);
+                        const float4 k = load4(k0 + tok * stride + (i & 3u) * (D / 4) + 4u * (i >> 2));
+                        dot += (q.x * k.x + q.y * k.y) + (q.z * k.z + q.w * k.w);
+                    }
+                    s[tile][2 * r + c] = dot;
+                }
+    }
 #pragma unroll
     for (int tile = 0; tile < 2; ++tile)
 #pragma unroll
@@ -383,7 +416,9 @@ __device__ __forceinline__ void tail_group(Rows<D, NR> &st, const cf_kv_paged_at
             for (int r = 0; r < NR; ++r)
                 if (!(in_tail < count && token >= first[r] && token <= qtok[r])) s[tile][2 * r + c] = -CUDART_INF_F;
         }
-    const float unit = st.v_unit == 0.0f ? 1.0f : st.v_unit, to_unit = kWeightScale / unit;
+    // The tail comes after the pages and its weights stay in fp32: O goes over to plain units, in which nothing overflows that the
+    // sums themselves do not (in units of pages with tiny scales an ordinary value would).
+    const float unit = fmaxf(st.v_unit, kWeightScale), to_unit = kWeightScale / unit;
     st.softmax(s, unit, [&](int, int) { return to_unit; });
 #pragma unroll 1
     for (int tile = 0; tile < 2; ++tile) {   // k index t = token 2t, t + 4 = token 2t + 1 of the tile
@@ -393,14 +428,35 @@ __device__ __forceinline__ void tail_group(Rows<D, NR> &st, const cf_kv_paged_at
         tf32_split(w1, ah[2], al[2]), tf32_split(w3, ah[3], al[3]);
         const uint32_t tok = t0 + 8u * tile + 2u * t;
         const float *va = v0 + tok * stride + g * (D / 8), *vb = va + stride;
+        odd = false;
 #pragma unroll
         for (int j = 0; j < D / 8; j += 4) {
-            const float4 a = tok < count ? load4(va + j) : make_float4(0.f, 0.f, 0.f, 0.f);
-            const float4 b = tok + 1u < count ? load4(vb + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+            float4 a = tok < count ? load4(va + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+            float4 b = tok + 1u < count ? load4(vb + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+            if (!(top4(top4(0.0f, a), b) < CUDART_INF_F)) a = b = make_float4(0.f, 0.f, 0.f, 0.f), odd = true;
             mma_3xtf32(st.acc[j], ah, al, a.x, b.x);
             mma_3xtf32(st.acc[j + 1], ah, al, a.y, b.y);
             mma_3xtf32(st.acc[j + 2], ah, al, a.z, b.z);
             mma_3xtf32(st.acc[j + 3], ah, al, a.w, b.w);
+        }
+        if (!__any_sync(0xffffffffu, odd)) continue;
+#pragma unroll 1
+        for (uint32_t i = 0; i < 8u; ++i) {   // what was left out above (four channels of two tokens), for the rows and columns whose sums this lane holds
+            const uint32_t at = t0 + 8u * tile + i, pair = at ^ 1u, from = (lane & 28u) | (i >> 1);
+            const float wa = __shfl_sync(0xffffffffu, i & 1u ? w1 : w0, from), wb = __shfl_sync(0xffffffffu, i & 1u ? w3 : w2, from);
+            if (at >= count) continue;
+#pragma unroll
+            for (int c = 0; c < 2; ++c)
+#pragma unroll
+                for (int j = 0; j < D / 8; j += 4) {
+                    const uint32_t channel = (2u * t + c) * (D / 8) + j;
+                    const float4 v = load4(v0 + at * stride + channel);
+                    const float4 other = pair < count ? load4(v0 + pair * stride + channel) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (top4(top4(0.0f, v), other) < CUDART_INF_F) continue;
+                    if (wa != 0.0f) st.acc[j][c] += wa * v.x, st.acc[j + 1][c] += wa * v.y, st.acc[j + 2][c] += wa * v.z, st.acc[j + 3][c] += wa * v.w;
+                    if (NR == 2 && wb != 0.0f)
+                        st.acc[j][2 + c] += wb * v.x, st.acc[j + 1][2 + c] += wb * v.y, st.acc[j + 2][2 + c] += wb * v.z, st.acc[j + 3][2 + c] += wb * v.w;
+                }
         }
     }
 }

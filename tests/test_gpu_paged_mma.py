@@ -107,6 +107,82 @@ def test_paged_attention_on_the_tensor_cores(native, oracle, case):
     assert np.abs(got - want).max() <= 1e-5 * np.abs(want).max(), np.abs(got - want).max() / np.abs(want).max()
 
 
+def _tail_only(native, q, k, v, first, pages=None, sealed=0):
+    """cf_kv_paged_attention_async over an fp32 tail [token][kv head][D] (and pages in front of it), one query head per kv head."""
+    import torch
+    dev = lambda a: torch.from_numpy(np.array(a, copy=True)).cuda()
+    out = torch.full(q.shape, 3.0, device="cuda")
+    d_q, d_k, d_v = dev(q), dev(k), dev(v)
+    desc = PagedAttentionDesc()
+    desc.struct_size, desc.abi_version = C.sizeof(desc), 0
+    if pages:
+        table = dev(np.frombuffer(bytes((DevicePage * len(pages))(*pages)), np.uint8))
+        desc.pages, desc.page_count = table.data_ptr(), len(pages)
+    desc.kv_head_count, desc.query_head_count, desc.gqa_group_size = k.shape[1], q.shape[1], q.shape[1] // k.shape[1]
+    desc.active_k, desc.active_v, desc.active_token_begin, desc.active_token_count = d_k.data_ptr(), d_v.data_ptr(), sealed, k.shape[0]
+    desc.queries, desc.output, desc.query_token_begin, desc.query_count = d_q.data_ptr(), out.data_ptr(), first, q.shape[0]
+    desc.head_dim, desc.softmax_scale = q.shape[2], 1.0 / np.sqrt(q.shape[2])
+    assert native.lib().cf_kv_paged_attention_async(C.byref(desc), None) == 0
+    torch.cuda.synchronize()
+    return out.cpu().numpy()
+
+
+@pytest.mark.parametrize("d,hq,hkv,tokens,nq", [(128, 4, 1, 21, 1), (64, 2, 2, 40, 1), (128, 4, 1, 33, 20), (64, 16, 1, 16, 9)], ids=str)
+def test_infinities_and_nan_in_the_tail_stay_where_fp32_puts_them(native, d, hq, hkv, tokens, nq):
+    rng = np.random.default_rng(d + nq)
+    q = rng.standard_normal((nq, hq, d)).astype(np.float32)
+    k, v = (rng.standard_normal((tokens, hkv, d)).astype(np.float32) for _ in range(2))
+    first, group = tokens - nq, hq // hkv
+    q[..., 5] = np.abs(q[..., 5]) + 0.1
+    k[0, :, 5] = -np.inf                        # a score of -inf: the token weighs nothing
+    v[2, :, 3], v[3, :, 60] = np.inf, -np.inf   # of visible tokens: the channels become infinite, no other does
+    if nq > 1:                                  # tokens that the first rows do not see
+        k[first + 2, :, 7], v[first + 2, :, 11] = np.nan, np.nan
+        v[first + 1, :, 20] = np.inf
+    got = _tail_only(native, q, k, v, first)
+    with np.errstate(invalid="ignore"):
+        for i in range(nq):
+            for h in range(hq):
+                kk, vv = (x[:first + i + 1, h // group].astype(np.float64) for x in (k, v))
+                s = kk @ q[i, h].astype(np.float64) / np.sqrt(d)
+                if np.isnan(s).any():
+                    continue
+                w = np.exp(s - s.max())
+                want = np.where(w[:, None] == 0, 0, w[:, None] * vv).sum(0) / w.sum()
+                finite = np.isfinite(want)
+                assert np.array_equal(np.isnan(want), np.isnan(got[i, h])) and np.array_equal(want[~finite], got[i, h][~finite], equal_nan=True)
+                if finite.any():
+                    assert np.abs(got[i, h] - want)[finite].max() <= 2e-5 * np.abs(want[finite]).max()
+
+
+@pytest.mark.parametrize("scale", [1e-36, 0.0, 1e34])
+def test_a_tail_behind_pages_of_any_scale(native, scale):
+    """V scales far from the tail's magnitudes: neither side of the sum overflows or vanishes."""
+    import torch
+    d, page = 128, 16
+    rng = np.random.default_rng(8)
+    dev = lambda a: torch.from_numpy(np.array(a, copy=True)).cuda()
+    held = [dev(rng.integers(0, 1 << 32, page * d // 4, dtype=np.uint32).view(np.int32)), dev(np.full(d, 1e-3, np.float32)), dev(np.full(page, scale, np.float32)),
+            dev(np.zeros(page * d // 64, np.int32))]
+    pg = DevicePage()
+    pg.k_words = pg.v_words = held[0].data_ptr()
+    pg.k_scales, pg.v_scales = held[1].data_ptr(), held[2].data_ptr()
+    pg.k_block_offsets = pg.v_block_offsets = pg.k_lut = pg.v_lut = held[3].data_ptr()
+    pg.token_count, pg.head_dim, pg.block_size = page, d, 64
+    pg.k_max_code_length = pg.v_max_code_length = pg.fixed_code_length = 8
+    pg.zero_point = 128
+    codes = held[0].cpu().numpy().view(np.uint32)
+    codes = np.stack([(codes >> s) & 255 for s in (24, 16, 8, 0)], 1).reshape(page, d).astype(np.float64) - 128
+    tail = 30
+    q, k, v = (rng.standard_normal((n, 1, d)).astype(np.float32) for n in (1, tail, tail))
+    v *= 1e5 if scale < 1 else 1.0
+    got = _tail_only(native, q, k, v, page + tail - 1, [pg], page)[0, 0]
+    s = np.concatenate([codes * np.float64(np.float32(1e-3)), k[:, 0]]) @ q[0, 0].astype(np.float64) / np.sqrt(d)
+    w = np.exp(s - s.max())
+    want = (w[:, None] * np.concatenate([codes * np.float64(np.float32(scale)), v[:, 0]])).sum(0) / w.sum()
+    assert np.abs(got - want).max() <= 1e-5 * np.abs(want).max()
+
+
 def test_paged_attention_from_several_threads(native):
     """Callers on streams of their own share the slots in which splits leave their partials: every call, whatever its number of
     splits, gives what it gives alone."""
