@@ -623,7 +623,7 @@ __global__ void __launch_bounds__(kThreadsOf<NG, NB, kSplitQ, kDim>, 1) lanes_at
                     if constexpr (!kProbe) {
                     // ---- online softmax for this page (fp32), per group of four heads ----
                     const uint32_t page_token = (page_begin + i) * 16u;
-                    const uint32_t seen_end = min(min(sealed, qpos + 1u), page_token + token_count);   // tokens [first_token, seen_end)
+                    const uint32_t seen_end = min(qpos < sealed ? qpos + 1u : sealed, page_token + token_count);   // tokens [first_token, seen_end)
                     const bool visible = page_token + my_token >= first_token && page_token + my_token < seen_end;
                     float s0[NS], s1[NS];
                     bool higher = false;

@@ -798,7 +798,8 @@ __device__ __forceinline__ void softmax_role(const AttentionParams &p, uint8_t *
                 v_unit = 0.0f;
                 // entries of one sequence see its pages up to their own position; entries of several see every shared page
                 const uint32_t row = min((u.tile_index * kCluster + rank) * 128u + row_in_tile, rows_total - 1u);
-                seen = p.one_slot ? static_cast<int32_t>(__ldcg(&seq_info(p)[row / G].qpos)) + 1 - static_cast<int32_t>(16u * u.page_begin)
+                // (a position may be anything up to 2^32 - 1; pages end below 2^30 tokens)
+                seen = p.one_slot ? static_cast<int32_t>(min(__ldcg(&seq_info(p)[row / G].qpos), 0x3fffffffu)) + 1 - static_cast<int32_t>(16u * u.page_begin)
                                   : 0x40000000;
             }
             tmem_load_wait();

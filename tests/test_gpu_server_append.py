@@ -137,3 +137,19 @@ def test_outputs_may_overlap_the_queries_of_the_batch(native, shift):
     torch.cuda.synchronize()
     assert torch.equal(room[shift:], alone)
     server.lib.cf_llama_server_runtime_destroy(server.rt, None)
+
+
+@pytest.mark.parametrize("rows,position", [(1, 0xffffffff), (8, 3_000_000_000), (40, 0x7fffffe0), (2, 0xfffffffe)])
+def test_positions_far_beyond_the_context_see_all_of_it(native, rows, position):
+    import torch
+    hq, hkv, d, page = 8, 2, 128, 16
+    server = Server(native, hq, hkv, d, page)
+    assert server.lib.cf_llama_server_slot_create(server.rt, i64(1)) == 0
+    k, v = _rows(300, hkv, d, 30)
+    assert server.append(1, k, v, 0) == 0, server.error()
+    g = torch.Generator(device="cuda")
+    g.manual_seed(7)
+    q = torch.randn((rows, hq, d), generator=g, device="cuda")
+    near, far = server.attend(1, q, 300), server.attend(1, q, position)
+    assert torch.equal(near, far)
+    server.lib.cf_llama_server_runtime_destroy(server.rt, None)
