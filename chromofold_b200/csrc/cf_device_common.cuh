@@ -133,7 +133,8 @@ __host__ __device__ inline WorkspaceLayout workspace_layout(uint32_t seq_count, 
     WorkspaceLayout w;
     w.prefix_offset = sizeof(PlanHeader);
     w.info_offset = (w.prefix_offset + 4ull * (seq_count + 1) + 31ull) / 32ull * 32ull;
-    w.partials_offset = (w.info_offset + sizeof(SeqInfo) * seq_count + 255ull) / 256ull * 256ull;
+    // (32 bytes: a layout of coarser alignment would refuse workspaces that were just large enough for one record per slot)
+    w.partials_offset = (w.info_offset + sizeof(SeqInfo) * seq_count + 31ull) / 32ull * 32ull;
     w.partial_stride_floats = head_dim + 2ull;
     w.shared_offset = 0;
     if (shared_prefix) {

@@ -123,3 +123,20 @@ def test_every_c_header_compiles_as_c11():
                               input=f'#include "chromofold_b200/{h}"\nint main(void) {{ return 0; }}\n', text=True,
                               capture_output=True)
         assert done.returncode == 0, f"{h}: {done.stderr[:400]}"
+
+
+def test_workspaces_that_held_one_record_per_partial_are_still_large_enough(native):
+    """The smallest workspace: line positions of every sequence (256-byte aligned), and for each of them a 32-byte record and one
+    partial per query head. No layout of the same contents may ask for more."""
+    lib = native.lib()
+    d = native.SealedAttentionDesc()
+    d.struct_size, d.abi_version = C.sizeof(d), native.ABI_VERSION
+    d.softmax_scale, d.query_type, d.output_type = 0.088, native.F16, native.F32
+    for f in ("queries", "output", "workspace", "seq_sealed_tokens", "k_tables", "v_tables"):
+        setattr(d, f, 0x1000)
+    for kv, group, dim in ((1, 1, 30), (8, 4, 128), (2, 7, 64), (1, 16, 96)):
+        d.kv_head_count, d.query_head_count, d.head_dim, d.page_tokens, d.block_size = kv, kv * group, dim, 16, 64
+        for n in list(range(1, 300)) + [1000, 4095, 4096, 60000]:
+            d.seq_count = n
+            d.workspace_bytes = (64 + 4 * (n + 1) + 255) // 256 * 256 + 32 + n * (4 * (dim + 2) * kv * group + 32)
+            assert lib.cf_b200_sealed_attention_validate(C.byref(d)) == native.CF_OK, (kv, group, dim, n)
