@@ -133,8 +133,11 @@ __host__ __device__ inline WorkspaceLayout workspace_layout(uint32_t seq_count, 
     WorkspaceLayout w;
     w.prefix_offset = sizeof(PlanHeader);
     w.info_offset = (w.prefix_offset + 4ull * (seq_count + 1) + 31ull) / 32ull * 32ull;
-    // (32 bytes: a layout of coarser alignment would refuse workspaces that were just large enough for one record per slot)
-    w.partials_offset = (w.info_offset + sizeof(SeqInfo) * seq_count + 31ull) / 32ull * 32ull;
+    // Partials begin at a 256-byte boundary where that asks for no more room than an aligned prefix and a record per partial would.
+    const uint64_t records_end = w.info_offset + sizeof(SeqInfo) * seq_count;
+    const uint64_t most = (w.prefix_offset + 4ull * (seq_count + 1) + 255ull) / 256ull * 256ull + sizeof(SeqInfo) * (seq_count + 1ull);
+    w.partials_offset = (records_end + 255ull) / 256ull * 256ull;
+    if (w.partials_offset > most) w.partials_offset = most;
     w.partial_stride_floats = head_dim + 2ull;
     w.shared_offset = 0;
     if (shared_prefix) {
