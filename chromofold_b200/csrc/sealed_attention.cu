@@ -69,6 +69,25 @@ __device__ __forceinline__ uint32_t block_scan(uint32_t value, uint32_t *warp_to
     return incl + (warp ? before : 0u);
 }
 
+// A workspace with `room` stretches for more warps than that: an even cut leaves warps idle, because a stretch may need a slot in
+// every sequence it meets. Units of a fixed size inside their sequence need one slot each. Returns their size in pages where they end
+// sooner, 0 where the even cut does: in the built-in workspace (8 MiB) 250 sequences of 1024 tokens on 64 query heads take 485 us in
+// units, 34.5 ms in the three stretches there is room for. Whole block; begin and end are this thread's entries.
+__device__ uint32_t pages_per_unit_in_small_workspace(const SeqInfo *info, uint32_t begin, uint32_t end, uint32_t pages, uint32_t room, uint32_t capacity,
+                                                      uint32_t warps, uint32_t *warp_totals) {
+    uint32_t grain = max((pages + capacity - 1u) / capacity, 1u);
+    for (;; grain += (grain + 3u) / 4u) {   // from one unit per sequence on they fit
+        uint32_t mine = 0, units;
+        for (uint32_t s = begin; s < end; ++s) mine += (info[s].page_end - info[s].first_page + grain - 1u) / grain;
+        block_scan(mine, warp_totals, &units);
+        if (units > capacity) continue;
+        return static_cast<uint64_t>((units + warps - 1u) / warps) * grain < (pages + room - 1u) / room ? grain : 0u;
+    }
+}
+
+// kSmall: the workspace may leave warps without a stretch. (A kernel of its own: the plan is one block whose instructions come from
+// memory, and the few for this case cost a step of one sequence 0.3 us.)
+template <bool kSmall>
 __global__ void __launch_bounds__(kPlanThreads) plan_kernel(AttentionParams p) {
     __shared__ uint32_t warp_totals[kPlanThreads / 32];
     allow_dependent_launch();
@@ -120,23 +139,26 @@ __global__ void __launch_bounds__(kPlanThreads) plan_kernel(AttentionParams p) {
     }
     PageLine line = {};
     line.grain = 1;
-    line.by_position = p.min_pages_per_unit != 0u;
-    uint32_t incl, total;
+    uint32_t incl, total, pages_per_unit = p.min_pages_per_unit;
     const uint32_t capacity = static_cast<uint32_t>(min(p.layout.chunk_capacity, static_cast<uint64_t>(0x7fffffffu)));
-    if (!line.by_position) {
+    if (pages_per_unit == 0u) {
         // One stretch per resident warp for the units of a stretch (kv heads x passes), where there is a page for each and a
         // partial slot: the last slot is stretches * pieces + seq_count - 2. The capacity is at least seq_count.
         incl = block_scan(local, warp_totals, &total);
-        const uint32_t room = capacity - (p.seq_count - 1u);
-        line.stretches = min(min(max(p.plan_warps / p.unit_lanes, 1u), total), room);
+        const uint32_t room = capacity - (p.seq_count - 1u), warps = max(p.plan_warps / p.unit_lanes, 1u);
+        line.stretches = min(min(warps, total), room);
+        if (kSmall && room < min(warps, total)) pages_per_unit = pages_per_unit_in_small_workspace(info, begin, end, total, room, capacity, warps, warp_totals);
         if (line.stretches) {
             line.base = total / line.stretches;
             line.longer = total % line.stretches;
             const uint32_t longest = line.base + (line.longer ? 1u : 0u);
             line.pieces = min(max(min((longest + kPiecePages - 1u) / kPiecePages, room / line.stretches), 1u), line.base);
         }
-    } else {
-        line.grain = p.min_pages_per_unit;
+    }
+    if (pages_per_unit != 0u) {
+        line.by_position = 1u;
+        line.longer = 0u;
+        line.grain = pages_per_unit;
         for (;;) {   // units grow until every one has a slot; from one unit per sequence on they do
             local = 0;
             for (uint32_t s = begin; s < end; ++s) {
@@ -958,7 +980,10 @@ cudaError_t launch_plan(const AttentionParams &p, cudaStream_t stream) {
     const bool verify = p.shared_prefix_pages != 0u && !p.one_slot;
     if (verify) verify_prefix_kernel<<<p.seq_count, 256, 0, stream>>>(p);
     const uint32_t threads = p.seq_count <= 128u ? 128u : kPlanThreads;   // small batches: fewer warps to start and to meet
-    return launch_kernel(plan_kernel, 1, threads, 0, stream, verify, p);
+    const bool small = p.min_pages_per_unit == 0u &&   // fewer stretches than warps and, as far as the host knows, pages
+                       p.layout.chunk_capacity < p.seq_count - 1ull + min(static_cast<uint64_t>(max(p.plan_warps / p.unit_lanes, 1u)),
+                                                                         static_cast<uint64_t>(p.seq_count) * p.page_table_stride);
+    return launch_kernel(small ? plan_kernel<true> : plan_kernel<false>, 1, threads, 0, stream, verify, p);
 }
 
 namespace {

@@ -119,3 +119,27 @@ def test_queries_that_begin_anywhere(native, heads, dim, f32, shift, shared):
     assert layer.device_status() == 0
     ok, err = attention_close(b, a, rel=2e-5, abs_=2e-5)
     assert ok, err
+
+
+@pytest.mark.parametrize("heads,dim,seqs,slots,coder", [((8, 2), 128, 40, 40, "rans4"), ((64, 8), 128, 24, 31, "huffman"), ((14, 2), 64, 300, 420, "rans"),
+                                                        ((4, 4), 48, 30, 33, "rans4"), ((8, 8), 128, 1, 1, "rans4")])
+def test_a_small_workspace_still_gives_every_sequence_a_unit(native, heads, dim, seqs, slots, coder):
+    """Room for `slots` partials per query head, the fewest that are accepted or a few more: the work is cut into no fewer units than
+    there are sequences, and the results are those of an ample workspace."""
+    import torch
+    from chromofold_b200.workloads import build_sealed_layer
+    hq, hkv = heads
+    rng = np.random.default_rng(seqs)
+    layer, _ = build_sealed_layer(16 * rng.integers(8, 60, seqs), query_heads=hq, kv_heads=hkv, head_dim=dim, coder=coder, seed=2)
+    q = torch.from_numpy(rng.standard_normal((seqs, hq, dim)).astype(np.float32)).cuda().half()
+    want = layer.attention(q).cpu().numpy()
+    bytes_ = (64 + 4 * (seqs + 1) + 255) // 256 * 256 + 32 * (seqs + 1) + slots * 4 * (dim + 2) * hq
+    layer.workspace = torch.zeros(bytes_ + 512, dtype=torch.uint8, device="cuda")
+    skip = -layer.workspace.data_ptr() % 256
+    layer.workspace = layer.workspace[skip:skip + bytes_]
+    got = layer.attention(q).cpu().numpy()
+    assert layer.device_status() == 0
+    header = layer.workspace[:28].cpu().numpy().view(np.uint32)      # positions, pages per position, stretches, ...
+    assert min(seqs, 444) <= header[2] and header[2] <= max(slots, seqs)
+    ok, err = attention_close(got, want, rel=2e-5, abs_=2e-5)
+    assert ok, err
