@@ -2,7 +2,7 @@
 // lane-per-block attention kernels read. It writes the same records as seal_pages_kernel (seal.cu), byte for byte.
 //
 // One WARP owns a (page, kv head) and a lane owns whole blocks, from the values to the coded bytes, so there is no barrier
-// anywhere: a K block is 64 consecutive values of a token row (or of two), a V block is four channels of all sixteen tokens.
+// anywhere (two warps, a stream each, where that ends sooner: see kPair): a K block is 64 consecutive values of a token row (or of two), a V block is four channels of all sixteen tokens.
 //   * head_dim 128: 32 blocks per stream, lane l codes K block l and V block l, interleaved (two independent chains);
 //     head_dim 64 and 32: at most 16 per stream, lanes 0..15 code K and lanes 16..31 code V.
 //   * values are loaded coalesced and quantised where they land, with a multiplication and the 1.5 * 2^23 rounding trick; the few whose quotient lies so close to
@@ -276,15 +276,32 @@ __device__ __forceinline__ void move_bytes(const uint8_t *src, uint8_t *dst, uin
 
 struct CursorPlacement {};   // the public entry point: room from the arena cursor, page ids from job_pages
 
-template <int D, bool kF32, class Placement>
+// What the two warps of a page-head tell each other (kPair).
+struct StreamResult {
+    uint32_t bytes, coder, scale_bits, magnitude;
+};
+__device__ __forceinline__ void pair_sync(uint32_t worker) { asm volatile("bar.sync %0, 64;" ::"r"(worker + 1u) : "memory"); }
+
+// kPair: two warps share a page-head, one per stream. A launch with few page-heads lasts as long as one of them, and a warp that
+// loads, quantises and codes both streams takes half as long again as two that take one each. Microseconds at head_dim 128 in
+// nibble-split rANS, binary16 | fp32 (a 128-thread CTA per page-head took 14.3, 16.4, 18.4, 28.7, 43 | 14.4, 16.4, 20.4, 30.7, 45):
+//                          8           512          1184         1600         2960 page-heads
+//   one warp each     18.4 | 17.4  20.5 | 21.4  22.5 | 24.6       | 30.8  30.8 | 34.8
+//   two warps each    12.3 | 12.3  12.3 | 14.3  16.4 | 18.4  22.5 |       28.7 | 36.9
+template <int D, bool kF32, class Placement, bool kPair>
 __global__ void __launch_bounds__(kThreads, 2) seal_blocks_kernel(const __grid_constant__ SealParams p, const __grid_constant__ Placement place) {
     using G = Geo<D>;
-    constexpr int kJobs = G::kJobs;
+    static_assert(!kPair || G::kJobs == 2, "a warp per stream needs blocks for all of its lanes");
+    constexpr int kJobs = kPair ? 1 : G::kJobs, kWorkers = kPair ? kWarps / 2 : kWarps;   // blocks per lane; page-heads at a time
+    constexpr int kScan = G::kJobs == 2 ? 32 : 16;                                         // lanes that hold a stream's blocks
     constexpr bool kPlaced = std::is_same<Placement, SealPlacement>::value;
+    __shared__ StreamResult s_result[kPair ? kWorkers : 1][2];
+    __shared__ unsigned long long s_offset[kPair ? kWorkers : 1];
     extern __shared__ __align__(16) uint8_t smem[];
     uint4 *s_enc = reinterpret_cast<uint4 *>(smem);   // [K | V][256]
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    uint8_t *parts = smem + 2 * 256 * 16 + warp * G::kWarpBytes, *slots = parts + 2 * G::kPart;
+    const uint32_t worker = kPair ? warp >> 1 : warp, role = kPair ? warp & 1u : 0u;   // role: the stream of a pair's warp
+    uint8_t *parts = smem + 2 * 256 * 16 + worker * G::kWarpBytes, *slots = parts + 2 * G::kPart;
     const bool split = split_coder(p.coder), rans = rans_family(p.coder), fixed = p.coder == CF_B200_CODER_FIXED8;
     for (uint32_t i = tid; i < 512u; i += kThreads) {
         s_enc[i] = coder_entry(i < 256u ? p.k_tables : p.v_tables, i & 255u, rans);
@@ -301,16 +318,16 @@ __global__ void __launch_bounds__(kThreads, 2) seal_blocks_kernel(const __grid_c
     bool active[kJobs];
 #pragma unroll
     for (int j = 0; j < kJobs; ++j) {
-        stream[j] = kJobs == 2 ? j : lane >> 4;
-        block[j] = kJobs == 2 ? lane : lane & 15u;
+        stream[j] = kPair ? role : kJobs == 2 ? j : lane >> 4;
+        block[j] = lane & (kScan - 1u);
         active[j] = block[j] < G::kBlocks;
-        slot[j] = slots + (j * 32u + lane) * kSlot;
+        slot[j] = slots + ((kPair ? role : j) * 32u + lane) * kSlot;
         enc[j] = s_enc + 256u * stream[j];
     }
 
     // unit = job * heads + kv head; both move on by fixed steps
-    const uint32_t stride = gridDim.x * kWarps, stride_jobs = stride / heads, stride_heads = stride % heads;
-    const uint32_t first = blockIdx.x * kWarps + warp;
+    const uint32_t stride = gridDim.x * kWorkers, stride_jobs = stride / heads, stride_heads = stride % heads;
+    const uint32_t first = kPair ? worker * gridDim.x + blockIdx.x : blockIdx.x * kWorkers + worker;   // (few: spread over the SMs)
     uint32_t job = first / heads, head_at = first % heads;
     for (; job < p.job_count; job += stride_jobs, head_at += stride_heads, job += head_at >= heads, head_at -= head_at >= heads ? heads : 0u) {
         const uint32_t kv_head = p.job_heads ? p.job_heads[job] : head_at;
@@ -332,15 +349,31 @@ __global__ void __launch_bounds__(kThreads, 2) seal_blocks_kernel(const __grid_c
                 for (uint32_t i = lane; i < 16u * kLines; i += 32u)
                     if (i / kLines < next_rows) {
                         const uint64_t line = (next + (i / kLines) * p.row_stride) * kElem + (i % kLines) * 128u;
-                        asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const uint8_t *>(p.tail_k) + line));
-                        asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const uint8_t *>(p.tail_v) + line));
+                        if (!kPair || role == 0u) asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const uint8_t *>(p.tail_k) + line));
+                        if (!kPair || role == 1u) asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const uint8_t *>(p.tail_v) + line));
                     }
             }
         }
         __syncwarp();   // the previous page's slots and parts have been read
         uint32_t k_mag, v_mag;
         uint16_t k_bits, v_bits;
-        {   // fp32 tiles one after the other: a lane holds 64 values of either
+        if constexpr (kPair) {   // this warp's stream alone; what the other finds comes with its length
+            Quantiser q;
+            auto quantise = [&](auto &tile, const uint8_t *base, uint8_t *to) {
+                tile.load(base, row_bytes, rows, lane);
+                k_mag = v_mag = __reduce_max_sync(0xffffffffu, tile.absmax());
+                k_bits = v_bits = scale_bits_from_absmax(__uint_as_float(k_mag));
+                q.set(k_bits, k_mag);
+                tile.quantise(q, to, lane);
+            };
+            if (role == 0u) {
+                KTile<D, kF32> k;
+                quantise(k, k_base, slots);
+            } else {
+                VTile<D, kF32> v;
+                quantise(v, v_base, slots + 32u * kSlot);
+            }
+        } else {   // fp32 tiles one after the other: a lane holds 64 values of either
             KTile<D, kF32> k;
             VTile<D, kF32> v;
             k.load(k_base, row_bytes, rows, lane);
@@ -356,14 +389,15 @@ __global__ void __launch_bounds__(kThreads, 2) seal_blocks_kernel(const __grid_c
             q.set(v_bits, v_mag);
             v.quantise(q, slots + (kJobs == 2 ? 32u : 16u) * kSlot, lane);
         }
-        if (rows == 0 || k_mag >= 0x7f800000u || v_mag >= 0x7f800000u) {   // finite validation failed: nothing is published
+        if (rows == 0 || (!kPair && (k_mag >= 0x7f800000u || v_mag >= 0x7f800000u))) {   // finite validation failed: nothing is published
             if (lane == 0) {
                 if (!kPlaced && p.status) atomicOr(p.status, CF_B200_DEVSTAT_NONFINITE);
                 if constexpr (kPlaced) place.used[job * heads + head_at] = kSealRefused;
             }
             continue;
         }
-        for (uint32_t i = lane; i < 2u * G::kPart / 16u; i += 32u) reinterpret_cast<uint4 *>(parts)[i] = make_uint4(0u, 0u, 0u, 0u);
+        for (uint32_t i = lane; i < (kPair ? 1u : 2u) * G::kPart / 16u; i += 32u)
+            reinterpret_cast<uint4 *>(parts + role * G::kPart)[i] = make_uint4(0u, 0u, 0u, 0u);
         __syncwarp();
         uint32_t w[kJobs][16], len[kJobs], state[kJobs];
 #pragma unroll
@@ -398,13 +432,13 @@ __global__ void __launch_bounds__(kThreads, 2) seal_blocks_kernel(const __grid_c
             if (!active[j]) len[j] = 0u;
             uint32_t incl = len[j];
 #pragma unroll
-            for (int d = 1; d < (kJobs == 2 ? 32 : 16); d <<= 1) {
-                const uint32_t up = __shfl_up_sync(0xffffffffu, incl, d, kJobs == 2 ? 32 : 16);
+            for (int d = 1; d < kScan; d <<= 1) {
+                const uint32_t up = __shfl_up_sync(0xffffffffu, incl, d, kScan);
                 if (block[j] >= static_cast<uint32_t>(d)) incl += up;
             }
             off[j] = incl - len[j];
-            if constexpr (kJobs == 2) {
-                run[j] = __shfl_sync(0xffffffffu, incl, 31);
+            if constexpr (kScan == 32) {
+                run[kPair ? role : j] = __shfl_sync(0xffffffffu, incl, 31);
             } else {
                 run[0] = __shfl_sync(0xffffffffu, incl, 15);
                 run[1] = __shfl_sync(0xffffffffu, incl, 31);
@@ -417,9 +451,21 @@ __global__ void __launch_bounds__(kThreads, 2) seal_blocks_kernel(const __grid_c
             coder[s] = p.coder;
             if (fixed || bytes[s] > G::kSyms) bytes[s] = G::kSyms, coder[s] = CF_B200_CODER_FIXED8;   // would not shrink
         }
+        if constexpr (kPair) {
+            if (lane == 0) s_result[worker][role] = {role ? bytes[1] : bytes[0], role ? coder[1] : coder[0], k_bits, k_mag};
+            pair_sync(worker);
+            const StreamResult k = s_result[worker][0], v = s_result[worker][1];
+            bytes[0] = k.bytes, bytes[1] = v.bytes, coder[0] = k.coder, coder[1] = v.coder;
+            k_bits = static_cast<uint16_t>(k.scale_bits), v_bits = static_cast<uint16_t>(v.scale_bits);
+            if (k.magnitude >= 0x7f800000u || v.magnitude >= 0x7f800000u) {
+                if (role == 0u && lane == 0 && p.status) atomicOr(p.status, CF_B200_DEVSTAT_NONFINITE);
+                pair_sync(worker);   // both have read the results
+                continue;
+            }
+        }
         const uint32_t k_units = bytes[0] / 16u, units = 1u + k_units + bytes[1] / 16u;
         unsigned long long taken = 0;   // room in the arena: on its way while the parts are put together
-        if (!kPlaced && lane == 0) taken = atomicAdd(p.cursor, static_cast<unsigned long long>(units));
+        if (!kPlaced && role == 0u && lane == 0) taken = atomicAdd(p.cursor, static_cast<unsigned long long>(units));
         __syncwarp();   // (a split stream that falls back overwrites the plane its part already holds)
 #pragma unroll
         for (int j = 0; j < kJobs; ++j) {
@@ -448,16 +494,22 @@ __global__ void __launch_bounds__(kThreads, 2) seal_blocks_kernel(const __grid_c
             page = page_slot * place.tiles_per_page + 1u + tile;
             offset = 1ull + (static_cast<uint64_t>(page_slot) * place.tiles_per_page + tile) * heads * place.record_units + kv_head * place.record_units;
         } else {
-            offset = __shfl_sync(0xffffffffu, taken, 0);
+            if constexpr (kPair) {
+                if (role == 0u && lane == 0) s_offset[worker] = taken;
+                pair_sync(worker);
+                offset = s_offset[worker];
+            } else {
+                offset = __shfl_sync(0xffffffffu, taken, 0);
+            }
             page = p.job_pages[job];
             if (offset + units > p.arena_units) {
-                if (lane == 0 && p.status) atomicOr(p.status, CF_B200_DEVSTAT_ARENA_FULL);
+                if (role == 0u && lane == 0 && p.status) atomicOr(p.status, CF_B200_DEVSTAT_ARENA_FULL);
                 continue;
             }
         }
         __syncwarp();   // the parts are complete
         uint4 *dst = reinterpret_cast<uint4 *>(p.arena + 16ull * offset);
-        if (lane == 0) {
+        if (role == 0u && lane == 0) {
             cf_b200_record_header h;
             h.k_part_units = static_cast<uint16_t>(k_units);
             h.v_part_units = static_cast<uint16_t>(bytes[1] / 16u);
@@ -471,11 +523,12 @@ __global__ void __launch_bounds__(kThreads, 2) seal_blocks_kernel(const __grid_c
             h.version = CF_B200_FORMAT_VERSION;
             dst[0] = *reinterpret_cast<const uint4 *>(&h);
         }
-        for (uint32_t i = lane; i + 1u < units; i += 32u)
+        for (uint32_t i = lane + (kPair && role ? k_units : 0u); i + 1u < (kPair && !role ? 1u + k_units : units); i += 32u)
             dst[1u + i] = *reinterpret_cast<const uint4 *>(i < k_units ? parts + 16u * i : parts + G::kPart + 16u * (i - k_units));
         __threadfence();   // the record is in place before its directory entry is
-        __syncwarp();
-        if (lane == 0) {
+        if constexpr (kPair) pair_sync(worker);
+        else __syncwarp();
+        if (role == 0u && lane == 0) {
             p.page_dir[static_cast<uint64_t>(page) * p.kv_head_count + kv_head] = CF_B200_DIR_ENTRY(offset, units);
             if constexpr (kPlaced) {
                 place.used[job * heads + head_at] = units;
@@ -485,29 +538,50 @@ __global__ void __launch_bounds__(kThreads, 2) seal_blocks_kernel(const __grid_c
     }
 }
 
-template <int D, bool kF32, class Placement>
+template <int D, bool kF32, bool kPair = false, class Placement>
 cudaError_t launch_one(const SealParams &p, const Placement &place, cudaStream_t stream) {
     static LauncherState table[64];
     cudaError_t e;
     LauncherState *state = launcher_state(table, &e);
     if (!state) return e;
     if (!state->configured) {
-        e = cudaFuncSetAttribute(seal_blocks_kernel<D, kF32, Placement>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(Geo<D>::kSmem));
+        e = cudaFuncSetAttribute(seal_blocks_kernel<D, kF32, Placement, kPair>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(Geo<D>::kSmem));
         if (e != cudaSuccess) return e;
         state->configured = true;
     }
     const uint64_t units = static_cast<uint64_t>(p.job_count) * (p.job_heads ? 1u : p.kv_head_count);
-    const uint64_t wanted = (units + kWarps - 1) / kWarps;
+    const uint64_t wanted = kPair ? units : (units + kWarps - 1) / kWarps;
     const uint32_t grid = static_cast<uint32_t>(wanted < 2ull * state->sm_count ? wanted : 2ull * state->sm_count);
-    seal_blocks_kernel<D, kF32, Placement><<<grid, kThreads, Geo<D>::kSmem, stream>>>(p, place);
+    seal_blocks_kernel<D, kF32, Placement, kPair><<<grid, kThreads, Geo<D>::kSmem, stream>>>(p, place);
     return cudaPeekAtLastError();
+}
+
+// Head_dim 128 through the public entry point, where launches of a page are usual: two warps per page-head for binary16 tiles; for fp32
+// tiles, of which a lane holds twice as many registers, as long as all page-heads are resident at once (one warp each
+// beyond that: 34.8 against 36.9 us for 2960, 64.4 against 62.3 for 5920).
+template <bool kF32>
+cudaError_t launch_128(const SealParams &p, const CursorPlacement &place, cudaStream_t stream) {
+    if constexpr (!kF32) {
+        return launch_one<128, false, true>(p, place, stream);
+    } else {
+        static LauncherState table[64];
+        cudaError_t e;
+        LauncherState *state = launcher_state(table, &e);
+        if (!state) return e;
+        const uint64_t units = static_cast<uint64_t>(p.job_count) * (p.job_heads ? 1u : p.kv_head_count);
+        return units <= static_cast<uint64_t>(state->sm_count) * kWarps ? launch_one<128, true, true>(p, place, stream) : launch_one<128, true>(p, place, stream);
+    }
+}
+template <bool kF32>
+cudaError_t launch_128(const SealParams &p, const SealPlacement &place, cudaStream_t stream) {
+    return launch_one<128, kF32>(p, place, stream);
 }
 
 template <class Placement>
 cudaError_t launch_for(const SealParams &p, const Placement &place, cudaStream_t stream) {
     const bool f32 = p.tail_type == CF_B200_F32;
     switch (p.head_dim) {
-        case 128: return f32 ? launch_one<128, true>(p, place, stream) : launch_one<128, false>(p, place, stream);
+        case 128: return f32 ? launch_128<true>(p, place, stream) : launch_128<false>(p, place, stream);
         case 96: return f32 ? launch_one<96, true>(p, place, stream) : launch_one<96, false>(p, place, stream);
         case 80: return f32 ? launch_one<80, true>(p, place, stream) : launch_one<80, false>(p, place, stream);
         case 64: return f32 ? launch_one<64, true>(p, place, stream) : launch_one<64, false>(p, place, stream);

@@ -69,3 +69,56 @@ def test_more_pages_than_warps_and_odd_head_counts(native):
     k, v = layer.decode_pages(np.arange(1, n + 1))
     assert torch.equal(k, (codes[0] + 128).to(torch.uint8).reshape(n, hkv, -1))
     assert torch.equal(v, (codes[1] + 128).to(torch.uint8).transpose(-1, -2).reshape(n, hkv, -1))
+
+
+@pytest.mark.parametrize("coder", range(5))
+@pytest.mark.parametrize("f32", [False, True])
+def test_few_page_heads_and_many_are_sealed_alike(native, coder, f32):
+    """Two warps share a page-head where a launch has few of them: the same records as of a launch with many, refusals (NaN in K or V
+    alone, no rows, no room in the arena) included."""
+    import torch
+    from chromofold_b200.cache import SealedKvLayer
+    from helpers import hist_for_coder, laplace_codes
+    n, hkv, d = 400, 8, 128
+    rng = np.random.default_rng(coder)
+    hist = hist_for_coder(laplace_codes(rng, 1 << 15, 9.0).astype(np.int16) + 128, coder)
+    kinds = ["codes", "noise", "halves", "tiny"]
+    k, v = (np.stack([_values(rng, kinds[i % 4], (hkv, 16, d)) for i in range(n)]) for _ in range(2))
+    k[10, 3, 2, 5], v[11, 0, 15, 127] = np.nan, np.inf
+    rows = rng.integers(1, 17, n)
+    rows[[10, 11]], rows[12] = 16, 0
+    dk, dv = (torch.from_numpy(x if f32 else x.astype(np.float16)).cuda() for x in (k, v))
+    layers = []
+    for step in (n, 29, 1):
+        layer = SealedKvLayer(kv_heads=hkv, query_heads=hkv, head_dim=d, page_tokens=16, block_size=64, coder=coder, max_sequences=1,
+                              max_pages_per_sequence=n, max_pages=n + 1, arena_bytes=n * hkv * 4112 + 4096)
+        layer.set_codebooks(hist, hist)
+        for begin in range(0, n if step > 1 else 40, step):
+            jobs = torch.arange(begin, min(begin + step, n), dtype=torch.int32, device="cuda")
+            desc = layer._seal_desc(jobs, jobs + 1, torch.as_tensor(rows[begin:begin + step], dtype=torch.int32, device="cuda"))
+            desc.tail_k, desc.tail_v, desc.tail_type = dk.data_ptr(), dv.data_ptr(), native.F32 if f32 else native.F16
+            assert native.lib().cf_b200_seal_pages_async(C.byref(desc), None) == 0
+        torch.cuda.synchronize()
+        assert layer.device_status() == native.DEVSTAT_NONFINITE
+        layers.append(layer)
+    directory = [layer.page_dir.cpu().numpy().reshape(-1, hkv) for layer in layers]
+    missing = {(11, 3), (12, 0)} | {(13, h) for h in range(hkv)}
+    for page in list(range(1, 41)) + [57, 399, 400]:
+        for h in range(hkv):
+            there = [bool(x[page, h]) for x in directory[:2]] + [bool(directory[2][page, h])] * (page <= 40)
+            assert all(t == ((page, h) not in missing) for t in there), (page, h)
+            if there[0]:
+                records = [layer.record_bytes(page, h) for layer in layers[:2 + (page <= 40)]]
+                assert all(np.array_equal(records[0], r) for r in records[1:])
+    layer = layers[2]      # room for some of the records of one more launch
+    layer.status.zero_()
+    layer.cursor.fill_(layer.arena_units - 1000)
+    layer.page_dir.zero_()
+    jobs = torch.arange(20, dtype=torch.int32, device="cuda")
+    desc = layer._seal_desc(jobs, jobs + 1, torch.full((20,), 16, dtype=torch.int32, device="cuda"))
+    desc.tail_k, desc.tail_v, desc.tail_type = dk.data_ptr(), dv.data_ptr(), native.F32 if f32 else native.F16
+    assert native.lib().cf_b200_seal_pages_async(C.byref(desc), None) == 0
+    torch.cuda.synchronize()
+    assert layer.device_status() & native.DEVSTAT_ARENA_FULL
+    entries = layer.page_dir.cpu().numpy()
+    assert 0 < np.count_nonzero(entries) < 20 * hkv
