@@ -32,15 +32,20 @@ inline __attribute__((always_inline)) uint32_t pass(float *dst, const float *src
     return top;
 }
 
+#if defined(__x86_64__) || defined(__i386__)
 __attribute__((target("avx2"))) uint32_t copy_avx2(float *dst, const float *src, size_t n) { return pass<true>(dst, src, n); }
 __attribute__((target("avx2"))) uint32_t look_avx2(float *dst, const float *src, size_t n) { return pass<false>(dst, src, n); }
-uint32_t copy_any(float *dst, const float *src, size_t n) { return pass<true>(dst, src, n); }
-uint32_t look_any(float *dst, const float *src, size_t n) { return pass<false>(dst, src, n); }
-
 bool has_avx2() {
     static const bool yes = __builtin_cpu_supports("avx2") != 0;
     return yes;
 }
+#else   // (a GPU beside Arm cores: what the compiler assumes everywhere there is four values wide already)
+uint32_t copy_avx2(float *, const float *, size_t) { return 0; }
+uint32_t look_avx2(float *, const float *, size_t) { return 0; }
+constexpr bool has_avx2() { return false; }
+#endif
+uint32_t copy_any(float *dst, const float *src, size_t n) { return pass<true>(dst, src, n); }
+uint32_t look_any(float *dst, const float *src, size_t n) { return pass<false>(dst, src, n); }
 
 }  // namespace
 
