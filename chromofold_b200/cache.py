@@ -45,6 +45,11 @@ def _on_own_device(method):
 
 
 _DESC_BYTES = C.sizeof(N.SealedAttentionDesc)
+# _attention_desc gives these by position, the quickest way: they have to be the struct's first fields in this order
+_DESC_HEAD = ("struct_size", "abi_version", "kv_head_count", "query_head_count", "head_dim", "page_tokens", "block_size", "kv_head_begin",
+              "kv_head_span", "codebook_id", "arena", "page_dir", "page_table", "seq_sealed_tokens", "seq_slots", "page_table_stride",
+              "seq_count", "k_tables", "v_tables", "tail_k", "tail_v", "tail_tokens")
+assert tuple(field[0] for field in N.SealedAttentionDesc._fields_[:len(_DESC_HEAD)]) == _DESC_HEAD
 
 
 class SealedKvLayer:

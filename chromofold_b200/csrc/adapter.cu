@@ -1008,7 +1008,7 @@ extern "C" int cf_llama_kv_attention(cf_llama_kv_adapter *adapter, uint32_t laye
         d.softmax_scale = softmax_scale;
         d.causal_window = causal_window;
         // Prefill (llama.cpp evaluates a prompt in batches of query tokens): they share the layer's sealed records, which the
-        // shared-prefix kernel then decodes once per 128 query rows instead of once per query token, masking what the
+        // shared-prefix kernel then decodes once per 256 query rows instead of once per query token, masking what the
         // earlier tokens must not see. Given where it pays and the workspace has or can get the room.
         if (query_count >= 4 && causal_window == 0) {
             const uint32_t tiles = std::min(h0.sealed / adapter->tile_tokens, (query_token_begin + query_count - 1u) / adapter->tile_tokens + 1u);

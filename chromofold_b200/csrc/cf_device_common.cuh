@@ -173,8 +173,8 @@ inline LauncherState *launcher_state(LauncherState (&table)[64], cudaError_t *er
     return state;
 }
 
-// Partial slots a launch over at most total_pages pages can need: with the library's own cut one per stretch (a warp of the 148 x
-// 24 resident ones, for one kv head of the span), per kPiecePages pages and per sequence; with the caller's one per unit.
+// Partial slots a launch over at most total_pages pages can need (asked without a device at hand, so for a whole B200; with fewer slots
+// the cut is coarser): with the library's own cut one per stretch (a warp of the 148 x 24 resident ones, for one kv head of the span), per kPiecePages pages and per sequence; with the caller's one per unit.
 __host__ __device__ inline uint64_t partial_slots_for(uint64_t total_pages, uint32_t seq_count, uint32_t kv_head_span, uint32_t min_pages_per_unit) {
     if (min_pages_per_unit) return total_pages / min_pages_per_unit + seq_count + 1ull;   // each sequence may round up once
     const uint64_t warps = 148ull * 24ull / (kv_head_span ? kv_head_span : 1u) + 1ull;

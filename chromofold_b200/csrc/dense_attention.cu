@@ -284,6 +284,11 @@ extern "C" cf_status cf_b200_dense_attention_async(const cf_b200_dense_attention
     p.pool_k = static_cast<const __half *>(d->pool_k);
     p.pool_v = static_cast<const __half *>(d->pool_v);
     if (p.layout.chunk_capacity < d->seq_count) return CF_ERR_INVALID_ARGUMENT;
+    static cfb::LauncherState table[64];
+    cudaError_t e;
+    const cfb::LauncherState *state = cfb::launcher_state(table, &e);
+    if (!state) return CF_ERR_CUDA;
+    p.sm_count = static_cast<uint32_t>(state->sm_count);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (cfb::launch_plan(p, s) != cudaSuccess) return CF_ERR_CUDA;
     if (cfb::launch_dense_attention(p, s) != cudaSuccess) return CF_ERR_CUDA;

@@ -314,7 +314,7 @@ void core_attention(Core &c, uint32_t layer, const void *q, uint32_t q_type, flo
     d.output_type = CF_B200_F32;
     d.softmax_scale = softmax_scale;
     d.causal_window = window;
-    // Prefill: the query tokens of one call share the layer's sealed records, which are decoded once per 128 query rows by
+    // Prefill: the query tokens of one call share the layer's sealed records, which are decoded once per 256 query rows by
     // the shared-prefix kernel instead of once per query token: all of them up to the last token's position, the kernel masks
     // what the earlier tokens must not see. Given where it pays and where the workspace has or can get room for the extra partials.
     if (count >= 4 && window == 0) {

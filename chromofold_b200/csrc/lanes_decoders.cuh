@@ -130,13 +130,7 @@ struct RansLaneT {
     __device__ __forceinline__ uint32_t symbol(int) {
         uint32_t e;
         asm volatile("ld.shared.u32 %0, [%1];" : "=r"(e) : "r"(imad(x & (CF_B200_RANS_M - 1u), 4u, table)));
-#ifdef CFB_RANS_MADHI
-        uint32_t t;
-        asm("mad.hi.u32 %0, %1, %2, %3;" : "=r"(t) : "r"(x), "r"(1u << (32 - CF_B200_RANS_PROB_BITS)), "r"(0u - CF_B200_RANS_M));
-        x = imad(e >> 20, t, e >> 8);
-#else
         x = imad(e >> 20, imad(x >> CF_B200_RANS_PROB_BITS, 1u, 0u - CF_B200_RANS_M), e >> 8);
-#endif
         const uint32_t shift = imad(static_cast<uint32_t>(__clz(x)), 1u, 0xffffffffu) & 24u;
         x = __funnelshift_l(__byte_perm(w0, w1, sel), x, shift);
         sel = imad(shift, 0x1110u / 8u, sel);

@@ -990,7 +990,7 @@ extern "C" int cf_ms_cuda_copy_sequence_async(cf_ms_cuda_resolver *r, int64_t so
 
 // Sealed records that every row of a layer's batch shares: sequences forked from one prompt reference the same pages
 // (copy shares pages by reference), and the query tokens of one prefill item all see the item's sealed history. Such
-// records are decoded once per 128 query rows by the shared-prefix kernel instead of once per row; the number returned
+// records are decoded once per 256 query rows by the shared-prefix kernel instead of once per row; the number returned
 // here is only a hint, the plan kernel checks it against the page tables. 0 = not worth it or not applicable.
 static uint32_t shared_leading_tiles(cf_ms_cuda_resolver *r, const cf_ms_batch_item *items, uint32_t item_count, uint32_t layer,
                                      uint32_t rows, uint32_t window, bool *one_sequence) {

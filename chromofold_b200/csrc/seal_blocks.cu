@@ -13,9 +13,10 @@
 //   * block lengths become offsets with a warp scan, a lane moves its bytes into the part word by word (the words it shares
 //     with a neighbour by atomicOr), the part leaves for the arena with 16-byte stores.
 // Bound: the latency of a warp's own chain (table look-ups, one page's loads and stores) with 20 warps per SM to hide it: 3500
-// warp instructions per page-head, issue slots 45 % busy. 2048 pages x 8 kv heads of binary16 tiles per launch, before (a
-// 128-thread CTA per page-head, two of its warps coding and two waiting) -> now: nibble-split rANS 178 -> 125 us,
-// nibble-split Huffman 180 -> 137, rANS 278 -> 178, Huffman 253 -> 186, fixed 8-bit 127 -> 85.
+// warp instructions per page-head, issue slots 45 % busy (one warp per page-head). 2048 pages x 8 kv heads of binary16 tiles per
+// launch, a 128-thread CTA per page-head, two of its warps coding and two waiting -> one warp -> two: nibble-split rANS 178 ->
+// 133 -> 113 us, nibble-split Huffman 180 -> 140 -> 115, rANS 279 -> 176 -> 158, Huffman 253 -> 190 -> 168, fixed 8-bit 127 ->
+// 90 -> 66.
 
 #include <type_traits>
 

@@ -29,7 +29,7 @@ constexpr uint32_t kGenericMaxGroup = 16;
 //
 // Bound by the chain of dependent loads slot -> counts -> record, once per entry, and a block scan; the kernels behind it set
 // themselves up meanwhile (see launch_kernel). It used to write a record per unit of pages as well and to try 32 unit sizes:
-// 5.2 us for one sequence and 9.4 us for 64, against 3.5 and 4.3 us now.
+// 5.2 us for one sequence and 9.4 us for 64, against 3.5 and 3.4 us now (alone on the GPU, start-up included).
 // ---------------------------------------------------------------------------------------------------------------
 
 // Shared-prefix hint, part one: block s compares the first `shared_prefix_pages` ids of entry s's page-table row with the
@@ -382,9 +382,11 @@ __global__ void __launch_bounds__(kGenericThreads) generic_attention_kernel(Atte
 // tail is done before this kernel waits for the attention kernel. Everything the plan kernel wrote may be read before that wait:
 // the attention kernel lets this one start only after it has seen the plan's end itself.
 //
-// Every sum has an order of its own that the shape of the CTA does not change, so that a row's result depends on nothing
-// but the row: partials are added up in 32 consecutive strands, each relative to its own maximum, and the strands in
-// order; tail tokens in eight interleaved strands.
+// Every sum of combine_kernel has an order of its own that the shape of the CTA does not change, so that its forms agree to the bit for
+// given partials: they are added up in 32 consecutive strands, each relative to its own maximum, and the strands in order; tail
+// tokens in eight interleaved strands. Which pages a partial covers follows the batch (an even cut of its whole line; a caller's
+// min_pages_per_unit keeps the cut to the sequence), and combine_tile_kernel, which large prompts take, adds in another
+// order: the last bits of a row can differ with the batch it is in.
 // ---------------------------------------------------------------------------------------------------------------
 constexpr uint32_t kStrands = 32;
 
@@ -1016,20 +1018,20 @@ cudaError_t launch_combine_as(const AttentionParams &p, cudaStream_t stream, boo
 // Four rows per CTA where that still makes about a CTA per SM, or where a CTA per row would not find room for all at once, else one; 32 where all entries are query tokens of one sequence
 // (the caller says so), their tail is worth sharing and its rows can be read 16 bytes at a time.
 cudaError_t launch_combine(const AttentionParams &p, cudaStream_t stream, bool dependent) {
-    constexpr uint32_t kEnoughCtas = 120;
+    const uint32_t sms = p.sm_count, enough_ctas = sms * 13u / 16u;   // 120 of 148
     const uint32_t G = p.group, C = p.tail_capacity;
     const uint32_t tiles = (p.seq_count + kTileRows / G - 1u) / (kTileRows / G) * p.kv_head_span;
     const bool by_16 = p.tail_type == CF_B200_F32 && p.head_dim % 4u == 0u &&
                        ((reinterpret_cast<uintptr_t>(p.tail_k) | reinterpret_cast<uintptr_t>(p.tail_v)) & 15u) == 0u;
-    if (p.one_slot && C > 16u && by_16 && tiles >= kEnoughCtas / 2u && combine_tile_smem(C) <= kCombineSmemMax) {
+    if (p.one_slot && C > 16u && by_16 && tiles >= enough_ctas / 2u && combine_tile_smem(C) <= kCombineSmemMax) {
         static std::atomic<uint64_t> configured{0};
         const cudaError_t e = allow_shared_memory(combine_tile_kernel, configured);
         if (e != cudaSuccess) return e;
         return launch_kernel(combine_tile_kernel, dim3(tiles / p.kv_head_span, p.kv_head_span), kTileThreads, combine_tile_smem(C), stream, dependent, p);
     }
     const uint32_t fours = p.seq_count * p.kv_head_span * ((G + 3u) / 4u);
-    if ((fours >= kEnoughCtas || p.seq_count * p.kv_head_span * G > 2u * 148u) && CombineSmem<4, 512>::bytes(C) <= kCombineSmemMax / 2u)
-        return fours <= 2u * 148u ? launch_combine_as<4, 512>(p, stream, dependent) : launch_combine_as<4, 128>(p, stream, dependent);
+    if ((fours >= enough_ctas || p.seq_count * p.kv_head_span * G > 2u * sms) && CombineSmem<4, 512>::bytes(C) <= kCombineSmemMax / 2u)
+        return fours <= 2u * sms ? launch_combine_as<4, 512>(p, stream, dependent) : launch_combine_as<4, 128>(p, stream, dependent);
     return launch_combine_as<1, 1024>(p, stream, dependent);
 }
 

@@ -1,12 +1,12 @@
-// sealed_attention_lanes.cu — the hot kernel: decode-step attention over sealed pages for the geometry
-// head_dim 128, page_tokens 16, block_size 64 (32 blocks per stream). Query groups larger than 4 heads per kv head are
-// served four heads at a time (the unit is then decoded once per sub-group). Blocks of 128 and 256 symbols (16 and 8
-// blocks per stream) run the same kernel behind a staging step, see stage_blocks below.
+// sealed_attention_lanes.cu — the hot kernel: decode-step attention over sealed pages of 16 tokens. What follows describes head_dim
+// 128 with blocks of 64 symbols (32 per stream); larger blocks, and head_dim 96, 80, 64 and 32, run the same kernel behind a
+// staging step, see stage_blocks below. One decode serves up to eight query heads of a kv head; a larger group takes
+// several passes, each with a decode of its own.
 //
 // What it computes is what src/cuda/paged_kv_attention.cu:183-276 computes for one query token; how it runs is new:
 //
 //   * One WARP owns one (stretch of the page line, kv head) unit. A page record arrives in shared memory as ONE bulk async copy
-//     (cp.async.bulk + mbarrier), double buffered per warp. Coding tables (rANS slot table, Huffman LUT) are loaded
+//     (cp.async.bulk + mbarrier); a warp has one place for it, free again once the record is decoded. Coding tables (rANS slot table, Huffman LUT) are loaded
 //     once per CTA. No thread ever reads page bytes from global memory directly.
 //   * Lane l decodes block l of the K stream and block l of the V stream, interleaved so that the two independent
 //     decoder chains overlap. Symbols never leave registers: four symbols are packed into one register, turned

@@ -114,12 +114,12 @@ typedef struct cf_b200_sealed_attention_desc {
     const uint32_t *query_positions;
     /* Shared prefix: the caller states that the first shared_prefix_pages entries of the page-table row of EVERY
      * listed sequence name the same pages (one sealed copy referenced by all, src/multisequence_cache.cpp:235-292).
-     * Such pages are then decoded once per 128 query rows instead of once per sequence, and the contraction with all
+     * Such pages are then decoded once per 256 query rows instead of once per sequence, and the contraction with all
      * the rows that share them runs on the tensor cores. Entries that name the SAME slot with different
      * query_positions (multi-query / prefill attention) share all of that slot's sealed pages this way. It is a
      * hint: the plan kernel checks the rows and that every entry's query position lies at or after the last shared
-     * token; if not, or the geometry is not the lanes kernel's, or causal_window is in use, every page is handled
-     * per entry as if the field were 0 (a failed check also raises CF_B200_DEVSTAT_PREFIX_MISMATCH).
+     * token; if not, or the geometry is not the lanes kernel's at head_dim 128 or 64, or causal_window is in use,
+     * or `queries` does not begin at a multiple of 16 bytes, every page is handled per entry as if the field were 0 (a failed check also raises CF_B200_DEVSTAT_PREFIX_MISMATCH).
      * The workspace must have been sized with the field set (cf_b200_sealed_attention_workspace_bytes). */
     uint32_t shared_prefix_pages;
     uint32_t reserved0;
