@@ -111,8 +111,8 @@ flat_rans_decode_kernel(const uint8_t *data, const int32_t *byte_off, const uint
                     b.advance();
                 }
             }
-            tile[lane * kTileWords + q] = pack_low_bytes(ea[0], ea[1], ea[2], ea[3]);
-            tile[(32u + lane) * kTileWords + q] = pack_low_bytes(eb[0], eb[1], eb[2], eb[3]);
+            tile[lane * kTileWords + q] = RansLane::pack(ea[0], ea[1], ea[2], ea[3]);
+            tile[(32u + lane) * kTileWords + q] = RansLane::pack(eb[0], eb[1], eb[2], eb[3]);
         }
         __syncwarp();
         // block r of the group: 64 symbols = two coalesced stores of 32 int32

@@ -79,11 +79,6 @@ __device__ __forceinline__ uint32_t imad(uint32_t a, uint32_t b, uint32_t c) {
     return r;
 }
 
-// The low bytes of four table entries as one register, first symbol in byte 0: three byte permutes.
-__device__ __forceinline__ uint32_t pack_low_bytes(uint32_t e0, uint32_t e1, uint32_t e2, uint32_t e3) {
-    return __byte_perm(__byte_perm(e0, e1, 0x0040), __byte_perm(e2, e3, 0x0040), 0x5410);
-}
-
 __device__ __forceinline__ uint32_t lds_u32(uint32_t address) {
     uint32_t w;
     asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w) : "r"(address));
@@ -136,6 +131,15 @@ struct RansLaneT {
         sel = imad(shift, 0x1110u / 8u, sel);
         return e;
     }
+    // The symbols of four entries as one register, first in byte 0.
+    static __device__ __forceinline__ uint32_t pack(uint32_t e0, uint32_t e1, uint32_t e2, uint32_t e3) {
+        return __byte_perm(__byte_perm(e0, e1, 0x0040), __byte_perm(e2, e3, 0x0040), 0x5410);
+    }
+    // Two pair symbols A:B as the high nibbles of four bytes, (A0, B0, A1, B1) from byte 0; the low nibbles are anything.
+    static __device__ __forceinline__ uint32_t high_nibbles(uint32_t e0, uint32_t e1) {
+        const uint32_t t = __byte_perm(e0, e1, 0x4400);             // A0:B0 A0:B0 A1:B1 A1:B1
+        return __byte_perm(t, imad(t, 16u, 0u), 0x7250);            // bytes 1 and 3 of t * 16 start with B
+    }
     // At most three bytes of w0 were used before two symbols, so at most seven of the eight are now: every byte a step looks
     // at was in w0 or w1.
     __device__ __forceinline__ void advance() {
@@ -153,18 +157,16 @@ struct RansLaneT {
         advance();
         const uint32_t e2 = symbol(0), e3 = symbol(1);
         advance();
-        return pack_low_bytes(e0, e1, e2, e3);
+        return pack(e0, e1, e2, e3);
     }
 };
 using RansLane = RansLaneT<32>;
 
 // Low nibbles of the four symbols of a quad (in the low nibble of each byte of w; its high nibbles are ignored) under
-// the two pair symbols that hold their high nibbles (table entries, pair A:B in the low byte): four symbols, first in byte 0.
+// the two pair symbols of decoder Lane that hold their high nibbles (table entries e0, e1): four symbols, first in byte 0.
+template <class Lane>
 __device__ __forceinline__ uint32_t merge_split_quad(uint32_t e0, uint32_t e1, uint32_t w) {
-    const uint32_t t = __byte_perm(e0, e1, 0x4400);             // (s1, s1, s0, s0), s = A:B
-    const uint32_t t4 = imad(t, 16u, 0u);                       // bytes 1 and 3 now start with B
-    const uint32_t h = __byte_perm(t, t4, 0x7250);              // (B1:*, A1:*, B0:*, A0:*)
-    return (h & 0xf0f0f0f0u) | (w & 0x0f0f0f0fu);
+    return (Lane::high_nibbles(e0, e1) & 0xf0f0f0f0u) | (w & 0x0f0f0f0fu);
 }
 
 // Nibble-split rANS (CF_B200_CODER_RANS_SPLIT4): the low nibble of every symbol is stored raw in a lane-interleaved
@@ -189,7 +191,7 @@ struct RansSplitLaneT : RansLaneT<NB> {
     __device__ __forceinline__ uint32_t quad(int q) {   // one stream on its own (mixed-coder records)
         const uint32_t e0 = Base::symbol(0), e1 = Base::symbol(1);
         Base::advance();
-        return merge_split_quad(e0, e1, lo_word(q >> 1) >> (4 * (q & 1)));
+        return merge_split_quad<Base>(e0, e1, lo_word(q >> 1) >> (4 * (q & 1)));
     }
 };
 using RansSplitLane = RansSplitLaneT<32>;
@@ -198,7 +200,8 @@ template <int NB>
 struct HuffLaneT {
     static constexpr bool kWholeQuads = false;
     static constexpr uint32_t kHead = (2u * NB + 3u) / 4u * 4u;   // u16 bit_off[NB]
-    uint32_t w0, w1, off;   // the stream word that holds the next bit, the one after it, bits of w0 used
+    uint32_t w0, w1;        // the stream word that holds the next bit, and the one after it
+    uint32_t off;           // bits of w0 used, in the low byte; above it the sum of the symbols, which nothing looks at
     uint32_t view;          // the next bits, top aligned: 32 of them at an even symbol, what it left of them at the odd one
     uint32_t next;          // shared-memory byte address of the word after w1
     uint32_t table;
@@ -216,20 +219,28 @@ struct HuffLaneT {
         open_at(smem_addr(part) + kHead, min(static_cast<uint32_t>(reinterpret_cast<const uint16_t *>(part)[lane]), payload_bits), lut);
     }
     // include/chromofold/detail/block_huffman_device.cuh:12-19: the next 12 bits, MSB-first, index the LUT. A code takes at
-    // most 12 bits, so 32 bits serve two of them.
+    // most 12 bits, so 32 bits serve two of them. The shared-memory LUT holds len | sym << 8: funnel shifts look at the low five
+    // bits of their distance, so an entry is one as it is, and at most 31 + 24 bits are in the low byte of `off` before advance().
+    // (With the length taken out first, a step had one shift more: 32 sequences of 8192 tokens 399 -> 395 us.)
     __device__ __forceinline__ uint32_t symbol(int odd) {
         if (!odd) view = __funnelshift_l(w1, w0, off);
         uint32_t e;
         asm volatile("ld.shared.u16 %0, [%1];" : "=r"(e) : "r"(imad(view >> (32u - CF_B200_HUFF_MAXLEN), 2u, table)));
-        const uint32_t len = e >> 8;
-        if (!odd) view <<= len;
-        off = imad(len, 1u, off);
+        if (!odd) view = __funnelshift_l(0u, view, e);
+        off = imad(e, 1u, off);
         return e;
+    }
+    static __device__ __forceinline__ uint32_t pack(uint32_t e0, uint32_t e1, uint32_t e2, uint32_t e3) {
+        return __byte_perm(__byte_perm(e0, e1, 0x0051), __byte_perm(e2, e3, 0x0051), 0x5410);
+    }
+    static __device__ __forceinline__ uint32_t high_nibbles(uint32_t e0, uint32_t e1) {   // as of RansLaneT
+        const uint32_t t = __byte_perm(e0, e1, 0x5511);
+        return __byte_perm(t, imad(t, 16u, 0u), 0x7250);
     }
     __device__ __forceinline__ void advance() {
         asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "setp.ge.u32 p, %3, 32;\n\t"
+            "{\n\t.reg .pred p;\n\t.reg .u32 t;\n\t"
+            "and.b32 t, %3, 32;\n\tsetp.ne.u32 p, t, 0;\n\t"
             "@p mov.u32 %0, %1;\n\t"
             "@p ld.shared.u32 %1, [%2];\n\t"
             "@p mad.lo.u32 %2, %2, 1, 4;\n\t"
@@ -241,7 +252,7 @@ struct HuffLaneT {
         advance();
         const uint32_t e2 = symbol(0), e3 = symbol(1);
         advance();
-        return pack_low_bytes(e0, e1, e2, e3);
+        return pack(e0, e1, e2, e3);
     }
 };
 using HuffLane = HuffLaneT<32>;
@@ -263,7 +274,7 @@ struct HuffSplitLaneT : HuffLaneT<NB> {
     __device__ __forceinline__ uint32_t quad(int q) {
         const uint32_t e0 = Base::symbol(0), e1 = Base::symbol(1);
         Base::advance();
-        return merge_split_quad(e0, e1, lo_word(q >> 1) >> (4 * (q & 1)));
+        return merge_split_quad<Base>(e0, e1, lo_word(q >> 1) >> (4 * (q & 1)));
     }
 };
 using HuffSplitLane = HuffSplitLaneT<32>;
@@ -282,7 +293,8 @@ struct FixedLaneT {
 using FixedLane = FixedLaneT<32>;
 
 // Coding tables into shared memory, once per CTA: [k rANS slots | v rANS slots | k Huffman LUT | v Huffman LUT].
-// Slot entries are re-packed for RansLane::symbol(): sym | (slot - cum) << 8 | freq << 20. All of a thread's loads are issued
+// Slot entries are re-packed for RansLane::symbol(): sym | (slot - cum) << 8 | freq << 20; LUT entries for HuffLane::symbol(): len |
+// sym << 8. All of a thread's loads are issued
 // before the first store: a launch that reads a page per warp would otherwise spend a third of its time here, one L2
 // latency after the other.
 template <uint32_t kThreads>
@@ -304,6 +316,7 @@ __device__ __forceinline__ void load_tables(uint8_t *smem, const AttentionParams
     for (uint32_t j = 0; j < kEach; ++j) {
         const uint32_t i = tid + j * kThreads;
         if (i < 2048u) w[j] = make_uint4(repack(w[j].x), repack(w[j].y), repack(w[j].z), repack(w[j].w));
+        else w[j] = make_uint4(__byte_perm(w[j].x, 0u, 0x2301), __byte_perm(w[j].y, 0u, 0x2301), __byte_perm(w[j].z, 0u, 0x2301), __byte_perm(w[j].w, 0u, 0x2301));
         if (i < kWords) dst[i] = w[j];
     }
 }

@@ -139,13 +139,13 @@ __device__ __forceinline__ void decode_fused(KLane &k, VLane &v, UnitState<NG> &
                 if ((i & 3) == 3) {
                     const int q = kEach * pass + (i >> 2);
                     if constexpr (kMode == kFold) {
-                        u.vq[0] ^= pack_low_bytes(ve[0], ve[1], ve[2], ve[3]) ^ pack_low_bytes(ke[0], ke[1], ke[2], ke[3]);
+                        u.vq[0] ^= VLane::pack(ve[0], ve[1], ve[2], ve[3]) ^ KLane::pack(ke[0], ke[1], ke[2], ke[3]);
                     } else if constexpr (kMode == kDump) {
-                        u.dump[q] = pack_low_bytes(ke[0], ke[1], ke[2], ke[3]);
-                        u.dump[512 + q] = pack_low_bytes(ve[0], ve[1], ve[2], ve[3]);
+                        u.dump[q] = KLane::pack(ke[0], ke[1], ke[2], ke[3]);
+                        u.dump[512 + q] = VLane::pack(ve[0], ve[1], ve[2], ve[3]);
                     } else {
-                        u.vq[16 - kEach + (i >> 2)] = pack_low_bytes(ve[0], ve[1], ve[2], ve[3]);
-                        score_quad(u, qs, q, pack_low_bytes(ke[0], ke[1], ke[2], ke[3]));
+                        u.vq[16 - kEach + (i >> 2)] = VLane::pack(ve[0], ve[1], ve[2], ve[3]);
+                        score_quad(u, qs, q, KLane::pack(ke[0], ke[1], ke[2], ke[3]));
                     }
                 }
             }
@@ -172,7 +172,7 @@ __device__ __forceinline__ void decode_fused_split(Lane &k, Lane &v, UnitState<N
                 kw >>= 4;
                 vw >>= 4;
             }
-            const uint32_t kq = merge_split_quad(ke[0], ke[1], kw), vq = merge_split_quad(ve[0], ve[1], vw);
+            const uint32_t kq = merge_split_quad<Lane>(ke[0], ke[1], kw), vq = merge_split_quad<Lane>(ve[0], ve[1], vw);
             if constexpr (kMode == kFold) {
                 u.vq[0] ^= kq ^ vq;
             } else if constexpr (kMode == kDump) {

@@ -240,8 +240,8 @@ __device__ __forceinline__ void decode_page(KLane &k, VLane &v, uint32_t (&kq)[1
                 k.advance();
                 v.advance();
                 const int j = 2 * pass + ((q - 12) >> 1), shift = 4 * (q & 1);
-                kq[q] = merge_split_quad(ke[0], ke[1], k.lo_word(j) >> shift);
-                vq[q] = merge_split_quad(ve[0], ve[1], v.lo_word(j) >> shift);
+                kq[q] = merge_split_quad<KLane>(ke[0], ke[1], k.lo_word(j) >> shift);
+                vq[q] = merge_split_quad<VLane>(ve[0], ve[1], v.lo_word(j) >> shift);
             } else if constexpr (KLane::kWholeQuads || VLane::kWholeQuads) {   // fixed width: a quad per call
                 kq[q] = k.quad(4 * pass + (q - 12));
                 vq[q] = v.quad(4 * pass + (q - 12));
@@ -256,8 +256,8 @@ __device__ __forceinline__ void decode_page(KLane &k, VLane &v, uint32_t (&kq)[1
                         v.advance();
                     }
                 }
-                kq[q] = pack_low_bytes(ke[0], ke[1], ke[2], ke[3]);
-                vq[q] = pack_low_bytes(ve[0], ve[1], ve[2], ve[3]);
+                kq[q] = KLane::pack(ke[0], ke[1], ke[2], ke[3]);
+                vq[q] = VLane::pack(ve[0], ve[1], ve[2], ve[3]);
             }
         }
     }
