@@ -11,7 +11,7 @@
 //   * Lane l decodes block l of the K stream and block l of the V stream, interleaved so that the two independent
 //     decoder chains overlap. Symbols never leave registers: four symbols are packed into one register, turned
 //     into two fp16 pairs with byte permutes (bias 1024, exact), and fed straight into mma.sync fragments.
-//       K block l = token l/2, channels 64*(l&1)..+63  -> A operand of S = K * Q^T   (16 mma per page)
+//       K block l = token l/2, channels 64*(l&1)..+63  -> B operand of S = Q * K^T   (16 mma per page)
 //       V block l = channels 4l..4l+3, all 16 tokens   -> B operand of O^T = P' * V  (16 mma per page)
 //     The query group is the other operand, laid out with zeros so that every lane's private slice of the
 //     contraction lands in its own output column/row. Tensor cores do the whole contraction for the group;
@@ -49,10 +49,11 @@ template <int NG, int NB, bool kSplitQ, int kDim> constexpr int kThreadsOf = kWa
 // every token).
 template <int NG, int kDim = 128>
 struct UnitState {
-    float score[NG][4];      // S fragments of the current page
+    static constexpr int kPairs = (NG + 1) / 2;   // of groups, one mma each
+    float score[kPairs][4];  // S fragments of the current page: the even group of a pair in rows 0..7, the odd one in rows 8..15
     float acc[NG][(kDim + 31) / 32][4];   // O fragments: [group][channel of the lane's V block][fragment register]
     uint32_t vq[4 * ((kDim + 31) / 32)];   // V symbols of the current page, [channel*4 + token quad]
-    float m0[NG], m1[NG], l0[NG], l1[NG];  // running max / partial sum of the lane's two heads of each group
+    float m[NG], l[NG];      // running max / the lane's part of the running sum, of its head of each group
     uint32_t *dump;          // kDump only: where this lane's quads of the current record go (K at +0, V at +512 words)
 };
 
@@ -62,34 +63,33 @@ constexpr int kAttend = 0, kFold = 1, kDump = 2;
 // The softmax weights go to the tensor cores as binary16 (value + rounding residue) scaled by this power of two.
 constexpr float kWeightScale = 32768.0f;
 
-// Where a lane finds its B fragments of S = K * Q^T (column n = parity*4 + head; zero where the lane's slice of the
-// contraction belongs to the other token of the pair): the query rows of up to eight heads sit in the warp's shared memory as
-// [head][half][64 channels] with a row stride of 36 words, which puts the eight rows one load touches into different banks; a
-// lane reads two words of row (head g&3 of the group, half t&1), or of a zero row when the column is not its own. (Held in
-// registers instead, a group of four heads took 32 of them, and with that room for eight warps more per SM.)
+// Where a lane finds its A fragments of S = Q * K^T (row = parity of the token * 4 + head, eight rows further for the odd group of
+// a pair; zero where the lane's slice of the contraction belongs to the other token): the query rows of a pair of groups sit in
+// the warp's shared memory as [head][half] rows of [quad of channels]{even: channels 0, 1 | odd: 0, 1 | even: 2, 3 | odd: 2, 3},
+// one 16-byte load per quad and pair, 16 bytes of padding a row, which puts the rows that eight lanes touch into different banks; a
+// lane whose row is not its own reads zeros, from the banks that the other lanes of its eight leave alone. (Four binary16 heads have
+// no odd group: their rows hold channels only, eight bytes a load.)
+// With the codes as B operand one mma serves a pair of groups, where K * Q^T took one for each of them and two zero registers.
 struct QSmem {
-    uint32_t addr, group_stride;  // byte address of the lane's row for group 0; distance to the row for group 1 (0 on the zero row)
-    template <int GRP>
-    __device__ __forceinline__ void get(int q, uint32_t &b0, uint32_t &b1) const {
-        asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(b0), "=r"(b1) : "r"(addr + GRP * group_stride + 8u * q));
+    uint32_t addr, pair_stride;  // byte address of the lane's row for pair 0; distance to the row for pair 1 (0 on the zero row)
+    template <int NG, int PAIR>
+    __device__ __forceinline__ void get(int q, uint32_t (&a)[4]) const {
+        if constexpr (NG == 1) {
+            a[1] = a[3] = 0u;
+            asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(a[0]), "=r"(a[2]) : "r"(addr + 8u * q));
+        } else asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3]) : "r"(addr + PAIR * pair_stride + 16u * q));
     }
 };
 
 template <int NG, int kDim, class QSrc>
 __device__ __forceinline__ void score_quad(UnitState<NG, kDim> &u, const QSrc &qs, int q, uint32_t kq) {
-    uint32_t lo, hi, b0, b1;
+    uint32_t lo, hi, a[4];
     quad_to_half2(kq, lo, hi);
-    qs.template get<0>(q, b0, b1);
-    mma_16816(u.score[0], lo, 0u, hi, 0u, b0, b1);
-    if constexpr (NG >= 2) {
-        qs.template get<1>(q, b0, b1);
-        mma_16816(u.score[1], lo, 0u, hi, 0u, b0, b1);
-    }
+    qs.template get<NG, 0>(q, a);
+    mma_16816(u.score[0], a[0], a[1], a[2], a[3], lo, hi);
     if constexpr (NG == 4) {
-        qs.template get<2>(q, b0, b1);
-        mma_16816(u.score[2], lo, 0u, hi, 0u, b0, b1);
-        qs.template get<3>(q, b0, b1);
-        mma_16816(u.score[3], lo, 0u, hi, 0u, b0, b1);
+        qs.template get<NG, 1>(q, a);
+        mma_16816(u.score[1], a[0], a[1], a[2], a[3], lo, hi);
     }
 }
 
@@ -274,20 +274,22 @@ __device__ __forceinline__ void stage_blocks(const uint8_t *part, uint32_t part_
 // Shared memory of one warp: one record, the softmax scratch, an mbarrier and the query rows. A record is decoded before anything
 // else happens to its page, so its place is free for the next one while the scores and weights are worked out; a second place
 // would cost eight warps per SM.
-//   scratch: P rows fp16 high halves [4 NG][16] | low halves [4 NG][16] | 128 zero bytes
+//   scratch: P rows fp16 high halves [4 NG][16] | low halves [4 NG][16]
 template <int NG, int NB, bool kSplitQ, int kDim>
 struct WarpLayout {
     static constexpr uint32_t kStage = kDim == 128 ? kStageBytes : 16u + 32u * kDim + 48u;   // header, two streams, read-ahead
     static constexpr uint32_t kPRows = kStage;
     static constexpr uint32_t kPBytes = 4 * kHeadGroups<NG, kSplitQ> * 16 * 2;
     static constexpr uint32_t kPLo = kPRows + kPBytes;
-    static constexpr uint32_t kZero = kPLo + kPBytes;
-    static constexpr uint32_t kBar = kZero + 128;
+    static constexpr uint32_t kBar = kPLo + kPBytes;
     static constexpr uint32_t kQRows = kBar + 16;
-    static constexpr uint32_t kQRowWords = kDim / 4 + (kDim == 80 ? 8 : 4);
-    static constexpr uint32_t kTile = (kQRows + 8 * NG * kQRowWords * 4 + 15u) / 16u * 16u;   // NB != 32 only
+    static constexpr uint32_t kQRowWords = NG == 1 ? kDim / 4 + (kDim == 80 ? 8 : 4) : kDim / 2 + 4;
+    static constexpr uint32_t kQPairBytes = 8 * kQRowWords * 4;
+    static constexpr uint32_t kTile = kQRows + (NG + 1) / 2 * kQPairBytes;   // NB != 32 only
     static constexpr uint32_t kBytes = kTile + (NB != 32 ? kTileBytesOf<kDim> : 0u);
-    static constexpr uint32_t kSmem = kTableBytes + kWarpsOf<NG, NB, kSplitQ, kDim> * kBytes;
+    static constexpr uint32_t kZeroBytes = 2 * 128 + 128;   // the CTA's zero row, after the tables
+    static constexpr uint32_t kSmem = kTableBytes + kZeroBytes + kWarpsOf<NG, NB, kSplitQ, kDim> * kBytes;
+    static_assert(kBytes % 16 == 0 && kQRows % 16 == 0, "16-byte loads");
     static_assert(kSmem <= 232448, "a CTA has 227 KB of shared memory");
 };
 
@@ -313,10 +315,10 @@ __global__ void __launch_bounds__(kThreadsOf<NG, NB, kSplitQ, kDim>, 1) lanes_at
     uint16_t *v_lut = k_lut + 4096;
 
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    uint8_t *warp_mem = smem + kTableBytes + warp * L::kBytes;
+    uint8_t *warp_mem = smem + kTableBytes + L::kZeroBytes + warp * L::kBytes;
     __half *p_rows = reinterpret_cast<__half *>(warp_mem + L::kPRows);         // [4 NS][16] fp16(p)
     __half *p_rows_lo = reinterpret_cast<__half *>(warp_mem + L::kPLo);        // [4 NS][16] fp16(p - fp16(p))
-    const __half *zero_row = reinterpret_cast<const __half *>(warp_mem + L::kZero);
+    const __half *zero_row = reinterpret_cast<const __half *>(smem + kTableBytes);   // what inactive lanes read their fragments from
     uint64_t *bar = reinterpret_cast<uint64_t *>(warp_mem + L::kBar);
     uint32_t *q_rows = reinterpret_cast<uint32_t *>(warp_mem + L::kQRows);
 
@@ -326,7 +328,7 @@ __global__ void __launch_bounds__(kThreadsOf<NG, NB, kSplitQ, kDim>, 1) lanes_at
         return;
     }
     load_tables<kThreadsOf<NG, NB, kSplitQ, kDim>>(smem, p, tid);   // coding tables: once per CTA
-    reinterpret_cast<uint32_t *>(warp_mem + L::kZero)[lane] = 0u;   // the zero row inactive lanes read their fragments from
+    if (tid < L::kZeroBytes / 4u) reinterpret_cast<uint32_t *>(smem + kTableBytes)[tid] = 0u;
     if (lane == 0) {
         mbar_init(bar, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -342,11 +344,9 @@ __global__ void __launch_bounds__(kThreadsOf<NG, NB, kSplitQ, kDim>, 1) lanes_at
     uint32_t phase = 0u;   // parity the next wait on the record's barrier expects
 
     // fixed lane roles
-    const uint32_t q_head_of_col = g & 3u;                 // S columns: n = parity*4 + head
-    const bool q_col_mine = (t >> 1) == (g >> 2);
-    const uint32_t my_token = 2u * g + (t >> 1);           // S fragment: row g, this lane's token
-    const uint32_t my_head0 = 2u * (t & 1u);               // S fragment: this lane's two heads (of each group)
-    const uint32_t o_head = g & 3u;                        // O fragments: all of this lane's outputs are one head per group
+    const bool q_row_mine = (t >> 1) == (g >> 2);          // S rows: parity of the token * 4 + head
+    const uint32_t my_token = 4u * t + (g >> 2);           // S fragment: this lane's tokens are this one and the second after it,
+    const uint32_t o_head = g & 3u;                        // its head (of each group) this one, and that of all its O fragments
     const bool row_lo_mine = t == (g >> 2), row_hi_mine = t == (g >> 2) + 2u;   // P rows with lane tag t
 
     // A unit is a stretch of the page line for one kv head (and one pass over its query group). The library's own cut makes at most
@@ -422,8 +422,10 @@ __global__ void __launch_bounds__(kThreadsOf<NG, NB, kSplitQ, kDim>, 1) lanes_at
                 const __half2 hi = __floats2half2_rn(x.x, x.y);
                 const float2 back = __half22float2(hi);
                 const __half2 lo = __floats2half2_rn(x.x - back.x, x.y - back.y);
-                q_rows[(i / kRowWords) * L::kQRowWords + i % kRowWords] = *reinterpret_cast<const uint32_t *>(&hi);
-                q_rows[(i / kRowWords + 8u * NS) * L::kQRowWords + i % kRowWords] = *reinterpret_cast<const uint32_t *>(&lo);
+                // four heads: value and residue are the groups of the one pair; eight: a pair of values, a pair of residues
+                uint32_t *row = q_rows + (i / kRowWords % 8u) * L::kQRowWords + (i % kRowWords) * 2u;
+                row[NS == 1 ? 0u : i / (8u * kRowWords)] = *reinterpret_cast<const uint32_t *>(&hi);
+                row[NS == 1 ? 1u : i / (8u * kRowWords) + L::kQPairBytes / 4u] = *reinterpret_cast<const uint32_t *>(&lo);
             }
             __syncwarp();
         } else {
@@ -432,12 +434,15 @@ __global__ void __launch_bounds__(kThreadsOf<NG, NB, kSplitQ, kDim>, 1) lanes_at
 #pragma unroll
             for (int j = 0; j < NG * kDim / 16; ++j) {   // 4 NG heads x kDim / 2 words; row = head*2 + half
                 const uint32_t i = lane + 32u * j, head = i / (2u * kRowWords);
-                q_rows[(i / kRowWords) * L::kQRowWords + i % kRowWords] = head < G ? qsrc[i] : 0u;
+                uint32_t *row = q_rows + (i / kRowWords % 8u) * L::kQRowWords + (i % kRowWords) * (NG == 1 ? 1u : 2u);
+                row[i / (8u * kRowWords)] = head < G ? qsrc[i] : 0u;
             }
         }
         __syncwarp();
-        qs.addr = q_col_mine ? smem_addr(q_rows + (q_head_of_col * 2u + (t & 1u)) * L::kQRowWords) : smem_addr(zero_row);
-        qs.group_stride = q_col_mine ? 8u * L::kQRowWords * 4u : 0u;
+        const uint32_t own = smem_addr(q_rows + (o_head * 2u + (t & 1u)) * L::kQRowWords);
+        // 16 banks of the rows of heads 0 and 1, which the lanes of eight that read zeros stay out of, or of heads 2 and 3
+        qs.addr = q_row_mine ? own : smem_addr(zero_row) + ((smem_addr(q_rows) - smem_addr(zero_row) + ((o_head & 2u) ? 0u : 64u)) & 112u);
+        qs.pair_stride = q_row_mine ? L::kQPairBytes : 0u;
 
         UnitState<NG, kDim> u;
         if constexpr (kProbe) u.vq[0] = 0u;
@@ -448,8 +453,8 @@ __global__ void __launch_bounds__(kThreadsOf<NG, NB, kSplitQ, kDim>, 1) lanes_at
             for (int a = 0; a < kVCh; ++a)
 #pragma unroll
                 for (int b = 0; b < 4; ++b) u.acc[n][a][b] = 0.0f;
-            u.m0[n] = u.m1[n] = -CUDART_INF_F;
-            u.l0[n] = u.l1[n] = 0.0f;
+            u.m[n] = -CUDART_INF_F;
+            u.l[n] = 0.0f;
         }
         // O is kept in units of a power of two at or above every V scale met so far; a page's scale relative to it rides on the
         // weights, together with kWeightScale. v_gain = kWeightScale / unit.
@@ -502,7 +507,7 @@ __global__ void __launch_bounds__(kThreadsOf<NG, NB, kSplitQ, kDim>, 1) lanes_at
                                           (p.softmax_scale * kLog2e);
                     const float v_scale = __half2float(__ushort_as_half(static_cast<unsigned short>(hv.z >> 16)));
 #pragma unroll
-                    for (int n = 0; n < NG; ++n) u.score[n][0] = u.score[n][1] = u.score[n][2] = u.score[n][3] = 0.0f;
+                    for (int n = 0; n < u.kPairs; ++n) u.score[n][0] = u.score[n][1] = u.score[n][2] = u.score[n][3] = 0.0f;
 
                     if constexpr (NB != 32) {
                         uint8_t *tile = warp_mem + L::kTile;
@@ -614,43 +619,36 @@ __global__ void __launch_bounds__(kThreadsOf<NG, NB, kSplitQ, kDim>, 1) lanes_at
                         if (i + 1 < n_pages) issue(entry_next);
                         next_issued = true;
                     }
-                    if constexpr (kSplitQ) {   // K q = K binary16(q) + K residue
-#pragma unroll
-                        for (int n = 0; n < NS; ++n)
-#pragma unroll
-                            for (int c = 0; c < 4; ++c) u.score[n][c] += u.score[n + NS][c];
-                    }
                     if constexpr (!kProbe) {
                     // ---- online softmax for this page (fp32), per group of four heads ----
                     const uint32_t page_token = (page_begin + i) * 16u;
                     const uint32_t seen_end = min(qpos < sealed ? qpos + 1u : sealed, page_token + token_count);   // tokens [first_token, seen_end)
-                    const bool visible = page_token + my_token >= first_token && page_token + my_token < seen_end;
+                    const bool visible0 = page_token + my_token >= first_token && page_token + my_token < seen_end;
+                    const bool visible1 = page_token + my_token + 2u >= first_token && page_token + my_token + 2u < seen_end;
                     float s0[NS], s1[NS];
                     bool higher = false;
 #pragma unroll
                     for (int n = 0; n < NS; ++n) {
-                        s0[n] = visible ? u.score[n][0] * k_scale : -CUDART_INF_F;
-                        s1[n] = visible ? u.score[n][1] * k_scale : -CUDART_INF_F;
-                        higher = higher || s0[n] > u.m0[n] || s1[n] > u.m1[n];
+                        s0[n] = u.score[0][2 * n], s1[n] = u.score[0][2 * n + 1];
+                        if constexpr (kSplitQ) {   // q k = binary16(q) k + residue k
+                            s0[n] += NS == 1 ? u.score[0][2] : u.score[u.kPairs - 1][2 * n];
+                            s1[n] += NS == 1 ? u.score[0][3] : u.score[u.kPairs - 1][2 * n + 1];
+                        }
+                        s0[n] = visible0 ? s0[n] * k_scale : -CUDART_INF_F;
+                        s1[n] = visible1 ? s1[n] * k_scale : -CUDART_INF_F;
+                        higher = higher || s0[n] > u.m[n] || s1[n] > u.m[n];
                     }
                     // The maximum moves on few pages (about one in n after n pages of a head): only then is it worked out, and O rescaled.
                     if (__any_sync(0xffffffffu, higher)) {
 #pragma unroll
                         for (int n = 0; n < NS; ++n) {
-                            float r0 = s0[n], r1 = s1[n];
-#pragma unroll
-                            for (int o = 2; o <= 16; o <<= 1) {  // lanes that hold the same two heads
-                                r0 = fmaxf(r0, __shfl_xor_sync(0xffffffffu, r0, o));
-                                r1 = fmaxf(r1, __shfl_xor_sync(0xffffffffu, r1, o));
-                            }
-                            const float n0 = fmaxf(u.m0[n], r0), n1 = fmaxf(u.m1[n], r1);
-                            const float a0 = n0 == -CUDART_INF_F ? 0.0f : exp2f(u.m0[n] - n0), a1 = n1 == -CUDART_INF_F ? 0.0f : exp2f(u.m1[n] - n1);
-                            u.l0[n] *= a0;
-                            u.l1[n] *= a1;
-                            u.m0[n] = n0;
-                            u.m1[n] = n1;
-                            const float b0 = __shfl_sync(0xffffffffu, a0, o_head >> 1), b1 = __shfl_sync(0xffffffffu, a1, o_head >> 1);
-                            const float alpha = (o_head & 1u) ? b1 : b0;
+                            float top = fmaxf(s0[n], s1[n]);
+                            top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1));   // over the lanes of the same head
+                            top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 2));
+                            top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 16));
+                            const float raised = fmaxf(u.m[n], top), alpha = raised == -CUDART_INF_F ? 0.0f : exp2f(u.m[n] - raised);
+                            u.l[n] *= alpha;
+                            u.m[n] = raised;
 #pragma unroll
                             for (int dd = 0; dd < kVCh; ++dd)
 #pragma unroll
@@ -674,20 +672,19 @@ __global__ void __launch_bounds__(kThreadsOf<NG, NB, kSplitQ, kDim>, 1) lanes_at
                     __syncwarp();  // the previous page's readers of the scratch are done
 #pragma unroll
                     for (int n = 0; n < NS; ++n) {
-                        const float p0 = visible ? exp2f(s0[n] - u.m0[n]) : 0.0f, p1 = visible ? exp2f(s1[n] - u.m1[n]) : 0.0f;
-                        u.l0[n] += p0;
-                        u.l1[n] += p1;
+                        const float p0 = visible0 ? exp2f(s0[n] - u.m[n]) : 0.0f, p1 = visible1 ? exp2f(s1[n] - u.m[n]) : 0.0f;
+                        u.l[n] += p0 + p1;
                         // P goes to the tensor cores as fp16; the rounding residue is fed as a second operand so that
                         // P V is accurate to fp32 level whatever the magnitude of V
                         // The weights (at most 1) are scaled by 2^15 on the way, O by 2^-15 at the partial's end, both exact:
                         // binary16 then resolves weights down to 2^-40 of the row maximum instead of 2^-25.
-                        const uint32_t h0 = 4u * n + my_head0;
+                        const uint32_t at = (4u * n + o_head) * 16u + my_token;
                         const float w0 = p0 * weight_scale, w1 = p1 * weight_scale;
                         const __half p0h = __float2half_rn(w0), p1h = __float2half_rn(w1);
-                        p_rows[h0 * 16u + my_token] = p0h;
-                        p_rows[(h0 + 1u) * 16u + my_token] = p1h;
-                        p_rows_lo[h0 * 16u + my_token] = __float2half_rn(w0 - __half2float(p0h));
-                        p_rows_lo[(h0 + 1u) * 16u + my_token] = __float2half_rn(w1 - __half2float(p1h));
+                        p_rows[at] = p0h;
+                        p_rows[at + 2u] = p1h;
+                        p_rows_lo[at] = __float2half_rn(w0 - __half2float(p0h));
+                        p_rows_lo[at + 2u] = __float2half_rn(w1 - __half2float(p1h));
                     }
                     __syncwarp();
                     // P rows as A fragments. Rows g / g+8 of the fragment belong to lane tags g>>2 / (g>>2)+2; a lane
@@ -749,24 +746,14 @@ __global__ void __launch_bounds__(kThreadsOf<NG, NB, kSplitQ, kDim>, 1) lanes_at
         } else {
 #pragma unroll
         for (int n = 0; n < NS; ++n) {
-            float l0 = u.l0[n], l1 = u.l1[n];
-#pragma unroll
-            for (int o = 2; o <= 16; o <<= 1) {
-                l0 += __shfl_xor_sync(0xffffffffu, l0, o);
-                l1 += __shfl_xor_sync(0xffffffffu, l1, o);
-            }
-            const uint32_t h0 = 4u * n + my_head0;
-            if (g == 0 && t < 2) {
-                if (h0 < G) {
-                    float *dst = partial_ptr(p, partial, out_head_base + h0);
-                    dst[0] = u.m0[n];
-                    dst[1] = l0;
-                }
-                if (h0 + 1u < G) {
-                    float *dst = partial_ptr(p, partial, out_head_base + h0 + 1u);
-                    dst[0] = u.m1[n];
-                    dst[1] = l1;
-                }
+            float sum = u.l[n];
+            sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+            sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+            sum += __shfl_xor_sync(0xffffffffu, sum, 16);
+            if (t == 0 && g < 4u && 4u * n + g < G) {
+                float *dst = partial_ptr(p, partial, out_head_base + 4u * n + g);
+                dst[0] = u.m[n];
+                dst[1] = sum;
             }
             if (4u * n + o_head < G) {
                 float *dst = partial_ptr(p, partial, out_head_base + 4u * n + o_head) + 2;
