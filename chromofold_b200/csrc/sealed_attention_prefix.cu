@@ -838,7 +838,11 @@ __device__ __forceinline__ void softmax_role(const AttentionParams &p, uint8_t *
 #pragma unroll
         for (uint32_t pg = 0; pg < kRoundPages; ++pg)
             if (__float_as_uint(meta[4 * pg + 2]) != 0u) round_scale = fmaxf(round_scale, meta[4 * pg + 1]);
-        const float m_new = fmaxf(m_run, fmaxf(row_max[row_in_tile], row_max[128u + row_in_tile]));
+        // The maximum that the weights are relative to follows the true one only when that has risen by 0.9 in the exponent of two:
+        // a weight is then at most 2^0.9, 2^15.9 scaled, which binary16 holds, and O is rescaled on few rounds (every second
+        // one of the first hundred met a higher maximum in one of a warp's 32 rows: 582 -> 560 us for 500 rows after 16384 tokens).
+        float m_new = fmaxf(m_run, fmaxf(row_max[row_in_tile], row_max[128u + row_in_tile]));
+        if (m_new - m_run < 0.9f) m_new = m_run;
         const float z = m_new == -CUDART_INF_F ? 0.0f : m_new;
         const float alpha = fast_exp2(m_run - z);   // m_run = -inf gives 0
         m_run = m_new;
@@ -857,7 +861,7 @@ __device__ __forceinline__ void softmax_role(const AttentionParams &p, uint8_t *
             const uint32_t pg = 4u * half + q;
             const uint32_t count = seen_of(pg, __float_as_uint(meta[4 * pg + 2]));
             const float ks = meta[4 * pg];
-            // the weights (at most 1) also carry 2^15, exactly, which O sheds at the unit's end: binary16 then resolves
+            // the weights (at most 2^0.9) also carry 2^15, exactly, which O sheds at the unit's end: binary16 then resolves
             // weights down to 2^-40 of the row maximum instead of 2^-25
             const float ratio = count ? __fdividef(meta[4 * pg + 1], v_unit) * kWeightScale : 0.0f;
             uint32_t hi[8], lo[8];
