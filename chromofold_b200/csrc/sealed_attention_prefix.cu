@@ -35,7 +35,10 @@
 // Tensor memory (512 columns): scores and weights of even rounds 0..127, of odd rounds 128..255 (P 64 columns of binary16 pairs, then
 // its residue), O 256..383, Q 384..447, Q residue 448..511 (fp32 queries only: the row is split into binary16(q) and its
 // rounding residue, S = Q K^T + Q residue K^T). Row = lane. B tiles use the no-swizzle K-major canonical layout: 8 rows x 16
-// bytes core matrices, element (row r, 16-byte chunk c) at (r % 8) * 16 + (r / 8) * 2048 + c * 128 bytes.
+// bytes core matrices, element (row r, 16-byte chunk c) at (r % 8) * 16 + (r / 8) * 2048 + c * 128 bytes in the K tile and at
+// (r % 8) * 16 + (r / 8) * 128 + c * 2048 in the V tile: a page (16 rows of K, two chunks of V) is then 4096 bytes in a row in
+// either, which a pair's CTA sends to the other one by bulk copies. (Stored there 16 bytes at a time, a page took its warp 4000 of
+// the 22000 clocks between two pages, and the tensor core waited for it: a round took 8950 clocks.)
 // Head_dim 64 runs the same kernel on the left half of the K tile and the upper half of the V tile.
 // The page's V scale relative to the largest one met so far in the unit rides on P (never above 1, so the binary16
 // weights cannot overflow); O is kept in units of that scale and rescaled when a larger one arrives.
@@ -89,20 +92,21 @@ static_assert(kLaunchRegs * kTcThreads <= 65536 && kDecoderRegs % 8 == 0 && kSof
 constexpr uint32_t kIdescS = (1u << 4) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
 template <int kDim> constexpr uint32_t kIdescO = (1u << 4) | ((static_cast<uint32_t>(kDim) >> 3) << 17) | ((128u >> 4) << 24);
 
-__device__ __forceinline__ uint32_t tile_offset(uint32_t row, uint32_t chunk) {
-    return (row & 7u) * 16u + (row >> 3) * 2048u + chunk * 128u;
-}
+__device__ __forceinline__ uint32_t k_tile_offset(uint32_t row, uint32_t chunk) { return (row & 7u) * 16u + (row >> 3) * 2048u + chunk * 128u; }
+__device__ __forceinline__ uint32_t v_tile_offset(uint32_t row, uint32_t chunk) { return (row & 7u) * 16u + (row >> 3) * 128u + chunk * 2048u; }
 // Row of the V tile (= column of O) that holds channel 4 * lane + c, the c-th channel of the block lane decodes: the 32
 // lanes of one store spread over all 8 rows of a core matrix, so a 16-byte store per lane meets no bank conflict.
 // Inverse: column n of O is channel 4 * ((n & 7) + 8 * (n >> 5)) + ((n >> 3) & 3).
 __device__ __forceinline__ uint32_t v_tile_row(uint32_t lane, uint32_t c) {
     return (lane & 7u) + 8u * c + 32u * (lane >> 3);
 }
-// shared-memory matrix descriptor: start address, leading (K) offset 128 B, stride (row group) offset 2048 B, version 1
-__device__ __forceinline__ uint64_t tile_desc(uint32_t smem_address) {
-    return static_cast<uint64_t>((smem_address >> 4) & 0x3fffu) | (static_cast<uint64_t>(128u >> 4) << 16) |
-           (static_cast<uint64_t>(2048u >> 4) << 32) | (1ull << 46);
+// shared-memory matrix descriptor: start address, leading (K) offset, stride (row group) offset, version 1
+__device__ __forceinline__ uint64_t tile_desc(uint32_t smem_address, uint32_t chunk_stride, uint32_t group_stride) {
+    return static_cast<uint64_t>((smem_address >> 4) & 0x3fffu) | (static_cast<uint64_t>(chunk_stride >> 4) << 16) |
+           (static_cast<uint64_t>(group_stride >> 4) << 32) | (1ull << 46);
 }
+__device__ __forceinline__ uint64_t k_desc(uint32_t k_tile, uint32_t step) { return tile_desc(k_tile + 256u * step, 128u, 2048u); }     // 16 channels
+__device__ __forceinline__ uint64_t v_desc(uint32_t v_tile, uint32_t step) { return tile_desc(v_tile + 4096u * step, 2048u, 128u); }   // 16 tokens
 // D[tmem_d] (+)= A[tmem_a: 128 lanes x 8 columns of binary16 pairs] x B[shared-memory tile]^T, one K step of 16
 __device__ __forceinline__ void umma(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t accumulate, uint32_t idesc) {
     asm volatile(
@@ -130,6 +134,15 @@ __device__ __forceinline__ void store_peer(uint32_t address, uint4 v) {
 }
 __device__ __forceinline__ void mbar_arrive_peer(uint32_t address) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(address) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive_expect_peer(uint32_t address, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.release.cluster.shared::cluster.b64 _, [%0], %1;" ::"r"(address), "r"(bytes) : "memory");
+}
+// Shared memory of this CTA to the other one's, counted by a barrier there.
+__device__ __forceinline__ void copy_to_peer(uint32_t to, uint32_t from, uint32_t bytes, uint32_t peer_bar) {
+    asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(to), "r"(from), "r"(bytes),
+                 "r"(peer_bar)
+                 : "memory");
 }
 __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -199,11 +212,7 @@ __device__ __forceinline__ void tmem_store32(uint32_t taddr, const uint32_t (&v)
         "r"(v[31])
         : "memory");
 }
-template <int kCluster>
-__device__ __forceinline__ void fence_async_smem() {
-    if constexpr (kCluster == 1) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    else asm volatile("fence.proxy.async;" ::: "memory");
-}
+__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
@@ -270,25 +279,19 @@ __device__ __forceinline__ void decode_stream(Lane &s, uint32_t (&quads)[16]) {
 // The decoded page goes into slot `slot` of the round's tiles as exact binary16 codes. K quad q of lane l = token l/2,
 // channels 64(l&1)+4q..+3 -> K tile row 16*slot + l/2; V quad q of lane l = channel 4l + q/4, tokens 4(q%4)..+3 -> V tile
 // row v_tile_row(l, q/4), token chunks 2*slot and 2*slot+1.
-template <int kCluster>
-__device__ __forceinline__ void store_codes(uint8_t *at, uint4 codes, uint32_t peer_delta) {
-    *reinterpret_cast<uint4 *>(at) = codes;
-    if constexpr (kCluster == 2) store_peer(smem_addr(at) + peer_delta, codes);
-}
 // A page that is absent (past the unit's end, or refused) leaves zeros in its slot of both tiles.
-template <int kCluster>
 __device__ __forceinline__ void store_tiles(const uint32_t (&kq)[16], const uint32_t (&vq)[16], bool present, uint8_t *k_tile, uint8_t *v_tile,
-                                            uint32_t slot, uint32_t lane, uint32_t peer_delta) {
+                                            uint32_t slot, uint32_t lane) {
     const uint32_t k_row = 16u * slot + (lane >> 1);
-    auto put = [&](uint8_t *at, uint32_t qa, uint32_t qb) { store_codes<kCluster>(at, present ? codes8(qa, qb) : make_uint4(0u, 0u, 0u, 0u), peer_delta); };
+    auto put = [&](uint8_t *at, uint32_t qa, uint32_t qb) { *reinterpret_cast<uint4 *>(at) = present ? codes8(qa, qb) : make_uint4(0u, 0u, 0u, 0u); };
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
         const uint32_t k_chunk = 8u * (lane & 1u) + 2u * c;
-        put(k_tile + tile_offset(k_row, k_chunk), kq[4 * c], kq[4 * c + 1]);
-        put(k_tile + tile_offset(k_row, k_chunk + 1u), kq[4 * c + 2], kq[4 * c + 3]);
+        put(k_tile + k_tile_offset(k_row, k_chunk), kq[4 * c], kq[4 * c + 1]);
+        put(k_tile + k_tile_offset(k_row, k_chunk + 1u), kq[4 * c + 2], kq[4 * c + 3]);
         const uint32_t v_row = v_tile_row(lane, c);
-        put(v_tile + tile_offset(v_row, 2u * slot), vq[4 * c], vq[4 * c + 1]);
-        put(v_tile + tile_offset(v_row, 2u * slot + 1u), vq[4 * c + 2], vq[4 * c + 3]);
+        put(v_tile + v_tile_offset(v_row, 2u * slot), vq[4 * c], vq[4 * c + 1]);
+        put(v_tile + v_tile_offset(v_row, 2u * slot + 1u), vq[4 * c + 2], vq[4 * c + 3]);
     }
 }
 // Head_dim 64: a stream has sixteen blocks, a lane decodes one block of one stream. K block l = token l, V block l = channels
@@ -317,15 +320,13 @@ __device__ __forceinline__ void decode_half(const uint8_t *part, uint32_t part_b
         decode_stream(d, quads);
     }
 }
-template <int kCluster>
-__device__ __forceinline__ void store_half(const uint32_t (&quads)[16], bool present, uint8_t *k_tile, uint8_t *v_tile, uint32_t slot, uint32_t lane,
-                                           uint32_t peer_delta) {
+__device__ __forceinline__ void store_half(const uint32_t (&quads)[16], bool present, uint8_t *k_tile, uint8_t *v_tile, uint32_t slot, uint32_t lane) {
     const uint32_t l = lane & 15u;
 #pragma unroll
     for (int c = 0; c < 8; ++c) {   // K: chunk c of token l's row; V: half c & 1 of channel 4 l + c / 2's sixteen tokens
         const uint4 codes = present ? codes8(quads[2 * c], quads[2 * c + 1]) : make_uint4(0u, 0u, 0u, 0u);
-        uint8_t *at = lane < 16u ? k_tile + tile_offset(16u * slot + l, c) : v_tile + tile_offset(v_tile_row(l, c >> 1), 2u * slot + (c & 1));
-        store_codes<kCluster>(at, codes, peer_delta);
+        uint8_t *at = lane < 16u ? k_tile + k_tile_offset(16u * slot + l, c) : v_tile + v_tile_offset(v_tile_row(l, c >> 1), 2u * slot + (c & 1));
+        *reinterpret_cast<uint4 *>(at) = codes;
     }
 }
 
@@ -583,8 +584,8 @@ __device__ __forceinline__ void decoder_role(const AttentionParams &p, uint8_t *
 
         wait_pair_free(it);
         uint8_t *k_tile = smem + kOffTiles + pair * 2u * kTileBytes, *v_tile = k_tile + kTileBytes;
-        if constexpr (kDim == 128) store_tiles<kCluster>(kq, vq, token_count != 0u, k_tile, v_tile, slot, lane, peer_delta);
-        else store_half<kCluster>(kq, token_count != 0u, k_tile, v_tile, slot, lane, peer_delta);
+        if constexpr (kDim == 128) store_tiles(kq, vq, token_count != 0u, k_tile, v_tile, slot, lane);
+        else store_half(kq, token_count != 0u, k_tile, v_tile, slot, lane);
         if (lane == 0) {
             uint4 *meta = reinterpret_cast<uint4 *>(smem + kOffMeta) + pair * 8u + slot;   // token count 0: the page contributes nothing
             const uint4 about = make_uint4(__float_as_uint(k_scale), __float_as_uint(v_scale), token_count, 0u);
@@ -592,28 +593,47 @@ __device__ __forceinline__ void decoder_role(const AttentionParams &p, uint8_t *
             if constexpr (kCluster == 2) store_peer(smem_addr(meta) + peer_delta, about);
             if (slot == 0) describe_round(pair, cur.unit, (in_unit < 8u ? kFirstRound : 0u) | (in_unit + 8u >= cur.slots ? kLastRound : 0u));
         }
-        fence_async_smem<kCluster>();   // the tiles were written through the generic proxy; the tensor core reads through the async one
+        fence_async_smem();   // the tiles were written through the generic proxy; the tensor core and the copies read through the async one
         __syncwarp();
-        if (lane == 0) arrive_full(pair);
+        if (lane == 0) {
+            mbar_arrive(&bar_full[pair]);
+            if constexpr (kCluster == 2) {
+                const uint32_t bar = smem_addr(&bar_full[pair]) + peer_delta;
+                if (failed) {
+                    mbar_arrive_peer(bar);
+                } else {   // the page's rows to the other CTA, whose round is full once they are there; its tiles are free, too
+                    constexpr uint32_t kPart = kDim == 128 ? 2048u : 1024u;   // of 2048 bytes of a row group, or a chunk
+                    mbar_arrive_expect_peer(bar, 4u * kPart);
+#pragma unroll
+                    for (uint32_t part = 0; part < 2u; ++part) {
+                        const uint32_t k_at = smem_addr(k_tile) + 4096u * slot + 2048u * part, v_at = smem_addr(v_tile) + 4096u * slot + 2048u * part;
+                        copy_to_peer(k_at + peer_delta, k_at, kPart, bar);
+                        copy_to_peer(v_at + peer_delta, v_at, kPart, bar);
+                    }
+                }
+            }
+        }
         cur = next;
         entry = next_entry;
     }
     // a copy whose wait ran out gets one more bounded chance to land before the CTA's shared memory is given back
     if (failed) mbar_wait(bar, copy_phase & 1u, p.wait_polls);
+    // ... and so do the copies to the other CTA, which only its barriers could tell of; they take a microsecond or two
+    for (int i = 0; kCluster == 2 && failed && i < 32; ++i) __nanosleep(1000);
 }
 
 // ---- tensor-core work, issued by one thread ----------------------------------------------------------------------------------
 // S of round r, whose tiles are there.
 template <int kDim, bool kSplitQ, int kCluster>
 __device__ __forceinline__ void issue_scores(uint8_t *smem, uint32_t tmem, uint64_t *bars, uint32_t r) {
-    fence_async_smem<kCluster>();
+    fence_async_smem();
     tc_fence_after();
     const uint32_t k_tile = smem_addr(smem + kOffTiles + (r & 1u) * 2u * kTileBytes), s_to = tmem + kColS + 128u * (r & 1u);
 #pragma unroll
-    for (uint32_t s = 0; s < kDim / 16; ++s) umma(s_to, tmem + kColQ + 8u * s, tile_desc(k_tile + 256u * s), s, kIdescS);
+    for (uint32_t s = 0; s < kDim / 16; ++s) umma(s_to, tmem + kColQ + 8u * s, k_desc(k_tile, s), s, kIdescS);
     if constexpr (kSplitQ) {
 #pragma unroll
-        for (uint32_t s = 0; s < kDim / 16; ++s) umma(s_to, tmem + kColQResidue + 8u * s, tile_desc(k_tile + 256u * s), 1u, kIdescS);
+        for (uint32_t s = 0; s < kDim / 16; ++s) umma(s_to, tmem + kColQResidue + 8u * s, k_desc(k_tile, s), 1u, kIdescS);
     }
     umma_commit(bars + kBarS + (r & 1u));
 }
@@ -623,9 +643,9 @@ __device__ __forceinline__ void issue_output(uint8_t *smem, uint32_t tmem, uint6
     tc_fence_after();
     const uint32_t v_tile = smem_addr(smem + kOffTiles + (r & 1u) * 2u * kTileBytes + kTileBytes), p_from = tmem + kColS + 128u * (r & 1u);
 #pragma unroll
-    for (uint32_t s = 0; s < 8; ++s) umma(tmem + kColO, p_from + 8u * s, tile_desc(v_tile + 256u * s), first && !s ? 0u : 1u, kIdescO<kDim>);
+    for (uint32_t s = 0; s < 8; ++s) umma(tmem + kColO, p_from + 8u * s, v_desc(v_tile, s), first && !s ? 0u : 1u, kIdescO<kDim>);
 #pragma unroll
-    for (uint32_t s = 0; s < 8; ++s) umma(tmem + kColO, p_from + 64u + 8u * s, tile_desc(v_tile + 256u * s), 1u, kIdescO<kDim>);
+    for (uint32_t s = 0; s < 8; ++s) umma(tmem + kColO, p_from + 64u + 8u * s, v_desc(v_tile, s), 1u, kIdescO<kDim>);
     if constexpr (kCluster == 1) umma_commit(bars + kBarFree + (r & 3u));   // the decoders may refill this pair of tiles
     else umma_commit_pair(bars + kBarFree + (r & 3u));
     umma_commit(bars + kBarO + (r & 1u));
