@@ -15,6 +15,7 @@
 #include <cuda_runtime.h>
 
 #include "attention_params.cuh"
+#include "copy_helpers.h"
 #include "host_rows.h"
 #include "chromofold_b200/compat_adapter.h"
 #include "chromofold_b200/compat_kv.h"
@@ -236,9 +237,8 @@ bool in_stream_order(const void *ptr) {
 }
 
 // Copies `rows` rows of `dim` floats and returns the first that holds NaN or Inf, or `rows`.
-uint32_t copy_rows_checked(float *dst, const float *src, uint32_t rows, uint32_t dim) {
-    const size_t n = static_cast<size_t>(rows) * dim;
-    if (chromofold_copy_max_magnitude(dst, src, n) < 0x7f800000u) return rows;   // inf and NaN lie above every finite magnitude
+uint32_t copy_rows_checked(cfb::CopyHelpers &helpers, float *dst, const float *src, uint32_t rows, uint32_t dim) {
+    if (helpers.copy(dst, src, static_cast<size_t>(rows) * dim) < 0x7f800000u) return rows;   // inf and NaN lie above every finite magnitude
     uint32_t r = 0;
     while (chromofold_copy_max_magnitude(dst + static_cast<size_t>(r) * dim, src + static_cast<size_t>(r) * dim, dim) < 0x7f800000u) ++r;
     return r;
@@ -385,6 +385,7 @@ struct cf_llama_kv_adapter {
     cudaEvent_t kivi_done[2] = {};           // the append that used pinned half i has ended
     uint32_t kivi_turn = 0;                  // pinned half of the next append
     StreamMarks kivi_written, kivi_read;     // appends and flushes, attention calls
+    cfb::CopyHelpers kivi_helpers;                // threads that share the copies there (a prompt's: a token's rows are too few)
     static constexpr size_t kKiviStageBytes = 1u << 20;   // of one stream, staged at a time (at least one page): the next turn copies meanwhile
 
     ~cf_llama_kv_adapter() {
@@ -619,7 +620,7 @@ struct cf_llama_kv_adapter {
                     const float *half = source[stream];
                     if (!ordered) {
                         float *pinned = kivi_pinned + (2u * kivi_turn + stream) * kivi_stage_floats;
-                        bad = std::min(bad, copy_rows_checked(pinned, half, rows, D));
+                        bad = std::min(bad, copy_rows_checked(kivi_helpers, pinned, half, rows, D));
                         half = pinned;
                     }
                     cuda_check(cudaMemcpyAsync(kivi_stage.ptr + stream * kivi_stage_floats, half, floats * sizeof(float), cudaMemcpyHostToDevice, s), "stage rows");

@@ -1,0 +1,47 @@
+"""Checked copies of host rows shared by several threads (chromofold_b200/csrc/copy_helpers.h): every size around the pieces' edges, one
+copy after the other and after pauses in which the helpers fall asleep; a value that is not finite is found wherever it lies."""
+import os
+import shutil
+import subprocess
+
+import pytest
+
+SRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "chromofold_b200", "csrc")
+
+PROGRAM = r"""
+#include "copy_helpers.h"
+#include <cstdio>
+#include <cstring>
+#include <limits>
+using cfb::CopyHelpers;
+int main() {
+    const size_t piece = CopyHelpers::kPieceFloats, least = CopyHelpers::kLeastFloats;
+    for (int object = 0; object < 3; ++object) {
+        CopyHelpers helpers;   // one of them ends without a copy, and one that is asleep
+        for (int turn = 0; object < 2 && turn < 60; ++turn)
+            for (size_t n : {size_t{1}, least - 1, least, least + 1, 5 * piece - 1, 5 * piece, 5 * piece + 1, 33 * piece + 7}) {
+                std::vector<float> a(n + 1), b(n + 1, 7.0f);
+                for (size_t i = 0; i < n; ++i) a[i] = static_cast<float>((i * 31 + turn) % 1000) - 500.0f;
+                const bool finite = turn % 3 != 0;
+                if (!finite) a[(n * static_cast<size_t>(turn)) / 60] = -std::numeric_limits<float>::infinity();
+                if ((helpers.copy(b.data(), a.data(), n) < 0x7f800000u) != finite) return 1;
+                if (std::memcmp(a.data(), b.data(), n * sizeof(float)) != 0 || b[n] != 7.0f) return 2;
+                if (turn % 20 == 7) std::this_thread::sleep_for(2 * CopyHelpers::kAwake);
+            }
+        if (object == 1) std::this_thread::sleep_for(20 * CopyHelpers::kAwake);
+    }
+    std::puts("ok");
+    return 0;
+}
+"""
+
+
+def test_shared_copies_are_exact(tmp_path):
+    gxx = shutil.which("g++")
+    if not gxx:
+        pytest.skip("g++ not found")
+    src, exe = tmp_path / "copies.cpp", tmp_path / "copies"
+    src.write_text(PROGRAM)
+    subprocess.run([gxx, "-std=c++17", "-O2", "-pthread", "-I", SRC, os.path.join(SRC, "host_rows.cpp"), str(src), "-o", str(exe)], check=True)
+    out = subprocess.run([str(exe)], capture_output=True, text=True, timeout=60)
+    assert out.stdout == "ok\n", out.returncode
