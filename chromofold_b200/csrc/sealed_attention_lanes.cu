@@ -95,92 +95,66 @@ __device__ __forceinline__ void score_quad(UnitState<NG, kDim> &u, const QSrc &q
 
 // kFold: the symbols are only folded into a checksum (u.vq[0]) — the decode work of the kernel without its attention.
 // kDump: lane l's quad q of a stream holds the symbols 64 l + 4 q .. + 3 of that stream, first symbol in byte 0.
-// kRolled: the page in four passes of four quads, a quarter of the code, so that more of it stays in the instruction cache; the V
+// kPasses: a page in four passes of four quads, a quarter of the code, so that more of it stays in the instruction cache; the V
 // quads shift down, so that quad q ends in element q. Taken by the eight-head kernel of binary16 queries, whose 16 warps hide
 // less of the fetches: 64 sequences of rANS pages 1403 -> 1335 us, of Huffman pages 1098 -> 1022. Half as many steps, as
 // nibble-split pages have, gain nothing by it, and neither the 24 warps of the four-head kernels nor eight heads of split
-// queries have registers to spare for it (821 -> 901, 1102 -> 1202 us).
+// queries have registers to spare for it (64 sequences, nibble-split rANS, 32 heads: 1351 us in one pass, 1413 in two, 1410 in four).
 template <int kEach>
 __device__ __forceinline__ void shift_quads(uint32_t (&vq)[16]) {
 #pragma unroll
     for (int i = 0; i < 16 - kEach; ++i) vq[i] = vq[i + kEach];
 }
-template <int kMode = kAttend, bool kRolled = false, class KLane, class VLane, int NG, class QSrc>
-__device__ __forceinline__ void decode_fused(KLane &k, VLane &v, UnitState<NG> &u, const QSrc &qs) {
-    if constexpr (KLane::kWholeQuads || VLane::kWholeQuads) {
-#pragma unroll
-        for (int q = 0; q < 16; ++q) {
-            const uint32_t kq = k.quad(q);
-            if constexpr (kMode == kFold) {
-                u.vq[0] ^= kq ^ v.quad(q);
-            } else if constexpr (kMode == kDump) {
-                u.dump[q] = kq;
-                u.dump[512 + q] = v.quad(q);
-            } else {
-                u.vq[q] = v.quad(q);
-                score_quad(u, qs, q, kq);
-            }
-        }
+template <int kMode, int NG, class QSrc>
+__device__ __forceinline__ void take_quads(UnitState<NG> &u, const QSrc &qs, int q, int at, uint32_t kq, uint32_t vq) {
+    if constexpr (kMode == kFold) {
+        u.vq[0] ^= kq ^ vq;
+    } else if constexpr (kMode == kDump) {
+        u.dump[q] = kq;
+        u.dump[512 + q] = vq;
     } else {
-        // two independent decoder chains, interleaved symbol by symbol; four symbols make one packed register
-        constexpr int kPasses = kRolled ? 4 : 1, kEach = 16 / kPasses;   // quads of a pass
-#pragma unroll 1
-        for (int pass = 0; pass < kPasses; ++pass) {
-            if constexpr (kRolled) shift_quads<kEach>(u.vq);
-            uint32_t ke[4], ve[4];
-#pragma unroll
-            for (int i = 0; i < 4 * kEach; ++i) {
-                ke[i & 3] = k.symbol(i & 1);
-                ve[i & 3] = v.symbol(i & 1);
-                if (i & 1) {
-                    k.advance();
-                    v.advance();
-                }
-                if ((i & 3) == 3) {
-                    const int q = kEach * pass + (i >> 2);
-                    if constexpr (kMode == kFold) {
-                        u.vq[0] ^= VLane::pack(ve[0], ve[1], ve[2], ve[3]) ^ KLane::pack(ke[0], ke[1], ke[2], ke[3]);
-                    } else if constexpr (kMode == kDump) {
-                        u.dump[q] = KLane::pack(ke[0], ke[1], ke[2], ke[3]);
-                        u.dump[512 + q] = VLane::pack(ve[0], ve[1], ve[2], ve[3]);
-                    } else {
-                        u.vq[16 - kEach + (i >> 2)] = VLane::pack(ve[0], ve[1], ve[2], ve[3]);
-                        score_quad(u, qs, q, KLane::pack(ke[0], ke[1], ke[2], ke[3]));
-                    }
-                }
-            }
-        }
+        u.vq[at] = vq;
+        score_quad(u, qs, q, kq);
     }
 }
-
-// Both streams nibble-split with the same coder: 32 interleaved steps per stream, a quad from every two of them.
-template <int kMode = kAttend, class Lane, int NG, class QSrc>
-__device__ __forceinline__ void decode_fused_split(Lane &k, Lane &v, UnitState<NG> &u, const QSrc &qs) {
-    uint32_t ke[2], ve[2], kw = 0u, vw = 0u;
+// Both streams with the same coder: two independent decoder chains, interleaved symbol by symbol.
+template <int kMode, int kPasses, class Lane, int NG, class QSrc>
+__device__ __forceinline__ void decode_fused(Lane &k, Lane &v, UnitState<NG> &u, const QSrc &qs) {
+    constexpr int kEach = 16 / kPasses;   // quads of a pass
+#pragma unroll 1
+    for (int pass = 0; pass < kPasses; ++pass) {
+        if constexpr (kPasses > 1) shift_quads<kEach>(u.vq);
+        uint32_t kw = 0u, vw = 0u;
 #pragma unroll
-    for (int i = 0; i < 32; ++i) {
-        ke[i & 1] = k.symbol(i & 1);
-        ve[i & 1] = v.symbol(i & 1);
-        if (i & 1) {
-            k.advance();
-            v.advance();
-            const int q = i >> 1;
-            if ((q & 1) == 0) {
-                kw = k.lo_word(q >> 1);
-                vw = v.lo_word(q >> 1);
+        for (int j = 0; j < kEach; ++j) {
+            const int q = kEach * pass + j, at = 16 - kEach + j;
+            if constexpr (requires { k.lo_word(0); }) {   // nibble-split: a quad from every two steps
+                uint32_t ke[2], ve[2];
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    ke[i] = k.symbol(i);
+                    ve[i] = v.symbol(i);
+                }
+                k.advance();
+                v.advance();
+                kw = j & 1 ? kw >> 4 : k.lo_word(q >> 1);
+                vw = j & 1 ? vw >> 4 : v.lo_word(q >> 1);
+                take_quads<kMode>(u, qs, q, at, merge_split_quad<Lane>(ke[0], ke[1], kw), merge_split_quad<Lane>(ve[0], ve[1], vw));
+            } else if constexpr (Lane::kWholeQuads) {
+                const uint32_t kq = k.quad(q);
+                take_quads<kMode>(u, qs, q, at, kq, v.quad(q));
             } else {
-                kw >>= 4;
-                vw >>= 4;
-            }
-            const uint32_t kq = merge_split_quad<Lane>(ke[0], ke[1], kw), vq = merge_split_quad<Lane>(ve[0], ve[1], vw);
-            if constexpr (kMode == kFold) {
-                u.vq[0] ^= kq ^ vq;
-            } else if constexpr (kMode == kDump) {
-                u.dump[q] = kq;
-                u.dump[512 + q] = vq;
-            } else {
-                u.vq[q] = vq;
-                score_quad(u, qs, q, kq);
+                uint32_t ke[4], ve[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    ke[i] = k.symbol(i & 1);
+                    ve[i] = v.symbol(i & 1);
+                    if (i & 1) {
+                        k.advance();
+                        v.advance();
+                    }
+                }
+                take_quads<kMode>(u, qs, q, at, Lane::pack(ke[0], ke[1], ke[2], ke[3]), Lane::pack(ve[0], ve[1], ve[2], ve[3]));
             }
         }
     }
@@ -307,7 +281,7 @@ __global__ void __launch_bounds__(kThreadsOf<NG, NB, kSplitQ, kDim>, 1) lanes_at
     using L = WarpLayout<NG, NB, kSplitQ, kDim>;
     constexpr int NS = kHeadGroups<NG, kSplitQ>;
     constexpr uint32_t kPassHeads = 4u * NS;
-    constexpr bool kRolled = NS == 2 && !kSplitQ && kMode == kAttend;
+    constexpr int kPasses = NS == 2 && !kSplitQ && kMode == kAttend ? 4 : 1;   // of decode_fused
     extern __shared__ __align__(128) uint8_t smem[];
     uint32_t *k_slot = reinterpret_cast<uint32_t *>(smem);
     uint32_t *v_slot = k_slot + 4096;
@@ -580,27 +554,27 @@ __global__ void __launch_bounds__(kThreadsOf<NG, NB, kSplitQ, kDim>, 1) lanes_at
                         RansSplitLane k, v;
                         k.open(k_part, k_bytes, lane, k_slot);
                         v.open(v_part, v_bytes, lane, v_slot);
-                        decode_fused_split<kMode>(k, v, u, qs);
+                        decode_fused<kMode, 1>(k, v, u, qs);
                     } else if (k_coder == CF_B200_CODER_HUFFMAN_SPLIT4 && v_coder == CF_B200_CODER_HUFFMAN_SPLIT4) {
                         HuffSplitLane k, v;
                         k.open(k_part, k_bytes, lane, k_lut);
                         v.open(v_part, v_bytes, lane, v_lut);
-                        decode_fused_split<kMode>(k, v, u, qs);
+                        decode_fused<kMode, 1>(k, v, u, qs);
                     } else if (k_coder == CF_B200_CODER_RANS && v_coder == CF_B200_CODER_RANS) {
                         RansLane k, v;
                         k.open(k_part, k_bytes, lane, k_slot);
                         v.open(v_part, v_bytes, lane, v_slot);
-                        decode_fused<kMode, kRolled>(k, v, u, qs);
+                        decode_fused<kMode, kPasses>(k, v, u, qs);
                     } else if (k_coder == CF_B200_CODER_HUFFMAN && v_coder == CF_B200_CODER_HUFFMAN) {
                         HuffLane k, v;
                         k.open(k_part, k_bytes, lane, k_lut);
                         v.open(v_part, v_bytes, lane, v_lut);
-                        decode_fused<kMode, kRolled>(k, v, u, qs);
+                        decode_fused<kMode, kPasses>(k, v, u, qs);
                     } else if (k_coder == CF_B200_CODER_FIXED8 && v_coder == CF_B200_CODER_FIXED8) {
                         FixedLane k, v;
                         k.open(k_part, k_bytes, lane);
                         v.open(v_part, v_bytes, lane);
-                        decode_fused<kMode, kRolled>(k, v, u, qs);
+                        decode_fused<kMode, kPasses>(k, v, u, qs);
                     } else {  // mixed coders (one stream fell back to fixed width): one stream after the other
                         if (k_coder == CF_B200_CODER_RANS) { RansLane k; k.open(k_part, k_bytes, lane, k_slot); decode_k_only<kMode>(k, u, qs); }
                         else if (k_coder == CF_B200_CODER_HUFFMAN) { HuffLane k; k.open(k_part, k_bytes, lane, k_lut); decode_k_only<kMode>(k, u, qs); }
