@@ -1,5 +1,7 @@
 """The benchmark configurations as parity cases (seeded synthetic inputs with their shapes and distributions), through
 the C ABI, against the CPU oracle reading the same sealed bytes. Config 2 runs at its full size."""
+import math
+
 import numpy as np
 import pytest
 
@@ -410,3 +412,31 @@ def test_shared_prefix_whose_first_page_has_a_tiny_v_scale(native, oracle):
     assert ok, err
     ok, err = attention_close(shared, oracle_from_layer(layer, q.cpu().numpy()))
     assert ok, err
+
+
+@pytest.mark.parametrize("rows", [8, 40])   # one CTA, a pair of them
+@pytest.mark.parametrize("step", [0.3, 0.85, 0.95, 20.0])
+def test_shared_prefix_whose_maxima_rise(native, step, rows):
+    """The maximum that the shared-prefix kernel's weights are relative to follows the true one only when that has risen by 0.9
+    in the exponent of two: scores that rise by less, by little more and by far more from round to round (128 tokens). The scores are
+    fp32-accurate in both kernels and the weights exact to 2^-22 of the largest: 2e-5 as for other fp32 queries."""
+    import torch
+    from chromofold_b200.workloads import build_sealed_layer
+    pages = 80
+    layer, _ = build_sealed_layer(np.array([0] * rows), coder="rans4", seed=130, extra_pages_per_sequence=pages + 2, reserve_pages=2 * rows)
+    layer.set_codebooks(np.ones(256, np.uint64), np.ones(256, np.uint64))
+    g = torch.Generator(device="cuda")
+    g.manual_seed(131)
+    rounds = torch.arange(pages, device="cuda") // 8
+    per_unit = 128 / math.sqrt(128) * math.log2(math.e)   # exponent of a key of ones under a query of ones
+    k = (rounds * (step / per_unit)).reshape(-1, 1, 1, 1).expand(pages, 8, 16, 128).half().contiguous()
+    v = (torch.randn((pages, 8, 16, 128), generator=g, device="cuda") * 0.7).half()
+    layer.seal_tiles(np.zeros(pages, np.int64), k, v)
+    for s in range(1, rows):
+        layer.copy_sequence(0, s)
+    q = 1.0 + 0.1 * torch.randn((rows, 32, 128), generator=g, device="cuda")
+    q[:, 1::4] *= -1.0   # the first round holds the maximum
+    shared = layer.attention(q, shared_prefix_pages=pages).cpu().numpy()
+    want = layer.attention(q, kernel=native.KERNEL_GENERIC).cpu().numpy()
+    assert layer.device_status() == 0
+    assert np.abs(shared - want).max() <= 2e-5
