@@ -423,7 +423,7 @@ def test_shared_prefix_whose_maxima_rise(native, step, rows):
     import torch
     from chromofold_b200.workloads import build_sealed_layer
     pages = 80
-    layer, _ = build_sealed_layer(np.array([0] * rows), coder="rans4", seed=130, extra_pages_per_sequence=pages + 2, reserve_pages=2 * rows)
+    layer, _ = build_sealed_layer(np.array([0] * rows), coder="rans4", seed=130, extra_pages_per_sequence=pages + 2, reserve_pages=pages + 2 * rows)
     layer.set_codebooks(np.ones(256, np.uint64), np.ones(256, np.uint64))
     g = torch.Generator(device="cuda")
     g.manual_seed(131)
