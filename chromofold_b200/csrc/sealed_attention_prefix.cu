@@ -10,7 +10,7 @@
 // One CTA of 20 warps per SM. The work is cut evenly (SharedSplit): the rounds (8 pages = 128 tokens) of every
 // (kv head, row tile) pair form one line and each CTA takes an equal stretch of it; the part of a stretch inside one
 // pair is a unit, which ends in one partial per row. From two row tiles on, two CTAs (a cluster) take a stretch together, a row
-// tile each: each decodes half of every round's pages and stores them in both, so that a page is decoded once per 256 rows.
+// tile each: each decodes half of every round's pages and sends them to the other, so that a page is decoded once per 256 rows.
 // The warps are specialised:
 //   decoder warps 0..11  the page slots of the CTA's units form one sequence; warp w takes slots w, w + 12, ... It
 //                        receives the record by one bulk async copy (mbarrier, bounded wait), decodes it with the
@@ -23,7 +23,7 @@
 //   softmax warps 12..19 a thread owns one row (= tensor-memory lane, in its warp's quarter) and half of the round's
 //                        128 score columns: one tcgen05.ld of its 64 scores (kept in registers), page K scales and masks,
 //                        the row's two threads share their maxima through shared memory, running max / sum updated,
-//                        O rescaled in tensor memory (tcgen05.ld / .st) only when some row of the warp moved its max,
+//                        O rescaled in tensor memory (tcgen05.ld / .st) only when some row of the warp moved its max by 2^0.9,
 //                        P and its residue written over the scores (tcgen05.st) as the next A operands.
 //                        Thread 0 of the group (in a pair of CTAs: warp 11) issues the tensor-core work (M 128, K 16):
 //                          S     Q from tensor memory x K tile -> one of two sets of 128 score columns
