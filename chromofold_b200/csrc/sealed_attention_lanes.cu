@@ -36,7 +36,9 @@ using namespace lanes;
 // (kSplitQ) take two groups for four heads, value and residue, and four for eight. NS = groups that go through softmax and P V.
 template <int NG, bool kSplitQ> constexpr int kHeadGroups = kSplitQ ? NG / 2 : NG;
 // Warps per CTA, one CTA per SM: what registers (65536, no spill worth the name) and shared memory (227 KB) leave. The
-// decoders want as many warps as they can get: 16 -> 24 of them took 8 % off a launch, 24 -> 28 do not fit.
+// decoders want warps, but not at the price of spilled registers, and as many on each of the four schedulers: 64 sequences of
+// nibble-split rANS, 32 heads, take 1381, 1530, 1470, 1351, 1459, 1445 us with 20, 21, 22, 24, 26, 28 warps; 8 x 131072 tokens, 64
+// heads, 2269, 2441, 2149 with 12, 14, 16.
 template <int NG, int NB, bool kSplitQ, int kDim>
 constexpr int kWarpsOf = NB == 32                ? (kHeadGroups<NG, kSplitQ> == 1 ? 24 : 16)
                          : kDim <= 64            ? 20
