@@ -98,6 +98,11 @@ __host__ __device__ inline uint32_t shared_tile_groups(uint32_t rows) {
     return (rows + per_group - 1u) / per_group;
 }
 
+// The page slots of a pair's CTA: its half of the eight of every round. The m-th of them is slot pair_slot(m, rank) of the pair's
+// sequence and lies in round pair_round(m); decoder warp w takes m = w, w + warps, ... in this order.
+__host__ __device__ inline uint32_t pair_slot(uint32_t m, uint32_t rank) { return (m >> 2) * 8u + 4u * rank + (m & 3u); }
+__host__ __device__ inline uint32_t pair_round(uint32_t m) { return m >> 2; }
+
 // The barrier on which a pair's CTA of the shared-prefix kernel is told that the weights of round r are stored, and the parity of
 // that arrival. The issuing thread sends the scores of round r + 1 before the output of round r, so the softmax warps can have
 // arrived for both before it looks: on one barrier the second arrival hides the first (the phase is back at the parity it waits

@@ -43,9 +43,9 @@
 // The page's V scale relative to the largest one met so far in the unit rides on P (never above 1, so the binary16
 // weights cannot overflow); O is kept in units of that scale and rescaled when a larger one arrives.
 // Every mbarrier wait is bounded. A warp whose wait ran out raises CF_B200_DEVSTAT_WAIT_EXPIRED and skips all later
-// waits and work; a decoder warp still arrives for each of its slots, a softmax warp still takes part in the barrier with its
-// partner, which OR-reduces the failure so that both leave their loops at the same point, and the roles that wait for
-// them run out of their own waits; the CTA then frees its tensor memory.
+// waits and work, but a decoder warp whose record never came, which goes on with absent pages, and a softmax warp still takes
+// part in the barrier with its partner, which OR-reduces the failure so that both leave their loops at the same point; the roles
+// that wait for one that left run out of their own waits; the CTA then frees its tensor memory.
 
 #include "lanes_decoders.cuh"
 
@@ -404,7 +404,7 @@ __device__ __forceinline__ void decoder_role(const AttentionParams &p, uint8_t *
     const uint32_t worker = blockIdx.x / kCluster, rank = kCluster == 1 ? 0u : cluster_rank();
     const uint32_t peer_delta = kCluster == 1 ? 0u : peer_address(smem_addr(smem), rank ^ 1u) - smem_addr(smem);   // own place -> the peer's
     // this CTA's m-th slot: all of them, or its half of every round
-    auto slot_number = [&](uint32_t m) { return kCluster == 1 ? m : (m >> 2) * 8u + 4u * rank + (m & 3u); };
+    auto slot_number = [&](uint32_t m) { return kCluster == 1 ? m : pair_slot(m, rank); };
     const uint32_t *k_slot = reinterpret_cast<const uint32_t *>(smem);
     const uint32_t *v_slot = k_slot + 4096;
     const uint16_t *k_lut = reinterpret_cast<const uint16_t *>(v_slot + 4096);
@@ -450,13 +450,17 @@ __device__ __forceinline__ void decoder_role(const AttentionParams &p, uint8_t *
         }
     };
     uint32_t copy_phase = 0;
-    bool failed = false;   // warp-uniform; once set, the warp waits for nothing and decodes nothing, but keeps arriving
+    // Warp-uniform. kNoRecord: a record never came; the warp decodes nothing more, but goes on by the rules: its pages are absent, and
+    // both CTAs' tiles get zeros for them (zero weights alone would not do: what lies there from before may be NaN).
+    // kNoTiles: no tiles were freed; the warp leaves, and arrives for nothing more.
+    constexpr uint32_t kNoRecord = 1u, kNoTiles = 2u;
+    uint32_t failed = 0u;
     // The pair of round `it` is free once the tensor core (of both CTAs) has finished round it - 2, which the barrier of that round's
     // number modulo four tells. The parity wait is sound because a warp's slots are at most three rounds apart, so that it has
     // seen the end of a round later than it - 6, the barrier's previous one.
     auto wait_pair_free = [&](uint32_t it) {
-        if (it >= 2u && !failed && !__all_sync(0xffffffffu, mbar_wait_pair(&bar_free[(it - 2u) & 3u], ((it - 2u) >> 2) & 1u, p.wait_polls))) {
-            failed = true;
+        if (it >= 2u && !__all_sync(0xffffffffu, mbar_wait_pair(&bar_free[(it - 2u) & 3u], ((it - 2u) >> 2) & 1u, p.wait_polls))) {
+            failed = kNoTiles;
             if (lane == 0) raise_status(p, CF_B200_DEVSTAT_WAIT_EXPIRED);
         }
     };
@@ -485,7 +489,7 @@ __device__ __forceinline__ void decoder_role(const AttentionParams &p, uint8_t *
         if (!cur.valid) {   // past the last unit: the eight slots after it make the round that tells the softmax group to stop
             if (n < cur.first_slot + 8u) {
                 wait_pair_free(cur.first_round);
-                if (lane == 0) {
+                if (lane == 0 && failed != kNoTiles) {
                     if (n == cur.first_slot) describe_round(cur.first_round & 1u, kStopUnit, 0u);
                     arrive_full(cur.first_round & 1u);
                 }
@@ -506,7 +510,7 @@ __device__ __forceinline__ void decoder_role(const AttentionParams &p, uint8_t *
             if (!entry_ok(entry)) {
                 if (lane == 0) raise_status(p, CF_B200_DEVSTAT_BAD_RECORD);
             } else if (!__all_sync(0xffffffffu, mbar_wait(bar, copy_phase & 1u, p.wait_polls))) {
-                failed = true;
+                failed = kNoRecord;
                 if (lane == 0) raise_status(p, CF_B200_DEVSTAT_WAIT_EXPIRED);
             } else {
                 copy_phase ^= 1u;
@@ -583,6 +587,7 @@ __device__ __forceinline__ void decoder_role(const AttentionParams &p, uint8_t *
         if (!failed) issue(next_entry);
 
         wait_pair_free(it);
+        if (failed == kNoTiles) break;
         uint8_t *k_tile = smem + kOffTiles + pair * 2u * kTileBytes, *v_tile = k_tile + kTileBytes;
         if constexpr (kDim == 128) store_tiles(kq, vq, token_count != 0u, k_tile, v_tile, slot, lane);
         else store_half(kq, token_count != 0u, k_tile, v_tile, slot, lane);
@@ -598,18 +603,15 @@ __device__ __forceinline__ void decoder_role(const AttentionParams &p, uint8_t *
         if (lane == 0) {
             mbar_arrive(&bar_full[pair]);
             if constexpr (kCluster == 2) {
+                // the page's rows to the other CTA, whose round is full once they are there; its tiles are free, too
+                constexpr uint32_t kPart = kDim == 128 ? 2048u : 1024u;   // of 2048 bytes of a row group, or a chunk
                 const uint32_t bar = smem_addr(&bar_full[pair]) + peer_delta;
-                if (failed) {
-                    mbar_arrive_peer(bar);
-                } else {   // the page's rows to the other CTA, whose round is full once they are there; its tiles are free, too
-                    constexpr uint32_t kPart = kDim == 128 ? 2048u : 1024u;   // of 2048 bytes of a row group, or a chunk
-                    mbar_arrive_expect_peer(bar, 4u * kPart);
+                mbar_arrive_expect_peer(bar, 4u * kPart);
 #pragma unroll
-                    for (uint32_t part = 0; part < 2u; ++part) {
-                        const uint32_t k_at = smem_addr(k_tile) + 4096u * slot + 2048u * part, v_at = smem_addr(v_tile) + 4096u * slot + 2048u * part;
-                        copy_to_peer(k_at + peer_delta, k_at, kPart, bar);
-                        copy_to_peer(v_at + peer_delta, v_at, kPart, bar);
-                    }
+                for (uint32_t part = 0; part < 2u; ++part) {
+                    const uint32_t k_at = smem_addr(k_tile) + 4096u * slot + 2048u * part, v_at = smem_addr(v_tile) + 4096u * slot + 2048u * part;
+                    copy_to_peer(k_at + peer_delta, k_at, kPart, bar);
+                    copy_to_peer(v_at + peer_delta, v_at, kPart, bar);
                 }
             }
         }
