@@ -102,6 +102,8 @@ __host__ __device__ inline uint32_t shared_tile_groups(uint32_t rows) {
 // sequence and lies in round pair_round(m); decoder warp w takes m = w, w + warps, ... in this order.
 __host__ __device__ inline uint32_t pair_slot(uint32_t m, uint32_t rank) { return (m >> 2) * 8u + 4u * rank + (m & 3u); }
 __host__ __device__ inline uint32_t pair_round(uint32_t m) { return m >> 2; }
+// Rounds up to the last one in which a warp whose next slot is m has arrived.
+__host__ __device__ inline uint32_t pair_rounds_arrived(uint32_t m, uint32_t warps) { return m < warps ? 0u : pair_round(m - warps) + 1u; }
 
 // The barrier on which a pair's CTA of the shared-prefix kernel is told that the weights of round r are stored, and the parity of
 // that arrival. The issuing thread sends the scores of round r + 1 before the output of round r, so the softmax warps can have

@@ -72,8 +72,11 @@ constexpr uint32_t kOffRound = kOffMeta + 2 * kRoundPages * 16;    // [pair]: un
 constexpr uint32_t kOffBars = kOffRound + 2 * 16;              // 12 copy barriers, full[2], free[4], S[2], O[2], P[2], Q
 constexpr uint32_t kBarFull = kDecodeWarps, kBarFree = kBarFull + 2, kBarS = kBarFree + 4, kBarO = kBarS + 2, kBarP = kBarO + 2, kBarQ = kBarP + kWeightBarriers,
                    kBarCount = kBarQ + 1;
-constexpr uint32_t kOffMisc = kOffBars + kBarCount * 8;        // [0] tmem base
-constexpr uint32_t kOffRowMax = kOffMisc + 32;                 // [round parity][2 column halves][128 rows]
+constexpr uint32_t kOffMisc = kOffBars + kBarCount * 8;        // [0] tmem base, [kMiscRounds], [kMiscGaveUp], [kMiscNext + warp]
+constexpr uint32_t kMiscRounds = 1;   // pair of CTAs: rounds in which some decoder warp of either has arrived, known once all have left
+constexpr uint32_t kMiscGaveUp = 2;   // ... an issuing thread of either has left before the last round
+constexpr uint32_t kMiscNext = 4;     // ... the first of its slots that decoder warp has not arrived for
+constexpr uint32_t kOffRowMax = kOffMisc + 64;                 // [round parity][2 column halves][128 rows]
 constexpr uint32_t kTcSmem = kOffRowMax + 4 * 128 * 4;
 static_assert(kTcSmem <= 232448, "the shared-prefix kernel must fit the 227 KB of one CTA");
 constexpr uint32_t kTmemColumns = 512;
@@ -118,7 +121,7 @@ __device__ __forceinline__ void umma(uint32_t tmem_d, uint32_t tmem_a, uint64_t 
 __device__ __forceinline__ void umma_commit(uint64_t *bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_addr(bar)) : "memory");
 }
-// A pair of CTAs (a cluster of two) shares the decoded pages: each decodes every other half round and stores it in both.
+// A pair of CTAs (a cluster of two) shares the decoded pages: each decodes half of every round and sends it to the other.
 __device__ __forceinline__ uint32_t cluster_rank() {
     uint32_t r;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
@@ -131,6 +134,12 @@ __device__ __forceinline__ uint32_t peer_address(uint32_t smem_address, uint32_t
 }
 __device__ __forceinline__ void store_peer(uint32_t address, uint4 v) {
     asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(address), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+__device__ __forceinline__ void store_peer(uint32_t address, uint32_t v) {
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(address), "r"(v) : "memory");
+}
+__device__ __forceinline__ void max_peer(uint32_t address, uint32_t v) {
+    asm volatile("red.relaxed.cluster.shared::cluster.max.u32 [%0], %1;" ::"r"(address), "r"(v) : "memory");
 }
 __device__ __forceinline__ void mbar_arrive_peer(uint32_t address) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(address) : "memory");
@@ -493,6 +502,7 @@ __device__ __forceinline__ void decoder_role(const AttentionParams &p, uint8_t *
                     if (n == cur.first_slot) describe_round(cur.first_round & 1u, kStopUnit, 0u);
                     arrive_full(cur.first_round & 1u);
                 }
+                if (failed != kNoTiles) m += kDecoders<kCluster>;
             }
             break;
         }
@@ -620,8 +630,13 @@ __device__ __forceinline__ void decoder_role(const AttentionParams &p, uint8_t *
     }
     // a copy whose wait ran out gets one more bounded chance to land before the CTA's shared memory is given back
     if (failed) mbar_wait(bar, copy_phase & 1u, p.wait_polls);
-    // ... and so do the copies to the other CTA, which only its barriers could tell of; they take a microsecond or two
-    for (int i = 0; kCluster == 2 && failed && i < 32; ++i) __nanosleep(1000);
+    if (kCluster == 2 && lane == 0) {   // for leave_pair
+        uint32_t *misc = reinterpret_cast<uint32_t *>(smem + kOffMisc);
+        const uint32_t rounds = pair_rounds_arrived(m, kDecoders<2>);
+        misc[kMiscNext + warp] = m;
+        atomicMax(misc + kMiscRounds, rounds);
+        max_peer(smem_addr(misc + kMiscRounds) + peer_delta, rounds);
+    }
 }
 
 // ---- tensor-core work, issued by one thread ----------------------------------------------------------------------------------
@@ -684,7 +699,12 @@ __device__ __forceinline__ void issuer_role(const AttentionParams &p, uint8_t *s
             ok = false;
         }
     }
-    if (!ok) raise_status(p, CF_B200_DEVSTAT_WAIT_EXPIRED);
+    if (!ok) {
+        raise_status(p, CF_B200_DEVSTAT_WAIT_EXPIRED);
+        uint32_t *gave_up = reinterpret_cast<uint32_t *>(smem + kOffMisc) + kMiscGaveUp;
+        *gave_up = 1u;
+        store_peer(peer_address(smem_addr(gave_up), cluster_rank() ^ 1u), 1u);
+    }
     // What the other CTA of the pair still signals here has to land before this one leaves; leaving early, the last product of
     // this one as well. Bounded, whatever happened.
     for (uint32_t r = o_round < 2u ? 0u : o_round - 2u; ok && r < o_round; ++r) mbar_wait_pair(bars + kBarFree + (r & 3u), (r >> 2) & 1u, p.wait_polls);
@@ -984,6 +1004,31 @@ __device__ __forceinline__ void softmax_role(const AttentionParams &p, uint8_t *
     if (issuer && rounds && failed) mbar_wait(&bar_o[(rounds - 1u) & 1u], ((rounds - 1u) >> 1) & 1u, p.wait_polls);
 }
 
+// A CTA of a pair may leave once nothing is on its way into its shared memory or, to the other one, out of it. If both issuing threads have
+// taken every round, they have seen all of it arrive. If one has not, the full barriers of the last two rounds that any decoder warp has
+// arrived for tell (of the ones before, the tiles were freed): the warps that left before make up the arrivals that
+// these lack, and then they complete when the pages that were sent are there.
+__device__ __forceinline__ void leave_pair(const AttentionParams &p, uint8_t *smem, uint32_t warp, uint32_t lane) {
+    constexpr uint32_t kWarps = kDecoders<2>;
+    uint64_t *bar_full = reinterpret_cast<uint64_t *>(smem + kOffBars) + kBarFull;
+    uint32_t *misc = reinterpret_cast<uint32_t *>(smem + kOffMisc);
+    __syncwarp();
+    cluster_sync();   // every role of both CTAs is done
+    if (misc[kMiscGaveUp] == 0u) return;
+    const uint32_t rounds = misc[kMiscRounds];
+    if (warp < kWarps && lane == 0) {
+        const uint32_t peer_delta = peer_address(smem_addr(smem), cluster_rank() ^ 1u) - smem_addr(smem);
+        for (uint32_t next_slot = misc[kMiscNext + warp]; pair_round(next_slot) < rounds; next_slot += kWarps) {
+            mbar_arrive(&bar_full[pair_round(next_slot) & 1u]);
+            mbar_arrive_peer(smem_addr(&bar_full[pair_round(next_slot) & 1u]) + peer_delta);
+        }
+    } else if (warp == kWarps && lane == 0) {
+        for (uint32_t r = rounds < 2u ? 0u : rounds - 2u; r < rounds; ++r) mbar_wait_pair(&bar_full[r & 1u], (r >> 1) & 1u, p.wait_polls);
+    }
+    __syncwarp();
+    cluster_sync();
+}
+
 template <int kDim, bool kSplitQ, int kCluster>
 __global__ void __launch_bounds__(kTcThreads, 1) prefix_attention_kernel(AttentionParams p) {
     extern __shared__ __align__(1024) uint8_t smem[];
@@ -1000,6 +1045,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) prefix_attention_kernel(Attenti
     if (hdr->shared_pages == 0 || blockIdx.x / kCluster >= hdr->shared_ctas) return;   // both CTAs of a pair alike
 
     if (tid == 0) {
+        misc[kMiscRounds] = misc[kMiscGaveUp] = 0u;
         for (uint32_t w = 0; w < kDecodeWarps; ++w) mbar_init(bars + w, 1);   // copies
         mbar_init(bars + kBarFull, kRoundPages);                    // full[0], full[1]: one arrival per page slot of the round
         mbar_init(bars + kBarFull + 1, kRoundPages);
@@ -1036,10 +1082,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) prefix_attention_kernel(Attenti
         softmax_role<kDim, kSplitQ, kCluster>(p, smem, hdr, tmem, warp, lane, tile_groups, split);
     }
 
-    if constexpr (kCluster == 2) {   // the peer may still store into this CTA's tiles
-        __syncwarp();
-        cluster_sync();
-    }
+    if constexpr (kCluster == 2) leave_pair(p, smem, warp, lane);
     tc_fence_before();
     __syncthreads();
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemColumns));

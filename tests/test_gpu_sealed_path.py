@@ -596,6 +596,36 @@ def test_a_wait_that_runs_out_is_reported_and_the_next_call_is_right(native, ora
     assert layer.device_status() == 0 and np.array_equal(again, good)
 
 
+@pytest.mark.parametrize("head_dim,queries,pages,skipped", [(128, "f16", 600, 300), (128, "f32", 600, 1), (64, "f32", 600, 590), (64, "f16", 80, 3)])
+def test_a_pair_whose_wait_runs_out_reports_it_and_the_next_call_is_right(native, head_dim, queries, pages, skipped):
+    """The same for pairs of CTAs (more than 128 rows), which send each other pages: eight rounds for each pair, or one or two; a page
+    of an early round, of one in the middle and of one of the last is never fetched."""
+    import torch
+    from chromofold_b200.workloads import build_sealed_layer
+    rows = 40
+    layer, _ = build_sealed_layer(np.array([16 * pages] + [0] * (rows - 1)), head_dim=head_dim, coder="rans4", seed=36)
+    for s in range(1, rows):
+        layer.copy_sequence(0, s)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(37)
+    q = torch.randn((rows, 32, head_dim), generator=g, device="cuda")
+    q = q if queries == "f32" else q.half()
+    good = layer.attention(q, shared_prefix_pages=pages).cpu().numpy()
+    assert layer.device_status() == 0
+    page_id = int(layer.page_table[0, skipped])
+    lib = native.lib()
+    try:
+        assert lib.cf_b200_test_wait_expiry(page_id, 2000) == 0
+        layer.attention(q, shared_prefix_pages=pages)
+        torch.cuda.synchronize()
+        assert layer.device_status() & native.DEVSTAT_WAIT_EXPIRED
+    finally:
+        assert lib.cf_b200_test_wait_expiry(0, 0) == 0
+    layer.status.zero_()
+    again = layer.attention(q, shared_prefix_pages=pages).cpu().numpy()
+    assert layer.device_status() == 0 and np.array_equal(again, good)
+
+
 def test_append_rows_entry_point_fills_the_tails_and_reports_a_full_one(native):
     """cf_b200_append_rows_async: one launch stores a token's K and V rows (binary16 or fp32 rows) at each listed slot's
     tail position and raises the count; a slot whose tail is full takes nothing and raises CF_B200_DEVSTAT_TAIL_FULL."""

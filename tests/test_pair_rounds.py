@@ -1,8 +1,9 @@
 """How the decoder warps of a pair of CTAs hand pages to each other in the shared-prefix kernel (pair_slot, pair_round,
-chromofold_b200/csrc/cf_device_common.cuh), played on the host in random order with mbarriers as the PTX manual describes them: each
+pair_rounds_arrived, chromofold_b200/csrc/cf_device_common.cuh), played on the host in random order with mbarriers as the PTX manual describes them: each
 round's barrier takes eight arrivals and the bytes of the other CTA's pages. Warps may leave at any slot and issuing threads at any
 round, as they do when a wait runs out. A warp arrives for a round only when the tiles of the one two before are free in both CTAs, so
-no arrival may meet a barrier that has had its eight; a warp whose record never came sends pages all the same."""
+no arrival may meet a barrier that has had its eight; a warp whose record never came sends pages all the same. And what a pair
+waits for before it leaves early (pair_rounds_arrived) tells when the pages that were sent have landed."""
 import os
 import shutil
 import subprocess
@@ -13,6 +14,7 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 PROGRAM = r"""
 #include "cf_device_common.cuh"
+#include <algorithm>
 #include <random>
 #include <vector>
 using namespace cfb;
@@ -37,6 +39,7 @@ int main() {
     for (uint32_t rank = 0; rank < 2; ++rank)   // the two CTAs' slots are those of the pair's sequence, each once
         for (uint32_t m = 0; m < 1000; ++m)
             if (pair_slot(m, rank) / 8 != pair_round(m) || pair_slot(m, rank) % 8 != 4 * rank + m % 4) return 1;
+    int left_early = 0;
     for (int game = 0; game < 20000; ++game) {
         const uint32_t rounds = 1 + below(12);   // with the one that tells to stop
         const bool trouble = game % 4 != 0;
@@ -78,13 +81,43 @@ int main() {
         }
         for (auto &cta : full) for (const Barrier &b : cta) if (b.overrun) return 2;
         if (!gave_up[0] && !gave_up[1] && !flying.empty()) return 3;   // issuers that took every round have seen every page land
+        if (!gave_up[0] && !gave_up[1]) continue;
+        // Before they leave, the warps make up arrivals up to the last round that any has arrived for; then the barriers of the last
+        // two rounds must tell exactly when the last page has landed.
+        uint32_t arrived = 0;
+        for (auto &cta : next) for (uint32_t m : cta) arrived = std::max(arrived, pair_rounds_arrived(m, kWarps));
+        std::vector<uint32_t> missing[2];
+        for (uint32_t c = 0; c < 2; ++c)
+            for (uint32_t m : next[c]) for (; pair_round(m) < arrived; m += kWarps) missing[c].push_back(pair_round(m));
+        for (;;) {
+            for (uint32_t c = 0; c < 2; ++c) {
+                bool told = missing[0].empty() && missing[1].empty(), there = true;
+                for (uint32_t r = arrived < 2 ? 0 : arrived - 2; r < arrived; ++r) {
+                    told = told && full[c][r & 1].done(r);
+                    if (full[c][r & 1].phase > (r >> 1) + 1) return 4;   // the parity would be that of a phase to come
+                }
+                for (const Copy &f : flying) there = there && f.to != c;
+                if (missing[0].empty() && missing[1].empty() && told != there) return 5;
+            }
+            if (flying.empty() && missing[0].empty() && missing[1].empty()) break;
+            const uint32_t c = below(2);
+            if (!missing[c].empty() && below(2)) {
+                const uint32_t i = below(static_cast<uint32_t>(missing[c].size()));
+                for (auto &cta : full) cta[missing[c][i] & 1].arrive(0);
+                missing[c].erase(missing[c].begin() + i);
+            } else if (!flying.empty()) {
+                land(below(static_cast<uint32_t>(flying.size())));
+            }
+        }
+        for (auto &cta : full) for (const Barrier &b : cta) if (b.overrun) return 6;
+        ++left_early;
     }
-    return 0;
+    return left_early > 5000 ? 0 : 7;
 }
 """
 
 
-def test_no_arrival_meets_a_full_round(tmp_path):
+def test_no_arrival_meets_a_full_round_and_no_page_lands_after_the_end(tmp_path):
     nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
     if not os.path.exists(nvcc):
         pytest.skip("nvcc not found")
