@@ -119,7 +119,19 @@ __device__ __forceinline__ void take_quads(UnitState<NG> &u, const QSrc &qs, int
         score_quad(u, qs, q, kq);
     }
 }
-// Both streams with the same coder: two independent decoder chains, interleaved symbol by symbol.
+// Both streams of fixed width: nothing to decode, and no passes: their words lie one after the other and sixteen lanes' words share a
+// bank, so that it matters that several go in one load, as the compiler makes them here, but not in the loop below (16 sequences of
+// 2048 to 6144 tokens, 32 fp32 heads: 72 us here, 70 with 16-byte loads written out, 114 there; 64 binary16 heads 82, 81, 125. The
+// written loads took the registers of the other coders' kernels: 8 x 131072 tokens, 64 heads, 2149 -> 2157).
+template <int kMode, int NG, class QSrc>
+__device__ __forceinline__ void decode_fixed(FixedLane &k, FixedLane &v, UnitState<NG> &u, const QSrc &qs) {
+#pragma unroll
+    for (int q = 0; q < 16; ++q) {
+        const uint32_t kq = k.quad(q);
+        take_quads<kMode>(u, qs, q, q, kq, v.quad(q));
+    }
+}
+// Both streams with the same other coder: two independent decoder chains, interleaved symbol by symbol.
 template <int kMode, int kPasses, class Lane, int NG, class QSrc>
 __device__ __forceinline__ void decode_fused(Lane &k, Lane &v, UnitState<NG> &u, const QSrc &qs) {
     constexpr int kEach = 16 / kPasses;   // quads of a pass
@@ -142,9 +154,6 @@ __device__ __forceinline__ void decode_fused(Lane &k, Lane &v, UnitState<NG> &u,
                 kw = j & 1 ? kw >> 4 : k.lo_word(q >> 1);
                 vw = j & 1 ? vw >> 4 : v.lo_word(q >> 1);
                 take_quads<kMode>(u, qs, q, at, merge_split_quad<Lane>(ke[0], ke[1], kw), merge_split_quad<Lane>(ve[0], ve[1], vw));
-            } else if constexpr (Lane::kWholeQuads) {
-                const uint32_t kq = k.quad(q);
-                take_quads<kMode>(u, qs, q, at, kq, v.quad(q));
             } else {
                 uint32_t ke[4], ve[4];
 #pragma unroll
@@ -576,7 +585,7 @@ __global__ void __launch_bounds__(kThreadsOf<NG, NB, kSplitQ, kDim>, 1) lanes_at
                         FixedLane k, v;
                         k.open(k_part, k_bytes, lane);
                         v.open(v_part, v_bytes, lane);
-                        decode_fused<kMode, kPasses>(k, v, u, qs);
+                        decode_fixed<kMode>(k, v, u, qs);
                     } else {  // mixed coders (one stream fell back to fixed width): one stream after the other
                         if (k_coder == CF_B200_CODER_RANS) { RansLane k; k.open(k_part, k_bytes, lane, k_slot); decode_k_only<kMode>(k, u, qs); }
                         else if (k_coder == CF_B200_CODER_HUFFMAN) { HuffLane k; k.open(k_part, k_bytes, lane, k_lut); decode_k_only<kMode>(k, u, qs); }

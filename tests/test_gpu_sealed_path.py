@@ -626,6 +626,30 @@ def test_a_pair_whose_wait_runs_out_reports_it_and_the_next_call_is_right(native
     assert layer.device_status() == 0 and np.array_equal(again, good)
 
 
+@pytest.mark.parametrize("heads,queries", [(32, "f16"), (32, "f32"), (64, "f16")])
+def test_fixed_width_pages_are_read_faster_than_coded_ones(native, heads, queries):
+    """Fixed-width pages have nothing to decode: a decode step over them takes about 0.75 to 0.8 times as long as over nibble-split
+    Huffman pages, the fastest of the coded ones (with their quads in the decoders' loop it took 0.97 to 1.2 times as long)."""
+    import torch
+    from chromofold_b200.workloads import build_sealed_layer
+    times = {}
+    for coder in ("fixed8", "huffman4"):
+        layer, _ = build_sealed_layer(np.full(16, 4096), query_heads=heads, coder=coder, seed=38)
+        q = torch.randn((16, heads, 128), device="cuda")
+        q, out = q if queries == "f32" else q.half(), torch.empty((16, heads, 128), device="cuda")
+        runs = []
+        for _ in range(6):
+            begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            begin.record()
+            for _ in range(20):
+                layer.attention(q, out=out)
+            end.record()
+            end.synchronize()
+            runs.append(begin.elapsed_time(end))
+        times[coder] = min(runs)
+    assert times["fixed8"] < 0.9 * times["huffman4"], times
+
+
 def test_append_rows_entry_point_fills_the_tails_and_reports_a_full_one(native):
     """cf_b200_append_rows_async: one launch stores a token's K and V rows (binary16 or fp32 rows) at each listed slot's
     tail position and raises the count; a slot whose tail is full takes nothing and raises CF_B200_DEVSTAT_TAIL_FULL."""
