@@ -12,8 +12,8 @@
 #include <atomic>
 #include <chrono>
 #include <condition_variable>
+#include <exception>
 #include <mutex>
-#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -90,7 +90,7 @@ private:
         const unsigned processors = std::thread::hardware_concurrency();
         try {
             while (threads_.size() < kHelpers && threads_.size() + 1u < processors) threads_.emplace_back(&CopyHelpers::help, this);
-        } catch (const std::system_error &) {   // no more threads to be had: those there are will do
+        } catch (const std::exception &) {   // no more threads, or no memory, to be had: those there are will do
         }
     }
     static void pause(unsigned turn) {

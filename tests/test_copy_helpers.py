@@ -1,5 +1,6 @@
 """Checked copies of host rows shared by several threads (chromofold_b200/csrc/copy_helpers.h): every size around the pieces' edges, one
-copy after the other and after pauses in which the helpers fall asleep; a value that is not finite is found wherever it lies."""
+copy after the other and after pauses in which the helpers fall asleep; a value that is not finite is found wherever it lies. Without
+memory for the helpers the caller copies alone."""
 import os
 import shutil
 import subprocess
@@ -36,12 +37,53 @@ int main() {
 """
 
 
-def test_shared_copies_are_exact(tmp_path):
+NO_MEMORY = r"""
+#include "copy_helpers.h"
+#include <cstdio>
+#include <cstdlib>
+#include <new>
+using cfb::CopyHelpers;
+static int allocations = -1;   // that still succeed, -1: all
+void *operator new(std::size_t n) {
+    if (allocations == 0) throw std::bad_alloc();
+    if (allocations > 0) --allocations;
+    return std::malloc(n);
+}
+void operator delete(void *p) noexcept { std::free(p); }
+void operator delete(void *p, std::size_t) noexcept { std::free(p); }
+int main() {
+    const size_t n = CopyHelpers::kLeastFloats + 5;
+    std::vector<float> a(n, 1.0f), b(n);
+    for (int left = 0; left < 12; ++left) {
+        std::fill(b.begin(), b.end(), 0.0f);
+        CopyHelpers helpers;
+        for (int turn = 0; turn < 3; ++turn) {
+            allocations = left;
+            const uint32_t top = helpers.copy(b.data(), a.data(), n);
+            allocations = -1;
+            if (top != 0x3f800000u || a != b) return 1;
+        }
+    }
+    std::puts("ok");
+    return 0;
+}
+"""
+
+
+def _run(tmp_path, program):
     gxx = shutil.which("g++")
     if not gxx:
         pytest.skip("g++ not found")
     src, exe = tmp_path / "copies.cpp", tmp_path / "copies"
-    src.write_text(PROGRAM)
+    src.write_text(program)
     subprocess.run([gxx, "-std=c++17", "-O2", "-pthread", "-I", SRC, os.path.join(SRC, "host_rows.cpp"), str(src), "-o", str(exe)], check=True)
     out = subprocess.run([str(exe)], capture_output=True, text=True, timeout=60)
     assert out.stdout == "ok\n", out.returncode
+
+
+def test_shared_copies_are_exact(tmp_path):
+    _run(tmp_path, PROGRAM)
+
+
+def test_a_caller_without_memory_for_helpers_copies_alone(tmp_path):
+    _run(tmp_path, NO_MEMORY)
