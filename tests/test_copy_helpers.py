@@ -1,6 +1,6 @@
 """Checked copies of host rows shared by several threads (chromofold_b200/csrc/copy_helpers.h): every size around the pieces' edges, one
 copy after the other and after pauses in which the helpers fall asleep; a value that is not finite is found wherever it lies. Without
-memory for the helpers the caller copies alone."""
+memory for the helpers, and in a process that was forked and has none, the caller copies alone."""
 import os
 import shutil
 import subprocess
@@ -40,6 +40,7 @@ int main() {
 NO_MEMORY = r"""
 #include "copy_helpers.h"
 #include <cstdio>
+#include <algorithm>
 #include <cstdlib>
 #include <new>
 using cfb::CopyHelpers;
@@ -70,6 +71,41 @@ int main() {
 """
 
 
+FORKED = r"""
+#include "copy_helpers.h"
+#include <algorithm>
+#include <cstdio>
+#include <sys/wait.h>
+#include <unistd.h>
+using cfb::CopyHelpers;
+int main() {
+    const size_t n = 40 * CopyHelpers::kPieceFloats;
+    std::vector<float> a(n, 1.0f), b(n);
+    for (int turn = 0; turn < 20; ++turn) {
+        CopyHelpers *helpers = new CopyHelpers;
+        if (turn % 5) helpers->copy(b.data(), a.data(), n);
+        if (turn % 2) std::this_thread::sleep_for(20 * CopyHelpers::kAwake);   // they are asleep, or awake
+        const pid_t child = fork();
+        if (child == 0) {
+            alarm(10);
+            std::fill(b.begin(), b.end(), 0.0f);
+            const uint32_t top = helpers->copy(b.data(), a.data(), n);
+            const bool right = top == 0x3f800000u && a == b;
+            delete helpers;
+            _exit(right ? 0 : 1);
+        }
+        int status = 0;
+        if (waitpid(child, &status, 0) != child || status != 0) return 1;
+        std::fill(b.begin(), b.end(), 0.0f);   // and in the one that has them all goes on
+        if (helpers->copy(b.data(), a.data(), n) != 0x3f800000u || a != b) return 2;
+        delete helpers;
+    }
+    std::puts("ok");
+    return 0;
+}
+"""
+
+
 def _run(tmp_path, program):
     gxx = shutil.which("g++")
     if not gxx:
@@ -87,3 +123,7 @@ def test_shared_copies_are_exact(tmp_path):
 
 def test_a_caller_without_memory_for_helpers_copies_alone(tmp_path):
     _run(tmp_path, NO_MEMORY)
+
+
+def test_a_forked_process_copies_alone_and_ends(tmp_path):
+    _run(tmp_path, FORKED)
