@@ -50,6 +50,7 @@ public:
         if (!team_ || owner_ != getpid()) return chromofold_copy_max_magnitude(dst, src, n);
         return team_->copy(dst, src, n);
     }
+    uint32_t asleep() const { return team_ ? team_->asleep() : 0u; }   // helpers that sleep
 
 private:
     class Team {
@@ -83,6 +84,7 @@ private:
             for (unsigned turn = 0; finished_.load(std::memory_order_acquire) != pieces; ++turn) pause(turn);
             return top_.load(std::memory_order_relaxed);
         }
+        uint32_t asleep() const { return asleep_.load(); }
 
     private:
         // Claims a piece and copies it; false if none is left. A claim holds the copy open (finished_), so that what it reads of it stays.
@@ -99,9 +101,12 @@ private:
         }
         void help() {
             for (;;) {
-                const auto until = std::chrono::steady_clock::now() + kAwake;
+                auto until = std::chrono::steady_clock::now() + kAwake;
                 do {
-                    while (work()) {}
+                    if (work()) {
+                        while (work()) {}
+                        until = std::chrono::steady_clock::now() + kAwake;
+                    }
                     for (unsigned turn = 0; turn < 64u && static_cast<uint32_t>(left_.load(std::memory_order_relaxed)) == 0u; ++turn) pause(0);
                 } while (!stop_.load(std::memory_order_relaxed) && std::chrono::steady_clock::now() < until);
                 std::unique_lock<std::mutex> hold(lock_);
