@@ -131,6 +131,26 @@ int main() {
 """
 
 
+SMALL = r"""
+#include "copy_helpers.h"
+#include <cstdio>
+#include <filesystem>
+#include <iterator>
+using cfb::CopyHelpers;
+static long threads() { return std::distance(std::filesystem::directory_iterator("/proc/self/task"), std::filesystem::directory_iterator()); }
+int main() {
+    CopyHelpers helpers;
+    std::vector<float> a(256 * 128, 1.0f), b(256 * 128);
+    helpers.copy(b.data(), a.data(), 160 * 128);
+    if (threads() != 1) return 1;
+    helpers.copy(b.data(), a.data(), 256 * 128);
+    if (threads() == 1) return 2;
+    std::puts("ok");
+    return 0;
+}
+"""
+
+
 def _run(tmp_path, program):
     gxx = shutil.which("g++")
     if not gxx:
@@ -157,3 +177,9 @@ def test_a_forked_process_copies_alone_and_ends(tmp_path):
 @pytest.mark.skipif((os.cpu_count() or 1) < 4, reason="needs a processor for each helper")
 def test_helpers_look_for_the_next_copy_after_a_long_one(tmp_path):
     _run(tmp_path, AWAKE)
+
+
+@pytest.mark.skipif((os.cpu_count() or 1) < 2 or not os.path.isdir("/proc/self/task"), reason="counts threads")
+def test_small_copies_start_no_helpers(tmp_path):
+    """160 rows of 128 channels are copied faster by the caller alone, 256 with helpers."""
+    _run(tmp_path, SMALL)
