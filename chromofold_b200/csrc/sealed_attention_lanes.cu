@@ -308,8 +308,11 @@ __global__ void __launch_bounds__(kThreadsOf<NG, NB, kSplitQ, kDim>, 1) lanes_at
     uint32_t *q_rows = reinterpret_cast<uint32_t *>(warp_mem + L::kQRows);
 
     if (after_prefix && __ldcg(&plan_header(p)->line.stretches) == 0u) {   // the shared-prefix kernel has taken every page
-        allow_dependent_launch();
+        // Only now may the combine kernel start: placed while these CTAs still held the SMs until the prefix kernel's end, and left all at
+        // once, it went onto those of one die that were free first, six or eight CTAs each (64 rows after 16384 tokens 134 -> 120 us,
+        // 100 rows of 12 heads after 8192 tokens 93 -> 82).
         wait_for_previous_kernel();
+        allow_dependent_launch();
         return;
     }
     load_tables<kThreadsOf<NG, NB, kSplitQ, kDim>>(smem, p, tid);   // coding tables: once per CTA

@@ -238,3 +238,39 @@ def test_prefill_through_the_dataplane_takes_the_shared_prefix_path(native, orac
     assert lib.cf_device_kv_attention_async(p, 0, C.c_void_p(q.data_ptr()), C.c_void_p(out.data_ptr()), nq, tokens - nq, scale, 100, None) == 0
     assert lib.cf_b200_shared_prefix_launches() == before + 1
     lib.cf_device_kv_destroy(p, None)
+
+
+def test_a_short_chunk_takes_its_share_of_a_long_ones_time(native):
+    """A chunk whose history the shared-prefix kernel takes whole: the combine kernel behind it has to find all SMs free. Placed while
+    they were still held it ended up on half of them, and 64 rows took 0.75 of the time of 128 rows, not 0.68."""
+    import torch
+    lib = native.lib()
+    lib.cf_device_kv_create.restype = C.c_void_p
+    hq, hkv, d, page, tokens = 32, 8, 128, 128, 16384
+    cfg = DeviceKvConfig(1, hkv, hq, d, page, hq // hkv, 1)
+    times = []
+    for count in (64, 128):
+        kv = C.c_void_p(lib.cf_device_kv_create(C.byref(cfg)))
+        n = tokens + count
+        g = torch.Generator(device="cuda").manual_seed(5)
+        k, v = (torch.randn((n, hkv, d), generator=g, device="cuda") * 0.2 for _ in range(2))
+        q, out = torch.randn((count, hq, d), generator=g, device="cuda"), torch.empty((count, hq, d), device="cuda")
+        view = lambda t: TensorView(t.data_ptr(), 3, t.shape[0], hkv, d, hkv * d * 4, d * 4, 4, 0)
+        for begin in range(0, n, page):
+            part = [view(t[begin:begin + page]) for t in (k, v)]
+            assert lib.cf_device_kv_append_async(kv, 0, begin, C.byref(part[0]), C.byref(part[1]), None) == 0
+            assert lib.cf_device_kv_seal_full_pages_async(kv, None) == 0
+        runs = []
+        for _ in range(9):
+            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            e0.record()
+            for _ in range(12):
+                assert lib.cf_device_kv_attention_async(kv, 0, C.c_void_p(q.data_ptr()), C.c_void_p(out.data_ptr()), count, tokens,
+                                                        C.c_float(d ** -0.5), 0, None) == 0
+            e1.record()
+            e1.synchronize()
+            runs.append(e0.elapsed_time(e1))
+        times.append(sorted(runs)[4])
+        torch.cuda.synchronize()
+        lib.cf_device_kv_destroy(kv, None)
+    assert times[0] < 0.715 * times[1], times[0] / times[1]
