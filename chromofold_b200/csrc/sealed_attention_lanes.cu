@@ -120,15 +120,18 @@ __device__ __forceinline__ void take_quads(UnitState<NG> &u, const QSrc &qs, int
     }
 }
 // Both streams of fixed width: nothing to decode, and no passes: their words lie one after the other and sixteen lanes' words share a
-// bank, so that it matters that several go in one load, as the compiler makes them here, but not in the loop below (16 sequences of
-// 2048 to 6144 tokens, 32 fp32 heads: 72 us here, 70 with 16-byte loads written out, 114 there; 64 binary16 heads 82, 81, 125. The
-// written loads took the registers of the other coders' kernels: 8 x 131072 tokens, 64 heads, 2149 -> 2157).
+// bank, so that it matters that four of them go in one load, as the compiler makes them here, but not in the loop below (16 sequences
+// of 2048 to 6144 tokens, 32 fp32 heads: 69 us here, 114 there; 64 binary16 heads 81 and 125). With all sixteen of a stream asked
+// for at once the fp32 kernel spilled more (32 server slots of 900 to 8200 tokens: 201.6 -> 202.4 us).
 template <int kMode, int NG, class QSrc>
 __device__ __forceinline__ void decode_fixed(FixedLane &k, FixedLane &v, UnitState<NG> &u, const QSrc &qs) {
 #pragma unroll
-    for (int q = 0; q < 16; ++q) {
-        const uint32_t kq = k.quad(q);
-        take_quads<kMode>(u, qs, q, q, kq, v.quad(q));
+    for (int q = 0; q < 16; q += 4) {
+        uint32_t kq[4], vq[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) kq[j] = k.quad(q + j), vq[j] = v.quad(q + j);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) take_quads<kMode>(u, qs, q + j, q + j, kq[j], vq[j]);
     }
 }
 // Both streams with the same other coder: two independent decoder chains, interleaved symbol by symbol.
