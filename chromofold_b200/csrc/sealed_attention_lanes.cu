@@ -70,7 +70,8 @@ constexpr float kWeightScale = 32768.0f;
 // the warp's shared memory as [head][half] rows of [quad of channels]{even: channels 0, 1 | odd: 0, 1 | even: 2, 3 | odd: 2, 3},
 // one 16-byte load per quad and pair, 16 bytes of padding a row, which puts the rows that eight lanes touch into different banks; a
 // lane whose row is not its own reads zeros, from the banks that the other lanes of its eight leave alone. (Four binary16 heads have
-// no odd group: their rows hold channels only, eight bytes a load.)
+// no odd group: their rows hold channels only, eight bytes a load, which serves sixteen lanes at a time; there the zeros share two
+// banks with rows of their own, and a load takes four wavefronts where two would do.)
 // With the codes as B operand one mma serves a pair of groups, where K * Q^T took one for each of them and two zero registers.
 struct QSmem {
     uint32_t addr, pair_stride;  // byte address of the lane's row for pair 0; distance to the row for pair 1 (0 on the zero row)
@@ -262,7 +263,7 @@ __device__ __forceinline__ void stage_blocks(const uint8_t *part, uint32_t part_
 // Shared memory of one warp: one record, the softmax scratch, an mbarrier and the query rows. A record is decoded before anything
 // else happens to its page, so its place is free for the next one while the scores and weights are worked out; a second place
 // would cost eight warps per SM.
-//   scratch: P rows fp16 high halves [4 NG][16] | low halves [4 NG][16]
+//   scratch: P rows fp16 high halves [4 NS][16] | low halves [4 NS][16], NS = kHeadGroups
 template <int NG, int NB, bool kSplitQ, int kDim>
 struct WarpLayout {
     static constexpr uint32_t kStage = kDim == 128 ? kStageBytes : 16u + 32u * kDim + 48u;   // header, two streams, read-ahead
@@ -281,9 +282,9 @@ struct WarpLayout {
     static_assert(kSmem <= 232448, "a CTA has 227 KB of shared memory");
 };
 
-// kSplitQ: the queries are fp32. Their rows are split into binary16(q) and binary16(q - binary16(q)), stored as the rows of the
-// first and of the last NS groups, the two score fragments of a head are added, and one softmax / P V follows: the scores
-// equal fp32-query scores to 2^-22 relative, at the cost of a second score mma.
+// kSplitQ: the queries are fp32. Their rows are split into binary16(q) and binary16(q - binary16(q)): with four heads the two groups
+// of the one pair, which one mma serves, with eight a pair of values and a pair of residues, a second score mma. The two score
+// fragments of a head are added, and one softmax / P V follows: the scores equal fp32-query scores to 2^-22 relative.
 template <int NG, int kMode, bool kSplitQ, int NB, int kDim>
 __global__ void __launch_bounds__(kThreadsOf<NG, NB, kSplitQ, kDim>, 1) lanes_attention_kernel(AttentionParams p, uint32_t after_prefix) {
     constexpr bool kProbe = kMode != kAttend;
@@ -407,7 +408,7 @@ __global__ void __launch_bounds__(kThreadsOf<NG, NB, kSplitQ, kDim>, 1) lanes_at
             const float2 *qsrc = reinterpret_cast<const float2 *>(
                 reinterpret_cast<const float *>(p.queries) + (static_cast<uint64_t>(q_row) * p.query_head_count + q_head_base) * kDim);
 #pragma unroll
-            for (int j = 0; j < NS * kDim / 16; ++j) {    // 4 NS heads x kDim / 2 channel pairs; row = head*2 + half, residues 8 NS rows further
+            for (int j = 0; j < NS * kDim / 16; ++j) {    // 4 NS heads x kDim / 2 channel pairs; row = head*2 + half
                 const uint32_t i = lane + 32u * j, head = i / (2u * kRowWords);
                 const float2 x = head < G ? qsrc[i] : make_float2(0.0f, 0.0f);
                 const __half2 hi = __floats2half2_rn(x.x, x.y);

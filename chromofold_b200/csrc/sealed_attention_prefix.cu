@@ -37,11 +37,12 @@
 // rounding residue, S = Q K^T + Q residue K^T). Row = lane. B tiles use the no-swizzle K-major canonical layout: 8 rows x 16
 // bytes core matrices, element (row r, 16-byte chunk c) at (r % 8) * 16 + (r / 8) * 2048 + c * 128 bytes in the K tile and at
 // (r % 8) * 16 + (r / 8) * 128 + c * 2048 in the V tile: a page (16 rows of K, two chunks of V) is then 4096 bytes in a row in
-// either, which a pair's CTA sends to the other one by bulk copies. (Stored there 16 bytes at a time, a page took its warp 4000 of
-// the 22000 clocks between two pages, and the tensor core waited for it: a round took 8950 clocks.)
+// either, which a pair's CTA sends to the other one by bulk copies. (Against storing them there 16 bytes at a time: 500 rows after
+// 16384 tokens 560 -> 544 us. A decoder warp itself gains nothing by it: of its 22000 clocks per page the stores to both CTAs took
+// 4000, now stores, fence and copies take 2200 and 2400.)
 // Head_dim 64 runs the same kernel on the left half of the K tile and the upper half of the V tile.
-// The page's V scale relative to the largest one met so far in the unit rides on P (never above 1, so the binary16
-// weights cannot overflow); O is kept in units of that scale and rescaled when a larger one arrives.
+// The page's V scale relative to the largest one met so far in the unit rides on P (never above 1); O is kept in units of
+// that scale and rescaled when a larger one arrives.
 // Every mbarrier wait is bounded. A warp whose wait ran out raises CF_B200_DEVSTAT_WAIT_EXPIRED and skips all later
 // waits and work, but a decoder warp whose record never came, which goes on with absent pages, and a softmax warp still takes
 // part in the barrier with its partner, which OR-reduces the failure so that both leave their loops at the same point; the roles
@@ -83,6 +84,10 @@ constexpr uint32_t kTmemColumns = 512;
 constexpr uint32_t kColS = 0, kColO = 256, kColQ = 384, kColQResidue = 448;
 constexpr uint32_t kStopUnit = 0xffffffffu;
 constexpr float kWeightScale = 32768.0f;   // power of two the binary16 weights are scaled by (O sheds it at a unit's end)
+// The maximum that the weights are relative to follows the true one only when that has risen by this much in the exponent of two. A
+// weight is then at most 2^0.9 = 1.8661, and 2^(1/16) more where the maximum itself was rounded (products of 2^20).
+constexpr float kMaxLag = 0.9f, kLargestWeight = 1.8661f * 1.0443f;
+static_assert(kMaxLag <= 0.9f && kWeightScale * kLargestWeight < 65504.0f, "binary16 has to hold the scaled weights");
 constexpr uint32_t kFirstRound = 1u, kLastRound = 2u;   // round flags
 // Register split (setmaxnreg). A CTA can only redistribute the registers it was launched with: kLaunchRegs per thread,
 // the most that 640 threads can have. What the softmax warps ask for must not exceed what the decoders give back, or
@@ -641,7 +646,7 @@ __device__ __forceinline__ void decoder_role(const AttentionParams &p, uint8_t *
 
 // ---- tensor-core work, issued by one thread ----------------------------------------------------------------------------------
 // S of round r, whose tiles are there.
-template <int kDim, bool kSplitQ, int kCluster>
+template <int kDim, bool kSplitQ>
 __device__ __forceinline__ void issue_scores(uint8_t *smem, uint32_t tmem, uint64_t *bars, uint32_t r) {
     fence_async_smem();
     tc_fence_after();
@@ -690,7 +695,7 @@ __device__ __forceinline__ void issuer_role(const AttentionParams &p, uint8_t *s
             const bool first = (round_desc[4 * pair + 1] & kFirstRound) != 0u;
             fresh = first ? fresh | 1u << pair : fresh & ~(1u << pair);
             if (first) ok = mbar_wait(bars + kBarQ, units++ & 1u, p.wait_polls);   // the unit's queries are in tensor memory
-            if (ok) issue_scores<kDim, kSplitQ, kCluster>(smem, tmem, bars, s_round++);
+            if (ok) issue_scores<kDim, kSplitQ>(smem, tmem, bars, s_round++);
         } else if (o_round < s_round && mbar_test_pair(bars + kBarP + weights_barrier(o_round).index, weights_barrier(o_round).parity)) {
             polls = 0;
             issue_output<kDim, kCluster>(smem, tmem, bars, o_round, (fresh >> (o_round & 1u) & 1u) != 0u);
@@ -786,7 +791,7 @@ __device__ __forceinline__ void softmax_role(const AttentionParams &p, uint8_t *
             if (lane == 0) mbar_arrive(bars + kBarQ);
         }
     };
-    auto issue_s = [&](uint32_t r) { issue_scores<kDim, kSplitQ, kCluster>(smem, tmem, bars, r); };   // issuer only
+    auto issue_s = [&](uint32_t r) { issue_scores<kDim, kSplitQ>(smem, tmem, bars, r); };   // issuer only
     uint32_t rounds = 0;    // whose O has been issued
     uint32_t s_round = 0;   // issuer: the next round whose S is due
     // Issuer only: S of round r ahead of its turn, unless its tiles are not there yet or its queries are another unit's.
@@ -880,11 +885,11 @@ __device__ __forceinline__ void softmax_role(const AttentionParams &p, uint8_t *
 #pragma unroll
         for (uint32_t pg = 0; pg < kRoundPages; ++pg)
             if (__float_as_uint(meta[4 * pg + 2]) != 0u) round_scale = fmaxf(round_scale, meta[4 * pg + 1]);
-        // The maximum that the weights are relative to follows the true one only when that has risen by 0.9 in the exponent of two:
-        // a weight is then at most 2^0.9, 2^15.9 scaled, which binary16 holds, and O is rescaled on few rounds (every second
-        // one of the first hundred met a higher maximum in one of a warp's 32 rows: 582 -> 560 us for 500 rows after 16384 tokens).
+        // With the lag O is rescaled on few rounds (every second one of the first hundred met a higher maximum in one of a warp's 32
+        // rows: 582 -> 560 us for 500 rows after 16384 tokens). The result is as close to double precision as without it (the error
+        // over 351 stores and queries is 0.9994 +- 0.0009 of what it was); a maximum kept whole, for exact rescaling, was 0.6 % worse.
         float m_new = fmaxf(m_run, fmaxf(row_max[row_in_tile], row_max[128u + row_in_tile]));
-        if (m_new - m_run < 0.9f) m_new = m_run;
+        if (m_new - m_run < kMaxLag) m_new = m_run;
         const float z = m_new == -CUDART_INF_F ? 0.0f : m_new;
         const float alpha = fast_exp2(m_run - z);   // m_run = -inf gives 0
         m_run = m_new;
@@ -903,7 +908,7 @@ __device__ __forceinline__ void softmax_role(const AttentionParams &p, uint8_t *
             const uint32_t pg = 4u * half + q;
             const uint32_t count = seen_of(pg, __float_as_uint(meta[4 * pg + 2]));
             const float ks = meta[4 * pg];
-            // the weights (at most 2^0.9) also carry 2^15, exactly, which O sheds at the unit's end: binary16 then resolves
+            // the weights (at most 2^kMaxLag) also carry 2^15, exactly, which O sheds at the unit's end: binary16 then resolves
             // weights down to 2^-40 of the row maximum instead of 2^-25
             const float ratio = count ? __fdividef(meta[4 * pg + 1], v_unit) * kWeightScale : 0.0f;
             uint32_t hi[8], lo[8];
